@@ -1296,6 +1296,18 @@ int cuvgls_gls_direct_batch(cuvgls_handle *h, const cuvgls_gls_input *b,
     size_t need = align_up(nc * sizeof(DevCurve)) + kAlign;
     if (hin) need += align_up(b->n_points_total * 8) + 2 * align_up(b->n_points_total * 4);
     if (hout) need += align_up(b->n_out_total * 4);
+    // few frequencies: the points cut into parts, when their sums fit
+    long long bins = 0, max_n = 0;
+    for (DevCurve &cv : cvs) {
+        cv.inter_off = bins;
+        bins += cv.nf;
+        max_n = std::max(max_n, (long long)cv.n);
+    }
+    int splits = direct_splits(bins, gls_direct_bins(), max_n);
+    const size_t part_bytes = (size_t)splits * bins * 3 * sizeof(double2);
+    if (splits > 1 && (long long)(need + part_bytes + kAlign) > h->opts.workspace_bytes) splits = 1;
+    if (splits > 1) need += align_up(part_bytes);
+    for (DevCurve &cv : cvs) cv.aux = (int)std::min<long long>(splits, (cv.n + 255) / 256);
     rc = ensure_ws(h, need);
     if (rc) return rc;
     rc = ensure_host_cv(h, nc);
@@ -1316,6 +1328,7 @@ int cuvgls_gls_direct_batch(cuvgls_handle *h, const cuvgls_gls_input *b,
         t = dt; yw = dy; w = dw;
     }
     float *dout = hout ? (float *)take(b->n_out_total * 4) : p_out;
+    double2 *part = splits > 1 ? (double2 *)take(part_bytes) : nullptr;
     int max_nf = 0;
     for (int i = 0; i < nc; ++i) { h->h_cv[i] = cvs[i]; max_nf = std::max(max_nf, cvs[i].nf); }
     CK(cudaMemcpyAsync(d_cv, h->h_cv, nc * sizeof(DevCurve), cudaMemcpyHostToDevice, s),
@@ -1325,7 +1338,8 @@ int cuvgls_gls_direct_batch(cuvgls_handle *h, const cuvgls_gls_input *b,
     for (int c0 = 0; c0 < nc; c0 += 65535) {
         int cnt = std::min(65535, nc - c0);
         LAUNCH(CUVGLS_STAGE_DIRECT, s,
-               launch_gls_direct(d_cv + c0, cnt, max_nf, t, yw, w, dout, g, s), "k_gls_direct");
+               launch_gls_direct(d_cv + c0, cnt, max_nf, splits, t, yw, w, dout, part, bins, g, s),
+               "k_gls_direct");
     }
     if (hout)
         CK(cudaMemcpyAsync(p_out, dout, b->n_out_total * 4, cudaMemcpyDeviceToHost, s), "D2H");
@@ -1427,7 +1441,7 @@ int cuvgls_nfft_adjoint_fp64(cuvgls_handle *h, const cuvgls_nfft_input *b, const
     if (rc) return rc;
     const int nc = b->n_curves;
     std::vector<Direct64Curve> hc(nc);
-    long long max_nf = 0;
+    long long max_nf = 0, bins = 0, max_n = 0;
     for (int i = 0; i < nc; ++i) {
         const cuvgls_nfft_curve &c = b->curves[i];
         if (c.n < 1 || c.nf < 1 || c.pt_off < 0 || c.out_off < 0 ||
@@ -1435,8 +1449,10 @@ int cuvgls_nfft_adjoint_fp64(cuvgls_handle *h, const cuvgls_nfft_input *b, const
             !(c.df > 0) || !is_fin(c.df) || !is_fin(c.f0))
             return fail(h, CUVGLS_EINVAL,
                         "curve " + std::to_string(i) + ": bad size, range or frequency grid");
-        hc[i] = Direct64Curve{c.pt_off, c.n, c.nf, c.out_off, c.f0, c.df};
+        hc[i] = Direct64Curve{c.pt_off, c.n, c.nf, c.out_off, c.f0, c.df, bins, 1};
         max_nf = std::max(max_nf, (long long)c.nf);
+        max_n = std::max(max_n, (long long)c.n);
+        bins += c.nf;
     }
     const bool hin = b->flags & CUVGLS_HOST_INPUT, hout = b->flags & CUVGLS_HOST_OUTPUT;
     const size_t npts = (size_t)b->n_points_total, nout = (size_t)b->n_out_total;
@@ -1445,6 +1461,12 @@ int cuvgls_nfft_adjoint_fp64(cuvgls_handle *h, const cuvgls_nfft_input *b, const
     if (hout) need += align_up(nout * 16);
     if ((long long)need > h->opts.workspace_bytes)
         return fail(h, CUVGLS_EBUDGET, "batch inputs/outputs exceed the workspace budget");
+    // few frequencies: the points cut into parts, when their sums fit
+    int splits = direct_splits(bins, nfft_direct64_bins(), max_n);
+    const size_t part_bytes = (size_t)splits * bins * sizeof(double2);
+    if (splits > 1 && (long long)(need + part_bytes + kAlign) > h->opts.workspace_bytes) splits = 1;
+    if (splits > 1) need += align_up(part_bytes);
+    for (Direct64Curve &c : hc) c.splits = (int)std::min<long long>(splits, (c.n + 255) / 256);
     rc = ensure_ws(h, need);
     if (rc) return rc;
     char *base = h->ws;
@@ -1464,10 +1486,12 @@ int cuvgls_nfft_adjoint_fp64(cuvgls_handle *h, const cuvgls_nfft_input *b, const
         dy = c;
     }
     double2 *dout = hout ? (double2 *)take(nout * 16) : (double2 *)out;
+    double2 *part = splits > 1 ? (double2 *)take(part_bytes) : nullptr;
     for (int c0 = 0; c0 < nc; c0 += 65535) {
         const int cnt = std::min(65535, nc - c0);
         LAUNCH(CUVGLS_STAGE_DIRECT, s,
-               launch_nfft_direct64(d_cv + c0, cnt, max_nf, dt, dy, dout, s), "k_nfft_direct64");
+               launch_nfft_direct64(d_cv + c0, cnt, max_nf, splits, dt, dy, dout, part, bins, s),
+               "k_nfft_direct64");
     }
     if (hout) CK(cudaMemcpyAsync(out, dout, nout * 16, cudaMemcpyDeviceToHost, s), "D2H");
     CK(cudaEventRecord(h->done, s), "record done");

@@ -1,0 +1,635 @@
+// Direct sums in FP64: use_fft=False (k_gls_direct), use_double
+// (k_nfft_direct64) and the multi-harmonic model (k_mhgls_direct).
+//
+// GB300 issues about two FP64 multiply-adds per clock and SM, so these
+// kernels are bound by their FP64 instruction count and by nothing else; a
+// sincospi per (point, frequency) alone is some 25 of them.  On a uniform
+// frequency grid the phasors factor instead.  A lane owns the 2 M + 1
+// consecutive bins K - M .. K + M; with E = v exp(i K x) and the step phasors
+// cos bx, sin bx (b = 1 .. M), which are the same for every lane,
+//   sum v exp(i (K + b) x) = (P1 - P2) + i (P3 + P4),
+//   sum v exp(i (K - b) x) = (P1 + P2) + i (P3 - P4),
+//   P1 = sum Re E cos bx, P2 = sum Im E sin bx,
+//   P3 = sum Im E cos bx, P4 = sum Re E sin bx,
+// which is two multiply-adds per complex bin and point.  exp(i K x) is the
+// product of a coarse and a fine table entry (32 centres from 4 + 8).
+#include <cuda_runtime.h>
+#include <math.h>
+
+#include <algorithm>
+
+#include "gls_math.cuh"
+#include "kernels.cuh"
+
+namespace cuvgls {
+
+namespace {
+
+constexpr int kDirThreads = 256;
+constexpr int kDirWarps = kDirThreads / 32;
+constexpr int kCoarse = 4, kFine = 8;  // 32 centres
+
+__device__ __forceinline__ double2 zmul(double2 a, double2 b) {
+    return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));
+}
+__device__ __forceinline__ double2 zturn(double turns) {  // exp(2 pi i turns)
+    double s, c;
+    sincospi(2.0 * (turns - floor(turns)), &s, &c);
+    return make_double2(c, s);
+}
+
+// Phasor tables of a warp's tile of 32 points, one entry row of 32 points
+// each: NB step phasors exp(i b x), kCoarse centres exp(i (K0 + 8 W g) x),
+// kFine offsets exp(i W f x), W = 2 M + 1.
+template <int M, int NB>
+struct DirTable {
+    static constexpr int kRows = NB + kCoarse + kFine;
+    double2 row[kRows][32];
+
+    // This lane's point: x in turns per bin, th0 the phase of K0 in turns.
+    // Two sincospi, the rest by products of depth at most 8.
+    __device__ __forceinline__ void build(int lane, double x, double th0) {
+        static_assert(NB >= M, "the centre step is built from step phasor M");
+        double2 z[NB + 1];
+        z[1] = zturn(x);
+#pragma unroll
+        for (int b = 2; b <= NB; ++b) z[b] = zmul(z[b / 2], z[b - b / 2]);
+#pragma unroll
+        for (int b = 1; b <= NB; ++b) row[b - 1][lane] = z[b];
+        const double2 w1 = zmul(zmul(z[M], z[M]), z[1]);  // exp(i W x)
+        double2 f[kFine];
+        f[0] = make_double2(1.0, 0.0);
+        f[1] = w1;
+#pragma unroll
+        for (int k = 2; k < kFine; ++k) f[k] = zmul(f[k / 2], f[k - k / 2]);
+#pragma unroll
+        for (int k = 0; k < kFine; ++k) row[NB + kCoarse + k][lane] = f[k];
+        const double2 w8 = zmul(f[kFine / 2], f[kFine / 2]);
+        double2 c = zturn(th0);
+#pragma unroll
+        for (int k = 0; k < kCoarse; ++k) {
+            row[NB + k][lane] = c;
+            c = zmul(c, w8);
+        }
+    }
+    // exp(i K x) of this lane's centre K = K0 + W lane at point p
+    __device__ __forceinline__ double2 centre(int lane, int p) const {
+        return zmul(row[NB + lane / kFine][p], row[NB + kCoarse + lane % kFine][p]);
+    }
+};
+
+// The sums of one value kind over a lane's 2 M + 1 bins.
+template <int M>
+struct DirSums {
+    double c0 = 0.0, s0 = 0.0, p1[M], p2[M], p3[M], p4[M];
+    __device__ __forceinline__ DirSums() {
+#pragma unroll
+        for (int b = 0; b < M; ++b) p1[b] = p2[b] = p3[b] = p4[b] = 0.0;
+    }
+    __device__ __forceinline__ void centre(double2 e) { c0 += e.x; s0 += e.y; }
+    __device__ __forceinline__ void pair(int b, double2 e, double2 st) {
+        p1[b] = fma(e.x, st.x, p1[b]);
+        p2[b] = fma(e.y, st.y, p2[b]);
+        p3[b] = fma(e.y, st.x, p3[b]);
+        p4[b] = fma(e.x, st.y, p4[b]);
+    }
+    // real and imaginary parts of the lane's bins into re[0 .. 2 M], im[...]
+    __device__ __forceinline__ void bins(double *re, double *im) const {
+        re[M] = c0;
+        im[M] = s0;
+#pragma unroll
+        for (int b = 0; b < M; ++b) {
+            re[M + 1 + b] = p1[b] - p2[b];
+            im[M + 1 + b] = p3[b] + p4[b];
+            re[M - 1 - b] = p1[b] + p2[b];
+            im[M - 1 - b] = p3[b] - p4[b];
+        }
+    }
+};
+
+// Sum of a value kind over the CTA's warps: bin tid + 256 q of the CTA's
+// 32 W bins into (re[q], im[q]).  `red` holds 2 x kDirWarps x 32 W doubles.
+template <int M>
+__device__ __forceinline__ void dir_reduce(const DirSums<M> &v, double *red, int tid,
+                                           double2 *out) {
+    constexpr int TB = 32 * (2 * M + 1);
+    const int lane = tid & 31, wid = tid >> 5;
+    __syncthreads();  // the tables (or the previous kind) are no longer read
+    v.bins(red + wid * TB + lane * (2 * M + 1), red + (kDirWarps + wid) * TB + lane * (2 * M + 1));
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < (TB + kDirThreads - 1) / kDirThreads; ++q) {
+        const int b = tid + q * kDirThreads;
+        double re = 0.0, im = 0.0;
+        if (b < TB)
+            for (int w = 0; w < kDirWarps; ++w) {
+                re += red[w * TB + b];
+                im += red[(kDirWarps + w) * TB + b];
+            }
+        out[q] = make_double2(re, im);
+    }
+}
+
+// Points [j0, j1) of split z of a curve of n points cut into `splits` equal
+// parts; false when the part is empty.
+__device__ __forceinline__ bool dir_part(long long n, int splits, int z, long long &j0,
+                                         long long &j1) {
+    if (z >= splits) return false;
+    const long long per = (n + splits - 1) / splits;
+    j0 = per * z;
+    j1 = min(n, j0 + per);
+    return true;
+}
+
+// ---------------------------------------------------------------------------
+// adjoint NFFT (use_double): M = 8, 544 bins per CTA
+// ---------------------------------------------------------------------------
+constexpr int kNfM = 8, kNfBins = 32 * (2 * kNfM + 1);
+using NfTable = DirTable<kNfM, kNfM>;
+constexpr int kNfSmem = kDirWarps * (int)sizeof(NfTable);
+static_assert(kNfSmem >= 2 * kDirWarps * kNfBins * 8, "the reduction reuses the tables");
+
+}  // namespace
+
+// One CTA per (544 bins, curve, part of its points); its eight warps take the
+// points 32 at a time in turn, each with tables of its own, and are summed in
+// shared memory at the end.  A curve cut into several parts leaves partial
+// sums for k_nfft_direct64_sum.  2.4 FP64 instructions per (point, bin)
+// against 12 with a sincospi pair per point and 8 bins: 4 curves of 300 to
+// 2,000 points and 20,000 bins, host to host, 5.68 -> 0.85 ms.
+__global__ void __launch_bounds__(kDirThreads, 2)
+k_nfft_direct64(const Direct64Curve *__restrict__ cvs, const double *__restrict__ t,
+                const double *__restrict__ y, double2 *__restrict__ out,
+                double2 *__restrict__ part, long long part_stride) {
+    extern __shared__ __align__(16) double sm[];
+    const Direct64Curve cv = cvs[blockIdx.y];
+    const long long k0 = (long long)blockIdx.x * kNfBins;
+    long long j0, j1;
+    if (k0 >= cv.nf || !dir_part(cv.n, cv.splits, blockIdx.z, j0, j1)) return;  // whole CTA
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    NfTable &tab = reinterpret_cast<NfTable *>(sm)[wid];
+    DirSums<kNfM> acc;
+    bool odd = false;  // a value that is not finite, added below bin by bin
+    const double kc = (double)(k0 + kNfM);
+    for (long long base = j0 + wid * 32; base < j1; base += kDirThreads) {
+        const int cnt = (int)min(32LL, j1 - base);
+        __syncwarp();  // the previous tile is consumed
+        if (lane < cnt) {
+            const double tj = t[cv.pt_off + base + lane];
+            double yj = y[cv.pt_off + base + lane];
+            if (!isfinite(yj)) {
+                odd = true;
+                yj = 0.0;
+            }
+            double a = cv.f0 * tj, b = cv.df * tj;
+            a -= floor(a);
+            b -= floor(b);
+            tab.build(lane, b, fma(kc, b, a));
+#pragma unroll
+            for (int g = 0; g < kCoarse; ++g) {  // y rides on the coarse centres
+                double2 &c = tab.row[kNfM + g][lane];
+                c = make_double2(c.x * yj, c.y * yj);
+            }
+        }
+        __syncwarp();
+        for (int p = 0; p < cnt; ++p) {
+            const double2 e = tab.centre(lane, p);
+            acc.centre(e);
+#pragma unroll
+            for (int b = 0; b < kNfM; ++b) acc.pair(b, e, tab.row[b][p]);
+        }
+    }
+    constexpr int NQ = (kNfBins + kDirThreads - 1) / kDirThreads;
+    double2 v[NQ];
+    dir_reduce<kNfM>(acc, sm, tid, v);
+    if (__syncthreads_or(odd)) {  // inf cos and inf sin keep their own signs
+        for (long long j = j0; j < j1; ++j) {
+            const double tj = t[cv.pt_off + j], yj = y[cv.pt_off + j];
+            if (isfinite(yj)) continue;
+            double a = cv.f0 * tj, b = cv.df * tj;
+            a -= floor(a);
+            b -= floor(b);
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) {
+                const double2 e = zturn(fma((double)(k0 + tid + q * kDirThreads), b, a));
+                v[q].x = fma(yj, e.x, v[q].x);
+                v[q].y = fma(yj, e.y, v[q].y);
+            }
+        }
+    }
+    double2 *dst = cv.splits > 1 ? part + blockIdx.z * part_stride + cv.part_off : out + cv.out_off;
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        const int b = tid + q * kDirThreads;
+        if (b < kNfBins && k0 + b < cv.nf) dst[k0 + b] = v[q];
+    }
+}
+
+// Parts of the split curves added in order.
+__global__ void __launch_bounds__(256)
+k_nfft_direct64_sum(const Direct64Curve *__restrict__ cvs, const double2 *__restrict__ part,
+                    long long part_stride, double2 *__restrict__ out) {
+    const Direct64Curve cv = cvs[blockIdx.y];
+    const long long k = (long long)blockIdx.x * 256 + threadIdx.x;
+    if (cv.splits <= 1 || k >= cv.nf) return;
+    double re = 0.0, im = 0.0;
+    for (int z = 0; z < cv.splits; ++z) {
+        const double2 v = part[z * part_stride + cv.part_off + k];
+        re += v.x;
+        im += v.y;
+    }
+    out[cv.out_off + k] = make_double2(re, im);
+}
+
+int direct_splits(long long bins, int bins_per_cta, long long max_n) {
+    // about eight CTAs per SM (152 SMs, one or two resident), so that curves
+    // of different lengths even out, and at least 256 points (one tile per
+    // warp) each; enough bins need no parts and no second kernel
+    const long long tiles = std::max(1LL, (bins + bins_per_cta - 1) / bins_per_cta);
+    const long long want = (8 * 152 + tiles - 1) / tiles;
+    return (int)std::max(1LL, std::min(std::min(want, (max_n + 255) / 256), 64LL));
+}
+int nfft_direct64_bins() { return kNfBins; }
+
+cudaError_t launch_nfft_direct64(const Direct64Curve *cv, int n_curves, long long max_nf,
+                                 int max_splits, const double *t, const double *y, double2 *out,
+                                 double2 *part, long long part_stride, cudaStream_t s) {
+    if (n_curves <= 0 || max_nf <= 0) return cudaSuccess;
+    const long long nb = (max_nf + kNfBins - 1) / kNfBins, nr = (max_nf + 255) / 256;
+    if (nr > 0x7fffffffLL || n_curves > 65535) return cudaErrorInvalidValue;
+    cudaError_t e = cudaFuncSetAttribute(
+        k_nfft_direct64, cudaFuncAttributeMaxDynamicSharedMemorySize, kNfSmem);
+    if (e != cudaSuccess) return e;
+    k_nfft_direct64<<<dim3((unsigned)nb, n_curves, max_splits), kDirThreads, kNfSmem, s>>>(
+        cv, t, y, out, part, part_stride);
+    e = cudaGetLastError();
+    if (e == cudaSuccess && max_splits > 1) {
+        k_nfft_direct64_sum<<<dim3((unsigned)nr, n_curves), 256, 0, s>>>(cv, part, part_stride, out);
+        e = cudaGetLastError();
+    }
+    return e;
+}
+
+// ---------------------------------------------------------------------------
+// GLS (use_fft=False): three sums, M = 4, 288 bins per CTA
+// ---------------------------------------------------------------------------
+namespace {
+constexpr int kGlM = 4, kGlBins = 32 * (2 * kGlM + 1);
+// step phasors up to 2 M: those of the 2x sums are the even ones
+using GlTable = DirTable<kGlM, 2 * kGlM>;
+struct GlTile {
+    GlTable tab;
+    double yw[32], w[32];
+};
+constexpr int kGlSmem = kDirWarps * (int)sizeof(GlTile);
+static_assert(kGlSmem >= 2 * kDirWarps * kGlBins * 8, "the reduction reuses the tables");
+
+__device__ __forceinline__ float gls_direct_power(const DevCurve &cv, const GlsParams &gp,
+                                                  double2 a, double2 b, double2 c) {
+    return (float)gls_from_sums<double>(a.x, a.y, b.x, b.y, c.x, c.y, gp.mode, (double)gp.reg,
+                                        (double)cv.w_sum, (double)cv.yw_sum, (double)cv.ybar,
+                                        (double)cv.yy_inv);
+}
+}  // namespace
+
+// As k_nfft_direct64 with the sums of yw and w at f and of w at 2 f (its
+// phasors are the squares of the others), then the power.  The times are
+// taken from the curve's first point (the power does not depend on the time
+// origin), so the phases stay small.  A curve cut into parts leaves its six
+// partial sums for k_gls_direct_sum.  7.7 FP64 instructions per (point,
+// frequency) against about 45 with a sincospi each: 8 curves of 300 to 2,000
+// points and 10,000 frequencies 9.62 -> 1.10 ms.
+__global__ void __launch_bounds__(kDirThreads, 1)
+k_gls_direct(const DevCurve *__restrict__ cvs, const double *__restrict__ t,
+             const float *__restrict__ yw, const float *__restrict__ w, float *__restrict__ out,
+             double2 *__restrict__ part, long long part_stride, GlsParams gp) {
+    extern __shared__ __align__(16) double sm[];
+    const DevCurve cv = cvs[blockIdx.y];
+    const long long k0 = (long long)blockIdx.x * kGlBins;
+    long long j0, j1;
+    if (k0 >= cv.nf || !dir_part(cv.n, cv.aux, blockIdx.z, j0, j1)) return;  // whole CTA
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    GlTile &tile = reinterpret_cast<GlTile *>(sm)[wid];
+    DirSums<kGlM> sa, sb, sc;
+    const double kc = cv.kc - (double)(cv.nf / 2) + (double)(k0 + kGlM);
+    const double t0 = t[cv.pt_off];
+    for (long long base = j0 + wid * 32; base < j1; base += kDirThreads) {
+        const int cnt = (int)min(32LL, j1 - base);
+        __syncwarp();  // the previous tile is consumed
+        if (lane < cnt) {
+            const long long j = cv.pt_off + base + lane;
+            const double x = (t[j] - t0) * cv.df;
+            tile.tab.build(lane, x, kc * x);
+            tile.yw[lane] = (double)yw[j];
+            tile.w[lane] = (double)w[j];
+        }
+        __syncwarp();
+#pragma unroll 1
+        for (int p = 0; p < cnt; ++p) {
+            const double2 e = tile.tab.centre(lane, p);
+            const double vy = tile.yw[p], vw = tile.w[p];
+            const double2 ea = make_double2(vy * e.x, vy * e.y);
+            const double2 eb = make_double2(vw * e.x, vw * e.y);
+            const double2 ec = make_double2(fma(eb.x, e.x, -eb.y * e.y), 2.0 * eb.x * e.y);
+            sa.centre(ea);
+            sb.centre(eb);
+            sc.centre(ec);
+#pragma unroll
+            for (int b = 0; b < kGlM; ++b) {
+                const double2 st = tile.tab.row[b][p];
+                sa.pair(b, ea, st);
+                sb.pair(b, eb, st);
+                sc.pair(b, ec, tile.tab.row[2 * b + 1][p]);
+            }
+        }
+    }
+    constexpr int NQ = (kGlBins + kDirThreads - 1) / kDirThreads;
+    double2 va[NQ], vb[NQ], vc[NQ];
+    dir_reduce<kGlM>(sa, sm, tid, va);
+    dir_reduce<kGlM>(sb, sm, tid, vb);
+    dir_reduce<kGlM>(sc, sm, tid, vc);
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        const int b = tid + q * kDirThreads;
+        if (b >= kGlBins || k0 + b >= cv.nf) continue;
+        if (cv.aux > 1) {
+            double2 *d = part + 3 * (blockIdx.z * part_stride + cv.inter_off + k0 + b);
+            d[0] = va[q];
+            d[1] = vb[q];
+            d[2] = vc[q];
+        } else {
+            out[cv.out_off + k0 + b] = gls_direct_power(cv, gp, va[q], vb[q], vc[q]);
+        }
+    }
+}
+
+// Parts of the split curves added in order, then the power.
+__global__ void __launch_bounds__(256)
+k_gls_direct_sum(const DevCurve *__restrict__ cvs, const double2 *__restrict__ part,
+                 long long part_stride, float *__restrict__ out, GlsParams gp) {
+    const DevCurve cv = cvs[blockIdx.y];
+    const long long k = (long long)blockIdx.x * 256 + threadIdx.x;
+    if (cv.aux <= 1 || k >= cv.nf) return;
+    double2 v[3] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
+    for (int z = 0; z < cv.aux; ++z) {
+        const double2 *d = part + 3 * (z * part_stride + cv.inter_off + k);
+#pragma unroll
+        for (int g = 0; g < 3; ++g) {
+            v[g].x += d[g].x;
+            v[g].y += d[g].y;
+        }
+    }
+    out[cv.out_off + k] = gls_direct_power(cv, gp, v[0], v[1], v[2]);
+}
+
+int gls_direct_bins() { return kGlBins; }
+
+cudaError_t launch_gls_direct(const DevCurve *cv, int n_curves, int max_nf, int max_splits,
+                              const double *t, const float *yw, const float *w, float *out,
+                              double2 *part, long long part_stride, GlsParams g, cudaStream_t s) {
+    if (n_curves <= 0 || max_nf <= 0) return cudaSuccess;
+    cudaError_t e =
+        cudaFuncSetAttribute(k_gls_direct, cudaFuncAttributeMaxDynamicSharedMemorySize, kGlSmem);
+    if (e != cudaSuccess) return e;
+    k_gls_direct<<<dim3((max_nf + kGlBins - 1) / kGlBins, n_curves, max_splits), kDirThreads,
+                   kGlSmem, s>>>(cv, t, yw, w, out, part, part_stride, g);
+    e = cudaGetLastError();
+    if (e == cudaSuccess && max_splits > 1) {
+        k_gls_direct_sum<<<dim3((max_nf + 255) / 256, n_curves), 256, 0, s>>>(cv, part, part_stride,
+                                                                              out, g);
+        e = cudaGetLastError();
+    }
+    return e;
+}
+
+// ---------------------------------------------------------------------------
+// multi-harmonic floating-mean GLS of one curve at any frequencies
+// ---------------------------------------------------------------------------
+namespace {
+
+constexpr int kTurn = 256;  // phasors of the shared turn table
+
+// exp(2 pi i p) from the phasor at the nearest multiple of 1 / kTurn and the
+// Taylor series of the remaining angle d, |d| <= pi / kTurn: the first terms
+// left out are d^7 / 7! < 9e-18 and d^8 / 8! < 2e-20.  16 FP64 instructions
+// with the product p = t f, against about 28 for floor and sincospi.
+__device__ __forceinline__ double2 table_turn(double p, const double2 *tab) {
+    // beyond 2^40 turns the index below would lose bits: reduce first
+    if (fabs(p) > 1099511627776.0) p -= floor(p);
+    constexpr double kRound = 6755399441055744.0;  // 1.5 2^52: adding it rounds to an integer
+    const double z = fma(p, (double)kTurn, kRound);
+    const double2 e = tab[__double2loint(z) & (kTurn - 1)];
+    const double d = fma(z - kRound, -1.0 / kTurn, p) * 6.283185307179586477;
+    const double d2 = d * d;
+    const double sn = fma(d * d2, fma(d2, 1.0 / 120.0, -1.0 / 6.0), d);
+    const double cm = d2 * fma(d2, fma(d2, -1.0 / 720.0, 1.0 / 24.0), -0.5);  // cos d - 1
+    return make_double2(fma(-e.y, sn, fma(e.x, cm, e.x)), fma(e.x, sn, fma(e.y, cm, e.y)));
+}
+
+// rows of sums a CTA reduces: c, s (2H each), yc, ys (H each), and sum w
+__host__ __device__ constexpr int mh_sums(int H) { return 6 * H + 1; }
+__host__ __device__ constexpr int mh_smem(int H) {
+    // turn table, the warps' point tiles, then (reused) the warps' sums
+    const int a = kTurn * 16 + kDirWarps * 32 * 24, b = (kDirWarps + 1) * mh_sums(H) * 32 * 8;
+    return a > b ? a : b;
+}
+
+}  // namespace
+
+// 32 frequencies per CTA, one per lane; the eight warps take the points 32 at
+// a time in turn and are summed in shared memory, so that a few thousand
+// frequencies already fill the chip evenly (with a thread per frequency,
+// 20,000 of them made 157 CTAs of 128 threads for 152 SMs).  Per point the
+// phasor from table_turn, its powers n = 2 .. 2H from half-way products (three
+// instructions for an even n), then the sums of
+// cuvarbase/lombscargle.py:337-400 (mhdirect_sums) with the regulariser of
+// :403-447, the 2H x 2H system solved by Gaussian elimination with partial
+// pivoting, and the power of :497-536.  H = 3, 1,000 points, 20,000
+// frequencies, host to host: 4.93 -> 2.55 ms.
+template <int H>
+__global__ void __launch_bounds__(kDirThreads, H <= 4 ? 2 : 1)
+k_mhgls_direct(const double *__restrict__ t, const double *__restrict__ yw,
+               const double *__restrict__ w, long long n, const double *__restrict__ freqs,
+               long long nf, MhParams mp, double *__restrict__ out) {
+    constexpr int NH = 2 * H, NS = mh_sums(H);
+    extern __shared__ __align__(16) double sm[];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    double2 *turn = reinterpret_cast<double2 *>(sm);
+    double *st = sm + 2 * kTurn + wid * 96, *sy = st + 32, *sw = st + 64;
+    for (int i = tid; i < kTurn; i += kDirThreads) turn[i] = zturn((double)i / kTurn);
+    __syncthreads();
+    const long long k = (long long)blockIdx.x * 32 + lane;
+    const double f = (k < nf) ? freqs[k] : 0.0;
+    double c[NH + 1], s[NH + 1], yc[H + 1], ys[H + 1];
+#pragma unroll
+    for (int m = 0; m <= NH; ++m) { c[m] = 0.0; s[m] = 0.0; }
+#pragma unroll
+    for (int m = 0; m <= H; ++m) { yc[m] = 0.0; ys[m] = 0.0; }
+    double ws = 0.0;  // of the points this lane staged
+    for (long long base = wid * 32; base < n; base += kDirThreads) {
+        const int cnt = (int)min(32LL, n - base);
+        __syncwarp();  // the previous tile is consumed
+        if (lane < cnt) {
+            st[lane] = t[base + lane];
+            sy[lane] = yw[base + lane];
+            sw[lane] = w[base + lane];
+            ws += sw[lane];
+        }
+        __syncwarp();
+#pragma unroll 1
+        for (int q = 0; q < cnt; ++q) {
+            const double wq = sw[q], yq = sy[q];
+            double2 z[NH + 1];
+            z[1] = table_turn(st[q] * f, turn);
+#pragma unroll
+            for (int m = 1; m <= NH; ++m) {
+                if (m > 1 && m % 2 == 0) {
+                    const double2 h = z[m / 2];
+                    const double hx = h.x + h.x;
+                    z[m] = make_double2(fma(hx, h.x, -1.0), hx * h.y);
+                } else if (m > 1) {
+                    z[m] = zmul(z[m / 2], z[m - m / 2]);
+                }
+                c[m] = fma(wq, z[m].x, c[m]);
+                s[m] = fma(wq, z[m].y, s[m]);
+                if (m <= H) {
+                    yc[m] = fma(yq, z[m].x, yc[m]);
+                    ys[m] = fma(yq, z[m].y, ys[m]);
+                }
+            }
+        }
+    }
+    // the eight warps' sums, in shared memory as [warp][sum][lane]
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ws += __shfl_xor_sync(0xffffffffu, ws, o);
+    __syncthreads();
+    {
+        double *r = sm + wid * NS * 32 + lane;
+#pragma unroll
+        for (int m = 1; m <= NH; ++m) {
+            r[(m - 1) * 32] = c[m];
+            r[(NH + m - 1) * 32] = s[m];
+        }
+#pragma unroll
+        for (int m = 1; m <= H; ++m) {
+            r[(2 * NH + m - 1) * 32] = yc[m];
+            r[(2 * NH + H + m - 1) * 32] = ys[m];
+        }
+        r[6 * H * 32] = ws;
+    }
+    __syncthreads();
+    double *tot = sm + kDirWarps * NS * 32;
+    for (int i = tid; i < NS * 32; i += kDirThreads) {
+        double v = 0.0;
+        for (int q = 0; q < kDirWarps; ++q) v += sm[q * NS * 32 + i];
+        tot[i] = v;
+    }
+    __syncthreads();
+    if (wid != 0 || k >= nf) return;
+#pragma unroll
+    for (int m = 1; m <= NH; ++m) {
+        c[m] = tot[(m - 1) * 32 + lane];
+        s[m] = tot[(NH + m - 1) * 32 + lane];
+    }
+#pragma unroll
+    for (int m = 1; m <= H; ++m) {
+        yc[m] = tot[(2 * NH + m - 1) * 32 + lane];
+        ys[m] = tot[(2 * NH + H + m - 1) * 32 + lane];
+    }
+    c[0] = tot[6 * H * 32 + lane];
+    // regularised blocks: M = [[CC, CS], [CS^T, SS]], rhs = [YC; YS]
+    double M[NH][NH], rhs[NH];
+#pragma unroll
+    for (int a = 1; a <= H; ++a) {
+#pragma unroll
+        for (int b = 1; b <= H; ++b) {
+            const int dd = a > b ? a - b : b - a;
+            const double sg = (a >= b) ? 1.0 : -1.0;  // sign(a - b), 1 at a == b
+            const double reg = (a == b) ? mp.d[a - 1] : 0.0;
+            const double cc = 0.5 * (c[a + b] + c[dd]) - c[a] * c[b] + reg;
+            const double cs = 0.5 * (s[a + b] - sg * s[dd]) - c[a] * s[b];
+            const double ss = 0.5 * (c[dd] - c[a + b]) - s[a] * s[b] + reg;
+            M[a - 1][b - 1] = cc;
+            M[a - 1][H + b - 1] = cs;
+            M[H + b - 1][a - 1] = cs;
+            M[H + a - 1][H + b - 1] = ss;
+        }
+        rhs[a - 1] = yc[a] - mp.ybar * c[a] + mp.d[a - 1] * mp.cn0[a - 1];
+        rhs[H + a - 1] = ys[a] - mp.ybar * s[a] + mp.d[a - 1] * mp.sn0[a - 1];
+    }
+    // Gaussian elimination with partial pivoting on a copy
+    double W[NH][NH + 1];
+#pragma unroll
+    for (int r = 0; r < NH; ++r) {
+#pragma unroll
+        for (int q = 0; q < NH; ++q) W[r][q] = M[r][q];
+        W[r][NH] = rhs[r];
+    }
+    bool singular = false;
+    for (int col = 0; col < NH; ++col) {
+        int piv = col;
+        double best = fabs(W[col][col]);
+        for (int r = col + 1; r < NH; ++r)
+            if (fabs(W[r][col]) > best) { best = fabs(W[r][col]); piv = r; }
+        if (!(best > 0.0)) { singular = true; break; }
+        if (piv != col)
+            for (int q = col; q <= NH; ++q) {
+                const double tmp = W[col][q];
+                W[col][q] = W[piv][q];
+                W[piv][q] = tmp;
+            }
+        for (int r = col + 1; r < NH; ++r) {
+            const double fct = W[r][col] / W[col][col];
+            for (int q = col; q <= NH; ++q) W[r][q] = fma(-fct, W[col][q], W[r][q]);
+        }
+    }
+    double th[NH];
+    if (!singular) {
+        for (int r = NH - 1; r >= 0; --r) {
+            double v = W[r][NH];
+            for (int q = r + 1; q < NH; ++q) v = fma(-W[r][q], th[q], v);
+            th[r] = v / W[r][r];
+        }
+    }
+    if (singular) {
+        out[k] = nan("");
+        return;
+    }
+    // P = (YX - sum XX) / YY with the regularised blocks
+    double xx = 0.0, yx = 0.0;
+#pragma unroll
+    for (int a = 0; a < H; ++a) {
+        yx += th[a] * rhs[a] + th[H + a] * rhs[H + a];
+#pragma unroll
+        for (int b = 0; b < H; ++b)
+            xx += th[a] * th[b] * M[a][b] + 2.0 * th[a] * th[H + b] * M[a][H + b] +
+                  th[H + a] * th[H + b] * M[H + a][H + b];
+    }
+    out[k] = (2.0 * yx - xx) / mp.yy;
+}
+
+cudaError_t launch_mhgls_direct(int nharms, const double *t, const double *yw, const double *w,
+                                long long n, const double *freqs, long long nf,
+                                const MhParams &mp, double *out, cudaStream_t s) {
+    if (n <= 0 || nf <= 0) return cudaSuccess;
+    const long long nb = (nf + 31) / 32;
+    if (nb > 0x7fffffffLL) return cudaErrorInvalidValue;
+    cudaError_t e = cudaErrorInvalidValue;
+    switch (nharms) {
+#define CUVGLS_MH(HH)                                                                             \
+    case HH:                                                                                      \
+        e = cudaFuncSetAttribute(k_mhgls_direct<HH>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+                                 mh_smem(HH));                                                    \
+        if (e != cudaSuccess) return e;                                                           \
+        k_mhgls_direct<HH><<<(unsigned)nb, kDirThreads, mh_smem(HH), s>>>(t, yw, w, n, freqs, nf, \
+                                                                          mp, out);               \
+        break;
+        CUVGLS_MH(1) CUVGLS_MH(2) CUVGLS_MH(3) CUVGLS_MH(4)
+        CUVGLS_MH(5) CUVGLS_MH(6) CUVGLS_MH(7) CUVGLS_MH(8)
+#undef CUVGLS_MH
+        default: return e;
+    }
+    return cudaGetLastError();
+}
+
+}  // namespace cuvgls

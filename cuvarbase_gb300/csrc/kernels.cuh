@@ -111,10 +111,18 @@ cudaError_t launch_spread_ref(const RefGridCurve *cv, int n_curves,
 struct Direct64Curve {
     long long pt_off, n, nf, out_off;
     double f0, df;
+    long long part_off;  // first partial sum of the curve within a part
+    int splits;          // parts its points are cut into
 };
+// Parts to cut the points of a direct-sum batch into, so that `bins`
+// frequencies in all still make enough CTAs of bins_per_cta (1: no parts).
+int direct_splits(long long bins, int bins_per_cta, long long max_n);
+int nfft_direct64_bins();
+int gls_direct_bins();
+// `part`: max_splits x part_stride partial sums (when max_splits > 1).
 cudaError_t launch_nfft_direct64(const Direct64Curve *cv, int n_curves, long long max_nf,
-                                 const double *t, const double *y, double2 *out,
-                                 cudaStream_t s);
+                                 int max_splits, const double *t, const double *y, double2 *out,
+                                 double2 *part, long long part_stride, cudaStream_t s);
 
 // Finish of a caller-given reference-convention grid g of length ng (the
 // reference's use_grid): shift by exp(2 pi i j ks / ng), inverse DFT, then
@@ -145,9 +153,11 @@ cudaError_t launch_mhgls_direct(int nharms, const double *t, const double *yw, c
                                 long long n, const double *freqs, long long nf,
                                 const MhParams &mp, double *out, cudaStream_t s);
 
-cudaError_t launch_gls_direct(const DevCurve *cv, int n_curves, int max_nf,
-                              const double *t, const float *yw, const float *w,
-                              float *out, GlsParams g, cudaStream_t s);
-
+// GLS powers by FP64 direct sums; aux of a descriptor holds its number of
+// parts and inter_off its first partial sum.  `part`: max_splits x part_stride
+// triples (when max_splits > 1).
+cudaError_t launch_gls_direct(const DevCurve *cv, int n_curves, int max_nf, int max_splits,
+                              const double *t, const float *yw, const float *w, float *out,
+                              double2 *part, long long part_stride, GlsParams g, cudaStream_t s);
 
 }  // namespace cuvgls
