@@ -19,8 +19,7 @@
 
 using namespace cuvgls;
 
-static_assert(CUVGLS_MAX_CURVE_POINTS + cuvgls::kSegPoints <= 0x7fffffffLL,
-              "segment arithmetic of a curve stays within int");
+static_assert(CUVGLS_MAX_CURVE_POINTS <= 0x7fffffffLL - 1024, "points of a curve fit an int");
 static_assert(sizeof(cuvgls_gridfin_curve) == 72, "cuvgls_gridfin_curve layout");
 static_assert(sizeof(cuvgls_raw_curve) == 48 && sizeof(cuvgls_raw_input) == 72,
               "raw input layout");
@@ -457,13 +456,17 @@ struct Group {
     size_t rec_bytes;          // records + bins of the group
     size_t inter_bytes;        // largest intermediate of its chunks
     std::vector<Chunk> chunks;
-    // Its binning, in one part per input phase that holds its curves: the
-    // descriptors [first, first + count) and their segments, [seg_b, seg_m)
-    // single-segment descriptors, [seg_m, seg_e) segments of longer curves.
-    struct Part {
-        int first, count, seg_b, seg_m, seg_e;
-    };
-    std::vector<Part> parts;
+};
+
+// Curves prepared together: the descriptors [first, first + count), their
+// lists by length class in the list table (fused[c] .. fused[c + 1]; then
+// the long ones up to long_e) and the segments of the long ones.
+struct Part {
+    int first, count;
+    int fused[kPrepClasses + 1];
+    int long_e;
+    int max_n[kPrepClasses];   // longest curve of each class
+    int seg_b, seg_e;
 };
 
 // Shared driver of the GLS and NFFT batches.
@@ -507,47 +510,54 @@ int run_batch(cuvgls_handle *h, const Work &wk, std::vector<DevCurve> &cvs,
     for (int i = 0; i < nc; ++i) order[i] = i;
     std::stable_sort(order.begin(), order.end(),
                      [&](int a, int b) { return cls[a] < cls[b]; });
-    // Preparation segments, in SegEntry tables copied with the descriptors,
-    // both built per input phase once the groups are known.  Binning: per
-    // group, the single-segment descriptors first (binned whole by
-    // k_bin_scatter), then the segments of its longer curves (counted and
-    // scanned first).  Raw input: the curves of one segment first (done whole
-    // by k_raw_finish), then the segments of the longer ones (summed first);
-    // every band of a curve refers to its curve's first entry.
+    // Preparation tables, copied with the descriptors: the descriptors by
+    // length class and the segments of long curves (binning), and of raw
+    // input the segments of the curves that k_prep does not weigh itself:
+    // long ones, and all of them when some curve has several bands (a curve
+    // is weighed once and binned per band).
     const bool raw = wk.ry != nullptr;
     long long nseg_bin = 0;
     for (int i = 0; i < nc; ++i) {
-        nseg_bin += seg_count(cvs[i].n);
-        cvs[i].flags = 0;
+        cvs[i].geom = pack_geom(cls[i]->plan.G1, cls[i]->plan.G2, cls[i]->plan.B);
+        if (cvs[i].n > kFusePoints) nseg_bin += seg_count(cvs[i].n);
     }
-    if (nseg_bin > 0x7fffffffLL) return fail(h, CUVGLS_ENOTSUP, "too many points");
-    // (the raw table itself is built once the input phases are known)
-    std::vector<int> bands;
-    long long nseg_raw = 0;
     bool multi_band = false;
     if (raw) {
-        bands.assign(wk.n_raw, 0);
+        std::vector<char> seen(wk.n_raw, 0);
         for (const DevCurve &cv : cvs) {
-            if (++bands[cv.best_slot] > 1) multi_band = true;
-            if (cv.best_off == 0) nseg_raw += seg_count(cv.n);
+            if (seen[cv.best_slot]) multi_band = true;
+            seen[cv.best_slot] = 1;
         }
     }
+    auto raw_apart = [&](const DevCurve &cv) {
+        return raw && (multi_band || cv.n > kFusePoints);
+    };
+    long long nseg_raw = 0;
+    for (const DevCurve &cv : cvs)
+        if (raw_apart(cv) && cv.best_off == 0) nseg_raw += seg_count(cv.n);
+    if (nseg_bin > 0x7fffffffLL || nseg_raw > 0x7fffffffLL)
+        return fail(h, CUVGLS_ENOTSUP, "too many points");
     // Budget: the arena holds the staged inputs / outputs, the descriptor and
     // segment tables ("fixed"), then the records and bins of one prep group, then the
     // intermediate of one FFT chunk (at most chunk_mb).  Preparing many
     // curves per launch keeps the prep kernel's grid deep.
     const size_t npts = (size_t)wk.n_points_total;
     const size_t in_bytes =
-        raw ? ((wk.flags & CUVGLS_HOST_INPUT) ? 3 * align_up(npts * 8) : 0) + align_up(npts * 8) +
-                  2 * align_up(npts * 4) + 2 * align_up(nseg_raw * sizeof(double4))
+        raw ? ((wk.flags & CUVGLS_HOST_INPUT) ? 3 * align_up(npts * 8) : 0) +
+                  (nseg_raw ? align_up(npts * 8) + 2 * align_up(npts * 4) +
+                                  2 * align_up(nseg_raw * sizeof(double4))
+                            : 0)
             : (wk.flags & CUVGLS_HOST_INPUT) ? align_up(npts * 8) + 2 * align_up(npts * 4) : 0;
     const bool best = wk.n_best > 0;
     const size_t out_bytes = !(wk.flags & CUVGLS_HOST_OUTPUT) ? 0
         : best ? align_up(wk.n_best * 8) + align_up(wk.n_best * 4)
                : align_up(wk.n_out_total * wk.out_elem);
     const size_t best_bytes = best ? align_up(wk.n_best * sizeof(unsigned long long)) : 0;
-    // descriptors, then the binning and raw segment tables, in one copy
-    const size_t tab_bytes = nc * sizeof(DevCurve) + (nseg_bin + nseg_raw) * sizeof(SegEntry);
+    // descriptors, then the binning and raw segment tables, the descriptors
+    // by length class and those of raw curves weighed apart, in one copy
+    const int nlist = nc + (nseg_raw ? nc : 0);
+    const size_t tab_bytes = nc * sizeof(DevCurve) + (nseg_bin + nseg_raw) * sizeof(SegEntry) +
+                             nlist * sizeof(int);
     const size_t cv_bytes = align_up(tab_bytes);
     const size_t aux_bytes = align_up(nc * sizeof(float4));
     const size_t fixed = in_bytes + out_bytes + best_bytes + cv_bytes + aux_bytes + kAlign;
@@ -671,37 +681,45 @@ int run_batch(cuvgls_handle *h, const Work &wk, std::vector<DevCurve> &cvs,
         }
     }
     const int nph = (int)pb.size() - 1;
-    // Raw segment table, per phase: the curves of one segment first (done
-    // whole by k_raw_finish), then the segments of the longer ones (summed
-    // first); every band of a curve refers to its curve's first entry.
-    // raw_ph[ph] = {first entry, first multi-segment entry, end}.
+    // Segments and descriptors of the raw curves weighed apart, per phase;
+    // every band of a curve refers to its curve's first entry.
+    // raw_ph[ph] = {first segment, end, first descriptor, end}.
     std::vector<SegEntry> raw_tab;
-    std::vector<std::array<int, 3>> raw_ph(nph, std::array<int, 3>{0, 0, 0});
-    bool need_fill = false;
-    if (raw) {
+    std::vector<int> raw_list;
+    std::vector<std::array<int, 4>> raw_ph(nph, std::array<int, 4>{0, 0, 0, 0});
+    if (nseg_raw) {
         raw_tab.reserve((size_t)nseg_raw);
         std::vector<int> first(wk.n_raw, 0);
         for (int ph = 0; ph < nph; ++ph) {
-            const int i0 = pb[ph], i1 = pb[ph + 1];
             raw_ph[ph][0] = (int)raw_tab.size();
-            for (int pass = 0; pass < 2; ++pass) {
-                if (pass == 1) raw_ph[ph][1] = (int)raw_tab.size();
-                for (int i = i0; i < i1; ++i) {
-                    DevCurve &cv = cvs[order[i]];
-                    const int ns = seg_count(cv.n);
-                    if (cv.best_off != 0 || (ns > 1) != (pass == 1)) continue;
-                    first[cv.best_slot] = (int)raw_tab.size();
-                    for (int k = 0; k < ns; ++k) raw_tab.push_back(SegEntry{i, k * kSegPoints});
-                    if (pass == 0 && bands[cv.best_slot] == 1) cv.flags = kDescFillHere;
-                }
+            raw_ph[ph][2] = (int)raw_list.size();
+            for (int i = pb[ph]; i < pb[ph + 1]; ++i) {
+                const DevCurve &cv = cvs[order[i]];
+                if (!raw_apart(cv)) continue;
+                raw_list.push_back(i);
+                if (cv.best_off != 0) continue;
+                first[cv.best_slot] = (int)raw_tab.size();
+                const int ns = seg_count(cv.n);
+                for (int k = 0; k < ns; ++k) raw_tab.push_back(SegEntry{i, k * kSegPoints});
             }
-            raw_ph[ph][2] = (int)raw_tab.size();
+            raw_ph[ph][1] = (int)raw_tab.size();
+            raw_ph[ph][3] = (int)raw_list.size();
         }
-        for (DevCurve &cv : cvs) {
-            cv.raw_seg = first[cv.best_slot];
-            if (!(cv.flags & kDescFillHere)) need_fill = true;
-        }
+        for (DevCurve &cv : cvs) cv.raw_seg = first[cv.best_slot];
     }
+    // One preparation serves all groups when their points arrive in one
+    // phase and the records of all of them fit beside the largest
+    // intermediate; else each group is prepared when its turn comes, over the
+    // same memory.
+    size_t all_rec = 0, max_inter = 0;
+    long long all_bins = 0;
+    for (const Group &g : groups) {
+        all_rec += g.rec_bytes;
+        max_inter = std::max(max_inter, g.inter_bytes);
+        all_bins += (long long)g.count * (g.cls->plan.nb + 1);
+    }
+    const bool merged = nph == 1 && all_rec + max_inter <= avail && all_bins < 0x7fffffffLL;
+    if (merged) max_group_bytes = all_rec + max_inter;
     if ((int)h->chunk_events.size() < 3 + nph) {
         // two for alternating chunk copies, the start of the later phases'
         // input copies, then the end of each later phase's copies
@@ -721,12 +739,13 @@ int run_batch(cuvgls_handle *h, const Work &wk, std::vector<DevCurve> &cvs,
     DevCurve *d_cv = (DevCurve *)take(tab_bytes);
     SegEntry *d_bseg = reinterpret_cast<SegEntry *>(d_cv + nc);
     SegEntry *d_rseg = d_bseg + nseg_bin;
+    int *d_list = reinterpret_cast<int *>(d_rseg + nseg_raw);
     float4 *d_aux = (float4 *)take(nc * sizeof(float4));
     const double *t = wk.t;
     const float *ya = wk.ya, *wv = wk.wv;
     const double *ry = wk.ry, *rdy = wk.rdy;
     double4 *partA = nullptr, *partB = nullptr;
-    double *d_ir = nullptr;  // dy^-2 of the raw points of longer curves
+    double *d_ir = nullptr;  // dy^-2 of the raw points weighed apart
     // Host input: phase 0's points on the work stream, then each later
     // phase's on the input stream (not behind the output copies), ending
     // with its event.  Those start once phase 0's copies are done, so that
@@ -776,11 +795,13 @@ int run_batch(cuvgls_handle *h, const Work &wk, std::vector<DevCurve> &cvs,
             copy_in(dd, wk.rdy, 8);
             t = dt; ry = dy; rdy = dd;
         }
-        ya = (const float *)take(npts * 4);
-        wv = (const float *)take(npts * 4);
-        d_ir = (double *)take(npts * 8);
-        partA = (double4 *)take(nseg_raw * sizeof(double4));
-        partB = (double4 *)take(nseg_raw * sizeof(double4));
+        if (nseg_raw) {
+            ya = (const float *)take(npts * 4);
+            wv = (const float *)take(npts * 4);
+            d_ir = (double *)take(npts * 8);
+            partA = (double4 *)take(nseg_raw * sizeof(double4));
+            partB = (double4 *)take(nseg_raw * sizeof(double4));
+        }
     } else if (wk.flags & CUVGLS_HOST_INPUT) {
         double *dt = (double *)take(npts * 8);
         float *dy = (float *)take(npts * 4);
@@ -811,43 +832,69 @@ int run_batch(cuvgls_handle *h, const Work &wk, std::vector<DevCurve> &cvs,
     rc = ensure_host_cv(h, (tab_bytes + sizeof(DevCurve) - 1) / sizeof(DevCurve));
     if (rc) return rc;
     SegEntry *h_bseg = reinterpret_cast<SegEntry *>(h->h_cv + nc);
-    int sidx = 0;
-    for (Group &g : groups) {
-        const Plan &p = g.cls->plan;
-        long long rec = 0;
-        for (int k = 0; k < g.count; ++k) {
-            DevCurve cv = cvs[order[g.first + k]];
-            cv.rec_off = rec;
-            cv.bin_off = (long long)k * (p.nb + 1);
-            cv.aux = g.first + k;
-            rec += cv.n;
-            h->h_cv[g.first + k] = cv;
-        }
-        for (const Chunk &ch : g.chunks)
-            for (int k = 0; k < ch.count; ++k)
-                h->h_cv[ch.first + k].inter_off = (long long)k * wk.ng * p.G;
-        // one binning part per input phase that holds curves of the group
-        g.parts.clear();
-        for (int ph = 0; ph < nph; ++ph) {
-            const int k0 = std::max(pb[ph], g.first) - g.first;
-            const int k1 = std::min(pb[ph + 1], g.first + g.count) - g.first;
-            if (k1 <= k0) continue;
-            Group::Part pt{g.first + k0, k1 - k0, sidx, 0, 0};
-            for (int k = k0; k < k1; ++k)
-                if (h->h_cv[g.first + k].n <= kSegPoints) h_bseg[sidx++] = SegEntry{g.first + k, 0};
-            pt.seg_m = sidx;
-            for (int k = k0; k < k1; ++k) {
-                const int ns = seg_count(h->h_cv[g.first + k].n);
-                if (ns > 1)
-                    for (int q = 0; q < ns; ++q)
-                        h_bseg[sidx++] = SegEntry{g.first + k, q * kSegPoints};
+    int *h_list = reinterpret_cast<int *>(h_bseg + nseg_bin + nseg_raw);
+    int sidx = 0, lidx = 0;
+    // descriptors [first, first + count) as one part
+    auto make_part = [&](int first, int count) {
+        Part pt;
+        pt.first = first;
+        pt.count = count;
+        for (int c = 0; c <= kPrepClasses; ++c) {
+            pt.fused[c] = lidx;
+            if (c < kPrepClasses) pt.max_n[c] = 0;
+            for (int k = first; k < first + count; ++k) {
+                const int n = h->h_cv[k].n;
+                if ((n > kFusePoints ? kPrepClasses : prep_class(n)) != c) continue;
+                h_list[lidx++] = k;
+                if (c < kPrepClasses) pt.max_n[c] = std::max(pt.max_n[c], n);
             }
-            pt.seg_e = sidx;
-            g.parts.push_back(pt);
+        }
+        pt.long_e = lidx;
+        pt.seg_b = sidx;
+        for (int k = pt.fused[kPrepClasses]; k < pt.long_e; ++k) {
+            const int ns = seg_count(h->h_cv[h_list[k]].n);
+            for (int q = 0; q < ns; ++q) h_bseg[sidx++] = SegEntry{h_list[k], q * kSegPoints};
+        }
+        pt.seg_e = sidx;
+        return pt;
+    };
+    std::vector<std::vector<Part>> parts(groups.size());  // of each group (all in the first)
+    {
+        long long rec = 0, bins = 0;
+        for (const Group &g : groups) {
+            const Plan &p = g.cls->plan;
+            if (!merged) rec = bins = 0;
+            for (int k = 0; k < g.count; ++k) {
+                DevCurve cv = cvs[order[g.first + k]];
+                cv.rec_off = rec;
+                cv.bin_off = (int)bins;
+                cv.aux = g.first + k;
+                rec += cv.n;
+                bins += p.nb + 1;
+                h->h_cv[g.first + k] = cv;
+            }
+            for (const Chunk &ch : g.chunks)
+                for (int k = 0; k < ch.count; ++k)
+                    h->h_cv[ch.first + k].inter_off = (long long)k * wk.ng * p.G;
+        }
+        if (merged) {
+            parts[0].push_back(make_part(0, nc));
+        } else {
+            for (size_t gi = 0; gi < groups.size(); ++gi) {
+                const Group &g = groups[gi];
+                // one part per input phase that holds curves of the group
+                for (int ph = 0; ph < nph; ++ph) {
+                    const int k0 = std::max(pb[ph], g.first);
+                    const int k1 = std::min(pb[ph + 1], g.first + g.count);
+                    if (k1 > k0) parts[gi].push_back(make_part(k0, k1 - k0));
+                }
+            }
         }
     }
-    if (nseg_raw > 0)
+    if (nseg_raw > 0) {
         memcpy(h_bseg + nseg_bin, raw_tab.data(), nseg_raw * sizeof(SegEntry));
+        memcpy(h_list + nc, raw_list.data(), raw_list.size() * sizeof(int));
+    }
     CK(cudaMemcpyAsync(d_cv, h->h_cv, tab_bytes, cudaMemcpyHostToDevice, s),
        "H2D descriptors");
     CK(cudaEventRecord(h->h_cv_free, s), "record");
@@ -857,23 +904,19 @@ int run_batch(cuvgls_handle *h, const Work &wk, std::vector<DevCurve> &cvs,
     // (1.3 ms on the bench workload) before the first chunk could start.
     CK(issue_in(), "H2D input");
     const bool in_copies = ninc > 0 && nph > 1;  // later phases wait for their copies
-    // weights, yw and statistics of one phase's raw curves on the device,
-    // then the descriptors' normalisation from them
+    // weights, yw and statistics of one phase's raw curves weighed apart
     auto prep_raw = [&](int ph) -> int {
-        const int b = raw_ph[ph][0], m = raw_ph[ph][1], e = raw_ph[ph][2];
-        if (m < e)
+        const std::array<int, 4> &r = raw_ph[ph];
+        if (r[1] > r[0])
             LAUNCH(CUVGLS_STAGE_PREP, s,
-                   launch_raw_sums(d_rseg + m, e - m, d_cv, ry, rdy, d_ir, partA, s),
-                   "k_raw_sums");
-        if (b < e)
+                   launch_raw_long(d_rseg + r[0], r[1] - r[0], d_cv, ry, rdy, d_ir, (float *)ya,
+                                   (float *)wv, partA, partB, s),
+                   "k_raw_sums, k_raw_finish");
+        if (r[1] > r[0]) h->launches[CUVGLS_STAGE_PREP] += 1;  // two kernels
+        if (r[3] > r[2])
             LAUNCH(CUVGLS_STAGE_PREP, s,
-                   launch_raw_finish(d_rseg + b, e - b, d_cv, ry, rdy, d_ir, (float *)ya,
-                                     (float *)wv, partA, partB, mode, s),
-                   "k_raw_finish");
-        const int c0 = pb[ph], c1 = pb[ph + 1];
-        if (need_fill && c1 > c0)
-            LAUNCH(CUVGLS_STAGE_PREP, s,
-                   launch_fill_desc(d_cv + c0, c1 - c0, partA, partB, mode, s), "k_fill_desc");
+                   launch_fill_desc(d_cv, d_list + nc + r[2], r[3] - r[2], partA, partB, mode, s),
+                   "k_fill_desc");
         return CUVGLS_OK;
     };
     // the phases up to the one of descriptor `first`, before its first
@@ -896,44 +939,58 @@ int run_batch(cuvgls_handle *h, const Work &wk, std::vector<DevCurve> &cvs,
         if (rc) return rc;
     }
     int evi = 0;
-    for (const Group &g : groups) {
+    const int fp32 = h->opts.precision == CUVGLS_PREC_FP32;
+    PrepArrays pa{d_cv, t, ry, rdy, ya, wv, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
+                  wk.ng == 1 ? d_aux : nullptr, h->d_flags, mode, 0};
+    RecAB *recAB = nullptr;
+    RecC *recC = nullptr;
+    int *binsAB = nullptr, *binsC = nullptr;
+    float2 *inter = nullptr;
+    for (size_t gi = 0; gi < groups.size(); ++gi) {
+        const Group &g = groups[gi];
         const Plan &p = g.cls->plan;
-        size_t o2 = 0;
-        auto gtake = [&](size_t bytes) { char *q = group_base + o2; o2 += align_up(bytes); return q; };
-        RecAB *recAB = (RecAB *)gtake(g.n_pts * sizeof(RecAB));
-        RecC *recC = (RecC *)gtake(g.n_pts * sizeof(RecC));
-        const size_t nbin = (size_t)g.count * (p.nb + 1);
-        int *binsAB = (int *)gtake(4 * nbin * sizeof(int));
-        int *binsC = binsAB + nbin, *curAB = binsC + nbin, *curC = curAB + nbin;
-        float2 *inter = (float2 *)gtake(g.inter_bytes);
-        const int fp32 = h->opts.precision == CUVGLS_PREC_FP32;
-        float4 *gaux = wk.ng == 1 ? d_aux : nullptr;
-        bool multi = false;  // curves longer than one segment
-        for (const Group::Part &pt : g.parts) multi = multi || pt.seg_e > pt.seg_m;
-        if (multi) CK(cudaMemsetAsync(binsAB, 0, 2 * nbin * sizeof(int), s), "zero bins");
-        auto bin_part = [&](const Group::Part &pt) -> int {
-            if (pt.seg_e > pt.seg_m) {
-                LAUNCH(CUVGLS_STAGE_PREP, s,
-                       launch_bin_count(d_bseg + pt.seg_m, pt.seg_e - pt.seg_m, d_cv, t, binsAB,
-                                        binsC, p, wk.ng, fp32, s),
-                       "k_bin_count");
-                LAUNCH(CUVGLS_STAGE_PREP, s,
-                       launch_bin_scan(d_cv + pt.first, pt.count, t, binsAB, binsC, curAB, curC,
-                                       gaux, p, wk.ng, s),
-                       "k_bin_scan");
+        if (!merged || gi == 0) {  // lay out the records and bins of the groups prepared now
+            size_t o2 = 0;
+            auto gtake = [&](size_t bytes) { char *q = group_base + o2; o2 += align_up(bytes); return q; };
+            long long pts = 0, nbin = 0;
+            bool multi = false;  // long curves
+            pa.max_nb = 0;
+            for (size_t k = gi; k < (merged ? groups.size() : gi + 1); ++k) {
+                pts += groups[k].n_pts;
+                nbin += (long long)groups[k].count * (groups[k].cls->plan.nb + 1);
+                pa.max_nb = std::max(pa.max_nb, groups[k].cls->plan.nb);
+                for (const Part &pt : parts[k]) multi = multi || pt.seg_e > pt.seg_b;
             }
-            LAUNCH(CUVGLS_STAGE_PREP, s,
-                   launch_bin_scatter(d_bseg + pt.seg_b, pt.seg_e - pt.seg_b, d_cv, t, ya, wv,
-                                      recAB, recC, binsAB, binsC, curAB, curC, gaux, p, wk.ng,
-                                      fp32, h->d_flags, s),
-                   "k_bin_scatter");
+            pa.recAB = recAB = (RecAB *)gtake(pts * sizeof(RecAB));
+            pa.recC = recC = (RecC *)gtake(pts * sizeof(RecC));
+            pa.binsAB = binsAB = (int *)gtake(4 * nbin * sizeof(int));
+            pa.binsC = binsC = binsAB + nbin;
+            pa.curAB = binsC + nbin;
+            pa.curC = pa.curAB + nbin;
+            inter = (float2 *)gtake(merged ? max_inter : g.inter_bytes);
+            if (multi) CK(cudaMemsetAsync(binsAB, 0, 2 * nbin * sizeof(int), s), "zero bins");
+        }
+        auto prep_part = [&](const Part &pt) -> int {
+            for (int c = 0; c < kPrepClasses; ++c)
+                if (pt.fused[c + 1] > pt.fused[c])
+                    LAUNCH(CUVGLS_STAGE_PREP, s,
+                           launch_prep(pa, d_list + pt.fused[c], pt.fused[c + 1] - pt.fused[c], c,
+                                       pt.max_n[c], raw && !multi_band, wk.ng, fp32, s),
+                           "k_prep");
+            if (pt.seg_e > pt.seg_b)
+                LAUNCH(CUVGLS_STAGE_PREP, s,
+                       launch_bin_long(pa, d_bseg + pt.seg_b, pt.seg_e - pt.seg_b,
+                                       d_list + pt.fused[kPrepClasses],
+                                       pt.long_e - pt.fused[kPrepClasses], wk.ng, fp32, s),
+                       "k_bin_count, k_bin_scan, k_bin_scatter");
+            if (pt.seg_e > pt.seg_b) h->launches[CUVGLS_STAGE_PREP] += 2;  // three kernels
             return CUVGLS_OK;
         };
-        size_t pi = 0;  // next binning part (each starts at a chunk)
+        size_t pi = 0;  // next part (each starts at a chunk)
         for (const Chunk &ch : g.chunks) {
-            while (pi < g.parts.size() && g.parts[pi].first < ch.first + ch.count) {
-                rc = reach(g.parts[pi].first);
-                if (!rc) rc = bin_part(g.parts[pi]);
+            while (pi < parts[gi].size() && parts[gi][pi].first < ch.first + ch.count) {
+                rc = reach(parts[gi][pi].first);
+                if (!rc) rc = prep_part(parts[gi][pi]);
                 if (rc) return rc;
                 ++pi;
             }
@@ -1798,10 +1855,9 @@ int cuvgls_batch_bytes(cuvgls_handle *h, int32_t n_curves, const int64_t *n,
         const int a = k.G1, b = k.G2, B = k.B;
         long long per = 3LL * a * b * (long long)sizeof(float2);
         per += n[i] * (long long)(sizeof(RecAB) + sizeof(RecC));
-        per += 4LL * (b / B + 1) * 4 + sizeof(DevCurve) + sizeof(float4) + 64;
+        per += 4LL * (b / B + 1) * 4 + sizeof(DevCurve) + sizeof(float4) + 72;
         // segment tables and the raw-preparation partials
-        per += (n[i] + kSegPoints - 1) / kSegPoints *
-               (long long)(2 * sizeof(SegEntry) + 2 * sizeof(double4));
+        per += (n[i] + 1023) / 1024 * (long long)(2 * sizeof(SegEntry) + 2 * sizeof(double4));
         tot += ns * per;
         // staged host input (raw t, y, dy in FP64, dy^-2, yw and w: 40 B per
         // point; prepared input needs 16) and the staged powers

@@ -13,31 +13,38 @@ struct RefGridCurve {  // device copy of cuvgls_grid_curve
     long long out_off;
 };
 
-// Segment tables of a descriptor table: binning segments of every
-// descriptor at its seg0 and, where raw_segs is given, the raw-preparation
-// segments of every curve (its band with best_off == 0) at raw_seg.
-cudaError_t launch_seg_fill(const DevCurve *cv, int n, SegEntry *bin_segs, SegEntry *raw_segs,
-                            cudaStream_t s);
+// Arrays of a preparation launch.  Records and bin offsets of a descriptor
+// start at its rec_off / bin_off.
+struct PrepArrays {
+    DevCurve *cv;
+    const double *t, *ry, *rdy;  // raw input: t, y, dy
+    const float *ya, *wv;        // prepared input: yw (or y) and w
+    RecAB *recAB;
+    RecC *recC;
+    int *binsAB, *binsC;         // nb + 1 offsets per descriptor
+    int *curAB, *curC;           // cursors (long curves)
+    float4 *aux;                 // output phases of the adjoint NFFT, or null
+    unsigned *errflag;
+    int mode;                    // GLS mode (raw input)
+    int max_nb;                  // most column blocks of the launch's plans
+};
 
-// Binning of a group (ngrids = 3, GLS: yw@x, w@x, w@2x; or 1, NFFT: y@x).
-// For curves longer than one segment: the count per segment into binsAB /
-// binsC (nb + 1 entries per descriptor at bin_off, zeroed by the caller),
-// then the scan per descriptor (offsets, cursors curAB / curC, aux).  Then
-// the scatter per segment, which also bins each curve of one segment
-// completely (offsets, records, aux).  Segment entries index cv; the scan
-// takes the group's own descriptors.  Count and scan skip single-segment
-// curves.
-cudaError_t launch_bin_count(const SegEntry *segs, int n_segs, const DevCurve *cv,
-                             const double *t, int *binsAB, int *binsC, const Plan &p,
-                             int ngrids, int fp32_positions, cudaStream_t s);
-cudaError_t launch_bin_scan(const DevCurve *cv, int n_curves, const double *t, int *binsAB,
-                            int *binsC, int *curAB, int *curC, float4 *aux, const Plan &p,
-                            int ngrids, cudaStream_t s);
-cudaError_t launch_bin_scatter(const SegEntry *segs, int n_segs, const DevCurve *cv,
-                               const double *t, const float *ya, const float *wv,
-                               RecAB *recAB, RecC *recC, int *binsAB, int *binsC, int *curAB,
-                               int *curC, float4 *aux, const Plan &p, int ngrids,
-                               int fp32_positions, unsigned *errflag, cudaStream_t s);
+// Curves of one length class (prep_class), each by one CTA or cluster: raw
+// weights and statistics (raw != 0), bin offsets and records.  `list`: their
+// descriptors (null: 0 .. n - 1); max_n: the longest; ngrids 3 (GLS: yw@x,
+// w@x, w@2x) or 1 (NFFT: y@x).
+cudaError_t launch_prep(const PrepArrays &a, const int *list, int n, int cls, int max_n, int raw,
+                        int ngrids, int fp32_positions, cudaStream_t s);
+
+// Binning of long curves: counts per segment (the counts of their
+// descriptors zeroed by the caller), scan per descriptor of `list`, records
+// per segment.
+cudaError_t launch_bin_long(const PrepArrays &a, const SegEntry *segs, int n_segs, const int *list,
+                            int n, int ngrids, int fp32_positions, cudaStream_t s);
+
+// Segment table of the descriptors 0 .. n - 1 filled on the device, each at
+// its raw_seg.
+cudaError_t launch_seg_fill(const DevCurve *cv, int n, SegEntry *segs, cudaStream_t s);
 
 // Dispatch on (G1, G2) to the compiled length templates; cudaErrorInvalidValue
 // if a length has no kernel.
@@ -79,22 +86,16 @@ cudaError_t launch_es_deconv(float *dst, long long G, int m, double beta, cudaSt
 // twiddles), fft_table_len(G1) + fft_table_len(G2) + G1 G2 entries at dst.
 cudaError_t launch_plan_tables(float2 *dst, int G1, int G2, int B, cudaStream_t s);
 
-// Host preparation of LombScargleMemory.setdata on the device for raw
-// (t, y, dy) input, over the raw-preparation segments (one double4 of
-// partA and partB each): k_raw_sums sums the segments of curves longer than
-// one segment; k_raw_finish does a curve of one segment completely
-// (w = dy^-2 / sum dy^-2 and yw = w (y - ybar) as FP32, the sums of YY, yw
-// and w, and the descriptor where flagged kDescFillHere) and writes w, yw
-// and the partial sums of the longer curves' segments; k_fill_desc gives
-// every unflagged descriptor its curve's statistics.
-cudaError_t launch_raw_sums(const SegEntry *segs, int n_segs, const DevCurve *cv,
-                            const double *y, const double *dy, double *ir, double4 *partA,
-                            cudaStream_t s);
-cudaError_t launch_raw_finish(const SegEntry *segs, int n_segs, DevCurve *cv, const double *y,
-                              const double *dy, const double *ir, float *yw, float *w,
-                              double4 *partA, double4 *partB, int mode, cudaStream_t s);
-cudaError_t launch_fill_desc(DevCurve *cv, int n, const double4 *partA, const double4 *partB,
-                             int mode, cudaStream_t s);
+// Host preparation of LombScargleMemory.setdata on the device for long raw
+// (t, y, dy) curves, over their segments (one double4 of partA and partB
+// each): k_raw_sums sums dy^-2, y dy^-2 and y; k_raw_finish writes w = dy^-2 /
+// sum dy^-2 and yw = w (y - ybar) as FP32 and their partial sums.
+cudaError_t launch_raw_long(const SegEntry *segs, int n_segs, const DevCurve *cv, const double *y,
+                            const double *dy, double *ir, float *yw, float *w, double4 *partA,
+                            double4 *partB, cudaStream_t s);
+// Statistics of the descriptors of `list` from their curves' partials.
+cudaError_t launch_fill_desc(DevCurve *cv, const int *list, int n, const double4 *partA,
+                             const double4 *partB, int mode, cudaStream_t s);
 
 // Per-curve best keys of k_pass2_gls to (index, power); -1 / -1 where a
 // curve had no valid power.

@@ -55,7 +55,7 @@ std::mutex g_scratch_mutex;
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
 // Descriptors handed to the device as a kernel parameter, kDescPerLaunch at
-// a time (32 x 104 bytes stays under the classic 4 KB parameter limit).
+// a time (32 x 96 bytes stays under the classic 4 KB parameter limit).
 constexpr int kDescPerLaunch = 32;
 struct DescChunk {
     DevCurve cv[kDescPerLaunch];
@@ -95,6 +95,7 @@ extern "C" int cuvgls_gls_noalloc(double sigma, int32_t m, const cuvgls_gls_inpu
     if (!(sigma >= 1.25 && sigma <= 16.0) || m < 2 || m > 16)
         return fail(CUVGLS_EINVAL, "sigma must be in [1.25, 16] and m in [2, 16]");
     long long max_nf = 0, n_tot = 0, n_seg = 0;
+    int max_n = 0;
     for (int i = 0; i < nc; ++i) {
         const cuvgls_curve &c = b->curves[i];
         if (c.n < 1 || c.nf < 1 || c.pt_off < 0 || c.out_off < 0 ||
@@ -106,6 +107,7 @@ extern "C" int cuvgls_gls_noalloc(double sigma, int32_t m, const cuvgls_gls_inpu
         max_nf = std::max(max_nf, (long long)c.nf);
         n_tot += c.n;
         n_seg += seg_count((int)c.n);
+        max_n = std::max(max_n, (int)c.n);
     }
     // one plan (the one for the largest nf) serves every curve of the call
     int G1, G2, B, R;
@@ -195,7 +197,8 @@ extern "C" int cuvgls_gls_noalloc(double sigma, int32_t m, const cuvgls_gls_inpu
             d.w_sum = (float)c.w_sum;
             d.rec_off = rec;
             d.bin_off = i * (p.nb + 1);
-            d.seg0 = seg;
+            d.geom = pack_geom(G1, G2, B);
+            d.raw_seg = seg;
             seg += seg_count(d.n);
             d.inter_off = (long long)i * 3 * G;
             d.aux = i;
@@ -212,20 +215,20 @@ extern "C" int cuvgls_gls_noalloc(double sigma, int32_t m, const cuvgls_gls_inpu
     int *binsAB = (int *)(base + o_bins);
     int *binsC = binsAB + nbin, *curAB = binsC + nbin, *curC = curAB + nbin;
     float2 *inter = (float2 *)(base + o_in);
-    // binning: the segment table is filled on the device (no host memory
-    // for it here); count and scan run only when a curve is longer than one
-    // segment, and skip the others
-    const int ns = (int)n_seg;
-    const bool multi = n_seg > nc;
-    if (e == cudaSuccess) e = launch_seg_fill(d_cv, nc, segs, nullptr, s);
-    if (e == cudaSuccess && multi) e = cudaMemsetAsync(binsAB, 0, 2 * nbin * sizeof(int), s);
-    if (e == cudaSuccess && multi)
-        e = launch_bin_count(segs, ns, d_cv, b->t, binsAB, binsC, p, 3, 0, s);
-    if (e == cudaSuccess && multi)
-        e = launch_bin_scan(d_cv, nc, b->t, binsAB, binsC, curAB, curC, nullptr, p, 3, s);
-    if (e == cudaSuccess)
-        e = launch_bin_scatter(segs, ns, d_cv, b->t, b->yw, b->w, recAB, recC, binsAB, binsC,
-                               curAB, curC, nullptr, p, 3, 0, d_flag, s);
+    // curves up to kFusePoints points in one launch; with a longer one all of
+    // them in segments, whose table is filled on the device (no host memory
+    // for it here)
+    const PrepArrays pa{d_cv, b->t, nullptr, nullptr, b->yw, b->w, recAB, recC, binsAB, binsC,
+                        curAB, curC, nullptr, d_flag, b->mode, p.nb};
+    if (max_n <= kFusePoints) {
+        if (e == cudaSuccess)
+            e = launch_prep(pa, nullptr, nc, prep_class(max_n), max_n, 0, 3, 0, s);
+    } else {
+        if (e == cudaSuccess) e = launch_seg_fill(d_cv, nc, segs, s);
+        if (e == cudaSuccess) e = cudaMemsetAsync(binsAB, 0, 2 * nbin * sizeof(int), s);
+        if (e == cudaSuccess)
+            e = launch_bin_long(pa, segs, (int)n_seg, nullptr, nc, 3, 0, s);
+    }
     if (e == cudaSuccess)
         e = launch_pass1(d_cv, nc, recAB, recC, binsAB, binsC, inter, p, 3, s);
     if (e == cudaSuccess)

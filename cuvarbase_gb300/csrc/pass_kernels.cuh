@@ -98,47 +98,6 @@ __device__ __forceinline__ void tile_fft2_a_occ(float2 *__restrict__ buf,
     }
 }
 
-// Exclusive scan of c[0..n) in place by the whole CTA of NT threads (each
-// thread a run of ceil(n / NT) consecutive entries), c[n] = total; ws holds
-// the 32 warp sums.  Ends with a barrier.
-template <int NT>
-__device__ __forceinline__ void block_scan_counts(int *c, int n, int *ws, int tid) {
-    static_assert(NT % 32 == 0 && NT <= 1024, "whole warps");
-    constexpr int NW = NT / 32;
-    const int per = (n + NT - 1) / NT;
-    const int i0 = min(tid * per, n), i1 = min(i0 + per, n);
-    int sum = 0;
-    for (int i = i0; i < i1; ++i) sum += c[i];
-    const int lane = tid & 31, wid = tid >> 5;
-    int inc = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += y;
-    }
-    if (lane == 31) ws[wid] = inc;
-    __syncthreads();
-    if (wid == 0) {
-        const int v = (lane < NW) ? ws[lane] : 0;
-        int iv = v;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, iv, o);
-            if (lane >= o) iv += y;
-        }
-        if (lane < NW) ws[lane] = iv - v;
-        if (lane == NW - 1) c[n] = iv;
-    }
-    __syncthreads();
-    int run = ws[wid] + inc - sum;
-    for (int i = i0; i < i1; ++i) {
-        const int v = c[i];
-        c[i] = run;
-        run += v;
-    }
-    __syncthreads();
-}
-
 // A record staged by pass 1: row << 16 | column of its cell, offset in the
 // cell, and its values (grids A and B, or grid C twice).
 struct StagedRec {
