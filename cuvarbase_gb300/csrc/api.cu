@@ -64,6 +64,12 @@ struct ClassTables {
 
 }  // namespace
 
+// Streams beside the caller's that the passes of a batch's groups (plans) are
+// spread over.  The kernels of one plan often fill a part of the chip for a
+// few tens of microseconds.  48 curves of 21 plans: 829 -> 510 us (with
+// the preparation of few points in one launch).
+constexpr int kSideStreams = 3;
+
 struct cuvgls_handle {
     cuvgls_opts opts;
     std::string err;
@@ -80,6 +86,10 @@ struct cuvgls_handle {
     cudaStream_t copy_stream = nullptr;   // device-to-host copies of the outputs
     cudaStream_t in_stream = nullptr;     // second-phase host-to-device input copies
     cudaStream_t table_stream = nullptr;  // builds the tables of new plan classes
+    // passes of groups that run beside the caller's stream (created when a
+    // batch first has several groups), with the events that fork and join them
+    cudaStream_t side[kSideStreams] = {};
+    cudaEvent_t side_ev[kSideStreams + 1] = {};
     cudaEvent_t done = nullptr;       // last enqueued work of this handle
     cudaStream_t last_stream = nullptr;
     bool have_last = false;
@@ -711,15 +721,32 @@ int run_batch(cuvgls_handle *h, const Work &wk, std::vector<DevCurve> &cvs,
     // phase and the records of all of them fit beside the largest
     // intermediate; else each group is prepared when its turn comes, over the
     // same memory.
-    size_t all_rec = 0, max_inter = 0;
+    size_t all_rec = 0, max_inter = 0, sum_inter = 0;
     long long all_bins = 0;
     for (const Group &g : groups) {
         all_rec += g.rec_bytes;
         max_inter = std::max(max_inter, g.inter_bytes);
+        sum_inter += align_up(g.inter_bytes);
         all_bins += (long long)g.count * (g.cls->plan.nb + 1);
     }
     const bool merged = nph == 1 && all_rec + max_inter <= avail && all_bins < 0x7fffffffLL;
     if (merged) max_group_bytes = all_rec + max_inter;
+    // Groups prepared together whose intermediates all fit run beside each
+    // other; else one after the other over one intermediate.
+    bool beside = merged && groups.size() > 1 && sum_inter <= inter_budget &&
+                  all_rec + sum_inter <= avail;
+    if (beside && !h->side[0]) {  // (nothing is created while the caller captures)
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        CK(cudaStreamIsCapturing(s, &cap), "capture status");
+        beside = cap == cudaStreamCaptureStatusNone;
+    }
+    if (beside) max_group_bytes = all_rec + sum_inter;
+    if (beside && !h->side[0]) {
+        for (cudaStream_t &x : h->side)
+            CK(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking), "side stream");
+        for (cudaEvent_t &x : h->side_ev)
+            CK(cudaEventCreateWithFlags(&x, cudaEventDisableTiming), "side event");
+    }
     if ((int)h->chunk_events.size() < 3 + nph) {
         // two for alternating chunk copies, the start of the later phases'
         // input copies, then the end of each later phase's copies
@@ -836,6 +863,9 @@ int run_batch(cuvgls_handle *h, const Work &wk, std::vector<DevCurve> &cvs,
     int sidx = 0, lidx = 0;
     // descriptors [first, first + count) as one part
     auto make_part = [&](int first, int count) {
+        long long pts = 0;
+        for (int k = first; k < first + count; ++k) pts += h->h_cv[k].n;
+        const bool spread = prep_spread(pts);
         Part pt;
         pt.first = first;
         pt.count = count;
@@ -844,7 +874,7 @@ int run_batch(cuvgls_handle *h, const Work &wk, std::vector<DevCurve> &cvs,
             if (c < kPrepClasses) pt.max_n[c] = 0;
             for (int k = first; k < first + count; ++k) {
                 const int n = h->h_cv[k].n;
-                if ((n > kFusePoints ? kPrepClasses : prep_class(n)) != c) continue;
+                if ((n > kFusePoints ? kPrepClasses : prep_class(n, spread)) != c) continue;
                 h_list[lidx++] = k;
                 if (c < kPrepClasses) pt.max_n[c] = std::max(pt.max_n[c], n);
             }
@@ -942,61 +972,62 @@ int run_batch(cuvgls_handle *h, const Work &wk, std::vector<DevCurve> &cvs,
     const int fp32 = h->opts.precision == CUVGLS_PREC_FP32;
     PrepArrays pa{d_cv, t, ry, rdy, ya, wv, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
                   wk.ng == 1 ? d_aux : nullptr, h->d_flags, mode, 0};
-    RecAB *recAB = nullptr;
-    RecC *recC = nullptr;
-    int *binsAB = nullptr, *binsC = nullptr;
     float2 *inter = nullptr;
-    for (size_t gi = 0; gi < groups.size(); ++gi) {
+    // records and bins of groups [gi, ge) and the intermediate after them
+    auto lay_out = [&](size_t gi, size_t ge, size_t inter_bytes) -> int {
+        size_t o2 = 0;
+        auto gtake = [&](size_t bytes) { char *q = group_base + o2; o2 += align_up(bytes); return q; };
+        long long pts = 0, nbin = 0;
+        bool multi = false;  // long curves
+        pa.max_nb = 0;
+        for (size_t k = gi; k < ge; ++k) {
+            pts += groups[k].n_pts;
+            nbin += (long long)groups[k].count * (groups[k].cls->plan.nb + 1);
+            pa.max_nb = std::max(pa.max_nb, groups[k].cls->plan.nb);
+            for (const Part &pt : parts[k]) multi = multi || pt.seg_e > pt.seg_b;
+        }
+        pa.recAB = (RecAB *)gtake(pts * sizeof(RecAB));
+        pa.recC = (RecC *)gtake(pts * sizeof(RecC));
+        pa.binsAB = (int *)gtake(4 * nbin * sizeof(int));
+        pa.binsC = pa.binsAB + nbin;
+        pa.curAB = pa.binsC + nbin;
+        pa.curC = pa.curAB + nbin;
+        inter = (float2 *)gtake(inter_bytes);
+        if (multi) CK(cudaMemsetAsync(pa.binsAB, 0, 2 * nbin * sizeof(int), s), "zero bins");
+        return CUVGLS_OK;
+    };
+    auto prep_part = [&](const Part &pt) -> int {
+        for (int c = 0; c < kPrepClasses; ++c)
+            if (pt.fused[c + 1] > pt.fused[c])
+                LAUNCH(CUVGLS_STAGE_PREP, s,
+                       launch_prep(pa, d_list + pt.fused[c], pt.fused[c + 1] - pt.fused[c], c,
+                                   pt.max_n[c], raw && !multi_band, wk.ng, fp32, s),
+                       "k_prep");
+        if (pt.seg_e > pt.seg_b)
+            LAUNCH(CUVGLS_STAGE_PREP, s,
+                   launch_bin_long(pa, d_bseg + pt.seg_b, pt.seg_e - pt.seg_b,
+                                   d_list + pt.fused[kPrepClasses],
+                                   pt.long_e - pt.fused[kPrepClasses], wk.ng, fp32, s),
+                   "k_bin_count, k_bin_scan, k_bin_scatter");
+        if (pt.seg_e > pt.seg_b) h->launches[CUVGLS_STAGE_PREP] += 2;  // three kernels
+        return CUVGLS_OK;
+    };
+    // preparation (of the parts not prepared before) and passes of a group
+    auto run_group = [&](size_t gi, float2 *inter, cudaStream_t gs) -> int {
         const Group &g = groups[gi];
         const Plan &p = g.cls->plan;
-        if (!merged || gi == 0) {  // lay out the records and bins of the groups prepared now
-            size_t o2 = 0;
-            auto gtake = [&](size_t bytes) { char *q = group_base + o2; o2 += align_up(bytes); return q; };
-            long long pts = 0, nbin = 0;
-            bool multi = false;  // long curves
-            pa.max_nb = 0;
-            for (size_t k = gi; k < (merged ? groups.size() : gi + 1); ++k) {
-                pts += groups[k].n_pts;
-                nbin += (long long)groups[k].count * (groups[k].cls->plan.nb + 1);
-                pa.max_nb = std::max(pa.max_nb, groups[k].cls->plan.nb);
-                for (const Part &pt : parts[k]) multi = multi || pt.seg_e > pt.seg_b;
-            }
-            pa.recAB = recAB = (RecAB *)gtake(pts * sizeof(RecAB));
-            pa.recC = recC = (RecC *)gtake(pts * sizeof(RecC));
-            pa.binsAB = binsAB = (int *)gtake(4 * nbin * sizeof(int));
-            pa.binsC = binsC = binsAB + nbin;
-            pa.curAB = binsC + nbin;
-            pa.curC = pa.curAB + nbin;
-            inter = (float2 *)gtake(merged ? max_inter : g.inter_bytes);
-            if (multi) CK(cudaMemsetAsync(binsAB, 0, 2 * nbin * sizeof(int), s), "zero bins");
-        }
-        auto prep_part = [&](const Part &pt) -> int {
-            for (int c = 0; c < kPrepClasses; ++c)
-                if (pt.fused[c + 1] > pt.fused[c])
-                    LAUNCH(CUVGLS_STAGE_PREP, s,
-                           launch_prep(pa, d_list + pt.fused[c], pt.fused[c + 1] - pt.fused[c], c,
-                                       pt.max_n[c], raw && !multi_band, wk.ng, fp32, s),
-                           "k_prep");
-            if (pt.seg_e > pt.seg_b)
-                LAUNCH(CUVGLS_STAGE_PREP, s,
-                       launch_bin_long(pa, d_bseg + pt.seg_b, pt.seg_e - pt.seg_b,
-                                       d_list + pt.fused[kPrepClasses],
-                                       pt.long_e - pt.fused[kPrepClasses], wk.ng, fp32, s),
-                       "k_bin_count, k_bin_scan, k_bin_scatter");
-            if (pt.seg_e > pt.seg_b) h->launches[CUVGLS_STAGE_PREP] += 2;  // three kernels
-            return CUVGLS_OK;
-        };
         size_t pi = 0;  // next part (each starts at a chunk)
         for (const Chunk &ch : g.chunks) {
-            while (pi < parts[gi].size() && parts[gi][pi].first < ch.first + ch.count) {
+            while (!merged && pi < parts[gi].size() && parts[gi][pi].first < ch.first + ch.count) {
                 rc = reach(parts[gi][pi].first);
                 if (!rc) rc = prep_part(parts[gi][pi]);
                 if (rc) return rc;
                 ++pi;
             }
             const DevCurve *dcv = d_cv + ch.first;
-            LAUNCH(CUVGLS_STAGE_PASS1, s,
-                   launch_pass1(dcv, ch.count, recAB, recC, binsAB, binsC, inter, p, wk.ng, s),
+            LAUNCH(CUVGLS_STAGE_PASS1, gs,
+                   launch_pass1(dcv, ch.count, pa.recAB, pa.recC, pa.binsAB, pa.binsC, inter, p,
+                                wk.ng, gs),
                    "k_pass1");
             // With host output, pass 2 runs in four launches over consecutive
             // curves, each followed by the copy of its powers: the copy stream
@@ -1010,19 +1041,19 @@ int run_batch(cuvgls_handle *h, const Work &wk, std::vector<DevCurve> &cvs,
                 const DevCurve *dq = dcv + a;
                 if (wk.ng == 3) {
                     GlsParams gp{mode, reg, keys};
-                    LAUNCH(CUVGLS_STAGE_PASS2, s,
-                           launch_pass2_gls(dq, e - a, inter, (float *)dev_out, p, gp, s),
+                    LAUNCH(CUVGLS_STAGE_PASS2, gs,
+                           launch_pass2_gls(dq, e - a, inter, (float *)dev_out, p, gp, gs),
                            "k_pass2_gls");
                 } else {
-                    LAUNCH(CUVGLS_STAGE_PASS2, s,
-                           launch_pass2_nfft(dq, e - a, inter, (float2 *)dev_out, d_aux, p, s),
+                    LAUNCH(CUVGLS_STAGE_PASS2, gs,
+                           launch_pass2_nfft(dq, e - a, inter, (float2 *)dev_out, d_aux, p, gs),
                            "k_pass2_nfft");
                 }
                 if (!hcopy) continue;
                 // copy these curves' outputs on the copy stream while later work runs
                 cudaEvent_t ev = h->chunk_events[evi];
                 evi ^= 1;
-                CK(cudaEventRecord(ev, s), "record chunk");
+                CK(cudaEventRecord(ev, gs), "record chunk");
                 CK(cudaStreamWaitEvent(h->copy_stream, ev, 0), "wait chunk");
                 std::vector<std::pair<long long, long long>> rng;
                 for (int k = ch.first + a; k < ch.first + e; ++k) {
@@ -1044,6 +1075,48 @@ int run_batch(cuvgls_handle *h, const Work &wk, std::vector<DevCurve> &cvs,
                 CK(flush(x0, x1), "D2H out");
             }
         }
+        return CUVGLS_OK;
+    };
+    if (merged) {
+        rc = lay_out(0, groups.size(), beside ? sum_inter : max_inter);
+        if (!rc) rc = prep_part(parts[0][0]);
+        if (rc) return rc;
+    }
+    if (!beside) {
+        for (size_t gi = 0; gi < groups.size(); ++gi) {
+            if (!merged) rc = lay_out(gi, gi + 1, groups[gi].inter_bytes);
+            if (!rc) rc = run_group(gi, inter, s);
+            if (rc) return rc;
+        }
+    } else {
+        // the largest groups first, each on the stream with the least work so
+        // far (cells; every group also costs its launches)
+        std::vector<size_t> by(groups.size()), at(groups.size());
+        size_t off2 = 0;
+        for (size_t gi = 0; gi < groups.size(); ++gi) {
+            by[gi] = gi;
+            at[gi] = off2;
+            off2 += align_up(groups[gi].inter_bytes);
+        }
+        std::stable_sort(by.begin(), by.end(), [&](size_t x, size_t y) {
+            return groups[x].inter_bytes > groups[y].inter_bytes;
+        });
+        double load[kSideStreams + 1] = {};
+        CK(cudaEventRecord(h->side_ev[kSideStreams], s), "fork");
+        for (cudaStream_t x : h->side)
+            CK(cudaStreamWaitEvent(x, h->side_ev[kSideStreams], 0), "fork");
+        for (size_t gi : by) {
+            const int k = (int)(std::min_element(load, load + kSideStreams + 1) - load);
+            load[k] += (double)groups[gi].inter_bytes + 4e6;
+            rc = run_group(gi, (float2 *)((char *)inter + at[gi]), k ? h->side[k - 1] : s);
+            if (rc) break;
+        }
+        // joined even after a failed launch: the arena is the next call's
+        for (int k = 0; k < kSideStreams; ++k) {
+            CK(cudaEventRecord(h->side_ev[k], h->side[k]), "join");
+            CK(cudaStreamWaitEvent(s, h->side_ev[k], 0), "join");
+        }
+        if (rc) return rc;
     }
     if (best) {
         CK(launch_best_finish(keys, wk.n_best, bk, bp, s), "best finish");
@@ -1137,6 +1210,10 @@ int cuvgls_destroy(cuvgls_handle *h) {
     if (h->copy_stream) cudaStreamDestroy(h->copy_stream);
     if (h->in_stream) cudaStreamDestroy(h->in_stream);
     if (h->table_stream) cudaStreamDestroy(h->table_stream);
+    for (cudaStream_t x : h->side)
+        if (x) cudaStreamDestroy(x);
+    for (cudaEvent_t x : h->side_ev)
+        if (x) cudaEventDestroy(x);
     delete h;
     return CUVGLS_OK;
 }

@@ -180,35 +180,41 @@ __device__ __forceinline__ double warp_sum4(double a, double b, double c, double
     for (int o = 4; o > 0; o >>= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
     return s0;
 }
-// Totals of four values over the CTA into part[0 .. 3] (written by threads
-// 0 .. 3; the caller synchronises before they are read).  wred: 4 NT / 32.
+// Totals of four values over the CTA's first `warps` warps (the others hold
+// none) into part[0 .. 3], written by threads 0 .. 3; the caller synchronises
+// before they are read.  wred: 4 NT / 32.
 template <int NT>
-__device__ __forceinline__ void block_sum4(double a, double b, double c, double d, double *wred,
-                                           double *part, int tid) {
+__device__ __forceinline__ void block_sum4(double a, double b, double c, double d, int warps,
+                                           double *wred, double *part, int tid) {
     const int lane = tid & 31, wid = tid >> 5;
-    const double v = warp_sum4(a, b, c, d, lane);
-    if ((lane & 7) == 0) wred[wid * 4 + (lane >> 3)] = v;
+    if (wid < warps) {
+        const double v = warp_sum4(a, b, c, d, lane);
+        if ((lane & 7) == 0) wred[wid * 4 + (lane >> 3)] = v;
+    }
     __syncthreads();
-    if (tid < 4) {
-        double s = 0.0;
+    if (wid == 0) {  // lane l: value l & 3 of warps l >> 2 (and 8 more)
+        double s = (lane >> 2) < warps ? wred[lane] : 0.0;
+        if (NT > 256 && warps > 8) s += 8 + (lane >> 2) < warps ? wred[32 + lane] : 0.0;
 #pragma unroll
-        for (int w = 0; w < NT / 32; ++w) s += wred[w * 4 + tid];
-        part[tid] = s;
+        for (int o = 16; o > 2; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane < 4) part[lane] = s;
     }
 }
 
 // Normalisation and statistics of a descriptor from its curve's totals a =
 // (sum dy^-2, sum y dy^-2, sum and count of the non-NaN y), b = (YY, sum yw,
-// sum w): ybar is relative to the unweighted nan-mean of y, as cuvarbase's
-// normalize_light_curves leaves it.
+// sum w).  ybar, which only the standard mode reads, is relative to the
+// unweighted nan-mean of y, as cuvarbase's normalize_light_curves leaves it.
 __device__ __forceinline__ void fill_stats(DevCurve &cv, double4 a, double4 b, int mode) {
     const double yy = b.x;
-    const double ybar = a.y / a.x - a.z / a.w;
     double norm = 1.0;
     if (mode == 1) norm = 1.0 / yy;
-    else if (mode == 0) norm = 1.0 / (yy + ybar * ybar);
+    else if (mode == 0) {
+        const double ybar = a.y / a.x - a.z / a.w;
+        norm = 1.0 / (yy + ybar * ybar);
+        cv.ybar = (float)ybar;
+    }
     cv.yy_inv = (float)norm;
-    cv.ybar = (float)ybar;
     cv.yw_sum = (float)b.y;
     cv.w_sum = (float)b.z;
 }
@@ -229,14 +235,15 @@ __host__ __device__ constexpr int prep_smem(int nb, bool cluster) {
 // points stay in registers (PPT per thread).  CL: the curve's points are
 // shared out over the first CTAs of a cluster, which exchange their partial
 // sums and counts through distributed shared memory (at most 2^15 points, so
-// a count fits 16 bits); CTAs without points leave at once.
+// a count fits 16 bits); CTAs without points leave at once.  `chunk` points go
+// to each CTA, or with 0 an even share of the curve (at least one per thread).
 //
 // Bound by the latency of its few steps (barriers, FP64 sums, shared
 // atomics) for one curve and by FP64 issue for many; one launch instead of
 // the three to six that passed yw, w, counts and cursors through memory.
 template <int NT, int PPT, bool CL, bool RAW, int NG, bool F32>
 __global__ void __launch_bounds__(NT)
-k_prep(const PrepArrays A, const int *__restrict__ list, int csize) {
+k_prep(const PrepArrays A, const int *__restrict__ list, int csize, int chunk) {
     extern __shared__ __align__(16) unsigned cnt[];
     __shared__ double wred[4 * NT / 32], part[8], mean[2];
     __shared__ int ws[32];
@@ -244,7 +251,8 @@ k_prep(const PrepArrays A, const int *__restrict__ list, int csize) {
     const int ci = CL ? blockIdx.x / csize : blockIdx.x, rank = CL ? blockIdx.x % csize : 0;
     DevCurve &cv = A.cv[list ? list[ci] : ci];
     const int n = cv.n;
-    const int na = CL ? (n - 1) / (NT * PPT) + 1 : 1;  // CTAs with points
+    if (CL && chunk == 0) chunk = max(NT, ((n - 1) / csize + 32) & ~31);
+    const int na = CL ? (n - 1) / chunk + 1 : 1;  // CTAs with points
     if (CL && rank >= na) return;
     const Geom g(cv.geom);
     const int nb = (int)(g.G2 >> g.lb);
@@ -253,7 +261,8 @@ k_prep(const PrepArrays A, const int *__restrict__ list, int csize) {
     const long long po = cv.pt_off;
     const double tref = A.t[po], df = cv.df, kc = cv.kc;
     const Centre k = centre_of<NG == 3>(kc);
-    const int j0 = rank * NT * PPT + tid;
+    const int j0 = rank * chunk + tid, j1 = CL ? min(n, (rank + 1) * chunk) : n;
+    const int warps = min(NT / 32, (j1 - j0 + tid + 31) / 32);  // with points
     float a[PPT], w[PPT];
     double y[RAW ? PPT : 1], ir[RAW ? PPT : 1];
     if (RAW) {
@@ -264,7 +273,7 @@ k_prep(const PrepArrays A, const int *__restrict__ list, int csize) {
             const int j = j0 + q * NT;
             ir[q] = 0.0;
             y[q] = 0.0;
-            if (j < n) {
+            if (j < j1) {
                 const double dj = A.rdy[po + j];
                 y[q] = A.ry[po + j];
                 ir[q] = 1.0 / (dj * dj);
@@ -273,40 +282,42 @@ k_prep(const PrepArrays A, const int *__restrict__ list, int csize) {
                 if (!isnan(y[q])) { sy += y[q]; ++cy; }
             }
         }
-        block_sum4<NT>(sw, swy, sy, (double)cy, wred, part, tid);
+        block_sum4<NT>(sw, swy, sy, (double)cy, warps, wred, part, tid);
         if (CL) cg::this_cluster().sync();
         else __syncthreads();
-        if (tid == 0 || tid == 32) {
+        if (tid == 0) {
             double tw = 0.0, ty = 0.0;
             for (int r = 0; r < na; ++r) {
                 const double *pr = CL ? cg::this_cluster().map_shared_rank(part, r) : part;
                 tw += pr[0];
                 ty += pr[1];
             }
-            if (tid == 0) mean[0] = ty / tw;
-            else mean[1] = 1.0 / tw;
+            mean[0] = ty / tw;
+            mean[1] = 1.0 / tw;
         }
         __syncthreads();
         const double ybar_w = mean[0], inv = mean[1];
         double yy = 0.0, ys = 0.0, wsum = 0.0;
 #pragma unroll
         for (int q = 0; q < PPT; ++q) {
-            const double wj = ir[q] * inv, d = y[q] - ybar_w, wd = wj * d;
-            a[q] = (float)wd;
-            w[q] = (float)wj;
-            if (j0 + q * NT < n) {
+            a[q] = 0.f;
+            w[q] = 0.f;
+            if (j0 + q * NT < j1) {
+                const double wj = ir[q] * inv, d = y[q] - ybar_w, wd = wj * d;
+                a[q] = (float)wd;
+                w[q] = (float)wj;
                 yy = fma(wd, d, yy);
                 ys += (double)a[q];
                 wsum += (double)w[q];
             }
         }
-        block_sum4<NT>(yy, ys, wsum, 0.0, wred, part + 4, tid);
+        block_sum4<NT>(yy, ys, wsum, 0.0, warps, wred, part + 4, tid);
     } else {
 #pragma unroll
         for (int q = 0; q < PPT; ++q) {
             const int j = j0 + q * NT;
-            a[q] = j < n ? A.ya[po + j] : 0.f;
-            w[q] = NG == 3 && j < n ? A.wv[po + j] : 0.f;
+            a[q] = j < j1 ? A.ya[po + j] : 0.f;
+            w[q] = NG == 3 && j < j1 ? A.wv[po + j] : 0.f;
         }
         __syncthreads();  // counts zeroed
     }
@@ -317,7 +328,7 @@ k_prep(const PrepArrays A, const int *__restrict__ list, int csize) {
     for (int q = 0; q < PPT; ++q) {
         const int j = j0 + q * NT;
         rank_ac[q] = 0;
-        if (j < n) {
+        if (j < j1) {
             double tj = A.t[po + j];
             if (!(isfinite(tj) && isfinite(a[q]) && isfinite(w[q]))) {
                 bad = true;
@@ -371,7 +382,7 @@ k_prep(const PrepArrays A, const int *__restrict__ list, int csize) {
     RecC *rC = A.recC + cv.rec_off;
 #pragma unroll
     for (int q = 0; q < PPT; ++q) {
-        if (j0 + q * NT >= n) continue;
+        if (j0 + q * NT >= j1) continue;
         const int binA = bin_of(p[q].a, g), binC = NG == 3 ? bin_of(p[q].c, g) : 0;
         const unsigned oa = off[binA] + (CL ? pre[binA] : 0);
         rA[(oa & 0xFFFFu) + (rank_ac[q] & 0xFFFF)] = rec_ab(p[q], a[q], w[q]);
@@ -458,9 +469,11 @@ k_bin_scan(const PrepArrays A, const int *__restrict__ list, int ngrids) {
 
 // One CTA per segment: a shared-memory rank of each point within its column
 // block, one global reservation per block for the segment's run, then the
-// records.
+// records.  Only the ranks stay in registers: the places are computed again
+// for the records, which costs two FP64 instructions a point and lets two
+// CTAs share an SM (102 registers and one CTA otherwise).
 template <int NG, bool F32>
-__global__ void __launch_bounds__(kSegThreads)
+__global__ void __launch_bounds__(kSegThreads, 2)
 k_bin_scatter(const PrepArrays A, const SegEntry *__restrict__ segs) {
     __shared__ unsigned h[kMaxBins];         // packed counts
     __shared__ int oA[kMaxBins], oC[kMaxBins];
@@ -475,8 +488,6 @@ k_bin_scatter(const PrepArrays A, const SegEntry *__restrict__ segs) {
     const double tref = A.t[cv.pt_off], df = cv.df, kc = cv.kc;
     const Centre k = centre_of<NG == 3>(kc);
     const int cntp = min(n - sg.start, kSegPoints);
-    Place p[kSegPpt];
-    float a[kSegPpt], w[kSegPpt];
     int rank_ac[kSegPpt];
     bool bad = false, lost = false;
 #pragma unroll
@@ -484,17 +495,10 @@ k_bin_scatter(const PrepArrays A, const SegEntry *__restrict__ segs) {
         const int i = tid + q * kSegThreads;
         if (i < cntp) {
             double tj = A.t[po + i];
-            a[q] = A.ya[po + i];
-            w[q] = NG == 3 ? A.wv[po + i] : 0.f;
-            if (!(isfinite(tj) && isfinite(a[q]) && isfinite(w[q]))) {
-                bad = true;
-                tj = isfinite(tj) ? tj : tref;
-                a[q] = 0.f;
-                w[q] = 0.f;
-            }
-            p[q] = place_of<NG, F32>(tj, tref, df, g, kc, k);
-            rank_ac[q] = atomicAdd(&h[bin_of(p[q].a, g)], 1u) & 0xFFFFu;
-            if (NG == 3) rank_ac[q] |= atomicAdd(&h[bin_of(p[q].c, g)], 0x10000u) & 0xFFFF0000u;
+            if (!isfinite(tj)) tj = tref;
+            const Place p = place_of<NG, F32>(tj, tref, df, g, kc, k);
+            rank_ac[q] = atomicAdd(&h[bin_of(p.a, g)], 1u) & 0xFFFFu;
+            if (NG == 3) rank_ac[q] |= atomicAdd(&h[bin_of(p.c, g)], 0x10000u) & 0xFFFF0000u;
         }
     }
     __syncthreads();
@@ -508,15 +512,25 @@ k_bin_scatter(const PrepArrays A, const SegEntry *__restrict__ segs) {
     RecC *rC = A.recC + cv.rec_off;
 #pragma unroll
     for (int q = 0; q < kSegPpt; ++q) {
-        if (tid + q * kSegThreads >= cntp) continue;
+        const int i = tid + q * kSegThreads;
+        if (i >= cntp) continue;
+        double tj = A.t[po + i];
+        float a = A.ya[po + i], w = NG == 3 ? A.wv[po + i] : 0.f;
+        if (!(isfinite(tj) && isfinite(a) && isfinite(w))) {
+            bad = true;
+            tj = isfinite(tj) ? tj : tref;
+            a = 0.f;
+            w = 0.f;
+        }
+        const Place p = place_of<NG, F32>(tj, tref, df, g, kc, k);
         // a slot outside the curve's n records would mean that the count and
         // the scatter binned a point differently: flag it, write nothing
-        const int sa = oA[bin_of(p[q].a, g)] + (rank_ac[q] & 0xFFFF);
-        if ((unsigned)sa < (unsigned)n) rA[sa] = rec_ab(p[q], a[q], w[q]);
+        const int sa = oA[bin_of(p.a, g)] + (rank_ac[q] & 0xFFFF);
+        if ((unsigned)sa < (unsigned)n) rA[sa] = rec_ab(p, a, w);
         else lost = true;
         if (NG == 3) {
-            const int sc = oC[bin_of(p[q].c, g)] + (int)((unsigned)rank_ac[q] >> 16);
-            if ((unsigned)sc < (unsigned)n) rC[sc] = rec_c(p[q], w[q]);
+            const int sc = oC[bin_of(p.c, g)] + (int)((unsigned)rank_ac[q] >> 16);
+            if ((unsigned)sc < (unsigned)n) rC[sc] = rec_c(p, w);
             else lost = true;
         }
     }
@@ -570,7 +584,7 @@ k_raw_sums(const SegEntry *__restrict__ segs, const DevCurve *__restrict__ cvs,
         swy = fma(wj, yj, swy);
         if (!isnan(yj)) { sy += yj; ++cy; }
     }
-    block_sum4<kSegThreads>(sw, swy, sy, (double)cy, wred, part, tid);
+    block_sum4<kSegThreads>(sw, swy, sy, (double)cy, kSegThreads / 32, wred, part, tid);
     __syncthreads();
     if (tid == 0)
         partA[cv.raw_seg + sg.start / kSegPoints] = make_double4(part[0], part[1], part[2], part[3]);
@@ -608,7 +622,7 @@ k_raw_finish(const SegEntry *__restrict__ segs, const DevCurve *__restrict__ cvs
         ys += (double)ywf;
         ws += (double)wf;
     }
-    block_sum4<kSegThreads>(yy, ys, ws, 0.0, wred, part, tid);
+    block_sum4<kSegThreads>(yy, ys, ws, 0.0, kSegThreads / 32, wred, part, tid);
     __syncthreads();
     if (tid == 0)
         partB[cv.raw_seg + sg.start / kSegPoints] = make_double4(part[0], part[1], part[2], 0.0);
@@ -635,7 +649,8 @@ k_fill_desc(DevCurve *__restrict__ cvs, const int *__restrict__ list, int n,
 namespace {
 
 template <int NT, int PPT, bool CL, bool RAW, int NG, bool F32>
-cudaError_t prep_t(const PrepArrays &a, const int *list, int n, int csize, cudaStream_t s) {
+cudaError_t prep_t(const PrepArrays &a, const int *list, int n, int csize, int chunk,
+                   cudaStream_t s) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)n * csize);
     cfg.blockDim = dim3(NT);
@@ -648,20 +663,20 @@ cudaError_t prep_t(const PrepArrays &a, const int *list, int n, int csize, cudaS
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = CL ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, k_prep<NT, PPT, CL, RAW, NG, F32>, a, list, csize);
+    return cudaLaunchKernelEx(&cfg, k_prep<NT, PPT, CL, RAW, NG, F32>, a, list, csize, chunk);
 }
 
 template <int NT, int PPT, bool CL>
-cudaError_t prep_kind(const PrepArrays &a, const int *list, int n, int csize, int raw, int ngrids,
-                      int f32, cudaStream_t s) {
+cudaError_t prep_kind(const PrepArrays &a, const int *list, int n, int csize, int chunk, int raw,
+                      int ngrids, int f32, cudaStream_t s) {
     if (raw)
-        return f32 ? prep_t<NT, PPT, CL, true, 3, true>(a, list, n, csize, s)
-                   : prep_t<NT, PPT, CL, true, 3, false>(a, list, n, csize, s);
+        return f32 ? prep_t<NT, PPT, CL, true, 3, true>(a, list, n, csize, chunk, s)
+                   : prep_t<NT, PPT, CL, true, 3, false>(a, list, n, csize, chunk, s);
     if (ngrids == 3)
-        return f32 ? prep_t<NT, PPT, CL, false, 3, true>(a, list, n, csize, s)
-                   : prep_t<NT, PPT, CL, false, 3, false>(a, list, n, csize, s);
-    return f32 ? prep_t<NT, PPT, CL, false, 1, true>(a, list, n, csize, s)
-               : prep_t<NT, PPT, CL, false, 1, false>(a, list, n, csize, s);
+        return f32 ? prep_t<NT, PPT, CL, false, 3, true>(a, list, n, csize, chunk, s)
+                   : prep_t<NT, PPT, CL, false, 3, false>(a, list, n, csize, chunk, s);
+    return f32 ? prep_t<NT, PPT, CL, false, 1, true>(a, list, n, csize, chunk, s)
+               : prep_t<NT, PPT, CL, false, 1, false>(a, list, n, csize, chunk, s);
 }
 
 }  // namespace
@@ -670,16 +685,26 @@ cudaError_t launch_prep(const PrepArrays &a, const int *list, int n, int cls, in
                         int ngrids, int fp32_positions, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
     if (a.max_nb > kMaxBins || max_n > kFusePoints) return cudaErrorInvalidValue;
-    const int pts = prep_points(cls);
-    int csize = 1;
-    while (csize * pts < max_n) csize *= 2;
-    if (csize > kMaxCluster || (cls == 0 && csize > 1)) return cudaErrorInvalidValue;
-    if (cls == 0)
-        return prep_kind<kPrepThreads, kPrepPpt, false>(a, list, n, 1, raw, ngrids, fp32_positions, s);
-    if (cls == 1)
-        return prep_kind<kPrepThreads, kPrepPpt, true>(a, list, n, csize, raw, ngrids,
+    if (cls == 0) {
+        if (max_n > kPrepPoints) return cudaErrorInvalidValue;
+        return prep_kind<kPrepThreads, kPrepPpt, false>(a, list, n, 1, kPrepPoints, raw, ngrids,
+                                                        fp32_positions, s);
+    }
+    if (cls == kPrepWide) {
+        int csize = 1;
+        while (csize * kWidePoints < max_n) csize *= 2;
+        return prep_kind<kWideThreads, kWidePpt, true>(a, list, n, csize, kWidePoints, raw, ngrids,
                                                        fp32_positions, s);
-    return prep_kind<kWideThreads, kWidePpt, true>(a, list, n, csize, raw, ngrids, fp32_positions, s);
+    }
+    if (max_n > kMaxCluster * kPrepPoints) return cudaErrorInvalidValue;
+    int csize = 1;
+    const bool spread = cls == kPrepSpread;
+    while (csize < kMaxCluster && csize * (spread ? kPrepThreads : kPrepPoints) < max_n) csize *= 2;
+    if (csize == 1)
+        return prep_kind<kPrepThreads, kPrepPpt, false>(a, list, n, 1, kPrepPoints, raw, ngrids,
+                                                        fp32_positions, s);
+    return prep_kind<kPrepThreads, kPrepPpt, true>(a, list, n, csize, spread ? 0 : kPrepPoints, raw,
+                                                   ngrids, fp32_positions, s);
 }
 
 cudaError_t launch_bin_long(const PrepArrays &a, const SegEntry *segs, int n_segs, const int *list,
