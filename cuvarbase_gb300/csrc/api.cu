@@ -390,18 +390,25 @@ int get_class(cuvgls_handle *h, long long nf, int ng, ClassTables **out) {
     // window the deconvolution of |k'| <= G / 2) built on the device
     const size_t n1 = (size_t)fft_table_len(G1), n2 = (size_t)fft_table_len(G2);
     const size_t nd = p.win == kWinES ? (size_t)(G / 2 + 2) / 2 : 0;  // in float2 units
-    CK(cudaMalloc(&c.d, (n1 + n2 + (size_t)G + nd) * sizeof(float2)), "cudaMalloc(plan tables)");
+    const size_t nr = p.win == kWinES && ng == 3 ? (size_t)(G + 1) / 2 : 0;
+    CK(cudaMalloc(&c.d, (n1 + n2 + (size_t)G + nd + nr) * sizeof(float2)),
+       "cudaMalloc(plan tables)");
     // on a stream of their own: a new class waits neither for batches nor for
     // result copies in flight
     CK(launch_plan_tables(c.d, G1, G2, B, h->table_stream), "plan tables");
     if (p.win == kWinES)
         CK(launch_es_deconv((float *)(c.d + n1 + n2 + G), G, p.m, beta, h->table_stream),
            "deconvolution table");
+    if (nr)
+        CK(launch_deconv_rows((const float *)(c.d + n1 + n2 + G), (float *)(c.d + n1 + n2 + G + nd),
+                              G1, G2, pass2_rows(ng, G2), h->table_stream),
+           "deconvolution rows");
     CK(cudaStreamSynchronize(h->table_stream), "plan tables");
     p.st1 = c.d;
     p.st2 = c.d + n1;
     p.itw = c.d + n1 + n2;
     p.dtab = p.win == kWinES ? (const float *)(c.d + n1 + n2 + G) : nullptr;
+    p.drow = nr ? (const float *)(c.d + n1 + n2 + G + nd) : nullptr;
     auto ins = h->classes.emplace(ck, c);
     *out = &ins.first->second;
     return CUVGLS_OK;
@@ -1040,9 +1047,9 @@ int run_batch(cuvgls_handle *h, const Work &wk, std::vector<DevCurve> &cvs,
                 const int e = (int)((long long)ch.count * (q + 1) / nsub);
                 const DevCurve *dq = dcv + a;
                 if (wk.ng == 3) {
-                    GlsParams gp{mode, reg, keys};
+                    GlsParams gp{mode, reg, keys, h->d_flags};
                     LAUNCH(CUVGLS_STAGE_PASS2, gs,
-                           launch_pass2_gls(dq, e - a, inter, (float *)dev_out, p, gp, gs),
+                           launch_pass2_gls(dq, e - a, a, inter, (float *)dev_out, p, gp, gs),
                            "k_pass2_gls");
                 } else {
                     LAUNCH(CUVGLS_STAGE_PASS2, gs,
@@ -1468,7 +1475,7 @@ int cuvgls_gls_direct_batch(cuvgls_handle *h, const cuvgls_gls_input *b,
     CK(cudaMemcpyAsync(d_cv, h->h_cv, nc * sizeof(DevCurve), cudaMemcpyHostToDevice, s),
        "H2D descriptors");
     CK(cudaEventRecord(h->h_cv_free, s), "record");
-    GlsParams g{b->mode, b->reg[0]};
+    GlsParams g{b->mode, b->reg[0], nullptr, h->d_flags};
     for (int c0 = 0; c0 < nc; c0 += 65535) {
         int cnt = std::min(65535, nc - c0);
         LAUNCH(CUVGLS_STAGE_DIRECT, s,

@@ -20,13 +20,17 @@
 //                evaluates the GLS power (3 grids) or applies the output phase
 //                of the adjoint NFFT (1 grid).
 // The grid itself never exists in HBM: spreading is fused into pass 1.
+#include <cuda.h>
+#include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 #include <math.h>
 
 #include <algorithm>
+#include <mutex>
 
 #include "gls_math.cuh"
 #include "kernels.cuh"
+#include "pass2_tma.cuh"
 
 namespace cuvgls {
 
@@ -236,6 +240,53 @@ cudaError_t launch_plan_tables(float2 *dst, int G1, int G2, int B, cudaStream_t 
     return cudaGetLastError();
 }
 
+__global__ void __launch_bounds__(256)
+k_deconv_rows(const float *__restrict__ dtab, float *__restrict__ dst, int G1, int G2, int R) {
+    const int G = G1 * G2;
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < G; e += gridDim.x * blockDim.x) {
+        const int r = e % R, q2 = e / R % G2, rb = e / (R * G2);
+        const int q = rb * R + r + G1 * q2;
+        dst[e] = dtab[min(q, G - q)];
+    }
+}
+
+cudaError_t launch_deconv_rows(const float *dtab, float *dst, int G1, int G2, int R,
+                               cudaStream_t s) {
+    if (G1 < R || G1 % R) return cudaErrorInvalidValue;
+    const int blocks = std::min((G1 * G2 + 255) / 256, 4096);
+    k_deconv_rows<<<blocks, 256, 0, s>>>(dtab, dst, G1, G2, R);
+    return cudaGetLastError();
+}
+
+// The driver's tensor-map encoder, looked up once (the library links no
+// driver symbols).
+static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
+    static std::once_flag once;
+    static void *fn = nullptr;
+    std::call_once(once, [] {
+        cudaDriverEntryPointQueryResult st;
+        void *f = nullptr;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault,
+                                             &st) == cudaSuccess &&
+            st == cudaDriverEntryPointSuccess)
+            fn = f;
+    });
+    return (PFN_cuTensorMapEncodeTiled_v12000)fn;
+}
+
+cudaError_t pass2_map(CUtensorMap &map, const float2 *inter, const Plan &p, int grids, int R) {
+    const PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
+    if (!enc) return cudaErrorNotSupported;
+    const cuuint64_t dims[3] = {(cuuint64_t)p.G1 * p.B * 2, (cuuint64_t)p.nb, (cuuint64_t)grids};
+    const cuuint64_t strides[2] = {(cuuint64_t)p.G1 * p.B * 8, (cuuint64_t)p.G * 8};
+    const cuuint32_t box[3] = {(cuuint32_t)(R * p.B * 2), (cuuint32_t)p.nb, 1};
+    const cuuint32_t es[3] = {1, 1, 1};
+    const CUresult r = enc(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, (void *)inter, dims, strides,
+                           box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
 cudaError_t launch_es_deconv(float *dst, long long G, int m, double beta, cudaStream_t s) {
     if (G < 2 || m < 1) return cudaErrorInvalidValue;
     const int n = (int)(G / 2 + 1);
@@ -282,11 +333,11 @@ cudaError_t preload_pass_kernels(int G1, int G2, int ngrids) {
 #undef CUVGLS_PL2
 }
 
-cudaError_t launch_pass2_gls(const DevCurve *cv, int n_curves,
+cudaError_t launch_pass2_gls(const DevCurve *cv, int n_curves, int first,
                              const float2 *inter, float *out, const Plan &p,
                              GlsParams g, cudaStream_t s) {
     if (n_curves <= 0) return cudaSuccess;
-#define CUVGLS_P2(L) case L: return launch_pass2_gls_t<L>(cv, n_curves, inter, out, p, g, s);
+#define CUVGLS_P2(L) case L: return launch_pass2_gls_t<L>(cv, n_curves, first, inter, out, p, g, s);
     switch (p.G2) {
         CUVGLS_ROW_LEN_CASES(CUVGLS_P2)
         default: return cudaErrorInvalidValue;

@@ -52,8 +52,8 @@ cudaError_t launch_pass1(const DevCurve *cv, int n_curves, const RecAB *recAB,
                          const RecC *recC, const int *binsAB, const int *binsC,
                          float2 *inter, const Plan &p, int ngrids, cudaStream_t s);
 
-cudaError_t launch_pass2_gls(const DevCurve *cv, int n_curves,
-                             const float2 *inter, float *out, const Plan &p,
+// (`first`: index of the first curve within the intermediate's chunk)
+cudaError_t launch_pass2_gls(const DevCurve *cv, int n_curves, int first, const float2 *inter, float *out, const Plan &p,
                              GlsParams g, cudaStream_t s);
 
 cudaError_t launch_pass2_nfft(const DevCurve *cv, int n_curves,
@@ -65,7 +65,7 @@ template <int NG, int L1>
 cudaError_t launch_pass1_t(const DevCurve *, int, const RecAB *, const RecC *,
                            const int *, const int *, float2 *, const Plan &, cudaStream_t);
 template <int L2>
-cudaError_t launch_pass2_gls_t(const DevCurve *, int, const float2 *, float *,
+cudaError_t launch_pass2_gls_t(const DevCurve *, int, int, const float2 *, float *,
                                const Plan &, GlsParams, cudaStream_t);
 template <int L2>
 cudaError_t launch_pass2_nfft_t(const DevCurve *, int, const float2 *, float2 *,
@@ -81,6 +81,8 @@ cudaError_t preload_pass_kernels(int G1, int G2, int ngrids);
 // Fill the deconvolution table of an ES-window plan: G / 2 + 1 floats
 // 1 / phihat(k'), |k'| <= G / 2 (kernels.cu: k_es_deconv).
 cudaError_t launch_es_deconv(float *dst, long long G, int m, double beta, cudaStream_t s);
+// The same by row blocks of R rows: dst[(rb L2 + q2) R + r], G floats.
+cudaError_t launch_deconv_rows(const float *dtab, float *dst, int G1, int G2, int R, cudaStream_t s);
 
 // Fill the tables of a plan (FFT tables of G1 and G2, then the inter-pass
 // twiddles), fft_table_len(G1) + fft_table_len(G2) + G1 G2 entries at dst.

@@ -233,7 +233,8 @@ extern "C" int cuvgls_gls_noalloc(double sigma, int32_t m, const cuvgls_gls_inpu
     if (e == cudaSuccess)
         e = launch_pass1(d_cv, nc, recAB, recC, binsAB, binsC, inter, p, 3, s);
     if (e == cudaSuccess)
-        e = launch_pass2_gls(d_cv, nc, inter, p_out, p, GlsParams{b->mode, b->reg[0]}, s);
+        e = launch_pass2_gls(d_cv, nc, 0, inter, p_out, p,
+                             GlsParams{b->mode, b->reg[0], nullptr, d_flag}, s);
     // this call's device error word (CUVGLS_DEVERR_*) to the caller's word
     if (e == cudaSuccess && device_flags)
         e = cudaMemcpyAsync(device_flags, d_flag, sizeof(unsigned), cudaMemcpyDefault, s);

@@ -1,0 +1,331 @@
+// Pass 2 of the GLS for rows whose outputs fit in registers.
+//
+//   k_pass2_gls_reg<L2, ES>  persistent CTAs; a task is R rows of one curve.
+//     The rows of its three grids arrive one after the other by TMA and each
+//     goes through the two-level row FFT:
+//       stage A  one unit (r, i) reads its LA inputs from the arrived tile,
+//                transforms them and writes them to the exchange tile;
+//       stage B  one thread per (r, qa) reads LB values and transforms them.
+//     A thread's outputs q2 = qa + LA qb of the three grids stay in its
+//     registers, so the power of those frequencies is evaluated and written
+//     without a further pass through shared memory.
+//
+// What it replaces (a CTA per R rows; the three grids' outputs back to shared
+// memory and read again) was held by the L1 data pipe: 75 % busy, of which a
+// third was the outputs' way through shared memory and the deconvolution
+// table's scattered reads.  2,000 curves of 320 x 400 cells 1.80 -> 1.61 ms
+// (now at 53 % issue, 51 % of the L1 pipe and of DRAM), 20,000 of 160 x 160
+// 4.11 -> 2.81 ms (the old tile also had two- to four-way bank conflicts).
+#pragma once
+
+#include <cuda.h>
+#include <cuda_runtime.h>
+
+#include "fft.cuh"
+#include "gls_math.cuh"
+#include "kernels.cuh"
+
+namespace cuvgls {
+
+// ---- mbarrier and TMA ----
+__device__ __forceinline__ unsigned smem_addr(const void *p) {
+    return (unsigned)__cvta_generic_to_shared(p);
+}
+__device__ __forceinline__ void mbar_init(unsigned long long *b) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(b)) : "memory");
+}
+__device__ __forceinline__ void mbar_expect(unsigned long long *b, unsigned bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(b)),
+                 "r"(bytes)
+                 : "memory");
+}
+// Waits for the phase of the given parity, a bounded number of times; false
+// when that ran out.
+__device__ __forceinline__ bool mbar_wait(unsigned long long *b, unsigned parity) {
+    constexpr int kTries = 1 << 18;  // each suspends for up to some microseconds
+    const unsigned a = smem_addr(b);
+    for (int k = 0; k < kTries; ++k) {
+        unsigned done;
+        asm volatile(
+            "{\n .reg .pred p;\n"
+            " mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+            " selp.u32 %0, 1, 0, p;\n}"
+            : "=r"(done)
+            : "r"(a), "r"(parity)
+            : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+__device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, int x, int y, int z,
+                                            unsigned long long *b) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
+        "[%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_addr(dst)),
+        "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_addr(b))
+        : "memory");
+}
+
+// Offset of row r in the exchange tile, beside r pitches: it spreads the
+// stores of stage A (four columns of four rows per half-warp) and the loads
+// of stage B (all rows at one or two qa) over the 16 bank pairs.
+template <int R>
+__device__ __forceinline__ int row_shift(int r) {
+    if constexpr (R == 16) return 4 * (r & 3) + (r >> 2);
+    else if constexpr (R == 8) return 4 * (r & 3) + 2 * (r >> 2);
+    else return 4 * (r & 3);
+}
+
+// P of two frequencies in packed FP32x2 arithmetic (floating mean), as
+// gls_from_sums: A, B, C are (re, im) per grid for the frequencies x and y.
+struct Fm2 {
+    float2 nyw, hw, pn;
+    __device__ __forceinline__ Fm2(const DevCurve &cv, float reg)
+        : nyw(make_float2(-cv.yw_sum, -cv.yw_sum)),
+          hw(make_float2(0.5f * cv.w_sum + reg, 0.5f * cv.w_sum + reg)),
+          pn(make_float2(cv.yy_inv, cv.yy_inv)) {}
+    __device__ __forceinline__ float2 power(float2 A0, float2 A1, float2 B0, float2 B1, float2 C0,
+                                            float2 C1, float2 D) const {
+        const float2 half = make_float2(0.5f, 0.5f), mhalf = make_float2(-0.5f, -0.5f);
+        const float2 mtwo = make_float2(-2.f, -2.f);
+        const float2 YCh = __fmul2_rn(make_float2(A0.x, A1.x), D);
+        const float2 YSh = __fmul2_rn(make_float2(A0.y, A1.y), D);
+        const float2 C = __fmul2_rn(make_float2(B0.x, B1.x), D);
+        const float2 S = __fmul2_rn(make_float2(B0.y, B1.y), D);
+        const float2 C2 = __fmul2_rn(make_float2(C0.x, C1.x), D);
+        const float2 S2 = __fmul2_rn(make_float2(C0.y, C1.y), D);
+        const float2 mC = make_float2(-C.x, -C.y), mS = make_float2(-S.x, -S.y);
+        const float2 YC = __ffma2_rn(nyw, C, YCh);
+        const float2 YS = __ffma2_rn(nyw, S, YSh);
+        const float2 CC = __ffma2_rn(mC, C, __ffma2_rn(half, C2, hw));
+        const float2 SS = __ffma2_rn(mS, S, __ffma2_rn(mhalf, C2, hw));
+        const float2 CS = __ffma2_rn(mC, S, __fmul2_rn(half, S2));
+        const float2 det = __ffma2_rn(make_float2(-CS.x, -CS.y), CS, __fmul2_rn(CC, SS));
+        const float2 a = __ffma2_rn(__fmul2_rn(mtwo, YS), CS, __fmul2_rn(YC, SS));
+        const float2 num = __ffma2_rn(YC, a, __fmul2_rn(__fmul2_rn(YS, YS), CC));
+        const float2 P = __fmul2_rn(
+            make_float2(__fdividef(num.x, det.x), __fdividef(num.y, det.y)), pn);
+        return make_float2((P.x >= 0.f && !isinf(P.x)) ? P.x : -1.f,
+                           (P.y >= 0.f && !isinf(P.y)) ? P.y : -1.f);
+    }
+};
+
+template <int L2, bool ES>
+__global__ void __launch_bounds__(pass2_reg_threads(L2), pass2_reg_ctas(L2))
+k_pass2_gls_reg(const __grid_constant__ CUtensorMap map, const DevCurve *__restrict__ cvs,
+                int n_curves, int first, float *__restrict__ out, const Plan p, const GlsParams gp) {
+    constexpr int LA = two_level_la(L2), LB = L2 / LA;
+    constexpr int R = pass2_rows(3, L2), NT = pass2_reg_threads(L2);
+    constexpr int PITCH = pass2_reg_pitch(L2), TILE = pass2_reg_tile(L2);
+    constexpr bool IP = pass2_reg_inplace(L2);
+    constexpr int NB = IP ? 1 : 2;  // tiles in flight
+    constexpr int AU = R * LB, UPT = (AU + NT - 1) / NT;  // stage-A units per grid and thread
+    // tiles in flight (at the 128 bytes a TMA tile needs: no static shared
+    // memory lies before them), exchange tile or parked outputs, barriers
+    extern __shared__ __align__(1024) unsigned char sm_tiles[];
+    float2 *tiles = reinterpret_cast<float2 *>(sm_tiles), *rest = tiles + NB * TILE;
+    unsigned long long *full = reinterpret_cast<unsigned long long *>(tiles + pass2_reg_elems(L2));
+    const int tid = threadIdx.x;
+    if (smem_addr(tiles) & 127) {  // uniform; a copy there would fault
+        if (tid == 0) atomicOr(gp.errflag, 2u);
+        return;
+    }
+    const int G1 = p.G1, G = (int)p.G, lb = p.B == 4 ? 2 : 1, nrb = G1 / R;
+    const int ntask = n_curves * nrb;
+    if (tid == 0) {
+        for (int b = 0; b < NB; ++b) mbar_init(&full[b]);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    __syncthreads();
+    // step s: grid s % 3 of this CTA's task s / 3, into tile s % NB
+    auto live = [&](int s) { return blockIdx.x + (s / 3) * (int)gridDim.x < ntask; };
+    auto issue = [&](int s) {
+        if (!live(s)) return;
+        const int t = blockIdx.x + (s / 3) * (int)gridDim.x, c = t / nrb, rb = t - c * nrb;
+        mbar_expect(&full[s % NB], R * L2 * 8);
+        tma_load_3d(tiles + (s % NB) * TILE, &map, rb * R * 2 * p.B, 0, (first + c) * 3 + s % 3,
+                    &full[s % NB]);
+    };
+    if (tid == 0)
+        for (int b = 0; b < NB; ++b) issue(b);
+    const int r = tid % R, qa = tid / R;  // stage-B unit of this thread
+    const bool act = NT == R * LA || tid < R * LA;
+    int s = 0;
+    for (int t = blockIdx.x; t < ntask; t += gridDim.x) {
+        const int ci = t / nrb, rb = t - ci * nrb;
+        float2 ya[LB], yb[LB], yc[LB];
+#pragma unroll
+        for (int g = 0; g < 3; ++g, ++s) {
+            const bool ok = mbar_wait(&full[s % NB], (s / NB) & 1);
+            float2 *in = tiles + (s % NB) * TILE;
+            float2 *ex = IP ? in : rest;
+            // stage A: unit u = (ih, r, c) reads in[u + k AU], i.e. elements
+            // i + LB k, i = ih B + c, of row r
+            auto load = [&](float2 (&x)[LA], int u) {
+#pragma unroll
+                for (int k = 0; k < LA; ++k) x[k] = in[u + k * AU];
+                fft2_stage_a_regs<L2>(x, p.st2, ((u >> lb) / R << lb) + (u & ((1 << lb) - 1)));
+            };
+            auto store = [&](const float2 (&x)[LA], int u) {
+                const int i = ((u >> lb) / R << lb) + (u & ((1 << lb) - 1)), ra = (u >> lb) % R;
+                float2 *d = ex + ra * PITCH + row_shift<R>(ra) + i;
+#pragma unroll
+                for (int q = 0; q < LA; ++q) d[(LB + 1) * q] = x[q];
+            };
+            float2 x[IP ? UPT : 1][LA];
+            if constexpr (IP) {  // all units read before the tile is written
+#pragma unroll
+                for (int v = 0; v < UPT; ++v)
+                    if (AU % NT == 0 || tid + v * NT < AU) load(x[v], tid + v * NT);
+            } else {
+#pragma unroll 1
+                for (int u = tid; u < AU; u += NT) {
+                    load(x[0], u);
+                    store(x[0], u);
+                }
+            }
+            if (__syncthreads_or(!ok)) {  // a copy never came: leave, all threads
+                if (tid == 0) {
+                    atomicOr(gp.errflag, 2u);
+                    for (int k = s; k < s + NB; ++k)
+                        if (live(k)) mbar_wait(&full[k % NB], (k / NB) & 1);
+                }
+                __syncthreads();
+                return;
+            }
+            if constexpr (IP) {
+#pragma unroll
+                for (int v = 0; v < UPT; ++v)
+                    if (AU % NT == 0 || tid + v * NT < AU) store(x[v], tid + v * NT);
+                __syncthreads();
+            } else {
+                if (tid == 0) issue(s + NB);  // into the tile just read
+            }
+            float2 *y = g == 0 ? ya : g == 1 ? yb : yc;
+            if (act) {
+                const float2 *e = ex + r * PITCH + row_shift<R>(r) + (LB + 1) * qa;
+#pragma unroll
+                for (int i = 0; i < LB; ++i) y[i] = e[i];
+            }
+            if constexpr (IP) {
+                __syncthreads();  // all read: the tile is free
+                if (tid == 0) issue(s + NB);
+            }
+            if (act) RegDFT<LB>::run(y);
+            if constexpr (IP) {
+                if (g == 0) {  // grid A parked, read back by the same thread
+#pragma unroll
+                    for (int qb = 0; qb < LB; ++qb) rest[qb * NT + tid] = ya[qb];
+                }
+            } else {
+                __syncthreads();  // the exchange tile is written next
+            }
+        }
+        // power of the outputs q2 = qa + LA qb
+        const DevCurve &cv = cvs[ci];
+        const int nf = cv.nf, h = nf / 2, lo_end = nf - h, hi_start = G - h;
+        const bool write = gp.best == nullptr || out != nullptr;
+        float *o = out + cv.out_off + h;
+        const int q0 = rb * R + r + G1 * qa;
+        const float *drow = ES ? p.drow + ((long long)rb * L2 + qa) * R + r : nullptr;
+        const Fm2 fm(cv, gp.reg);
+        unsigned long long key = 0;
+        const unsigned ibase = (unsigned)(cv.best_off + h);
+        auto emit = [&](float P, int k) {
+            if (write) o[k] = P;
+            if (gp.best != nullptr && P >= 0.f) {  // valid powers only
+                const unsigned long long kk = ((unsigned long long)__float_as_uint(P) << 32) |
+                                              (0xFFFFFFFFu - (ibase + (unsigned)k));
+                key = kk > key ? kk : key;
+            }
+        };
+        // two frequencies at a time; f(qb, ka, kb, ina, inb, D) for each pair
+        // with an output in band
+        auto pairs = [&](auto f) {
+#pragma unroll
+            for (int qb = 0; qb < LB; qb += 2) {
+                // (no band reaches the middle fifth of the grid: sigma >= 1.25)
+                if (5 * qb >= 2 * LB && 5 * (qb + 2) <= 3 * LB) continue;
+                const int qA = q0 + G1 * LA * qb, qB = qA + G1 * LA;
+                const bool ina = qA < lo_end || qA >= hi_start;
+                const bool inb = qB < lo_end || qB >= hi_start;
+                if (!ina && !inb) continue;
+                if constexpr (IP) {
+                    ya[qb] = rest[qb * NT + tid];
+                    ya[qb + 1] = rest[(qb + 1) * NT + tid];
+                }
+                const int ka = qA < lo_end ? qA : qA - G, kb = qB < lo_end ? qB : qB - G;
+                float2 D;
+                if constexpr (ES)
+                    D = make_float2(__ldg(drow + LA * R * qb), __ldg(drow + LA * R * (qb + 1)));
+                else
+                    D = make_float2(win_deconv<false>(ka, p), win_deconv<false>(kb, p));
+                f(qb, ka, kb, ina, inb, D);
+            }
+        };
+        if (act && gp.mode == 1) {
+            pairs([&](int qb, int ka, int kb, bool ina, bool inb, float2 D) {
+                const float2 P = fm.power(ya[qb], ya[qb + 1], yb[qb], yb[qb + 1], yc[qb],
+                                          yc[qb + 1], D);
+                if (ina) emit(P.x, ka);
+                if (inb) emit(P.y, kb);
+            });
+        } else if (act) {
+            auto one = [&](float2 A, float2 B, float2 C, float D) {
+                return gls_from_sums<float>(A.x * D, A.y * D, B.x * D, B.y * D, C.x * D, C.y * D,
+                                            gp.mode, gp.reg, cv.w_sum, cv.yw_sum, cv.ybar,
+                                            cv.yy_inv);
+            };
+            pairs([&](int qb, int ka, int kb, bool ina, bool inb, float2 D) {
+                if (ina) emit(one(ya[qb], yb[qb], yc[qb], D.x), ka);
+                if (inb) emit(one(ya[qb + 1], yb[qb + 1], yc[qb + 1], D.y), kb);
+            });
+        }
+        if (gp.best != nullptr) {
+#pragma unroll
+            for (int of = 16; of > 0; of >>= 1) {
+                const unsigned long long v = __shfl_xor_sync(0xffffffffu, key, of);
+                key = v > key ? v : key;
+            }
+            if ((tid & 31) == 0 && key != 0) atomicMax(gp.best + cv.best_slot, key);
+        }
+    }
+}
+
+// Tensor map of a chunk's intermediate for tiles of R rows of one grid:
+// (G1 B complex values of a column block, column blocks, curve x grid).
+cudaError_t pass2_map(CUtensorMap &map, const float2 *inter, const Plan &p, int grids, int R);
+
+template <int L2, bool ES>
+cudaError_t launch_pass2_reg_t(const DevCurve *cv, int n_curves, int first, const float2 *inter,
+                               float *out, const Plan &p, GlsParams g, cudaStream_t s) {
+    static int per_sm[64] = {0}, sms[64] = {0};  // per instantiation and device
+    constexpr int NT = pass2_reg_threads(L2);
+    const int smem = (int)pass2_smem(3, L2);
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+    if (per_sm[dev] == 0) {
+        cudaError_t e = cudaFuncSetAttribute(k_pass2_gls_reg<L2, ES>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return e;
+        int n = 0, m = 0;
+        e = cudaDeviceGetAttribute(&m, cudaDevAttrMultiProcessorCount, dev);
+        if (e == cudaSuccess)
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_pass2_gls_reg<L2, ES>, NT, smem);
+        if (e != cudaSuccess) return e;
+        sms[dev] = m;
+        per_sm[dev] = n > 0 ? n : 1;
+    }
+    CUtensorMap map;
+    cudaError_t e = pass2_map(map, inter, p, 3 * (first + n_curves), pass2_rows(3, L2));
+    if (e != cudaSuccess) return e;
+    const long long tasks = (long long)n_curves * (p.G1 / pass2_rows(3, L2));
+    if (tasks > 0x3fffffffLL) return cudaErrorInvalidValue;
+    const int grid = (int)(tasks < (long long)per_sm[dev] * sms[dev] ? tasks
+                                                                     : per_sm[dev] * sms[dev]);
+    k_pass2_gls_reg<L2, ES><<<grid, NT, smem, s>>>(map, cv, n_curves, first, out, p, g);
+    return cudaGetLastError();
+}
+
+}  // namespace cuvgls

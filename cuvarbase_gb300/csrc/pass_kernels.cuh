@@ -21,6 +21,7 @@
 #include "fft.cuh"
 #include "gls_math.cuh"
 #include "kernels.cuh"
+#include "pass2_tma.cuh"
 
 namespace cuvgls {
 
@@ -493,7 +494,7 @@ __device__ __forceinline__ void gls_epilogue(const float2 *tile, const DevCurve 
         if (q < lo_end) kp = q;
         else if (q >= hi_start) kp = q - G;
         else continue;
-        const float D = win_deconv<ES>(kp, p);
+        const float D = ES ? __ldg(p.drow + (long long)rb * R * L2 + e) : win_deconv<false>(kp, p);
         const int o = phys2<L2>(q2);
         const float2 A = tile[r * LDS + o];
         const float2 Bv = tile[(R + r) * LDS + o];
@@ -567,9 +568,9 @@ __device__ __forceinline__ void gls_epilogue_fm2(const float2 *tile, const DevCu
         // or the plan's table
         float2 D;
         if constexpr (ES) {
-            // (an out-of-band lane reads entry 0: |k'| <= G / 2 only in band)
-            D = make_float2(__ldg(p.dtab + (ina ? abs(ka) : 0)),
-                            __ldg(p.dtab + (inb ? abs(kb) : 0)));
+            // (a lane beyond the row repeats the first entry)
+            const float *dr = p.drow + (long long)rb * R * L2 + r;
+            D = make_float2(__ldg(dr + q2a * R), __ldg(dr + (q2b < L2 ? q2b : q2a) * R));
         } else {
             const float2 kf = make_float2((float)ka, (float)kb);
             const float2 ex = __fmul2_rn(__fmul2_rn(kf, kf), dc1);
@@ -741,15 +742,20 @@ cudaError_t launch_pass1_t(const DevCurve *cv, int n_curves, const RecAB *recAB,
 }
 
 template <int L2>
-cudaError_t launch_pass2_gls_t(const DevCurve *cv, int n_curves, const float2 *inter,
+cudaError_t launch_pass2_gls_t(const DevCurve *cv, int n_curves, int first, const float2 *inter,
                                float *out, const Plan &p, GlsParams g, cudaStream_t s) {
-    static size_t done[64] = {0};  // per instantiation
-    cudaError_t e = allow_smem(k_pass2_gls<L2>, (size_t)pass2_smem(3, L2), done);
-    if (e != cudaSuccess) return e;
-    dim3 grid(p.G1 / pass2_rows(3, L2), n_curves);
-    k_pass2_gls<L2><<<grid, pass2_threads(3, L2), (size_t)pass2_smem(3, L2), s>>>(
-        cv, inter, out, p, g);
-    return cudaGetLastError();
+    if constexpr (pass2_reg(3, L2)) {
+        return p.win == kWinES ? launch_pass2_reg_t<L2, true>(cv, n_curves, first, inter, out, p, g, s)
+                               : launch_pass2_reg_t<L2, false>(cv, n_curves, first, inter, out, p, g, s);
+    } else {
+        static size_t done[64] = {0};  // per instantiation
+        cudaError_t e = allow_smem(k_pass2_gls<L2>, (size_t)pass2_smem(3, L2), done);
+        if (e != cudaSuccess) return e;
+        dim3 grid(p.G1 / pass2_rows(3, L2), n_curves);
+        k_pass2_gls<L2><<<grid, pass2_threads(3, L2), (size_t)pass2_smem(3, L2), s>>>(
+            cv, inter, out, p, g);
+        return cudaGetLastError();
+    }
 }
 
 template <int L2>
@@ -777,12 +783,17 @@ cudaError_t preload_pass1_t() {
 template <int L2>
 cudaError_t preload_pass2_t(int ng) {
     cudaFuncAttributes a;
-    return ng == 3 ? cudaFuncGetAttributes(&a, k_pass2_gls<L2>)
-                   : cudaFuncGetAttributes(&a, k_pass2_nfft<L2>);
+    if (ng != 3) return cudaFuncGetAttributes(&a, k_pass2_nfft<L2>);
+    if constexpr (pass2_reg(3, L2)) {
+        const cudaError_t e = cudaFuncGetAttributes(&a, k_pass2_gls_reg<L2, true>);
+        return e != cudaSuccess ? e : cudaFuncGetAttributes(&a, k_pass2_gls_reg<L2, false>);
+    } else {
+        return cudaFuncGetAttributes(&a, k_pass2_gls<L2>);
+    }
 }
 
 #define CUVGLS_INSTANTIATE_ROW_LEN(L)                                               \
-    template cudaError_t launch_pass2_gls_t<L>(const DevCurve *, int, const float2 *, \
+    template cudaError_t launch_pass2_gls_t<L>(const DevCurve *, int, int, const float2 *, \
                                                float *, const Plan &, GlsParams,     \
                                                cudaStream_t);                        \
     template cudaError_t launch_pass2_nfft_t<L>(const DevCurve *, int, const float2 *, \
@@ -797,7 +808,7 @@ cudaError_t preload_pass2_t(int ng) {
     template cudaError_t launch_pass1_t<1, L>(const DevCurve *, int, const RecAB *, \
                                               const RecC *, const int *, const int *, \
                                               float2 *, const Plan &, cudaStream_t); \
-    template cudaError_t launch_pass2_gls_t<L>(const DevCurve *, int, const float2 *, \
+    template cudaError_t launch_pass2_gls_t<L>(const DevCurve *, int, int, const float2 *, \
                                                float *, const Plan &, GlsParams,     \
                                                cudaStream_t);                        \
     template cudaError_t launch_pass2_nfft_t<L>(const DevCurve *, int, const float2 *, \

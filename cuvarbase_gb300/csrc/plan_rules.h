@@ -190,12 +190,21 @@ CUVGLS_HD constexpr int pass1_cols(int ng, int L1) {
     return b;
 }
 
+// Whether the GLS rows of this length keep their outputs in registers
+// (k_pass2_gls_reg): a two-level split with at most 20 outputs of each grid
+// per thread.
+CUVGLS_HD constexpr bool pass2_reg(int ng, int L2) {
+    return ng == 3 && two_level_la(L2) > 0 && L2 / two_level_la(L2) <= 20;
+}
+
 // Rows per pass-2 CTA for ng grids of row length L2: 16 for short rows, so
-// that a CTA still transforms a few thousand elements; 4 for the three-grid
-// GLS rows of 256..1024 (more, smaller CTAs per SM overlap one CTA's loads
-// with another's arithmetic); 8 otherwise; halved until the tile fits (2 at
-// least, 1 only for the 4096-long rows).
+// that a CTA still transforms a few thousand elements; 8 for the other
+// register rows (32-byte runs of powers); 4 for the three-grid GLS rows of
+// 512..1024 (more, smaller CTAs per SM overlap one CTA's loads with another's
+// arithmetic); 8 otherwise; halved until the tile fits (2 at least, 1 only for
+// the 4096-long rows).
 CUVGLS_HD constexpr int pass2_rows(int ng, int L2) {
+    if (pass2_reg(ng, L2)) return L2 <= 160 ? 16 : 8;
     int r = (ng == 1 || L2 <= 160) ? 16 : (L2 <= 1024 ? 4 : 8);
     while (r > (L2 > 2048 ? 1 : 2) && !tile_fits(ng * r, L2)) r /= 2;
     return r;
@@ -204,6 +213,34 @@ CUVGLS_HD constexpr int pass2_rows(int ng, int L2) {
 CUVGLS_HD constexpr int pass1_threads(int ng, int L1) {
     return fft_threads(ng * pass1_cols(ng, L1), L1);
 }
+// k_pass2_gls_reg: a thread per stage-B unit; row pitch of the exchange tile
+// (room for row_shift).  Rows above 160 are exchanged in place, in the one
+// tile a grid arrives in, and park grid A's outputs in shared memory: 96
+// registers and four CTAs per SM, which matters more there than copies ahead
+// of their use (400: 1.66 ms per 2,000 curves of 320 x 400 cells; 1.77 with
+// two tiles and three CTAs, 2.02 with two tiles, an exchange tile of their own
+// and two CTAs).  Shorter rows have a tile to exchange in and two in flight
+// (160: 2.89 ms per 20,000 curves of 160 x 160 cells; 3.16 in place).
+CUVGLS_HD constexpr int pass2_reg_threads(int L2) {
+    return round32(pass2_rows(3, L2) * two_level_la(L2));
+}
+CUVGLS_HD constexpr int pass2_reg_pitch(int L2) { return (tile_len(L2) + 11 + 15) / 16 * 16; }
+CUVGLS_HD constexpr bool pass2_reg_inplace(int L2) { return L2 > 160; }
+CUVGLS_HD constexpr int pass2_reg_ctas(int L2) { return pass2_reg_inplace(L2) ? 4 : 3; }
+// elements of the exchange tile and of a tile in flight
+CUVGLS_HD constexpr int pass2_reg_exch(int L2) {
+    return pass2_rows(3, L2) * pass2_reg_pitch(L2) + 16;
+}
+CUVGLS_HD constexpr int pass2_reg_tile(int L2) {
+    return pass2_reg_inplace(L2) ? pass2_reg_exch(L2) : pass2_rows(3, L2) * L2;
+}
+// elements of shared memory before the barriers
+CUVGLS_HD constexpr int pass2_reg_elems(int L2) {
+    return pass2_reg_inplace(L2)
+               ? pass2_reg_tile(L2) + L2 / two_level_la(L2) * pass2_reg_threads(L2)
+               : 2 * pass2_reg_tile(L2) + pass2_reg_exch(L2);
+}
+
 CUVGLS_HD constexpr int pass2_threads(int ng, int L2) {
     return fft_threads(ng * pass2_rows(ng, L2), L2);
 }
@@ -286,6 +323,7 @@ CUVGLS_HD constexpr long long pass1_smem(int ng, int L1, long long G) {
 
 // Shared memory of a pass-2 CTA: ng * R padded rows and the stage twiddles.
 CUVGLS_HD constexpr long long pass2_smem(int ng, int L2) {
+    if (pass2_reg(ng, L2)) return (pass2_reg_elems(L2) + 2LL) * 8;
     return (long long)(ng * pass2_rows(ng, L2) * row_stride(L2) +
                        (two_level_la(L2) ? 0 : fft_table_len(L2))) * 8;
 }

@@ -1,0 +1,55 @@
+"""Pass 2 of the GLS at every row length, with the band as wide as the grid
+allows (sigma at its smallest) and much narrower, four and two columns per
+pass-1 block, several curves in one chunk, every mode and output kind, both
+windows, against the FP64 oracle."""
+import numpy as np
+import pytest
+
+from test_gpu_prep import _curve
+from test_gpu_raw import _raw
+
+pytestmark = pytest.mark.gpu
+
+ROWS = [16, 32, 64, 80, 128, 160, 256, 320, 400, 512, 640, 800, 1024, 1280, 1600, 2048, 4096]
+
+
+def _ref(oracle, c, k, mode):
+    t, y, dy, df = c
+    tt, yw, w, YY, ybar = oracle.prepare_curve(t, y, dy)
+    return oracle.gls_tau(tt, yw.astype(np.float64), w.astype(np.float64), df * (1 + k), YY, ybar,
+                          mode=mode)
+
+
+@pytest.mark.parametrize("G1", [64, 320, 1280])
+@pytest.mark.parametrize("G2", ROWS)
+def test_row_lengths(oracle, G2, G1):
+    from cuvarbase_gb300 import _lib
+    if G1 == 1280 and G2 > 640:
+        G1 = 64                       # (keeps the oracle's bands short)
+    curves = [_curve(n, n + G2) for n in (300, 90, 700)]
+    # the oracle's FP32 comparison values: 2e-5 for the Gaussian (FP32 rounding
+    # amplified at the band edge of sigma 2), 1e-4 for the ES budget
+    for sigma, tol in ((-1.0, 1e-4), (2.0, 2e-5)):
+        if sigma > 0 and G2 < 32:
+            continue                  # 16 taps of the Gaussian do not fit
+        h = _lib.Handle(sigma=sigma, m=8)
+        try:
+            G = G1 * G2
+            for nf in (int(G / (1.28 if sigma < 0 else 2.0)), G // 6):
+                h.plan_pin(nf, G1, G2)
+                assert h.plan(nf)[1:3] == (G1, G2)
+                k = np.unique(np.concatenate([np.arange(30, 130), np.arange(nf - 60, nf),
+                                              np.arange(nf // 2 - 40, nf // 2 + 40),
+                                              np.arange(31, nf, max(1, nf // 200))]))
+                for mode in (1, 0, 2):
+                    P = _raw(h, curves, nf, mode)
+                    for c, got in zip(curves, P):
+                        ref = _ref(oracle, c, k, mode)
+                        assert np.abs(got[k] - ref).max() <= tol * max(1.0, np.abs(ref).max())
+                P = _raw(h, curves, nf)
+                bk, bp = _raw(h, curves, nf, best=True)
+                for i in range(len(curves)):
+                    assert P[i][bk[i]] >= P[i].max() - 1e-6
+                    assert abs(float(bp[i]) - float(P[i].max())) <= 1e-6
+        finally:
+            h.close()
