@@ -390,7 +390,7 @@ int get_class(cuvgls_handle *h, long long nf, int ng, ClassTables **out) {
     // window the deconvolution of |k'| <= G / 2) built on the device
     const size_t n1 = (size_t)fft_table_len(G1), n2 = (size_t)fft_table_len(G2);
     const size_t nd = p.win == kWinES ? (size_t)(G / 2 + 2) / 2 : 0;  // in float2 units
-    const size_t nr = p.win == kWinES && ng == 3 ? (size_t)(G + 1) / 2 : 0;
+    const size_t nr = p.win == kWinES ? (size_t)(G + 1) / 2 : 0;
     CK(cudaMalloc(&c.d, (n1 + n2 + (size_t)G + nd + nr) * sizeof(float2)),
        "cudaMalloc(plan tables)");
     // on a stream of their own: a new class waits neither for batches nor for
@@ -774,7 +774,7 @@ int run_batch(cuvgls_handle *h, const Work &wk, std::vector<DevCurve> &cvs,
     SegEntry *d_bseg = reinterpret_cast<SegEntry *>(d_cv + nc);
     SegEntry *d_rseg = d_bseg + nseg_bin;
     int *d_list = reinterpret_cast<int *>(d_rseg + nseg_raw);
-    float4 *d_aux = (float4 *)take(nc * sizeof(float4));
+    ulonglong2 *d_aux = (ulonglong2 *)take(nc * sizeof(ulonglong2));
     const double *t = wk.t;
     const float *ya = wk.ya, *wv = wk.wv;
     const double *ry = wk.ry, *rdy = wk.rdy;
@@ -1053,7 +1053,8 @@ int run_batch(cuvgls_handle *h, const Work &wk, std::vector<DevCurve> &cvs,
                            "k_pass2_gls");
                 } else {
                     LAUNCH(CUVGLS_STAGE_PASS2, gs,
-                           launch_pass2_nfft(dq, e - a, inter, (float2 *)dev_out, d_aux, p, gs),
+                           launch_pass2_nfft(dq, e - a, a, inter, (float2 *)dev_out, d_aux,
+                                             h->d_flags, p, gs),
                            "k_pass2_nfft");
                 }
                 if (!hcopy) continue;

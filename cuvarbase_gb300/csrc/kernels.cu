@@ -345,11 +345,12 @@ cudaError_t launch_pass2_gls(const DevCurve *cv, int n_curves, int first,
 #undef CUVGLS_P2
 }
 
-cudaError_t launch_pass2_nfft(const DevCurve *cv, int n_curves,
-                              const float2 *inter, float2 *out,
-                              const float4 *aux, const Plan &p, cudaStream_t s) {
+cudaError_t launch_pass2_nfft(const DevCurve *cv, int n_curves, int first, const float2 *inter,
+                              float2 *out, const ulonglong2 *aux, unsigned *errflag, const Plan &p,
+                              cudaStream_t s) {
     if (n_curves <= 0) return cudaSuccess;
-#define CUVGLS_P2N(L) case L: return launch_pass2_nfft_t<L>(cv, n_curves, inter, out, aux, p, s);
+#define CUVGLS_P2N(L) \
+    case L: return launch_pass2_nfft_t<L>(cv, n_curves, first, inter, out, aux, errflag, p, s);
     switch (p.G2) {
         CUVGLS_ROW_LEN_CASES(CUVGLS_P2N)
         default: return cudaErrorInvalidValue;

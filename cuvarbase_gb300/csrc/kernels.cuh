@@ -23,7 +23,7 @@ struct PrepArrays {
     RecC *recC;
     int *binsAB, *binsC;         // nb + 1 offsets per descriptor
     int *curAB, *curC;           // cursors (long curves)
-    float4 *aux;                 // output phases of the adjoint NFFT, or null
+    ulonglong2 *aux;             // output phases of the adjoint NFFT, or null
     unsigned *errflag;
     int mode;                    // GLS mode (raw input)
     int max_nb;                  // most column blocks of the launch's plans
@@ -56,9 +56,9 @@ cudaError_t launch_pass1(const DevCurve *cv, int n_curves, const RecAB *recAB,
 cudaError_t launch_pass2_gls(const DevCurve *cv, int n_curves, int first, const float2 *inter, float *out, const Plan &p,
                              GlsParams g, cudaStream_t s);
 
-cudaError_t launch_pass2_nfft(const DevCurve *cv, int n_curves,
-                              const float2 *inter, float2 *out,
-                              const float4 *aux, const Plan &p, cudaStream_t s);
+cudaError_t launch_pass2_nfft(const DevCurve *cv, int n_curves, int first, const float2 *inter,
+                              float2 *out, const ulonglong2 *aux, unsigned *errflag, const Plan &p,
+                              cudaStream_t s);
 
 // Length templates (pass_kernels.cuh, instantiated in inst_*.cu).
 template <int NG, int L1>
@@ -68,8 +68,8 @@ template <int L2>
 cudaError_t launch_pass2_gls_t(const DevCurve *, int, int, const float2 *, float *,
                                const Plan &, GlsParams, cudaStream_t);
 template <int L2>
-cudaError_t launch_pass2_nfft_t(const DevCurve *, int, const float2 *, float2 *,
-                                const float4 *, const Plan &, cudaStream_t);
+cudaError_t launch_pass2_nfft_t(const DevCurve *, int, int, const float2 *, float2 *,
+                                const ulonglong2 *, unsigned *, const Plan &, cudaStream_t);
 
 template <int NG, int L1>
 cudaError_t preload_pass1_t();

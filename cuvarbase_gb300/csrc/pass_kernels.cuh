@@ -662,10 +662,9 @@ k_pass2_gls(const DevCurve *__restrict__ cvs, const float2 *__restrict__ inter,
 template <bool ES, int L2, int R, int NT, int LDS>
 __device__ __forceinline__ void nfft_finish(const float2 *tile, const DevCurve &cv,
                                             float2 *__restrict__ out,
-                                            const float4 *__restrict__ aux, const Plan &p,
+                                            const ulonglong2 *__restrict__ aux, const Plan &p,
                                             int rb, int tid) {
-    const float4 ax = aux[cv.aux];
-    const float2 base = make_float2(ax.x, ax.y);
+    const ulonglong2 ax = aux[cv.aux];
     const long long G = p.G;
     const int G1 = p.G1;
     const int nf = cv.nf, h = nf / 2;
@@ -673,15 +672,8 @@ __device__ __forceinline__ void nfft_finish(const float2 *tile, const DevCurve &
         const int r = e % R, q2 = e / R;
         const int kp = band_index((long long)(rb * R + r) + (long long)G1 * q2, nf, h, G);
         if (kp == INT_MIN) continue;
-        const float kf = (float)kp;
-        const float D = win_deconv<ES>(kp, p);
-        // frac(k' alpha) with alpha = hi + lo and k' alpha_hi split exactly
-        const float pr = kf * ax.z;
-        const float er = fmaf(kf, ax.z, -pr);
-        const float th = (pr - rintf(pr)) + (er + kf * ax.w);
-        float s, c;
-        sincospif(2.0f * th, &s, &c);
-        const float2 ph = cmul(base, make_float2(c, s));
+        const float D = ES ? __ldg(p.drow + (long long)rb * R * L2 + e) : win_deconv<false>(kp, p);
+        const float2 ph = turn_phasor(ax.x + (unsigned long long)(long long)kp * ax.y);
         out[cv.out_off + kp + h] = cmul(cscale(tile[r * LDS + phys2<L2>(q2)], D), ph);
     }
 }
@@ -689,7 +681,7 @@ __device__ __forceinline__ void nfft_finish(const float2 *tile, const DevCurve &
 template <int L2>
 __global__ void __launch_bounds__(pass2_threads(1, L2))
 k_pass2_nfft(const DevCurve *__restrict__ cvs, const float2 *__restrict__ inter,
-             float2 *__restrict__ out, const float4 *__restrict__ aux, Plan p) {
+             float2 *__restrict__ out, const ulonglong2 *__restrict__ aux, Plan p) {
     constexpr int R = pass2_rows(1, L2);
     constexpr int NT = pass2_threads(1, L2);
     constexpr int LDS = row_stride(L2);
@@ -759,16 +751,22 @@ cudaError_t launch_pass2_gls_t(const DevCurve *cv, int n_curves, int first, cons
 }
 
 template <int L2>
-cudaError_t launch_pass2_nfft_t(const DevCurve *cv, int n_curves, const float2 *inter,
-                                float2 *out, const float4 *aux, const Plan &p,
-                                cudaStream_t s) {
-    static size_t done[64] = {0};  // per instantiation
-    cudaError_t e = allow_smem(k_pass2_nfft<L2>, (size_t)pass2_smem(1, L2), done);
-    if (e != cudaSuccess) return e;
-    dim3 grid(p.G1 / pass2_rows(1, L2), n_curves);
-    k_pass2_nfft<L2><<<grid, pass2_threads(1, L2), (size_t)pass2_smem(1, L2), s>>>(
-        cv, inter, out, aux, p);
-    return cudaGetLastError();
+cudaError_t launch_pass2_nfft_t(const DevCurve *cv, int n_curves, int first, const float2 *inter,
+                                float2 *out, const ulonglong2 *aux, unsigned *errflag,
+                                const Plan &p, cudaStream_t s) {
+    if constexpr (pass2_reg(1, L2)) {
+        return p.win == kWinES
+                   ? launch_nfft_reg_t<L2, true>(cv, n_curves, first, inter, out, aux, errflag, p, s)
+                   : launch_nfft_reg_t<L2, false>(cv, n_curves, first, inter, out, aux, errflag, p, s);
+    } else {
+        static size_t done[64] = {0};  // per instantiation
+        cudaError_t e = allow_smem(k_pass2_nfft<L2>, (size_t)pass2_smem(1, L2), done);
+        if (e != cudaSuccess) return e;
+        dim3 grid(p.G1 / pass2_rows(1, L2), n_curves);
+        k_pass2_nfft<L2><<<grid, pass2_threads(1, L2), (size_t)pass2_smem(1, L2), s>>>(
+            cv, inter, out, aux, p);
+        return cudaGetLastError();
+    }
 }
 
 // Load the pass kernels of a length now (CUDA loads kernels lazily, at
@@ -783,12 +781,16 @@ cudaError_t preload_pass1_t() {
 template <int L2>
 cudaError_t preload_pass2_t(int ng) {
     cudaFuncAttributes a;
-    if (ng != 3) return cudaFuncGetAttributes(&a, k_pass2_nfft<L2>);
     if constexpr (pass2_reg(3, L2)) {
+        if (ng != 3) {
+            const cudaError_t e = cudaFuncGetAttributes(&a, k_pass2_nfft_reg<L2, true>);
+            return e != cudaSuccess ? e : cudaFuncGetAttributes(&a, k_pass2_nfft_reg<L2, false>);
+        }
         const cudaError_t e = cudaFuncGetAttributes(&a, k_pass2_gls_reg<L2, true>);
         return e != cudaSuccess ? e : cudaFuncGetAttributes(&a, k_pass2_gls_reg<L2, false>);
     } else {
-        return cudaFuncGetAttributes(&a, k_pass2_gls<L2>);
+        return ng == 3 ? cudaFuncGetAttributes(&a, k_pass2_gls<L2>)
+                       : cudaFuncGetAttributes(&a, k_pass2_nfft<L2>);
     }
 }
 
@@ -796,9 +798,9 @@ cudaError_t preload_pass2_t(int ng) {
     template cudaError_t launch_pass2_gls_t<L>(const DevCurve *, int, int, const float2 *, \
                                                float *, const Plan &, GlsParams,     \
                                                cudaStream_t);                        \
-    template cudaError_t launch_pass2_nfft_t<L>(const DevCurve *, int, const float2 *, \
-                                                float2 *, const float4 *, const Plan &, \
-                                                cudaStream_t);                       \
+    template cudaError_t launch_pass2_nfft_t<L>(const DevCurve *, int, int, const float2 *, \
+                                                float2 *, const ulonglong2 *, unsigned *, \
+                                                const Plan &, cudaStream_t);                       \
     template cudaError_t preload_pass2_t<L>(int);
 
 #define CUVGLS_INSTANTIATE_LEN(L)                                                   \
@@ -811,9 +813,9 @@ cudaError_t preload_pass2_t(int ng) {
     template cudaError_t launch_pass2_gls_t<L>(const DevCurve *, int, int, const float2 *, \
                                                float *, const Plan &, GlsParams,     \
                                                cudaStream_t);                        \
-    template cudaError_t launch_pass2_nfft_t<L>(const DevCurve *, int, const float2 *, \
-                                                float2 *, const float4 *, const Plan &, \
-                                                cudaStream_t);                       \
+    template cudaError_t launch_pass2_nfft_t<L>(const DevCurve *, int, int, const float2 *, \
+                                                float2 *, const ulonglong2 *, unsigned *, \
+                                                const Plan &, cudaStream_t);                       \
     template cudaError_t preload_pass1_t<3, L>();                                  \
     template cudaError_t preload_pass1_t<1, L>();                                  \
     template cudaError_t preload_pass2_t<L>(int);

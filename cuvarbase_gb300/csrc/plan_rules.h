@@ -190,11 +190,11 @@ CUVGLS_HD constexpr int pass1_cols(int ng, int L1) {
     return b;
 }
 
-// Whether the GLS rows of this length keep their outputs in registers
-// (k_pass2_gls_reg): a two-level split with at most 20 outputs of each grid
-// per thread.
+// Whether the rows of this length keep their outputs in registers
+// (k_pass2_gls_reg, k_pass2_nfft_reg): a two-level split with at most 20
+// outputs of each grid per thread.
 CUVGLS_HD constexpr bool pass2_reg(int ng, int L2) {
-    return ng == 3 && two_level_la(L2) > 0 && L2 / two_level_la(L2) <= 20;
+    return two_level_la(L2) > 0 && L2 / two_level_la(L2) <= 20;
 }
 
 // Rows per pass-2 CTA for ng grids of row length L2: 16 for short rows, so
@@ -233,6 +233,19 @@ CUVGLS_HD constexpr int pass2_reg_exch(int L2) {
 }
 CUVGLS_HD constexpr int pass2_reg_tile(int L2) {
     return pass2_reg_inplace(L2) ? pass2_reg_exch(L2) : pass2_rows(3, L2) * L2;
+}
+// k_pass2_nfft_reg: in place in one tile, four CTAs per SM (1,000 curves of
+// 512 x 400 cells 0.431 ms; 0.442 with a tile ahead, 0.452 with five CTAs).
+constexpr int kNfftCols = 8;  // columns per pass-1 block of every one-grid plan
+CUVGLS_HD constexpr bool nfft_cols_ok() {
+    for (int l : kLens)
+        if (pass1_cols(1, l) != kNfftCols) return false;
+    return true;
+}
+static_assert(nfft_cols_ok(), "k_pass2_nfft_reg reads blocks of eight columns");
+constexpr int kNfftRegCtas = 4;
+CUVGLS_HD constexpr int nfft_reg_elems(int L2) {
+    return pass2_reg_exch(L2) + L2 / two_level_la(L2);
 }
 // elements of shared memory before the barriers
 CUVGLS_HD constexpr int pass2_reg_elems(int L2) {
@@ -323,7 +336,8 @@ CUVGLS_HD constexpr long long pass1_smem(int ng, int L1, long long G) {
 
 // Shared memory of a pass-2 CTA: ng * R padded rows and the stage twiddles.
 CUVGLS_HD constexpr long long pass2_smem(int ng, int L2) {
-    if (pass2_reg(ng, L2)) return (pass2_reg_elems(L2) + 2LL) * 8;
+    if (pass2_reg(ng, L2))
+        return ((ng == 3 ? pass2_reg_elems(L2) : nfft_reg_elems(L2)) + 2LL) * 8;
     return (long long)(ng * pass2_rows(ng, L2) * row_stride(L2) +
                        (two_level_la(L2) ? 0 : fft_table_len(L2))) * 8;
 }

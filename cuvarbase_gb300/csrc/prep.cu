@@ -97,18 +97,7 @@ template <bool WHOLE>
 __device__ __forceinline__ float2 centre_phase(u64 f, double x, const Centre &k) {
     u64 th = (u64)k.ki * f;
     if (!WHOLE && k.kf != 0.0) th += turns64(k.kf * x);
-    // th in [-1/2, 1/2) as hi + lo floats, hi the nearest float to its upper
-    // half; sincospi(2 hi) corrected to first order in lo
-    const int h32 = (int)(th >> 32);
-    const float hf = (float)h32;
-    const int d32 = (int)((unsigned)h32 - (unsigned)(int)fminf(hf, 2147483520.f));
-    const float hi = fminf(hf, 2147483520.f) * 2.3283064365386963e-10f;  // 2^-32
-    const float lo = fmaf((float)(unsigned)th, 5.42101086242752217e-20f,  // 2^-64
-                          (float)d32 * 2.3283064365386963e-10f);
-    float s, c;
-    sincospif(2.0f * hi, &s, &c);
-    const float e = 6.283185307179586f * lo;
-    return make_float2(fmaf(-e, s, c), fmaf(e, c, s));
+    return turn_phasor(th);
 }
 
 // Cells (x and 2x) and centring phase of one point; a point whose t is not
@@ -150,19 +139,11 @@ __device__ __forceinline__ RecC rec_c(const Place &p, float w) {
 }
 
 // Output phase of the adjoint NFFT of a descriptor: out[k] needs
-// exp(2 pi i (kc + k') df t0): base = exp(2 pi i kc df t0), alpha =
-// frac(df t0) split into hi + lo floats.
+// exp(2 pi i (kc + k') df t0): the turns kc df t0 and df t0 as 64-bit
+// fractions.
 __device__ __forceinline__ void write_aux(const DevCurve &cv, double tref,
-                                          float4 *__restrict__ aux) {
-    double v = cv.kc * cv.df * tref;
-    v -= floor(v);
-    double s, c;
-    sincospi(2.0 * v, &s, &c);
-    double al = cv.df * tref;
-    al -= floor(al);
-    const float ah = (float)al;
-    const float alo = (float)(al - (double)ah);
-    aux[cv.aux] = make_float4((float)c, (float)s, ah, alo);
+                                          ulonglong2 *__restrict__ aux) {
+    aux[cv.aux] = make_ulonglong2(turns64(cv.kc * cv.df * tref), turns64(cv.df * tref));
 }
 
 // ---------------------------------------------------------------------------

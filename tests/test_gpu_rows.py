@@ -53,3 +53,26 @@ def test_row_lengths(oracle, G2, G1):
                     assert abs(float(bp[i]) - float(P[i].max())) <= 1e-6
         finally:
             h.close()
+
+
+@pytest.mark.parametrize("sigma", ["auto", 2])
+@pytest.mark.parametrize("nf", [150, 700, 2500, 5000, 12800, 20000, 31000, 50000, 100000, 160000,
+                                250000, 600000])
+def test_nfft_rows(oracle, sigma, nf):
+    """The adjoint NFFT on the grids of many frequency counts (rows of most
+    lengths), with a first frequency that is not a multiple of df and times
+    far from zero, several curves in one chunk."""
+    from cuvarbase_gb300.cunfft import NFFTAsyncProcess
+    data = [(t + 5.0e4, y, nf) for t, y, _, _ in (_curve(n, nf + n) for n in (200, 60, 500))]
+    p = NFFTAsyncProcess(sigma=sigma, m=8)
+    res = p.run(data, minimum_frequency=0.7531, samples_per_peak=3)
+    p.finish()
+    # the ES window's budget at the band edge against the Gaussian's rounding
+    tol = 2e-5 if sigma == "auto" else 2e-6
+    for (t, y, _), got in zip(data, res):
+        df = 1.0 / (3 * (t.max() - t.min()))
+        k = np.unique(np.concatenate([np.arange(60), np.arange(nf - 60, nf),
+                                      np.arange(nf // 2 - 30, nf // 2 + 30),
+                                      np.arange(0, nf, max(1, nf // 400))]))
+        ref = oracle.nfft_direct(t, y, 0.7531 + k * df)
+        assert np.abs(got[k] - ref).max() <= tol * np.abs(y).sum()
