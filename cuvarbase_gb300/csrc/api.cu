@@ -932,9 +932,24 @@ int run_batch(cuvgls_handle *h, const Work &wk, std::vector<DevCurve> &cvs,
         memcpy(h_bseg + nseg_bin, raw_tab.data(), nseg_raw * sizeof(SegEntry));
         memcpy(h_list + nc, raw_list.data(), raw_list.size() * sizeof(int));
     }
-    CK(cudaMemcpyAsync(d_cv, h->h_cv, tab_bytes, cudaMemcpyHostToDevice, s),
-       "H2D descriptors");
-    CK(cudaEventRecord(h->h_cv_free, s), "record");
+    // A small batch whose curves are all prepared by one launch hands its
+    // descriptors over as a kernel parameter; otherwise the tables are copied.
+    DescParam dp;
+    dp.n = 0;
+    const Part &p0 = parts[0].empty() ? Part{} : parts[0][0];
+    if (merged && nc <= kParamDesc && nseg_raw == 0 && p0.seg_e == p0.seg_b) {
+        int used = 0;
+        for (int c = 0; c < kPrepClasses; ++c) used += p0.fused[c + 1] > p0.fused[c];
+        if (used == 1) {
+            dp.n = nc;
+            std::copy(h->h_cv, h->h_cv + nc, dp.cv);
+        }
+    }
+    if (dp.n == 0) {
+        CK(cudaMemcpyAsync(d_cv, h->h_cv, tab_bytes, cudaMemcpyHostToDevice, s),
+           "H2D descriptors");
+        CK(cudaEventRecord(h->h_cv_free, s), "record");
+    }
     // The input copies after the descriptor table: host-to-device copies of
     // all streams share the copy engine in the order they are issued, so a
     // table issued after the later phases' input would wait for all of it
@@ -1007,7 +1022,8 @@ int run_batch(cuvgls_handle *h, const Work &wk, std::vector<DevCurve> &cvs,
         for (int c = 0; c < kPrepClasses; ++c)
             if (pt.fused[c + 1] > pt.fused[c])
                 LAUNCH(CUVGLS_STAGE_PREP, s,
-                       launch_prep(pa, d_list + pt.fused[c], pt.fused[c + 1] - pt.fused[c], c,
+                       launch_prep(pa, dp, dp.n ? nullptr : d_list + pt.fused[c],
+                                   pt.fused[c + 1] - pt.fused[c], c,
                                    pt.max_n[c], raw && !multi_band, wk.ng, fp32, s),
                        "k_prep");
         if (pt.seg_e > pt.seg_b)

@@ -27,14 +27,25 @@ struct PrepArrays {
     unsigned *errflag;
     int mode;                    // GLS mode (raw input)
     int max_nb;                  // most column blocks of the launch's plans
+    int trigger;                 // let the next kernel be set up early (small_launch)
 };
+
+// Descriptors of a small batch as a kernel parameter: k_prep then takes its
+// curves from here and writes the descriptors to a.cv itself, so the batch
+// needs no copy of its table before its first kernel.
+constexpr int kParamDesc = 32;
+struct DescParam {
+    int n;  // 0: none, the descriptors are in a.cv
+    DevCurve cv[kParamDesc];
+};
+static_assert(sizeof(DescParam) + sizeof(PrepArrays) <= 3584, "kernel parameters");
 
 // Curves of one length class (prep_class), each by one CTA or cluster: raw
 // weights and statistics (raw != 0), bin offsets and records.  `list`: their
 // descriptors (null: 0 .. n - 1); max_n: the longest; ngrids 3 (GLS: yw@x,
 // w@x, w@2x) or 1 (NFFT: y@x).
-cudaError_t launch_prep(const PrepArrays &a, const int *list, int n, int cls, int max_n, int raw,
-                        int ngrids, int fp32_positions, cudaStream_t s);
+cudaError_t launch_prep(const PrepArrays &a, const DescParam &d, const int *list, int n, int cls,
+                        int max_n, int raw, int ngrids, int fp32_positions, cudaStream_t s);
 
 // Binning of long curves: counts per segment (the counts of their
 // descriptors zeroed by the caller), scan per descriptor of `list`, records

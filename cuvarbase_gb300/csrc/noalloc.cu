@@ -222,7 +222,7 @@ extern "C" int cuvgls_gls_noalloc(double sigma, int32_t m, const cuvgls_gls_inpu
                         curAB, curC, nullptr, d_flag, b->mode, p.nb};
     if (max_n <= kFusePoints) {
         if (e == cudaSuccess)
-            e = launch_prep(pa, nullptr, nc, prep_class(max_n, prep_spread(n_tot)), max_n,
+            e = launch_prep(pa, DescParam{}, nullptr, nc, prep_class(max_n, prep_spread(n_tot)), max_n,
                             0, 3, 0, s);
     } else {
         if (e == cudaSuccess) e = launch_seg_fill(d_cv, nc, segs, s);

@@ -112,7 +112,7 @@ struct Fm2 {
 
 template <int L2, bool ES>
 __global__ void __launch_bounds__(pass2_reg_threads(L2), pass2_reg_ctas(L2))
-k_pass2_gls_reg(const __grid_constant__ CUtensorMap map, const DevCurve *__restrict__ cvs,
+k_pass2_gls_reg(const __grid_constant__ CUtensorMap map, const DevCurve *cvs,
                 int n_curves, int first, float *__restrict__ out, const Plan p, const GlsParams gp) {
     constexpr int LA = two_level_la(L2), LB = L2 / LA;
     constexpr int R = pass2_rows(3, L2), NT = pass2_reg_threads(L2);
@@ -126,6 +126,7 @@ k_pass2_gls_reg(const __grid_constant__ CUtensorMap map, const DevCurve *__restr
     float2 *tiles = reinterpret_cast<float2 *>(sm_tiles), *rest = tiles + NB * TILE;
     unsigned long long *full = reinterpret_cast<unsigned long long *>(tiles + pass2_reg_elems(L2));
     const int tid = threadIdx.x;
+    if (p.dependent) pdl_trigger();
     if (smem_addr(tiles) & 127) {  // uniform; a copy there would fault
         if (tid == 0) atomicOr(gp.errflag, 2u);
         return;
@@ -137,6 +138,8 @@ k_pass2_gls_reg(const __grid_constant__ CUtensorMap map, const DevCurve *__restr
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     __syncthreads();
+    if (p.dependent) pdl_wait();  // the intermediate and the descriptors
+    cvs = written(cvs);
     // step s: grid s % 3 of this CTA's task s / 3, into tile s % NB
     auto live = [&](int s) { return blockIdx.x + (s / 3) * (int)gridDim.x < ntask; };
     auto issue = [&](int s) {
@@ -222,7 +225,7 @@ k_pass2_gls_reg(const __grid_constant__ CUtensorMap map, const DevCurve *__restr
             }
         }
         // power of the outputs q2 = qa + LA qb
-        const DevCurve &cv = cvs[ci];
+        const DevCurve cv = cvs[ci];
         const int nf = cv.nf, h = nf / 2, lo_end = nf - h, hi_start = G - h;
         const bool write = gp.best == nullptr || out != nullptr;
         float *o = out + cv.out_off + h;
@@ -301,9 +304,9 @@ k_pass2_gls_reg(const __grid_constant__ CUtensorMap map, const DevCurve *__restr
 // the measured copy rate).
 template <int L2, bool ES>
 __global__ void __launch_bounds__(pass2_reg_threads(L2), kNfftRegCtas)
-k_pass2_nfft_reg(const __grid_constant__ CUtensorMap map, const DevCurve *__restrict__ cvs,
+k_pass2_nfft_reg(const __grid_constant__ CUtensorMap map, const DevCurve *cvs,
                  int n_curves, int first, float2 *__restrict__ out,
-                 const ulonglong2 *__restrict__ aux, unsigned *__restrict__ errflag, const Plan p) {
+                 const ulonglong2 *aux, unsigned *__restrict__ errflag, const Plan p) {
     constexpr int LA = two_level_la(L2), LB = L2 / LA;
     constexpr int R = pass2_rows(1, L2), NT = pass2_reg_threads(L2);
     constexpr int PITCH = pass2_reg_pitch(L2), TILE = pass2_reg_exch(L2);
@@ -312,6 +315,7 @@ k_pass2_nfft_reg(const __grid_constant__ CUtensorMap map, const DevCurve *__rest
     float2 *in = reinterpret_cast<float2 *>(sm_tiles), *step = in + TILE;
     unsigned long long *full = reinterpret_cast<unsigned long long *>(in + nfft_reg_elems(L2));
     const int tid = threadIdx.x;
+    if (p.dependent) pdl_trigger();
     if (smem_addr(in) & 127) {  // uniform; a copy there would fault
         if (tid == 0) atomicOr(errflag, 2u);
         return;
@@ -329,6 +333,9 @@ k_pass2_nfft_reg(const __grid_constant__ CUtensorMap map, const DevCurve *__rest
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     __syncthreads();
+    if (p.dependent) pdl_wait();  // the intermediate and the descriptors
+    cvs = written(cvs);
+    aux = written(aux);
     auto live = [&](int s) { return blockIdx.x + s * (int)gridDim.x < ntask; };
     auto issue = [&](int s) {  // this CTA's task s
         if (!live(s)) return;
@@ -341,7 +348,7 @@ k_pass2_nfft_reg(const __grid_constant__ CUtensorMap map, const DevCurve *__rest
     const bool act = NT == R * LA || tid < R * LA;
     for (int s = 0; live(s); ++s) {
         const int t = blockIdx.x + s * (int)gridDim.x, ci = t / nrb, rb = t - ci * nrb;
-        const DevCurve &cv = cvs[ci];
+        const DevCurve cv = cvs[ci];
         const ulonglong2 ax = aux[cv.aux];
         const bool ok = mbar_wait(full, s & 1);
         float2 x[UPT][LA];
@@ -449,9 +456,11 @@ cudaError_t launch_nfft_reg_t(const DevCurve *cv, int n_curves, int first, const
     if (e != cudaSuccess) return e;
     const long long tasks = (long long)n_curves * (p.G1 / R);
     if (tasks > 0x3fffffffLL || p.B != kNfftCols) return cudaErrorInvalidValue;
-    k_pass2_nfft_reg<L2, ES><<<(int)(tasks < slots[dev] ? tasks : slots[dev]), NT, smem, s>>>(
-        map, cv, n_curves, first, out, aux, errflag, p);
-    return cudaGetLastError();
+    Plan q = p;
+    q.dependent = small_launch(tasks);
+    return launch_pdl(k_pass2_nfft_reg<L2, ES>, q.dependent,
+                      dim3((int)(tasks < slots[dev] ? tasks : slots[dev])), NT, smem, s, map, cv,
+                      n_curves, first, out, aux, errflag, q);
 }
 
 template <int L2, bool ES>
@@ -469,9 +478,11 @@ cudaError_t launch_pass2_reg_t(const DevCurve *cv, int n_curves, int first, cons
     if (e != cudaSuccess) return e;
     const long long tasks = (long long)n_curves * (p.G1 / R);
     if (tasks > 0x3fffffffLL) return cudaErrorInvalidValue;
-    k_pass2_gls_reg<L2, ES><<<(int)(tasks < slots[dev] ? tasks : slots[dev]), NT, smem, s>>>(
-        map, cv, n_curves, first, out, p, g);
-    return cudaGetLastError();
+    Plan q = p;
+    q.dependent = small_launch(tasks);
+    return launch_pdl(k_pass2_gls_reg<L2, ES>, q.dependent,
+                      dim3((int)(tasks < slots[dev] ? tasks : slots[dev])), NT, smem, s, map, cv,
+                      n_curves, first, out, q, g);
 }
 
 }  // namespace cuvgls

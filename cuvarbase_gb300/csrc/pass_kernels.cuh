@@ -111,12 +111,9 @@ static_assert(sizeof(StagedRec) == kStageRecBytes, "staged record size");
 // One pass-1 CTA: column block blockIdx.x of curve blockIdx.y (the body of
 // both pass-1 kernels below).
 template <int NG, int L1>
-__device__ __forceinline__ void pass1_body(const DevCurve *__restrict__ cvs,
-                                           const RecAB *__restrict__ recAB,
-                                           const RecC *__restrict__ recC,
-                                           const int *__restrict__ binsAB,
-                                           const int *__restrict__ binsC,
-                                           float2 *__restrict__ inter, const Plan &p) {
+__device__ __forceinline__ void pass1_body(const DevCurve *cvs, const RecAB *recAB,
+                                           const RecC *recC, const int *binsAB, const int *binsC,
+                                           float2 *inter, const Plan &p) {
     constexpr int B = pass1_cols(NG, L1);
     constexpr int NT = pass1_threads(NG, L1);
     constexpr int GS = tile_len(L1) * B;
@@ -129,8 +126,16 @@ __device__ __forceinline__ void pass1_body(const DevCurve *__restrict__ cvs,
     float2 *tile = sm;
     const int tid = threadIdx.x;
     const int cb = blockIdx.x;
-    const DevCurve cv = cvs[blockIdx.y];
     const int c0 = cb * B;
+    if (p.dependent) {
+        pdl_trigger();
+        pdl_wait();  // descriptors and records; the intermediate read by earlier passes
+    }
+    recAB = written(recAB);
+    recC = written(recC);
+    binsAB = written(binsAB);
+    binsC = written(binsC);
+    const DevCurve cv = written(cvs)[blockIdx.y];  // in flight during the zero-fill
     const int G2 = p.G2, m = p.m;
     // FFT table: read through the read-only cache (two-level lengths) or
     // staged in shared memory (Stockham lengths)
@@ -375,9 +380,8 @@ __device__ __forceinline__ void pass1_body(const DevCurve *__restrict__ cvs,
 // Pass 1 with the compiler's own register choice ...
 template <int NG, int L1>
 __global__ void __launch_bounds__(pass1_threads(NG, L1))
-k_pass1(const DevCurve *__restrict__ cvs, const RecAB *__restrict__ recAB,
-        const RecC *__restrict__ recC, const int *__restrict__ binsAB,
-        const int *__restrict__ binsC, float2 *__restrict__ inter, Plan p) {
+k_pass1(const DevCurve *cvs, const RecAB *recAB, const RecC *recC, const int *binsAB,
+        const int *binsC, float2 *inter, Plan p) {
     pass1_body<NG, L1>(cvs, recAB, recC, binsAB, binsC, inter, p);
 }
 
@@ -387,9 +391,8 @@ k_pass1(const DevCurve *__restrict__ cvs, const RecAB *__restrict__ recAB,
 // registers (pass 1 of rows of 400: 60 -> 110 registers, half the CTAs).
 template <int NG, int L1>
 __global__ void __launch_bounds__(pass1_threads(NG, L1), pass1_min_ctas(NG, L1))
-k_pass1_occ(const DevCurve *__restrict__ cvs, const RecAB *__restrict__ recAB,
-            const RecC *__restrict__ recC, const int *__restrict__ binsAB,
-            const int *__restrict__ binsC, float2 *__restrict__ inter, Plan p) {
+k_pass1_occ(const DevCurve *cvs, const RecAB *recAB, const RecC *recC, const int *binsAB,
+            const int *binsC, float2 *inter, Plan p) {
     pass1_body<NG, L1>(cvs, recAB, recC, binsAB, binsC, inter, p);
 }
 
@@ -406,8 +409,8 @@ __device__ __forceinline__ void load_rows_b(float2 *tile, const float2 *__restri
         const int g = v / R, r = v - g * R;
         const int l2 = 2 * pr;
         const int cb = l2 / B, c = l2 % B;
-        const float4 val = *reinterpret_cast<const float4 *>(
-            src + g * G + ((long long)cb * G1 + (long long)rb * R + r) * B + c);
+        const float4 val = __ldg(reinterpret_cast<const float4 *>(
+            src + g * G + ((long long)cb * G1 + (long long)rb * R + r) * B + c));
         float2 *d = tile + v * LDS;
         d[phys2<L2>(l2)] = make_float2(val.x, val.y);
         d[phys2<L2>(l2 + 1)] = make_float2(val.z, val.w);
@@ -616,8 +619,8 @@ __device__ __forceinline__ void gls_epilogue_fm2(const float2 *tile, const DevCu
 
 template <int L2>
 __global__ void __launch_bounds__(pass2_threads(3, L2))
-k_pass2_gls(const DevCurve *__restrict__ cvs, const float2 *__restrict__ inter,
-            float *__restrict__ out, Plan p, GlsParams gp) {
+k_pass2_gls(const DevCurve *cvs, const float2 *inter, float *__restrict__ out, Plan p,
+            GlsParams gp) {
     constexpr int R = pass2_rows(3, L2);
     constexpr int NT = pass2_threads(3, L2);
     static_assert(NT % 32 == 0, "the best-power reduction needs full warps");
@@ -625,7 +628,12 @@ k_pass2_gls(const DevCurve *__restrict__ cvs, const float2 *__restrict__ inter,
     extern __shared__ __align__(16) float2 sm[];
     float2 *tile = sm;
     const int tid = threadIdx.x, rb = blockIdx.x;
-    const DevCurve cv = cvs[blockIdx.y];
+    if (p.dependent) {
+        pdl_trigger();
+        pdl_wait();
+    }
+    inter = written(inter);
+    const DevCurve cv = written(cvs)[blockIdx.y];
     const int G1 = p.G1;
     rows_fft<3, L2, R, NT, LDS>(tile, inter + cv.inter_off, p.st2, G1, p.G, p.B, rb, tid);
     // The packed finish is compiled only into the 4-row tiles (rows of 256 to
@@ -680,15 +688,21 @@ __device__ __forceinline__ void nfft_finish(const float2 *tile, const DevCurve &
 
 template <int L2>
 __global__ void __launch_bounds__(pass2_threads(1, L2))
-k_pass2_nfft(const DevCurve *__restrict__ cvs, const float2 *__restrict__ inter,
-             float2 *__restrict__ out, const ulonglong2 *__restrict__ aux, Plan p) {
+k_pass2_nfft(const DevCurve *cvs, const float2 *inter, float2 *__restrict__ out,
+             const ulonglong2 *aux, Plan p) {
     constexpr int R = pass2_rows(1, L2);
     constexpr int NT = pass2_threads(1, L2);
     constexpr int LDS = row_stride(L2);
     extern __shared__ __align__(16) float2 sm[];
     float2 *tile = sm;
     const int tid = threadIdx.x, rb = blockIdx.x;
-    const DevCurve cv = cvs[blockIdx.y];
+    if (p.dependent) {
+        pdl_trigger();
+        pdl_wait();
+    }
+    inter = written(inter);
+    aux = written(aux);
+    const DevCurve cv = written(cvs)[blockIdx.y];
     const int G1 = p.G1;
     rows_fft<1, L2, R, NT, LDS>(tile, inter + cv.inter_off, p.st2, G1, p.G, p.B, rb, tid);
 
@@ -719,18 +733,19 @@ cudaError_t launch_pass1_t(const DevCurve *cv, int n_curves, const RecAB *recAB,
     static size_t done[64] = {0};  // per instantiation
     const size_t smem = (size_t)pass1_smem(NG, L1, p.G);
     dim3 grid(p.G2 / pass1_cols(NG, L1), n_curves);
+    Plan q = p;
+    q.dependent = small_launch((long long)grid.x * grid.y);
     if constexpr (pass1_small_stage(NG, L1)) {
         cudaError_t e = allow_smem(k_pass1_occ<NG, L1>, smem, done);
         if (e != cudaSuccess) return e;
-        k_pass1_occ<NG, L1><<<grid, pass1_threads(NG, L1), smem, s>>>(cv, recAB, recC, binsAB,
-                                                                        binsC, inter, p);
+        return launch_pdl(k_pass1_occ<NG, L1>, q.dependent, grid, pass1_threads(NG, L1), smem, s, cv, recAB,
+                          recC, binsAB, binsC, inter, q);
     } else {
         cudaError_t e = allow_smem(k_pass1<NG, L1>, smem, done);
         if (e != cudaSuccess) return e;
-        k_pass1<NG, L1><<<grid, pass1_threads(NG, L1), smem, s>>>(cv, recAB, recC, binsAB,
-                                                                    binsC, inter, p);
+        return launch_pdl(k_pass1<NG, L1>, q.dependent, grid, pass1_threads(NG, L1), smem, s, cv, recAB, recC,
+                          binsAB, binsC, inter, q);
     }
-    return cudaGetLastError();
 }
 
 template <int L2>
@@ -743,10 +758,11 @@ cudaError_t launch_pass2_gls_t(const DevCurve *cv, int n_curves, int first, cons
         static size_t done[64] = {0};  // per instantiation
         cudaError_t e = allow_smem(k_pass2_gls<L2>, (size_t)pass2_smem(3, L2), done);
         if (e != cudaSuccess) return e;
-        dim3 grid(p.G1 / pass2_rows(3, L2), n_curves);
-        k_pass2_gls<L2><<<grid, pass2_threads(3, L2), (size_t)pass2_smem(3, L2), s>>>(
-            cv, inter, out, p, g);
-        return cudaGetLastError();
+        const dim3 grid(p.G1 / pass2_rows(3, L2), n_curves);
+        Plan q = p;
+        q.dependent = small_launch((long long)grid.x * grid.y);
+        return launch_pdl(k_pass2_gls<L2>, q.dependent, grid, pass2_threads(3, L2),
+                          (size_t)pass2_smem(3, L2), s, cv, inter, out, q, g);
     }
 }
 
@@ -762,10 +778,11 @@ cudaError_t launch_pass2_nfft_t(const DevCurve *cv, int n_curves, int first, con
         static size_t done[64] = {0};  // per instantiation
         cudaError_t e = allow_smem(k_pass2_nfft<L2>, (size_t)pass2_smem(1, L2), done);
         if (e != cudaSuccess) return e;
-        dim3 grid(p.G1 / pass2_rows(1, L2), n_curves);
-        k_pass2_nfft<L2><<<grid, pass2_threads(1, L2), (size_t)pass2_smem(1, L2), s>>>(
-            cv, inter, out, aux, p);
-        return cudaGetLastError();
+        const dim3 grid(p.G1 / pass2_rows(1, L2), n_curves);
+        Plan q = p;
+        q.dependent = small_launch((long long)grid.x * grid.y);
+        return launch_pdl(k_pass2_nfft<L2>, q.dependent, grid, pass2_threads(1, L2),
+                          (size_t)pass2_smem(1, L2), s, cv, inter, out, aux, q);
     }
 }
 

@@ -224,13 +224,16 @@ __host__ __device__ constexpr int prep_smem(int nb, bool cluster) {
 // the three to six that passed yw, w, counts and cursors through memory.
 template <int NT, int PPT, bool CL, bool RAW, int NG, bool F32>
 __global__ void __launch_bounds__(NT)
-k_prep(const PrepArrays A, const int *__restrict__ list, int csize, int chunk) {
+k_prep(const PrepArrays A, const __grid_constant__ DescParam D, const int *__restrict__ list,
+       int csize, int chunk) {
     extern __shared__ __align__(16) unsigned cnt[];
     __shared__ double wred[4 * NT / 32], part[8], mean[2];
     __shared__ int ws[32];
     const int tid = threadIdx.x;
+    if (A.trigger) pdl_trigger();  // pass 1 may be set up
     const int ci = CL ? blockIdx.x / csize : blockIdx.x, rank = CL ? blockIdx.x % csize : 0;
-    DevCurve &cv = A.cv[list ? list[ci] : ci];
+    const int di = list ? list[ci] : ci;
+    const DevCurve &cv = D.n ? D.cv[di] : A.cv[di];
     const int n = cv.n;
     if (CL && chunk == 0) chunk = max(NT, ((n - 1) / csize + 32) & ~31);
     const int na = CL ? (n - 1) / chunk + 1 : 1;  // CTAs with points
@@ -339,14 +342,17 @@ k_prep(const PrepArrays A, const int *__restrict__ list, int csize, int chunk) {
         __syncthreads();
         for (int i = tid; i < nb; i += NT) off[i] = cnt[i];
     }
-    if (RAW && rank == 0 && tid == 0) {
-        double4 ta = make_double4(0.0, 0.0, 0.0, 0.0), tb = ta;
-        for (int r = 0; r < na; ++r) {
-            const double *pr = CL ? cg::this_cluster().map_shared_rank(part, r) : part;
-            ta.x += pr[0]; ta.y += pr[1]; ta.z += pr[2]; ta.w += pr[3];
-            tb.x += pr[4]; tb.y += pr[5]; tb.z += pr[6];
+    if ((RAW || D.n) && rank == 0 && tid == 0) {
+        if (D.n) A.cv[di] = cv;
+        if (RAW) {
+            double4 ta = make_double4(0.0, 0.0, 0.0, 0.0), tb = ta;
+            for (int r = 0; r < na; ++r) {
+                const double *pr = CL ? cg::this_cluster().map_shared_rank(part, r) : part;
+                ta.x += pr[0]; ta.y += pr[1]; ta.z += pr[2]; ta.w += pr[3];
+                tb.x += pr[4]; tb.y += pr[5]; tb.z += pr[6];
+            }
+            fill_stats(A.cv[di], ta, tb, A.mode);
         }
-        fill_stats(cv, ta, tb, A.mode);
     }
     // after the last read of another CTA's shared memory
     if (CL) cg::this_cluster().barrier_arrive();
@@ -630,8 +636,8 @@ k_fill_desc(DevCurve *__restrict__ cvs, const int *__restrict__ list, int n,
 namespace {
 
 template <int NT, int PPT, bool CL, bool RAW, int NG, bool F32>
-cudaError_t prep_t(const PrepArrays &a, const int *list, int n, int csize, int chunk,
-                   cudaStream_t s) {
+cudaError_t prep_t(const PrepArrays &a, const DescParam &d, const int *list, int n, int csize,
+                   int chunk, cudaStream_t s) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)n * csize);
     cfg.blockDim = dim3(NT);
@@ -644,37 +650,39 @@ cudaError_t prep_t(const PrepArrays &a, const int *list, int n, int csize, int c
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = CL ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, k_prep<NT, PPT, CL, RAW, NG, F32>, a, list, csize, chunk);
+    PrepArrays b = a;
+    b.trigger = small_launch((long long)n * csize);
+    return cudaLaunchKernelEx(&cfg, k_prep<NT, PPT, CL, RAW, NG, F32>, b, d, list, csize, chunk);
 }
 
 template <int NT, int PPT, bool CL>
-cudaError_t prep_kind(const PrepArrays &a, const int *list, int n, int csize, int chunk, int raw,
+cudaError_t prep_kind(const PrepArrays &a, const DescParam &d, const int *list, int n, int csize, int chunk, int raw,
                       int ngrids, int f32, cudaStream_t s) {
     if (raw)
-        return f32 ? prep_t<NT, PPT, CL, true, 3, true>(a, list, n, csize, chunk, s)
-                   : prep_t<NT, PPT, CL, true, 3, false>(a, list, n, csize, chunk, s);
+        return f32 ? prep_t<NT, PPT, CL, true, 3, true>(a, d, list, n, csize, chunk, s)
+                   : prep_t<NT, PPT, CL, true, 3, false>(a, d, list, n, csize, chunk, s);
     if (ngrids == 3)
-        return f32 ? prep_t<NT, PPT, CL, false, 3, true>(a, list, n, csize, chunk, s)
-                   : prep_t<NT, PPT, CL, false, 3, false>(a, list, n, csize, chunk, s);
-    return f32 ? prep_t<NT, PPT, CL, false, 1, true>(a, list, n, csize, chunk, s)
-               : prep_t<NT, PPT, CL, false, 1, false>(a, list, n, csize, chunk, s);
+        return f32 ? prep_t<NT, PPT, CL, false, 3, true>(a, d, list, n, csize, chunk, s)
+                   : prep_t<NT, PPT, CL, false, 3, false>(a, d, list, n, csize, chunk, s);
+    return f32 ? prep_t<NT, PPT, CL, false, 1, true>(a, d, list, n, csize, chunk, s)
+               : prep_t<NT, PPT, CL, false, 1, false>(a, d, list, n, csize, chunk, s);
 }
 
 }  // namespace
 
-cudaError_t launch_prep(const PrepArrays &a, const int *list, int n, int cls, int max_n, int raw,
-                        int ngrids, int fp32_positions, cudaStream_t s) {
+cudaError_t launch_prep(const PrepArrays &a, const DescParam &d, const int *list, int n, int cls,
+                        int max_n, int raw, int ngrids, int fp32_positions, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
     if (a.max_nb > kMaxBins || max_n > kFusePoints) return cudaErrorInvalidValue;
     if (cls == 0) {
         if (max_n > kPrepPoints) return cudaErrorInvalidValue;
-        return prep_kind<kPrepThreads, kPrepPpt, false>(a, list, n, 1, kPrepPoints, raw, ngrids,
+        return prep_kind<kPrepThreads, kPrepPpt, false>(a, d, list, n, 1, kPrepPoints, raw, ngrids,
                                                         fp32_positions, s);
     }
     if (cls == kPrepWide) {
         int csize = 1;
         while (csize * kWidePoints < max_n) csize *= 2;
-        return prep_kind<kWideThreads, kWidePpt, true>(a, list, n, csize, kWidePoints, raw, ngrids,
+        return prep_kind<kWideThreads, kWidePpt, true>(a, d, list, n, csize, kWidePoints, raw, ngrids,
                                                        fp32_positions, s);
     }
     if (max_n > kMaxCluster * kPrepPoints) return cudaErrorInvalidValue;
@@ -682,9 +690,9 @@ cudaError_t launch_prep(const PrepArrays &a, const int *list, int n, int cls, in
     const bool spread = cls == kPrepSpread;
     while (csize < kMaxCluster && csize * (spread ? kPrepThreads : kPrepPoints) < max_n) csize *= 2;
     if (csize == 1)
-        return prep_kind<kPrepThreads, kPrepPpt, false>(a, list, n, 1, kPrepPoints, raw, ngrids,
+        return prep_kind<kPrepThreads, kPrepPpt, false>(a, d, list, n, 1, kPrepPoints, raw, ngrids,
                                                         fp32_positions, s);
-    return prep_kind<kPrepThreads, kPrepPpt, true>(a, list, n, csize, spread ? 0 : kPrepPoints, raw,
+    return prep_kind<kPrepThreads, kPrepPpt, true>(a, d, list, n, csize, spread ? 0 : kPrepPoints, raw,
                                                    ngrids, fp32_positions, s);
 }
 
