@@ -13,6 +13,7 @@
 //   P3 = sum Im E cos bx, P4 = sum Re E sin bx,
 // which is two multiply-adds per complex bin and point.  exp(i K x) is the
 // product of a coarse and a fine table entry (32 centres from 4 + 8).
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <math.h>
 
@@ -20,6 +21,8 @@
 
 #include "gls_math.cuh"
 #include "kernels.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace cuvgls {
 
@@ -156,7 +159,7 @@ static_assert(kNfSmem >= 2 * kDirWarps * kNfBins * 8, "the reduction reuses the 
 // shared memory at the end.  A curve cut into several parts leaves partial
 // sums for k_nfft_direct64_sum.  2.4 FP64 instructions per (point, bin)
 // against 12 with a sincospi pair per point and 8 bins: 4 curves of 300 to
-// 2,000 points and 20,000 bins, host to host, 5.68 -> 0.85 ms.
+// 2,000 points and 20,000 bins 5.33 -> 0.36 ms (FP64 pipes 93 % busy).
 __global__ void __launch_bounds__(kDirThreads, 2)
 k_nfft_direct64(const Direct64Curve *__restrict__ cvs, const double *__restrict__ t,
                 const double *__restrict__ y, double2 *__restrict__ out,
@@ -298,7 +301,7 @@ __device__ __forceinline__ float gls_direct_power(const DevCurve &cv, const GlsP
 // origin), so the phases stay small.  A curve cut into parts leaves its six
 // partial sums for k_gls_direct_sum.  7.7 FP64 instructions per (point,
 // frequency) against about 45 with a sincospi each: 8 curves of 300 to 2,000
-// points and 10,000 frequencies 9.62 -> 1.10 ms.
+// points and 10,000 frequencies 9.62 -> 1.10 ms (FP64 pipes 81 % busy).
 __global__ void __launch_bounds__(kDirThreads, 1)
 k_gls_direct(const DevCurve *__restrict__ cvs, const double *__restrict__ t,
              const float *__restrict__ yw, const float *__restrict__ w, float *__restrict__ out,
@@ -414,8 +417,9 @@ constexpr int kTurn = 256;  // phasors of the shared turn table
 // left out are d^7 / 7! < 9e-18 and d^8 / 8! < 2e-20.  16 FP64 instructions
 // with the product p = t f, against about 28 for floor and sincospi.
 __device__ __forceinline__ double2 table_turn(double p, const double2 *tab) {
-    // beyond 2^40 turns the index below would lose bits: reduce first
-    if (fabs(p) > 1099511627776.0) p -= floor(p);
+    // from 2^40 turns on the index below would lose bits: reduce first
+    // (the exponent compared as an integer: no FP64 instruction)
+    if ((__double2hiint(p) & 0x7ff00000) >= (1023 + 40) << 20) p -= floor(p);
     constexpr double kRound = 6755399441055744.0;  // 1.5 2^52: adding it rounds to an integer
     const double z = fma(p, (double)kTurn, kRound);
     const double2 e = tab[__double2loint(z) & (kTurn - 1)];
@@ -438,27 +442,32 @@ __host__ __device__ constexpr int mh_smem(int H) {
 
 // 32 frequencies per CTA, one per lane; the eight warps take the points 32 at
 // a time in turn and are summed in shared memory, so that a few thousand
-// frequencies already fill the chip evenly (with a thread per frequency,
-// 20,000 of them made 157 CTAs of 128 threads for 152 SMs).  Per point the
+// frequencies already fill the chip (with a thread per frequency, 20,000 of
+// them made 157 CTAs of 128 threads for 152 SMs).  Up to four CTAs of a
+// cluster share the points of the same frequencies, and the first adds their
+// sums and solves: 625 CTAs left a fifth of the FP64 pipes idle at the end
+// (4.1 CTAs per SM are 5 rounds).  Per point the
 // phasor from table_turn, its powers n = 2 .. 2H from half-way products (three
 // instructions for an even n), then the sums of
 // cuvarbase/lombscargle.py:337-400 (mhdirect_sums) with the regulariser of
 // :403-447, the 2H x 2H system solved by Gaussian elimination with partial
 // pivoting, and the power of :497-536.  H = 3, 1,000 points, 20,000
-// frequencies, host to host: 4.93 -> 2.55 ms.
+// frequencies, host to host: 4.93 -> 2.24 ms (the kernel 2.17 ms with the FP64
+// pipes 88 % busy: 54 instructions per point and frequency).
 template <int H>
 __global__ void __launch_bounds__(kDirThreads, H <= 4 ? 2 : 1)
 k_mhgls_direct(const double *__restrict__ t, const double *__restrict__ yw,
                const double *__restrict__ w, long long n, const double *__restrict__ freqs,
-               long long nf, MhParams mp, double *__restrict__ out) {
+               long long nf, MhParams mp, double *__restrict__ out, int csize) {
     constexpr int NH = 2 * H, NS = mh_sums(H);
+    const int rank = blockIdx.x % csize;
     extern __shared__ __align__(16) double sm[];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     double2 *turn = reinterpret_cast<double2 *>(sm);
     double *st = sm + 2 * kTurn + wid * 96, *sy = st + 32, *sw = st + 64;
     for (int i = tid; i < kTurn; i += kDirThreads) turn[i] = zturn((double)i / kTurn);
     __syncthreads();
-    const long long k = (long long)blockIdx.x * 32 + lane;
+    const long long k = (long long)(blockIdx.x / csize) * 32 + lane;
     const double f = (k < nf) ? freqs[k] : 0.0;
     double c[NH + 1], s[NH + 1], yc[H + 1], ys[H + 1];
 #pragma unroll
@@ -466,7 +475,7 @@ k_mhgls_direct(const double *__restrict__ t, const double *__restrict__ yw,
 #pragma unroll
     for (int m = 0; m <= H; ++m) { yc[m] = 0.0; ys[m] = 0.0; }
     double ws = 0.0;  // of the points this lane staged
-    for (long long base = wid * 32; base < n; base += kDirThreads) {
+    for (long long base = rank * kDirThreads + wid * 32; base < n; base += csize * kDirThreads) {
         const int cnt = (int)min(32LL, n - base);
         __syncwarp();  // the previous tile is consumed
         if (lane < cnt) {
@@ -523,6 +532,18 @@ k_mhgls_direct(const double *__restrict__ t, const double *__restrict__ yw,
         double v = 0.0;
         for (int q = 0; q < kDirWarps; ++q) v += sm[q * NS * 32 + i];
         tot[i] = v;
+    }
+    if (csize > 1) {
+        cg::cluster_group cl = cg::this_cluster();
+        cl.sync();
+        if (rank == 0)
+            for (int i = tid; i < NS * 32; i += kDirThreads) {
+                double v = tot[i];
+                for (int q = 1; q < csize; ++q) v += cl.map_shared_rank(tot, q)[i];
+                tot[i] = v;
+            }
+        cl.sync();  // the others' sums are read before they leave
+        if (rank != 0) return;
     }
     __syncthreads();
     if (wid != 0 || k >= nf) return;
@@ -614,6 +635,22 @@ cudaError_t launch_mhgls_direct(int nharms, const double *t, const double *yw, c
     if (n <= 0 || nf <= 0) return cudaSuccess;
     const long long nb = (nf + 31) / 32;
     if (nb > 0x7fffffffLL) return cudaErrorInvalidValue;
+    // enough CTAs already (16 per SM), or too few points for one tile per warp
+    int csize = 1;
+    while (csize < 4 && nb * csize < 16 * 152 && n >= 2LL * csize * kDirThreads) csize *= 2;
+    if (nb * csize > 0x7fffffffLL) return cudaErrorInvalidValue;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(nb * csize));
+    cfg.blockDim = dim3(kDirThreads);
+    cfg.dynamicSmemBytes = mh_smem(nharms);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = csize;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = csize > 1 ? 1 : 0;
     cudaError_t e = cudaErrorInvalidValue;
     switch (nharms) {
 #define CUVGLS_MH(HH)                                                                             \
@@ -621,15 +658,14 @@ cudaError_t launch_mhgls_direct(int nharms, const double *t, const double *yw, c
         e = cudaFuncSetAttribute(k_mhgls_direct<HH>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                                  mh_smem(HH));                                                    \
         if (e != cudaSuccess) return e;                                                           \
-        k_mhgls_direct<HH><<<(unsigned)nb, kDirThreads, mh_smem(HH), s>>>(t, yw, w, n, freqs, nf, \
-                                                                          mp, out);               \
+        e = cudaLaunchKernelEx(&cfg, k_mhgls_direct<HH>, t, yw, w, n, freqs, nf, mp, out, csize); \
         break;
         CUVGLS_MH(1) CUVGLS_MH(2) CUVGLS_MH(3) CUVGLS_MH(4)
         CUVGLS_MH(5) CUVGLS_MH(6) CUVGLS_MH(7) CUVGLS_MH(8)
 #undef CUVGLS_MH
-        default: return e;
+        default: break;
     }
-    return cudaGetLastError();
+    return e;
 }
 
 }  // namespace cuvgls
