@@ -1,6 +1,8 @@
 """Asynchronous-process base class (mirrors cuvarbase/core.py:13-56)."""
 from __future__ import annotations
 
+import sys
+
 from . import _lib
 
 
@@ -43,6 +45,21 @@ class GPUAsyncProcess:
                             workspace_bytes=workspace_bytes, precision=precision)
             self._handles[key] = h
         return h
+
+    def _result_buffer(self, nbytes):
+        """A page-locked result buffer of the process: a pooled one that no
+        earlier result views any more, else a new one (free buffers that are
+        too small are given back then).  Page-locking a megabyte takes a few
+        hundred microseconds, longer than most calls' kernels."""
+        pool = self.__dict__.setdefault('_result_pool', [])
+        for buf in pool:
+            # references: the pool, the loop variable, getrefcount's argument
+            if buf.nbytes >= nbytes and sys.getrefcount(buf) <= 3:
+                return buf
+        buf = None
+        new = _lib.PinnedBuffer(max(int(nbytes), 1 << 20))
+        pool[:] = [b for b in pool if sys.getrefcount(b) > 3] + [new]
+        return new
 
     def _compile_and_prepare_functions(self, **kwargs):
         """Kernels are compiled ahead of time into libcuvgls.so; this only

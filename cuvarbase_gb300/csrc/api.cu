@@ -1788,7 +1788,10 @@ int cuvgls_sync(cuvgls_handle *h, void *stream, int32_t timeout_ms) {
     // ev[0] marks the caller's work, ev[1] the copy of the flag word queued
     // behind it into page-locked memory: nothing here blocks (a blocking
     // copy would also wait for other streams' work).  The deadline applies
-    // to the work; the one-word copy then gets a bounded grace period.
+    // to the work; the one-word copy then gets a bounded grace period.  The
+    // first millisecond is polled without pause: a 50 us sleep takes about 57,
+    // twice in a call whose kernels take as long (one curve of 1,000 points
+    // and 50,000 frequencies, host to host: 205 -> 90 us).
     cudaEvent_t ev[2] = {nullptr, nullptr};
     auto release = [&]() {
         for (cudaEvent_t e : ev)
@@ -1801,7 +1804,7 @@ int cuvgls_sync(cuvgls_handle *h, void *stream, int32_t timeout_ms) {
         e = cudaMemcpyAsync(h->h_flags, h->d_flags, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaEventRecord(ev[1], s);
     if (e != cudaSuccess) { release(); return cuda_fail(h, e, "record sync"); }
-    constexpr double kCopyGraceMs = 1000.0;
+    constexpr double kCopyGraceMs = 1000.0, kSpinMs = 1.0;
     auto t0 = std::chrono::steady_clock::now();
     for (int k = 0; k < 2; ++k) {
         const double limit = k == 0 ? (double)timeout_ms : (double)timeout_ms + kCopyGraceMs;
@@ -1817,7 +1820,7 @@ int cuvgls_sync(cuvgls_handle *h, void *stream, int32_t timeout_ms) {
                 return fail(h, CUVGLS_ETIMEOUT,
                             "sync deadline of " + std::to_string(timeout_ms) + " ms passed");
             }
-            std::this_thread::sleep_for(std::chrono::microseconds(50));
+            if (ms > kSpinMs) std::this_thread::sleep_for(std::chrono::microseconds(50));
         }
     }
     release();

@@ -103,13 +103,15 @@ def nfft_adjoint_async(memory, functions, minimum_frequency=0., block_size=256,
     return memory.ghat_c
 
 
-def _launch_nfft(handle, stream, mems, minimum_frequency, samples_per_peak):
+def _launch_nfft(handle, stream, mems, minimum_frequency, samples_per_peak,
+                 buffer=_lib.PinnedBuffer):
+    """``buffer(nbytes)`` gives the page-locked result buffer."""
     n_tot = sum(len(m.t) for m in mems)
     nf_tot = sum(m.nf for m in mems)
     t = np.empty(n_tot, np.float64)
     y = np.empty(n_tot, np.float32)
     curves = (_lib.NfftCurve * len(mems))()
-    out = _lib.PinnedBuffer(nf_tot * 8)
+    out = buffer(nf_tot * 8)
     o, fo = 0, 0
     for i, m in enumerate(mems):
         n = len(m.t)
@@ -134,7 +136,8 @@ def _launch_nfft(handle, stream, mems, minimum_frequency, samples_per_peak):
                                                        out.ptr, stream), "nfft batch")
 
 
-def _launch_nfft64(handle, stream, mems, minimum_frequency, samples_per_peak):
+def _launch_nfft64(handle, stream, mems, minimum_frequency, samples_per_peak,
+                   buffer=_lib.PinnedBuffer):
     """use_double: FP64 direct sums (cuvgls_nfft_adjoint_fp64), results as
     complex128 in each memory's ``ghat_c`` (valid after finish())."""
     n_tot = sum(len(m.t) for m in mems)
@@ -142,7 +145,7 @@ def _launch_nfft64(handle, stream, mems, minimum_frequency, samples_per_peak):
     t = np.empty(n_tot, np.float64)
     y = np.empty(n_tot, np.float64)
     curves = (_lib.NfftCurve * len(mems))()
-    out = _lib.PinnedBuffer(nf_tot * 16)
+    out = buffer(nf_tot * 16)
     o, fo = 0, 0
     for i, m in enumerate(mems):
         n = len(m.t)
@@ -270,20 +273,27 @@ class NFFTAsyncProcess(GPUAsyncProcess):
 
     def allocate(self, data, **kwargs):
         """NFFTMemory objects for [(t, y, nf), ...] (cunfft.py:468-505)."""
+        return self._memories(data, True, **kwargs)
+
+    def _memories(self, data, allocate, **kwargs):
+        """The memory objects, with result buffers of their own or without
+        (run() binds them to one buffer for all curves)."""
         stream = self._stream()  # one stream serves the whole batched call
         mems = []
         for i, (t, y, nf) in enumerate(data):
             m = self.get_m(nf)
             mem = NFFTMemory(self.sigma, stream, m,
                              use_double=self.use_double, **kwargs)
-            mems.append(mem.fromdata(t, y, nf=nf, allocate=True, **kwargs))
+            mems.append(mem.fromdata(t, y, nf=nf, allocate=allocate, **kwargs))
+            if not allocate:
+                mem.n = int((2.0 if mem.sigma == 'auto' else mem.sigma) * mem.nf)
         return mems
 
     def run(self, data, memory=None, **kwargs):
         """Adjoint NFFTs of [(t, y, nf), ...] (cunfft.py:507-542)."""
         self._compile_and_prepare_functions()
         if memory is None:
-            memory = self.allocate(data, **kwargs)
+            memory = self._memories(data, False, **kwargs)
         spp = kwargs.get('samples_per_peak', 1)
         f0 = kwargs.get('minimum_frequency', 0.)
         by_m = {}
@@ -303,7 +313,7 @@ class NFFTAsyncProcess(GPUAsyncProcess):
         for m, mems in by_m.items():
             h = self._handle(self._lib_sigma(), m)
             if self.use_double:
-                _launch_nfft64(h, self._stream().ptr, mems, f0, spp)
+                _launch_nfft64(h, self._stream().ptr, mems, f0, spp, self._result_buffer)
             else:
-                _launch_nfft(h, self._stream().ptr, mems, f0, spp)
+                _launch_nfft(h, self._stream().ptr, mems, f0, spp, self._result_buffer)
         return [mem.ghat_c for mem in memory]

@@ -560,20 +560,6 @@ class LombScargleAsyncProcess(GPUAsyncProcess):
         return [(freqs, lsp) for lsp in lsps]
 
 
-def _raw_buffer(proc, nbytes):
-    """A page-locked result buffer of the process: a pooled one that no
-    earlier result views any more, else a new one."""
-    import sys
-    pool = proc.__dict__.setdefault('_raw_pool', [])
-    for buf in pool:
-        # references: the pool, the loop variable, getrefcount's argument
-        if buf.nbytes >= nbytes and sys.getrefcount(buf) <= 3:
-            return buf
-    buf = _lib.PinnedBuffer(max(int(nbytes), 1 << 20))
-    pool.append(buf)
-    return buf
-
-
 def _run_raw(proc, data, frqs, k0s, best=False, **kwargs):
     """One cuvgls_gls_raw call for a list of (t, y, dy) curves: the weights,
     ybar, yw and YY of every curve are computed on the GPU from the raw FP64
@@ -615,7 +601,7 @@ def _run_raw(proc, data, frqs, k0s, best=False, **kwargs):
                                  bp.ctypes.data, stream), "gls raw best")
         h.sync(stream, -1)
         return bk, bp
-    buf = _raw_buffer(proc, 4 * int(oo[-1]))
+    buf = proc._result_buffer(4 * int(oo[-1]))
     # the library copies pageable inputs before the call returns
     h.check(L.cuvgls_gls_raw(h.ptr, ctypes.byref(inp), buf.ptr, None, None, stream),
             "gls raw")
