@@ -66,9 +66,10 @@ struct ClassTables {
 
 // Streams beside the caller's that the passes of a batch's groups (plans) are
 // spread over.  The kernels of one plan often fill a part of the chip for a
-// few tens of microseconds.  48 curves of 21 plans: 829 -> 510 us (with
-// the preparation of few points in one launch).
-constexpr int kSideStreams = 3;
+// few tens of microseconds.  48 curves of 21 plans: 829 -> 510 us with
+// three of them (and the preparation of few points in one launch), 540 -> 457
+// from three to seven.
+constexpr int kSideStreams = 7;
 
 struct cuvgls_handle {
     cuvgls_opts opts;
@@ -870,9 +871,9 @@ int run_batch(cuvgls_handle *h, const Work &wk, std::vector<DevCurve> &cvs,
     int sidx = 0, lidx = 0;
     // descriptors [first, first + count) as one part
     auto make_part = [&](int first, int count) {
-        long long pts = 0;
-        for (int k = first; k < first + count; ++k) pts += h->h_cv[k].n;
-        const bool spread = prep_spread(pts);
+        long long ctas = 0;
+        for (int k = first; k < first + count; ++k) ctas += spread_ctas(h->h_cv[k].n);
+        const bool spread = prep_spread(ctas);
         Part pt;
         pt.first = first;
         pt.count = count;
@@ -1018,14 +1019,19 @@ int run_batch(cuvgls_handle *h, const Work &wk, std::vector<DevCurve> &cvs,
         if (multi) CK(cudaMemsetAsync(pa.binsAB, 0, 2 * nbin * sizeof(int), s), "zero bins");
         return CUVGLS_OK;
     };
+    // (the classes after a part's first run beside it; the longest curves first)
     auto prep_part = [&](const Part &pt) -> int {
-        for (int c = 0; c < kPrepClasses; ++c)
-            if (pt.fused[c + 1] > pt.fused[c])
-                LAUNCH(CUVGLS_STAGE_PREP, s,
-                       launch_prep(pa, dp, dp.n ? nullptr : d_list + pt.fused[c],
-                                   pt.fused[c + 1] - pt.fused[c], c,
-                                   pt.max_n[c], raw && !multi_band, wk.ng, fp32, s),
-                       "k_prep");
+        bool beside_first = false;
+        for (int k = 0; k < kPrepClasses; ++k) {
+            const int c = (kPrepWide + k) % kPrepClasses;
+            if (pt.fused[c + 1] == pt.fused[c]) continue;
+            LAUNCH(CUVGLS_STAGE_PREP, s,
+                   launch_prep(pa, dp, dp.n ? nullptr : d_list + pt.fused[c],
+                               pt.fused[c + 1] - pt.fused[c], c, pt.max_n[c],
+                               raw && !multi_band, wk.ng, fp32, beside_first, s),
+                   "k_prep");
+            beside_first = !h->prof_on;
+        }
         if (pt.seg_e > pt.seg_b)
             LAUNCH(CUVGLS_STAGE_PREP, s,
                    launch_bin_long(pa, d_bseg + pt.seg_b, pt.seg_e - pt.seg_b,
@@ -1113,8 +1119,7 @@ int run_batch(cuvgls_handle *h, const Work &wk, std::vector<DevCurve> &cvs,
             if (rc) return rc;
         }
     } else {
-        // the largest groups first, each on the stream with the least work so
-        // far (cells; every group also costs its launches)
+        // the longest groups first, each on the stream with the least work so far
         std::vector<size_t> by(groups.size()), at(groups.size());
         size_t off2 = 0;
         for (size_t gi = 0; gi < groups.size(); ++gi) {
@@ -1122,16 +1127,25 @@ int run_batch(cuvgls_handle *h, const Work &wk, std::vector<DevCurve> &cvs,
             at[gi] = off2;
             off2 += align_up(groups[gi].inter_bytes);
         }
-        std::stable_sort(by.begin(), by.end(), [&](size_t x, size_t y) {
-            return groups[x].inter_bytes > groups[y].inter_bytes;
-        });
+        // modelled time (us): 14 ps per cell, or the spreading of the group's
+        // longest curve by the CTAs of its column blocks
+        std::vector<double> cost(groups.size());
+        for (size_t gi = 0; gi < groups.size(); ++gi) {
+            const Group &g = groups[gi];
+            int n = 0;
+            for (int k = 0; k < g.count; ++k) n = std::max(n, h->h_cv[g.first + k].n);
+            cost[gi] = 10.0 + 1.4e-5 * (double)g.count * (double)g.cls->plan.G +
+                       0.075 * n / g.cls->plan.nb;
+        }
+        std::stable_sort(by.begin(), by.end(),
+                         [&](size_t x, size_t y) { return cost[x] > cost[y]; });
         double load[kSideStreams + 1] = {};
         CK(cudaEventRecord(h->side_ev[kSideStreams], s), "fork");
         for (cudaStream_t x : h->side)
             CK(cudaStreamWaitEvent(x, h->side_ev[kSideStreams], 0), "fork");
         for (size_t gi : by) {
             const int k = (int)(std::min_element(load, load + kSideStreams + 1) - load);
-            load[k] += (double)groups[gi].inter_bytes + 4e6;
+            load[k] += cost[gi];
             rc = run_group(gi, (float2 *)((char *)inter + at[gi]), k ? h->side[k - 1] : s);
             if (rc) break;
         }

@@ -27,7 +27,8 @@ struct PrepArrays {
     unsigned *errflag;
     int mode;                    // GLS mode (raw input)
     int max_nb;                  // most column blocks of the launch's plans
-    int trigger;                 // let the next kernel be set up early (small_launch)
+    int trigger;                 // let the next kernel be set up early
+    int beside;                  // run beside the k_prep before: wait for it at the end
 };
 
 // Descriptors of a small batch as a kernel parameter: k_prep then takes its
@@ -43,9 +44,12 @@ static_assert(sizeof(DescParam) + sizeof(PrepArrays) <= 3584, "kernel parameters
 // Curves of one length class (prep_class), each by one CTA or cluster: raw
 // weights and statistics (raw != 0), bin offsets and records.  `list`: their
 // descriptors (null: 0 .. n - 1); max_n: the longest; ngrids 3 (GLS: yw@x,
-// w@x, w@2x) or 1 (NFFT: y@x).
+// w@x, w@2x) or 1 (NFFT: y@x).  `beside`: the kernel before it in the stream
+// is a launch_prep of the same batch, which it does not wait for before its
+// end.
 cudaError_t launch_prep(const PrepArrays &a, const DescParam &d, const int *list, int n, int cls,
-                        int max_n, int raw, int ngrids, int fp32_positions, cudaStream_t s);
+                        int max_n, int raw, int ngrids, int fp32_positions, bool beside,
+                        cudaStream_t s);
 
 // Binning of long curves: counts per segment (the counts of their
 // descriptors zeroed by the caller), scan per descriptor of `list`, records

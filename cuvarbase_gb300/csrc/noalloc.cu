@@ -94,7 +94,7 @@ extern "C" int cuvgls_gls_noalloc(double sigma, int32_t m, const cuvgls_gls_inpu
         return fail(CUVGLS_EINVAL, "reg must be (lambda, lambda, 0) with lambda >= 0");
     if (!(sigma >= 1.25 && sigma <= 16.0) || m < 2 || m > 16)
         return fail(CUVGLS_EINVAL, "sigma must be in [1.25, 16] and m in [2, 16]");
-    long long max_nf = 0, n_tot = 0, n_seg = 0;
+    long long max_nf = 0, n_tot = 0, n_seg = 0, n_ctas = 0;
     int max_n = 0;
     for (int i = 0; i < nc; ++i) {
         const cuvgls_curve &c = b->curves[i];
@@ -108,6 +108,7 @@ extern "C" int cuvgls_gls_noalloc(double sigma, int32_t m, const cuvgls_gls_inpu
         n_tot += c.n;
         n_seg += seg_count((int)c.n);
         max_n = std::max(max_n, (int)c.n);
+        n_ctas += spread_ctas((int)c.n);
     }
     // one plan (the one for the largest nf) serves every curve of the call
     int G1, G2, B, R;
@@ -222,8 +223,8 @@ extern "C" int cuvgls_gls_noalloc(double sigma, int32_t m, const cuvgls_gls_inpu
                         curAB, curC, nullptr, d_flag, b->mode, p.nb};
     if (max_n <= kFusePoints) {
         if (e == cudaSuccess)
-            e = launch_prep(pa, DescParam{}, nullptr, nc, prep_class(max_n, prep_spread(n_tot)), max_n,
-                            0, 3, 0, s);
+            e = launch_prep(pa, DescParam{}, nullptr, nc, prep_class(max_n, prep_spread(n_ctas)), max_n,
+                            0, 3, 0, false, s);
     } else {
         if (e == cudaSuccess) e = launch_seg_fill(d_cv, nc, segs, s);
         if (e == cudaSuccess) e = cudaMemsetAsync(binsAB, 0, 2 * nbin * sizeof(int), s);

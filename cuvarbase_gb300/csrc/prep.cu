@@ -382,6 +382,8 @@ k_prep(const PrepArrays A, const __grid_constant__ DescParam D, const int *__res
     if (A.aux != nullptr && rank == 0 && tid == 0) write_aux(cv, tref, A.aux);
     // a CTA's shared memory stays until the others have read it
     if (CL) cg::this_cluster().barrier_wait();
+    // this kernel's end says that the one beside it has ended too
+    if (A.beside && rank == 0) pdl_wait();
 }
 
 // ---------------------------------------------------------------------------
@@ -637,53 +639,62 @@ namespace {
 
 template <int NT, int PPT, bool CL, bool RAW, int NG, bool F32>
 cudaError_t prep_t(const PrepArrays &a, const DescParam &d, const int *list, int n, int csize,
-                   int chunk, cudaStream_t s) {
+                   int chunk, bool beside, cudaStream_t s) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)n * csize);
     cfg.blockDim = dim3(NT);
     cfg.dynamicSmemBytes = prep_smem(a.max_nb, CL);
     cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = csize;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
+    cudaLaunchAttribute at[2];
     cfg.attrs = at;
-    cfg.numAttrs = CL ? 1 : 0;
+    if (CL) {
+        cudaLaunchAttribute &x = at[cfg.numAttrs++];
+        x.id = cudaLaunchAttributeClusterDimension;
+        x.val.clusterDim.x = csize;
+        x.val.clusterDim.y = 1;
+        x.val.clusterDim.z = 1;
+    }
+    if (beside) {
+        cudaLaunchAttribute &x = at[cfg.numAttrs++];
+        x.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        x.val.programmaticStreamSerializationAllowed = 1;
+    }
     PrepArrays b = a;
-    b.trigger = small_launch((long long)n * csize);
+    b.trigger = 1;
+    b.beside = beside;
     return cudaLaunchKernelEx(&cfg, k_prep<NT, PPT, CL, RAW, NG, F32>, b, d, list, csize, chunk);
 }
 
 template <int NT, int PPT, bool CL>
 cudaError_t prep_kind(const PrepArrays &a, const DescParam &d, const int *list, int n, int csize, int chunk, int raw,
-                      int ngrids, int f32, cudaStream_t s) {
+                      int ngrids, int f32, bool beside, cudaStream_t s) {
     if (raw)
-        return f32 ? prep_t<NT, PPT, CL, true, 3, true>(a, d, list, n, csize, chunk, s)
-                   : prep_t<NT, PPT, CL, true, 3, false>(a, d, list, n, csize, chunk, s);
+        return f32 ? prep_t<NT, PPT, CL, true, 3, true>(a, d, list, n, csize, chunk, beside, s)
+                   : prep_t<NT, PPT, CL, true, 3, false>(a, d, list, n, csize, chunk, beside, s);
     if (ngrids == 3)
-        return f32 ? prep_t<NT, PPT, CL, false, 3, true>(a, d, list, n, csize, chunk, s)
-                   : prep_t<NT, PPT, CL, false, 3, false>(a, d, list, n, csize, chunk, s);
-    return f32 ? prep_t<NT, PPT, CL, false, 1, true>(a, d, list, n, csize, chunk, s)
-               : prep_t<NT, PPT, CL, false, 1, false>(a, d, list, n, csize, chunk, s);
+        return f32 ? prep_t<NT, PPT, CL, false, 3, true>(a, d, list, n, csize, chunk, beside, s)
+                   : prep_t<NT, PPT, CL, false, 3, false>(a, d, list, n, csize, chunk, beside, s);
+    return f32 ? prep_t<NT, PPT, CL, false, 1, true>(a, d, list, n, csize, chunk, beside, s)
+               : prep_t<NT, PPT, CL, false, 1, false>(a, d, list, n, csize, chunk, beside, s);
 }
 
 }  // namespace
 
 cudaError_t launch_prep(const PrepArrays &a, const DescParam &d, const int *list, int n, int cls,
-                        int max_n, int raw, int ngrids, int fp32_positions, cudaStream_t s) {
+                        int max_n, int raw, int ngrids, int fp32_positions, bool beside,
+                        cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
     if (a.max_nb > kMaxBins || max_n > kFusePoints) return cudaErrorInvalidValue;
     if (cls == 0) {
         if (max_n > kPrepPoints) return cudaErrorInvalidValue;
         return prep_kind<kPrepThreads, kPrepPpt, false>(a, d, list, n, 1, kPrepPoints, raw, ngrids,
-                                                        fp32_positions, s);
+                                                        fp32_positions, beside, s);
     }
     if (cls == kPrepWide) {
         int csize = 1;
         while (csize * kWidePoints < max_n) csize *= 2;
         return prep_kind<kWideThreads, kWidePpt, true>(a, d, list, n, csize, kWidePoints, raw, ngrids,
-                                                       fp32_positions, s);
+                                                       fp32_positions, beside, s);
     }
     if (max_n > kMaxCluster * kPrepPoints) return cudaErrorInvalidValue;
     int csize = 1;
@@ -691,9 +702,9 @@ cudaError_t launch_prep(const PrepArrays &a, const DescParam &d, const int *list
     while (csize < kMaxCluster && csize * (spread ? kPrepThreads : kPrepPoints) < max_n) csize *= 2;
     if (csize == 1)
         return prep_kind<kPrepThreads, kPrepPpt, false>(a, d, list, n, 1, kPrepPoints, raw, ngrids,
-                                                        fp32_positions, s);
+                                                        fp32_positions, beside, s);
     return prep_kind<kPrepThreads, kPrepPpt, true>(a, d, list, n, csize, spread ? 0 : kPrepPoints, raw,
-                                                   ngrids, fp32_positions, s);
+                                                   ngrids, fp32_positions, beside, s);
 }
 
 cudaError_t launch_bin_long(const PrepArrays &a, const SegEntry *segs, int n_segs, const int *list,
