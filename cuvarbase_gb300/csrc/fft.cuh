@@ -21,6 +21,7 @@
 namespace cuvgls {
 
 template <int R> struct SmallDFT;
+template <int R> struct RegDFT;
 
 template <> struct SmallDFT<2> {
     static __device__ __forceinline__ void run(float2 *v) {
@@ -153,7 +154,7 @@ struct FftStage {
                     if (NS > 1 && r > 0) a = cmul(a, tws[TWO + (r - 1) * NS + k]);
                     v[it][r] = a;
                 }
-                SmallDFT<R>::run(v[it]);
+                RegDFT<R>::run(v[it]);
             }
         }
         __syncthreads();

@@ -6,13 +6,16 @@
 //                    L1 x B shared-memory tiles (shared-memory float atomics),
 //                    runs the length-L1 column FFTs, applies the inter-pass
 //                    twiddle exp(2 pi i q1 l2 / G) and writes the tile to the
-//                    intermediate buffer (row-major, rows of G2).
+//                    intermediate buffer ([column block][q1][column]).
+//   k_pass1_long<L1> the same for one grid of the long columns.
 //   k_pass2_gls<L2>  one CTA per (curve, block of R rows).  Loads R rows of
 //                    the three grids, runs the length-L2 row FFTs and, in the
-//                    same kernel, deconvolves the Gaussian window and
-//                    evaluates the GLS power of every in-band frequency.
+//                    same kernel, deconvolves the window and evaluates the
+//                    GLS power of every in-band frequency.
+//   k_pass2_gls_cube the same for rows of 4,096.
 //   k_pass2_nfft<L2> the same for one grid, writing complex adjoint-NFFT
 //                    values with the absolute-time phase.
+// (Rows up to 400: pass2_tma.cuh.)
 #pragma once
 
 #include <climits>
@@ -169,13 +172,14 @@ __device__ __forceinline__ void pass1_body(const DevCurve *cvs, const RecAB *rec
     const RecC *rcc = recC + cv.rec_off;
     StagedRec *st = reinterpret_cast<StagedRec *>(sm + STAGE);
     const int ntot = nab + nc;
-    // Dense column blocks of the long Stockham tiles (at least one record per
-    // row of the tile) are spread by gather: the staged records are sorted
+    // Dense column blocks of the long Stockham tiles of one grid (at least one
+    // record per row of the tile) are spread by gather: the staged records are sorted
     // by the row they land in (integer shared-memory atomics and a scan),
     // then each thread sums the taps of whole rows in registers and adds
     // them to the tile with plain stores; no float atomics, which serialise
     // when several records hit the same cells.
     constexpr bool GATHER = pass1_gather(NG, L1);
+    static_assert(!GATHER || NG == 1, "the three-grid columns of that length: k_pass1_long");
     int *rowcnt = reinterpret_cast<int *>(st + NSR);  // L1 + 1 (gather tiles)
     int *bucket = rowcnt + L1 + 1;                      // NSR
     int *wsum = bucket + NSR;                           // 32
@@ -253,13 +257,9 @@ __device__ __forceinline__ void pass1_body(const DevCurve *cvs, const RecAB *rec
             __syncthreads();
             // 4. whole rows per thread: taps summed in registers
             for (int r = tid; r < L1; r += NT) {
-                float2 aA[B], aB[B], aC[B];
+                float2 aA[B];
 #pragma unroll
-                for (int cc = 0; cc < B; ++cc) {
-                    aA[cc] = make_float2(0.f, 0.f);
-                    aB[cc] = make_float2(0.f, 0.f);
-                    aC[cc] = make_float2(0.f, 0.f);
-                }
+                for (int cc = 0; cc < B; ++cc) aA[cc] = make_float2(0.f, 0.f);
                 // (bounds: offsets within the round's records, indices of
                 // staged records)
                 const int g0 = max(rowcnt[r], 0), g1 = min(rowcnt[r + 1], cnt);
@@ -267,34 +267,19 @@ __device__ __forceinline__ void pass1_body(const DevCurve *cvs, const RecAB *rec
                     const int j = bucket[e];
                     if ((unsigned)j >= (unsigned)cnt) continue;
                     const StagedRec rec = st[j];
-                    const bool ab = base + j < nab;
 #pragma unroll
                     for (int cc = 0; cc < B; ++cc) {
                         const int d = rec.rc + cc;
                         if (d < 1 - m || d > m) continue;
                         const float dd = (float)d - rec.frac;
                         const float wg = win_tap(dd, p);
-                        if (ab) {
-                            aA[cc] = make_float2(fmaf(rec.v0.x, wg, aA[cc].x),
-                                                 fmaf(rec.v0.y, wg, aA[cc].y));
-                            if (NG == 3)
-                                aB[cc] = make_float2(fmaf(rec.v1.x, wg, aB[cc].x),
-                                                     fmaf(rec.v1.y, wg, aB[cc].y));
-                        } else {
-                            aC[cc] = make_float2(fmaf(rec.v0.x, wg, aC[cc].x),
-                                                 fmaf(rec.v0.y, wg, aC[cc].y));
-                        }
+                        aA[cc] = make_float2(fmaf(rec.v0.x, wg, aA[cc].x),
+                                             fmaf(rec.v0.y, wg, aA[cc].y));
                     }
                 }
                 float2 *rp = tile + phys2<L1>(r) * B;
 #pragma unroll
-                for (int cc = 0; cc < B; ++cc) {
-                    rp[cc] = cadd(rp[cc], aA[cc]);
-                    if (NG == 3) {
-                        rp[GS + cc] = cadd(rp[GS + cc], aB[cc]);
-                        rp[2 * GS + cc] = cadd(rp[2 * GS + cc], aC[cc]);
-                    }
-                }
+                for (int cc = 0; cc < B; ++cc) rp[cc] = cadd(rp[cc], aA[cc]);
             }
             __syncthreads();  // rows summed before the counts are reset
             for (int i = tid; i <= L1; i += NT) rowcnt[i] = 0;
@@ -394,6 +379,149 @@ __global__ void __launch_bounds__(pass1_threads(NG, L1), pass1_min_ctas(NG, L1))
 k_pass1_occ(const DevCurve *cvs, const RecAB *recAB, const RecC *recC, const int *binsAB,
             const int *binsC, float2 *inter, Plan p) {
     pass1_body<NG, L1>(cvs, recAB, recC, binsAB, binsC, inter, p);
+}
+
+// Pass 1 of the GLS for the long columns (1,280 to 2,048): one CTA per curve,
+// column block and grid.  The column FFT has three levels F0 F1 F2 with every
+// butterfly in registers and in place: n = i + N1 k (N1 = F1 F2), i = j + F2 k',
+// output q0 + F0 q1 + F0 F1 q2, which level 3 multiplies by the inter-pass
+// twiddle and stores.  A record's taps are spread by one thread, straight from
+// global memory: more of them are in flight than in rounds staged through
+// shared memory and sorted by row.  Three grids of two columns in one CTA per SM
+// (1,024 threads, that staging, Stockham stages) had nothing beside them to fill
+// their barriers; two CTAs of one grid and four columns also halve the records
+// read and give pass 2 whole 32-byte sectors.  10^6 points, 3 x 2048 x 4096
+// cells: 1.066 -> 0.590 ms (0.24 ms of it the transforms, whose floor is
+// 0.09 ms of stores; the rest the taps: window values and compare-and-swap
+// adds, 52 % issue, L1 63 %); 1,000 points 0.413 -> 0.240 ms.
+template <int L1>
+__global__ void __launch_bounds__(pass1_threads(3, L1), 65536 / (64 * pass1_threads(3, L1)))
+k_pass1_long(const DevCurve *cvs, const RecAB *recAB, const RecC *recC, const int *binsAB,
+             const int *binsC, float2 *inter, const Plan p) {
+    constexpr int B = kLongCols, NT = pass1_threads(3, L1);
+    constexpr int F0 = long_fac(L1, 0), F1 = long_fac(L1, 1), F2 = long_fac(L1, 2), N1 = F1 * F2;
+    static_assert(F0 * N1 == L1 && B == 4, "three levels, four columns");
+    extern __shared__ __align__(16) float2 sm[];
+    const int tid = threadIdx.x, cb = blockIdx.x / 3, g = blockIdx.x % 3, c0 = cb * B;
+    if (p.dependent) {
+        pdl_trigger();
+        pdl_wait();  // descriptors and records; the intermediate read by earlier passes
+    }
+    recAB = written(recAB);
+    recC = written(recC);
+    const int *bins = written(g < 2 ? binsAB : binsC);
+    const DevCurve cv = written(cvs)[blockIdx.y];  // in flight during the zero-fill
+    {
+        float4 *t4 = reinterpret_cast<float4 *>(sm);
+        for (int i = tid; i < (L1 + F0) * B / 2; i += NT) t4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    const int G2 = p.G2, m = p.m;
+    int a0, a1, b0, b1;
+    bin_ranges(bins + cv.bin_off, cb, -((m + B - 1) / B), (B + m - 2) / B, p.nb, a0, a1, b0, b1);
+    const int na = a1 - a0, ntot = na + (b1 - b0);
+    const RecAB *rab = recAB + cv.rec_off;
+    const RecC *rcc = recC + cv.rec_off;
+    struct Rec {
+        int rc;
+        float frac;
+        float2 v;
+    };
+    auto load = [&](int k) {
+        k = k < na ? a0 + k : b0 + (k - na);
+        Rec r;
+        if (g < 2) {
+            const RecAB *q = rab + k;
+            r.rc = q->rc; r.frac = q->frac; r.v = g == 0 ? q->a : q->b;
+        } else {
+            const RecC q = rcc[k];
+            r.rc = q.rc; r.frac = q.frac; r.v = q.c;
+        }
+        return r;
+    };
+    // The lanes of a warp start at different columns and halves of a value, so
+    // that their adds spread over the banks.
+    const int sw = (tid >> 2) & 1;
+    auto spread = [&](const Rec &r) {
+        // one wrap decision per record: with G2 >= 2 m + B the columns agree
+        // wherever a tap is inside the window
+        int row = r.rc >> 16, x = c0 - (r.rc & 0xFFFF);
+        if (x + B - 1 < 1 - m) { x += G2; row += 1; }
+        else if (x > m) { x -= G2; row -= 1; }
+        if (x + B - 1 < 1 - m || x > m) return;
+        if (row < 0) row += L1;
+        else if (row >= L1) row -= L1;
+        float *t = reinterpret_cast<float *>(sm + (row + row / N1) * B);
+        const float va = sw ? r.v.y : r.v.x, vb = sw ? r.v.x : r.v.y;
+#pragma unroll
+        for (int k = 0; k < B; ++k) {
+            const int cc = (k + tid) & (B - 1), d = x + cc;
+            if (d < 1 - m || d > m) continue;
+            const float wg = win_tap((float)d - r.frac, p);
+            atomicAdd(t + 2 * cc + sw, va * wg);
+            atomicAdd(t + 2 * cc + (sw ^ 1), vb * wg);
+        }
+    };
+    constexpr int U = 2;  // records in flight per thread
+    Rec nx[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+        if (tid + u * NT < ntot) nx[u] = load(tid + u * NT);
+    __syncthreads();  // the tile is cleared
+    for (int k0 = tid; k0 < ntot; k0 += U * NT) {
+        Rec r[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            r[u] = nx[u];
+            const int k = k0 + (u + U) * NT;
+            if (k < ntot) nx[u] = load(k);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (k0 + u * NT < ntot) spread(r[u]);
+    }
+    __syncthreads();
+    const int c = tid & (B - 1);
+    // level 1: unit (i, c), planes of N1 + 1 slots
+    const float2 *w1 = p.st1 + stage_tw_offset(L1, 2), *w2 = p.st1 + stage_tw_offset(L1, 1);
+#pragma unroll 1
+    for (int u = tid; u < N1 * B; u += NT) {
+        const int i = u / B;
+        float2 *e = sm + i * B + c, x[F0];
+#pragma unroll
+        for (int k = 0; k < F0; ++k) x[k] = e[k * (N1 + 1) * B];
+        RegDFT<F0>::run(x);
+        e[0] = x[0];
+#pragma unroll
+        for (int q = 1; q < F0; ++q) e[q * (N1 + 1) * B] = cmul(x[q], __ldg(w1 + (q - 1) * N1 + i));
+    }
+    __syncthreads();
+    {  // level 2: unit (q0, j, c), one per thread
+        const int j = tid / B % F2, q0 = tid / (B * F2);
+        float2 *e = sm + (q0 * (N1 + 1) + j) * B + c, x[F1];
+#pragma unroll
+        for (int k = 0; k < F1; ++k) x[k] = e[k * F2 * B];
+        RegDFT<F1>::run(x);
+        e[0] = x[0];
+#pragma unroll
+        for (int q = 1; q < F1; ++q) e[q * F2 * B] = cmul(x[q], __ldg(w2 + (q - 1) * F2 + j));
+    }
+    __syncthreads();
+    // level 3: unit (q1, q0, c): outputs v + F0 F1 q2, v = q0 + F0 q1
+    const long long blk = (long long)cb * L1 * B;
+    float2 *dst = inter + cv.inter_off + g * p.G + blk;
+    const float2 *itw = p.itw + blk;
+#pragma unroll 1
+    for (int u = tid; u < F0 * F1 * B; u += NT) {
+        const int v = u / B, q0 = v % F0, q1 = v / F0;
+        const float2 *e = sm + (q0 * (N1 + 1) + q1 * F2) * B + c;
+        float2 x[F2];
+#pragma unroll
+        for (int j = 0; j < F2; ++j) x[j] = e[j * B];
+        RegDFT<F2>::run(x);
+#pragma unroll
+        for (int q = 0; q < F2; ++q)
+            dst[u + q * F0 * F1 * B] = cmul(x[q], __ldg(itw + u + q * F0 * F1 * B));
+    }
 }
 
 template <int NG, int L2, int R, int NT, int LDS, int B>
@@ -665,6 +793,143 @@ k_pass2_gls(const DevCurve *cvs, const float2 *inter, float *__restrict__ out, P
     }
 }
 
+// Pass 2 of the GLS for rows of 4,096: one row of one curve per CTA of 256
+// threads.  Each grid's row is transformed in three levels of 16 with every
+// butterfly in registers: n = i + 256 k, i = j + 16 k', output
+// q2 = q0 + 16 q1 + 256 qb.
+//   level 1  thread i reads its 16 elements straight from the intermediate
+//            and leaves [q0][i] in the exchange tile;
+//   level 2  thread (q0, j), in place;
+//   level 3  thread (q1, q0) holds the outputs q0 + 16 q1 + 256 qb.
+// The outputs stay in registers (grid A's parked in shared memory and read
+// back by the same thread), so the powers need no further pass.  The planes'
+// pitch of 257 keeps all accesses free of bank conflicts.  3 x 2048 rows of
+// three grids: 0.631 -> 0.350 ms (0.406 with two columns per pass-1 block, 0.465
+// with 80 registers and three CTAs per SM); 604 MB read, 0.09 ms at the
+// measured copy rate: it is held by latency (two CTAs per SM) and by the L1
+// pipe (56 %: a row is 1,024 pieces of 32 bytes, its powers 4-byte stores).
+template <bool ES>
+__global__ void __launch_bounds__(256, 2)
+k_pass2_gls_cube(const DevCurve *cvs, const float2 *inter, float *__restrict__ out, const Plan p,
+                 const GlsParams gp) {
+    constexpr int L2 = 4096, P = kCubePitch;
+    extern __shared__ __align__(16) float2 sm[];
+    float2 *ex = sm, *park = sm + 16 * P;
+    const int tid = threadIdx.x, q1r = blockIdx.x;
+    if (p.dependent) {
+        pdl_trigger();
+        pdl_wait();
+    }
+    inter = written(inter);
+    const DevCurve cv = written(cvs)[blockIdx.y];
+    const int G1 = p.G1, G = (int)p.G, B = p.B;
+    const int lo = tid & 15, hi = tid >> 4;
+    // element l = tid + 256 k of the row lies at ((l / B) G1 + row) B + l % B
+    const float2 *src = inter + cv.inter_off + ((long long)(tid / B) * G1 + q1r) * B + tid % B;
+    const int kstride = 256 * G1;
+    const float2 *w1 = p.st2 + 240 + tid, *w2 = p.st2 + lo;  // Stockham tables of 4096
+    float2 y[16], yb[16], x[16];
+    // (volatile: the loads stay ahead of the levels they are to overlap)
+    auto fetch = [](const float2 *q) {
+        float2 v;
+        asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(q) : "memory");
+        return v;
+    };
+#pragma unroll
+    for (int k = 0; k < 16; ++k) x[k] = fetch(src + k * kstride);
+#pragma unroll
+    for (int g = 0; g < 3; ++g) {
+        RegDFT<16>::run(x);
+        if (g) __syncthreads();  // the grid before is read
+        ex[tid] = x[0];
+#pragma unroll
+        for (int q = 1; q < 16; ++q) ex[q * P + tid] = cmul(x[q], __ldg(w1 + (q - 1) * 256));
+        if (g < 2) {  // the next grid's row, in flight during levels 2 and 3
+            src += p.G;
+#pragma unroll
+            for (int k = 0; k < 16; ++k) x[k] = fetch(src + k * kstride);
+        }
+        __syncthreads();
+        float2 *e = ex + hi * P + lo;  // (q0, j) = (hi, lo)
+#pragma unroll
+        for (int k = 0; k < 16; ++k) y[k] = e[16 * k];
+        RegDFT<16>::run(y);
+        e[0] = y[0];
+#pragma unroll
+        for (int q = 1; q < 16; ++q) e[16 * q] = cmul(y[q], __ldg(w2 + (q - 1) * 16));
+        __syncthreads();
+        e = ex + lo * P + 16 * hi;  // (q0, q1) = (lo, hi)
+#pragma unroll
+        for (int j = 0; j < 16; ++j) y[j] = e[j];
+        RegDFT<16>::run(y);
+        if (g == 0) {
+#pragma unroll
+            for (int q = 0; q < 16; ++q) park[q * 256 + tid] = y[q];
+        } else if (g == 1) {
+#pragma unroll
+            for (int q = 0; q < 16; ++q) yb[q] = y[q];
+        }
+    }
+    const int nf = cv.nf, h = nf / 2, lo_end = nf - h, hi_start = G - h;
+    const bool write = gp.best == nullptr || out != nullptr;
+    float *o = out + cv.out_off + h;
+    const int q0 = q1r + G1 * tid;
+    const float *drow = ES ? p.drow + (long long)q1r * L2 + tid : nullptr;
+    const Fm2 fm(cv, gp.reg);
+    unsigned long long key = 0;
+    const unsigned ibase = (unsigned)(cv.best_off + h);
+    auto emit = [&](float P, int k) {
+        if (write) o[k] = P;
+        if (gp.best != nullptr && P >= 0.f) {  // valid powers only
+            const unsigned long long kk = ((unsigned long long)__float_as_uint(P) << 32) |
+                                          (0xFFFFFFFFu - (ibase + (unsigned)k));
+            key = kk > key ? kk : key;
+        }
+    };
+    // two frequencies at a time; f(qb, ka, kb, ina, inb, A0, A1, D)
+    auto pairs = [&](auto f) {
+#pragma unroll
+        for (int qb = 0; qb < 16; qb += 2) {
+            // (no band reaches the middle fifth of the grid: sigma >= 1.25)
+            if (5 * qb >= 2 * 16 && 5 * (qb + 2) <= 3 * 16) continue;
+            const int qA = q0 + G1 * 256 * qb, qB = qA + G1 * 256;
+            const bool ina = qA < lo_end || qA >= hi_start;
+            const bool inb = qB < lo_end || qB >= hi_start;
+            if (!ina && !inb) continue;
+            const float2 A0 = park[qb * 256 + tid], A1 = park[(qb + 1) * 256 + tid];
+            const int ka = qA < lo_end ? qA : qA - G, kb = qB < lo_end ? qB : qB - G;
+            float2 D;
+            if constexpr (ES) D = make_float2(__ldg(drow + 256 * qb), __ldg(drow + 256 * (qb + 1)));
+            else D = make_float2(win_deconv<false>(ka, p), win_deconv<false>(kb, p));
+            f(qb, ka, kb, ina, inb, A0, A1, D);
+        }
+    };
+    if (gp.mode == 1) {
+        pairs([&](int qb, int ka, int kb, bool ina, bool inb, float2 A0, float2 A1, float2 D) {
+            const float2 pw = fm.power(A0, A1, yb[qb], yb[qb + 1], y[qb], y[qb + 1], D);
+            if (ina) emit(pw.x, ka);
+            if (inb) emit(pw.y, kb);
+        });
+    } else {
+        auto one = [&](float2 A, float2 Bv, float2 C, float d) {
+            return gls_from_sums<float>(A.x * d, A.y * d, Bv.x * d, Bv.y * d, C.x * d, C.y * d,
+                                        gp.mode, gp.reg, cv.w_sum, cv.yw_sum, cv.ybar, cv.yy_inv);
+        };
+        pairs([&](int qb, int ka, int kb, bool ina, bool inb, float2 A0, float2 A1, float2 D) {
+            if (ina) emit(one(A0, yb[qb], y[qb], D.x), ka);
+            if (inb) emit(one(A1, yb[qb + 1], y[qb + 1], D.y), kb);
+        });
+    }
+    if (gp.best != nullptr) {
+#pragma unroll
+        for (int of = 16; of > 0; of >>= 1) {
+            const unsigned long long v = __shfl_xor_sync(0xffffffffu, key, of);
+            key = v > key ? v : key;
+        }
+        if ((tid & 31) == 0 && key != 0) atomicMax(gp.best + cv.best_slot, key);
+    }
+}
+
 // Adjoint-NFFT finish of a pass-2 tile: deconvolution and the phase of the
 // absolute time origin, complex output per in-band frequency.
 template <bool ES, int L2, int R, int NT, int LDS>
@@ -732,10 +997,16 @@ cudaError_t launch_pass1_t(const DevCurve *cv, int n_curves, const RecAB *recAB,
                            float2 *inter, const Plan &p, cudaStream_t s) {
     static size_t done[64] = {0};  // per instantiation
     const size_t smem = (size_t)pass1_smem(NG, L1, p.G);
-    dim3 grid(p.G2 / pass1_cols(NG, L1), n_curves);
+    constexpr int per = pass1_long(NG, L1) ? 3 : 1;  // CTAs per column block
+    dim3 grid(p.G2 / pass1_cols(NG, L1) * per, n_curves);
     Plan q = p;
     q.dependent = small_launch((long long)grid.x * grid.y);
-    if constexpr (pass1_small_stage(NG, L1)) {
+    if constexpr (pass1_long(NG, L1)) {
+        cudaError_t e = allow_smem(k_pass1_long<L1>, smem, done);
+        if (e != cudaSuccess) return e;
+        return launch_pdl(k_pass1_long<L1>, q.dependent, grid, pass1_threads(NG, L1), smem, s, cv,
+                          recAB, recC, binsAB, binsC, inter, q);
+    } else if constexpr (pass1_small_stage(NG, L1)) {
         cudaError_t e = allow_smem(k_pass1_occ<NG, L1>, smem, done);
         if (e != cudaSuccess) return e;
         return launch_pdl(k_pass1_occ<NG, L1>, q.dependent, grid, pass1_threads(NG, L1), smem, s, cv, recAB,
@@ -754,6 +1025,18 @@ cudaError_t launch_pass2_gls_t(const DevCurve *cv, int n_curves, int first, cons
     if constexpr (pass2_reg(3, L2)) {
         return p.win == kWinES ? launch_pass2_reg_t<L2, true>(cv, n_curves, first, inter, out, p, g, s)
                                : launch_pass2_reg_t<L2, false>(cv, n_curves, first, inter, out, p, g, s);
+    } else if constexpr (pass2_cube(3, L2)) {
+        static size_t done[2][64] = {{0}};  // per window and device
+        const bool es = p.win == kWinES;
+        const size_t smem = (size_t)pass2_smem(3, L2);
+        cudaError_t e = es ? allow_smem(k_pass2_gls_cube<true>, smem, done[1])
+                           : allow_smem(k_pass2_gls_cube<false>, smem, done[0]);
+        if (e != cudaSuccess) return e;
+        const dim3 grid(p.G1, n_curves);
+        Plan q = p;
+        q.dependent = small_launch((long long)grid.x * grid.y);
+        return es ? launch_pdl(k_pass2_gls_cube<true>, q.dependent, grid, 256, smem, s, cv, inter, out, q, g)
+                  : launch_pdl(k_pass2_gls_cube<false>, q.dependent, grid, 256, smem, s, cv, inter, out, q, g);
     } else {
         static size_t done[64] = {0};  // per instantiation
         cudaError_t e = allow_smem(k_pass2_gls<L2>, (size_t)pass2_smem(3, L2), done);
@@ -792,7 +1075,8 @@ cudaError_t launch_pass2_nfft_t(const DevCurve *cv, int n_curves, int first, con
 template <int NG, int L1>
 cudaError_t preload_pass1_t() {
     cudaFuncAttributes a;
-    if constexpr (pass1_small_stage(NG, L1)) return cudaFuncGetAttributes(&a, k_pass1_occ<NG, L1>);
+    if constexpr (pass1_long(NG, L1)) return cudaFuncGetAttributes(&a, k_pass1_long<L1>);
+    else if constexpr (pass1_small_stage(NG, L1)) return cudaFuncGetAttributes(&a, k_pass1_occ<NG, L1>);
     else return cudaFuncGetAttributes(&a, k_pass1<NG, L1>);
 }
 template <int L2>
@@ -805,6 +1089,10 @@ cudaError_t preload_pass2_t(int ng) {
         }
         const cudaError_t e = cudaFuncGetAttributes(&a, k_pass2_gls_reg<L2, true>);
         return e != cudaSuccess ? e : cudaFuncGetAttributes(&a, k_pass2_gls_reg<L2, false>);
+    } else if constexpr (pass2_cube(3, L2)) {
+        if (ng != 3) return cudaFuncGetAttributes(&a, k_pass2_nfft<L2>);
+        const cudaError_t e = cudaFuncGetAttributes(&a, k_pass2_gls_cube<true>);
+        return e != cudaSuccess ? e : cudaFuncGetAttributes(&a, k_pass2_gls_cube<false>);
     } else {
         return ng == 3 ? cudaFuncGetAttributes(&a, k_pass2_gls<L2>)
                        : cudaFuncGetAttributes(&a, k_pass2_nfft<L2>);

@@ -65,10 +65,11 @@ struct FacList {
 };
 
 // Radix sequence of L = 2^a 5^c: the radix-5 stages first, then 16s, then
-// the remaining power of two (2, 4, 8 or 16).
+// the remaining power of two (2, 4, 8 or 16); 1600 is 20 x 20 x 4.
 CUVGLS_HD constexpr FacList fft_factors(int L) {
     FacList f{0, {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0}};
     int x = L;
+    if (x == 1600) { f.r[f.n++] = 20; f.r[f.n++] = 20; x = 4; }
     while (x % 5 == 0) { f.r[f.n++] = 5; x /= 5; }
     while (x % 3 == 0) { f.r[f.n++] = 3; x /= 3; }
     while (x % 16 == 0 && x > 16) { f.r[f.n++] = 16; x /= 16; }
@@ -81,7 +82,7 @@ CUVGLS_HD constexpr bool len_ok(int L) {
     int p = 1;
     for (int i = 0; i < f.n; ++i) {
         int r = f.r[i];
-        if (r != 2 && r != 3 && r != 4 && r != 5 && r != 8 && r != 16) return false;
+        if (r != 2 && r != 3 && r != 4 && r != 5 && r != 8 && r != 16 && r != 20) return false;
         p *= r;
     }
     return p == L;
@@ -183,8 +184,16 @@ CUVGLS_HD constexpr bool tile_fits(int V, int L) {
     return two_level_la(L) ? V * two_level_la(L) <= kMaxThreads : V * L <= kMaxTile;
 }
 
+// Whether the columns of this length go through k_pass1_long (the three grids
+// of a column block in CTAs of their own): those without a two-level split,
+// in three levels F0, F1, F2, the Stockham radices in reverse.
+CUVGLS_HD constexpr bool pass1_long(int ng, int L1) { return ng == 3 && two_level_la(L1) == 0; }
+CUVGLS_HD constexpr int long_fac(int L1, int level) { return fft_factors(L1).r[2 - level]; }
+constexpr int kLongCols = 4;
+
 // Columns per pass-1 CTA for ng grids of column length L1.
 CUVGLS_HD constexpr int pass1_cols(int ng, int L1) {
+    if (pass1_long(ng, L1)) return kLongCols;
     int b = (ng == 1) ? 8 : 4;
     while (b > 2 && !tile_fits(ng * b, L1)) b /= 2;
     return b;
@@ -196,6 +205,11 @@ CUVGLS_HD constexpr int pass1_cols(int ng, int L1) {
 CUVGLS_HD constexpr bool pass2_reg(int ng, int L2) {
     return two_level_la(L2) > 0 && L2 / two_level_la(L2) <= 20;
 }
+
+// Whether the GLS rows of this length go through k_pass2_gls_cube: three
+// levels of 16, one row of one curve per CTA.
+CUVGLS_HD constexpr bool pass2_cube(int ng, int L2) { return ng == 3 && L2 == 4096; }
+constexpr int kCubePitch = 257;   // of its exchange tile: 16 planes of 256 elements
 
 // Rows per pass-2 CTA for ng grids of row length L2: 16 for short rows, so
 // that a CTA still transforms a few thousand elements; 8 for the other
@@ -211,6 +225,8 @@ CUVGLS_HD constexpr int pass2_rows(int ng, int L2) {
 }
 
 CUVGLS_HD constexpr int pass1_threads(int ng, int L1) {
+    // (one thread per level-2 butterfly)
+    if (pass1_long(ng, L1)) return kLongCols * L1 / long_fac(L1, 1);
     return fft_threads(ng * pass1_cols(ng, L1), L1);
 }
 // k_pass2_gls_reg: a thread per stage-B unit; row pitch of the exchange tile
@@ -271,7 +287,7 @@ CUVGLS_HD constexpr long long pass1_tile_bytes(int ng, int L1) {
 }
 
 // Records a pass-1 CTA stages per round: 256, or, for the 1024-thread CTAs
-// of the long Stockham columns (one CTA per SM), as many as fit (in steps of
+// of the long Stockham columns of one grid (one CTA per SM), as many as fit (in steps of
 // 256, up to 4096) beside the row counts and the row-sorted record list of
 // the gather spreading, so that a dense curve (tens of thousands of records
 // per column block) takes a few rounds rather than one barrier pair per 256
@@ -329,6 +345,8 @@ CUVGLS_HD constexpr int pass1_stage_recs(int ng, int L1) {
 }
 
 CUVGLS_HD constexpr long long pass1_smem(int ng, int L1, long long G) {
+    // (one slot of padding per level-1 plane)
+    if (pass1_long(ng, L1)) return (long long)kLongCols * (L1 + long_fac(L1, 0)) * 8;
     return pass1_tile_bytes(ng, L1) + (long long)pass1_stage_recs(ng, L1) * kStageRecBytes +
            (pass1_gather(ng, L1) ? pass1_gather_bytes(L1, pass1_stage_recs(ng, L1)) : 0) +
            kOccBytes;
@@ -338,6 +356,7 @@ CUVGLS_HD constexpr long long pass1_smem(int ng, int L1, long long G) {
 CUVGLS_HD constexpr long long pass2_smem(int ng, int L2) {
     if (pass2_reg(ng, L2))
         return ((ng == 3 ? pass2_reg_elems(L2) : nfft_reg_elems(L2)) + 2LL) * 8;
+    if (pass2_cube(ng, L2)) return (16LL * kCubePitch + L2) * 8;  // exchange tile, grid A
     return (long long)(ng * pass2_rows(ng, L2) * row_stride(L2) +
                        (two_level_la(L2) ? 0 : fft_table_len(L2))) * 8;
 }
