@@ -1054,8 +1054,10 @@ int run_batch(cuvgls_handle *h, const Work &wk, std::vector<DevCurve> &cvs,
                 ++pi;
             }
             const DevCurve *dcv = d_cv + ch.first;
+            int max_n = 0;
+            for (int k = 0; k < ch.count; ++k) max_n = std::max(max_n, h->h_cv[ch.first + k].n);
             LAUNCH(CUVGLS_STAGE_PASS1, gs,
-                   launch_pass1(dcv, ch.count, pa.recAB, pa.recC, pa.binsAB, pa.binsC, inter, p,
+                   launch_pass1(dcv, ch.count, max_n, pa.recAB, pa.recC, pa.binsAB, pa.binsC, inter, p,
                                 wk.ng, gs),
                    "k_pass1");
             // With host output, pass 2 runs in four launches over consecutive
@@ -1135,7 +1137,7 @@ int run_batch(cuvgls_handle *h, const Work &wk, std::vector<DevCurve> &cvs,
             int n = 0;
             for (int k = 0; k < g.count; ++k) n = std::max(n, h->h_cv[g.first + k].n);
             cost[gi] = 10.0 + 1.4e-5 * (double)g.count * (double)g.cls->plan.G +
-                       0.075 * n / g.cls->plan.nb;
+                       0.03 * n / g.cls->plan.nb;
         }
         std::stable_sort(by.begin(), by.end(),
                          [&](size_t x, size_t y) { return cost[x] > cost[y]; });

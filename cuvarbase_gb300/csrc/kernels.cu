@@ -301,13 +301,13 @@ cudaError_t launch_es_deconv(float *dst, long long G, int m, double beta, cudaSt
     X(400) X(512) X(640) X(800) X(1024) X(1280) X(1600) X(2048)
 #define CUVGLS_ROW_LEN_CASES(X) CUVGLS_LEN_CASES(X) X(4096)
 
-cudaError_t launch_pass1(const DevCurve *cv, int n_curves, const RecAB *recAB,
+cudaError_t launch_pass1(const DevCurve *cv, int n_curves, int max_n, const RecAB *recAB,
                          const RecC *recC, const int *binsAB, const int *binsC,
                          float2 *inter, const Plan &p, int ngrids, cudaStream_t s) {
     if (n_curves <= 0) return cudaSuccess;
 #define CUVGLS_P1(L) \
-    case L: return ngrids == 3 ? launch_pass1_t<3, L>(cv, n_curves, recAB, recC, binsAB, binsC, inter, p, s) \
-                               : launch_pass1_t<1, L>(cv, n_curves, recAB, recC, binsAB, binsC, inter, p, s);
+    case L: return ngrids == 3 ? launch_pass1_t<3, L>(cv, n_curves, max_n, recAB, recC, binsAB, binsC, inter, p, s) \
+                               : launch_pass1_t<1, L>(cv, n_curves, max_n, recAB, recC, binsAB, binsC, inter, p, s);
     switch (p.G1) {
         CUVGLS_LEN_CASES(CUVGLS_P1)
         default: return cudaErrorInvalidValue;

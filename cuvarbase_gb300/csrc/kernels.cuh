@@ -63,7 +63,8 @@ cudaError_t launch_seg_fill(const DevCurve *cv, int n, SegEntry *segs, cudaStrea
 
 // Dispatch on (G1, G2) to the compiled length templates; cudaErrorInvalidValue
 // if a length has no kernel.
-cudaError_t launch_pass1(const DevCurve *cv, int n_curves, const RecAB *recAB,
+// (`max_n`: points of the longest of the curves)
+cudaError_t launch_pass1(const DevCurve *cv, int n_curves, int max_n, const RecAB *recAB,
                          const RecC *recC, const int *binsAB, const int *binsC,
                          float2 *inter, const Plan &p, int ngrids, cudaStream_t s);
 
@@ -77,7 +78,7 @@ cudaError_t launch_pass2_nfft(const DevCurve *cv, int n_curves, int first, const
 
 // Length templates (pass_kernels.cuh, instantiated in inst_*.cu).
 template <int NG, int L1>
-cudaError_t launch_pass1_t(const DevCurve *, int, const RecAB *, const RecC *,
+cudaError_t launch_pass1_t(const DevCurve *, int, int, const RecAB *, const RecC *,
                            const int *, const int *, float2 *, const Plan &, cudaStream_t);
 template <int L2>
 cudaError_t launch_pass2_gls_t(const DevCurve *, int, int, const float2 *, float *,

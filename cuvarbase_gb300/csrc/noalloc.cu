@@ -232,7 +232,7 @@ extern "C" int cuvgls_gls_noalloc(double sigma, int32_t m, const cuvgls_gls_inpu
             e = launch_bin_long(pa, segs, (int)n_seg, nullptr, nc, 3, 0, s);
     }
     if (e == cudaSuccess)
-        e = launch_pass1(d_cv, nc, recAB, recC, binsAB, binsC, inter, p, 3, s);
+        e = launch_pass1(d_cv, nc, max_n, recAB, recC, binsAB, binsC, inter, p, 3, s);
     if (e == cudaSuccess)
         e = launch_pass2_gls(d_cv, nc, 0, inter, p_out, p,
                              GlsParams{b->mode, b->reg[0], nullptr, d_flag}, s);

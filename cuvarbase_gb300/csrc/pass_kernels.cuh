@@ -19,6 +19,7 @@
 #pragma once
 
 #include <climits>
+#include <type_traits>
 #include <cuda_runtime.h>
 
 #include "fft.cuh"
@@ -113,7 +114,7 @@ static_assert(sizeof(StagedRec) == kStageRecBytes, "staged record size");
 
 // One pass-1 CTA: column block blockIdx.x of curve blockIdx.y (the body of
 // both pass-1 kernels below).
-template <int NG, int L1>
+template <int NG, int L1, bool MANY>
 __device__ __forceinline__ void pass1_body(const DevCurve *cvs, const RecAB *recAB,
                                            const RecC *recC, const int *binsAB, const int *binsC,
                                            float2 *inter, const Plan &p) {
@@ -183,7 +184,7 @@ __device__ __forceinline__ void pass1_body(const DevCurve *cvs, const RecAB *rec
     int *rowcnt = reinterpret_cast<int *>(st + NSR);  // L1 + 1 (gather tiles)
     int *bucket = rowcnt + L1 + 1;                      // NSR
     int *wsum = bucket + NSR;                           // 32
-    const bool dense = GATHER && ntot >= L1;
+    const bool dense = GATHER ? ntot >= L1 : MANY && ntot >= 2 * NT;
     // Two-level column FFTs: occ[kind * 32 + i] is set when a tap of that
     // record kind (0: A and B, 1: C) lands in a row congruent to i modulo
     // LB, so stage A can skip the all-zero units; the dense path does not
@@ -193,7 +194,7 @@ __device__ __forceinline__ void pass1_body(const DevCurve *cvs, const RecAB *rec
     unsigned char *occ = reinterpret_cast<unsigned char *>(st + NSR) +
                          (GATHER ? pass1_gather_bytes(L1, NSR) : 0);  // kOccBytes
     if (LA1 && tid < kOccBytes) occ[tid] = 0;  // before the first round's barrier
-    if (dense) {  // uniform over the CTA
+    if (GATHER && dense) {  // uniform over the CTA
         for (int i = tid; i <= L1; i += NT) rowcnt[i] = 0;
         __syncthreads();  // counts zeroed before the first round's atomics
     }
@@ -212,7 +213,56 @@ __device__ __forceinline__ void pass1_body(const DevCurve *cvs, const RecAB *rec
         }
         return r;
     };
-    for (int base = 0;; base += NSR) {
+    // Blocks of many records otherwise: one thread per record, the next one in
+    // flight, its columns one after the other (no rounds, no barriers; the lanes
+    // start at different columns and halves of a value, so that their adds
+    // spread over the banks).
+    if (MANY && dense) {
+        __syncthreads();  // the tile is cleared
+        const int sw = (tid >> 2) & 1;
+        // adds the taps of a record's grids 0 .. n - 1 (values v[g], tiles GS apart)
+        auto spread = [&](float2 *t0, int rc, float frac, const float2 *v, auto n) {
+            int row = rc >> 16, x = c0 - (rc & 0xFFFF);
+            if (x + B - 1 < 1 - m) { x += G2; row += 1; }
+            else if (x > m) { x -= G2; row -= 1; }
+            if (x + B - 1 < 1 - m || x > m) return;
+            if (row < 0) row += L1;
+            else if (row >= L1) row -= L1;
+            float *t = reinterpret_cast<float *>(t0 + phys2<L1>(row) * B);
+#pragma unroll
+            for (int k = 0; k < B; ++k) {
+                const int cc = (k + tid) & (B - 1), d = x + cc;
+                if (d < 1 - m || d > m) continue;
+                const float wg = win_tap((float)d - frac, p);
+#pragma unroll
+                for (int g = 0; g < n; ++g) {
+                    const float va = sw ? v[g].y : v[g].x, vb = sw ? v[g].x : v[g].y;
+                    atomicAdd(t + 2 * (g * GS + cc) + sw, va * wg);
+                    atomicAdd(t + 2 * (g * GS + cc) + (sw ^ 1), vb * wg);
+                }
+            }
+        };
+        auto at = [](int k, int s0, int s1, int r0) { return k < s1 - s0 ? s0 + k : r0 + (k - (s1 - s0)); };
+        if (tid < nab) {
+            RecAB nx = rab[at(tid, a0, a1, b0)];
+            for (int k = tid; k < nab; k += NT) {
+                const RecAB r = nx;
+                if (k + NT < nab) nx = rab[at(k + NT, a0, a1, b0)];
+                const float2 v[2] = {r.a, r.b};
+                spread(tile, r.rc, r.frac, v, std::integral_constant<int, NG == 3 ? 2 : 1>());
+            }
+        }
+        if (NG == 3 && tid < nc) {
+            RecC nx = rcc[at(tid, e0, e1, f0)];
+            for (int k = tid; k < nc; k += NT) {
+                const RecC r = nx;
+                if (k + NT < nc) nx = rcc[at(k + NT, e0, e1, f0)];
+                spread(tile + 2 * GS, r.rc, r.frac, &r.c, std::integral_constant<int, 1>());
+            }
+        }
+        __syncthreads();
+    }
+    for (int base = 0; !MANY || !dense; base += NSR) {
         const int cnt = min(NSR, ntot - base);
         if (GATHER && dense) {
             constexpr int RPT = (NSR + NT - 1) / NT;
@@ -363,22 +413,22 @@ __device__ __forceinline__ void pass1_body(const DevCurve *cvs, const RecAB *rec
 }
 
 // Pass 1 with the compiler's own register choice ...
-template <int NG, int L1>
+template <int NG, int L1, bool MANY>
 __global__ void __launch_bounds__(pass1_threads(NG, L1))
 k_pass1(const DevCurve *cvs, const RecAB *recAB, const RecC *recC, const int *binsAB,
         const int *binsC, float2 *inter, Plan p) {
-    pass1_body<NG, L1>(cvs, recAB, recC, binsAB, binsC, inter, p);
+    pass1_body<NG, L1, MANY>(cvs, recAB, recC, binsAB, binsC, inter, p);
 }
 
 // ... and, for the tiles whose smaller staging fits one more CTA per SM
 // (pass1_small_stage), bound to that many CTAs per SM.  A minimum of one CTA
 // per SM is not the same as no bound: it lets the compiler spend up to 255
 // registers (pass 1 of rows of 400: 60 -> 110 registers, half the CTAs).
-template <int NG, int L1>
+template <int NG, int L1, bool MANY>
 __global__ void __launch_bounds__(pass1_threads(NG, L1), pass1_min_ctas(NG, L1))
 k_pass1_occ(const DevCurve *cvs, const RecAB *recAB, const RecC *recC, const int *binsAB,
             const int *binsC, float2 *inter, Plan p) {
-    pass1_body<NG, L1>(cvs, recAB, recC, binsAB, binsC, inter, p);
+    pass1_body<NG, L1, MANY>(cvs, recAB, recC, binsAB, binsC, inter, p);
 }
 
 // Pass 1 of the GLS for the long columns (1,280 to 2,048): one CTA per curve,
@@ -991,31 +1041,52 @@ static cudaError_t allow_smem(K kernel, size_t bytes, size_t (&done)[64]) {
     return e;
 }
 
+// Whether a launch takes the kernel that also spreads by records: it is
+// compiled apart, because the registers of that path cost the others 2 % to
+// 3 % (2,000 curves of 320 x 400 cells 1746 -> 1787 us).  It pays from a few
+// rounds per thread on: 16 curves of 50 to 5,000 points on 160 x 160 cells
+// 57 -> 43 us, 48 curves of 100 to 20,000 points 455 -> 379 us.
 template <int NG, int L1>
-cudaError_t launch_pass1_t(const DevCurve *cv, int n_curves, const RecAB *recAB,
-                           const RecC *recC, const int *binsAB, const int *binsC,
-                           float2 *inter, const Plan &p, cudaStream_t s) {
-    static size_t done[64] = {0};  // per instantiation
+bool pass1_many(int max_n, const Plan &p) {
+    constexpr int B = pass1_cols(NG, L1);
+    const int bins = (B + p.m - 2) / B + (p.m + B - 1) / B + 1;
+    const long long recs = (long long)max_n * (NG == 3 ? 2 : 1) * bins * B / p.G2;
+    return recs >= 4LL * pass1_threads(NG, L1);
+}
+
+template <int NG, int L1, typename K>
+cudaError_t launch_pass1_k(K kernel, size_t (&done)[64], int n_curves, const Plan &p, int per,
+                           cudaStream_t s, const DevCurve *cv, const RecAB *recAB, const RecC *recC,
+                           const int *binsAB, const int *binsC, float2 *inter) {
     const size_t smem = (size_t)pass1_smem(NG, L1, p.G);
-    constexpr int per = pass1_long(NG, L1) ? 3 : 1;  // CTAs per column block
-    dim3 grid(p.G2 / pass1_cols(NG, L1) * per, n_curves);
+    const cudaError_t e = allow_smem(kernel, smem, done);
+    if (e != cudaSuccess) return e;
+    const dim3 grid(p.G2 / pass1_cols(NG, L1) * per, n_curves);
     Plan q = p;
     q.dependent = small_launch((long long)grid.x * grid.y);
+    return launch_pdl(kernel, q.dependent, grid, pass1_threads(NG, L1), smem, s, cv, recAB, recC,
+                      binsAB, binsC, inter, q);
+}
+
+template <int NG, int L1>
+cudaError_t launch_pass1_t(const DevCurve *cv, int n_curves, int max_n, const RecAB *recAB,
+                           const RecC *recC, const int *binsAB, const int *binsC,
+                           float2 *inter, const Plan &p, cudaStream_t s) {
+    static size_t done[2][64] = {{0}};  // per instantiation
+    auto go = [&](auto kernel, int k) {
+        return launch_pass1_k<NG, L1>(kernel, done[k], n_curves, p, pass1_long(NG, L1) ? 3 : 1, s,
+                                      cv, recAB, recC, binsAB, binsC, inter);
+    };
     if constexpr (pass1_long(NG, L1)) {
-        cudaError_t e = allow_smem(k_pass1_long<L1>, smem, done);
-        if (e != cudaSuccess) return e;
-        return launch_pdl(k_pass1_long<L1>, q.dependent, grid, pass1_threads(NG, L1), smem, s, cv,
-                          recAB, recC, binsAB, binsC, inter, q);
+        return go(k_pass1_long<L1>, 0);
     } else if constexpr (pass1_small_stage(NG, L1)) {
-        cudaError_t e = allow_smem(k_pass1_occ<NG, L1>, smem, done);
-        if (e != cudaSuccess) return e;
-        return launch_pdl(k_pass1_occ<NG, L1>, q.dependent, grid, pass1_threads(NG, L1), smem, s, cv, recAB,
-                          recC, binsAB, binsC, inter, q);
+        return pass1_many<NG, L1>(max_n, p) ? go(k_pass1_occ<NG, L1, true>, 1)
+                                            : go(k_pass1_occ<NG, L1, false>, 0);
+    } else if constexpr (pass1_gather(NG, L1)) {
+        return go(k_pass1<NG, L1, false>, 0);
     } else {
-        cudaError_t e = allow_smem(k_pass1<NG, L1>, smem, done);
-        if (e != cudaSuccess) return e;
-        return launch_pdl(k_pass1<NG, L1>, q.dependent, grid, pass1_threads(NG, L1), smem, s, cv, recAB, recC,
-                          binsAB, binsC, inter, q);
+        return pass1_many<NG, L1>(max_n, p) ? go(k_pass1<NG, L1, true>, 1)
+                                            : go(k_pass1<NG, L1, false>, 0);
     }
 }
 
@@ -1075,9 +1146,16 @@ cudaError_t launch_pass2_nfft_t(const DevCurve *cv, int n_curves, int first, con
 template <int NG, int L1>
 cudaError_t preload_pass1_t() {
     cudaFuncAttributes a;
-    if constexpr (pass1_long(NG, L1)) return cudaFuncGetAttributes(&a, k_pass1_long<L1>);
-    else if constexpr (pass1_small_stage(NG, L1)) return cudaFuncGetAttributes(&a, k_pass1_occ<NG, L1>);
-    else return cudaFuncGetAttributes(&a, k_pass1<NG, L1>);
+    if constexpr (pass1_long(NG, L1)) {
+        return cudaFuncGetAttributes(&a, k_pass1_long<L1>);
+    } else if constexpr (pass1_small_stage(NG, L1)) {
+        const cudaError_t e = cudaFuncGetAttributes(&a, k_pass1_occ<NG, L1, false>);
+        return e != cudaSuccess ? e : cudaFuncGetAttributes(&a, k_pass1_occ<NG, L1, true>);
+    } else {
+        const cudaError_t e = cudaFuncGetAttributes(&a, k_pass1<NG, L1, false>);
+        if constexpr (pass1_gather(NG, L1)) return e;
+        else return e != cudaSuccess ? e : cudaFuncGetAttributes(&a, k_pass1<NG, L1, true>);
+    }
 }
 template <int L2>
 cudaError_t preload_pass2_t(int ng) {
@@ -1109,10 +1187,10 @@ cudaError_t preload_pass2_t(int ng) {
     template cudaError_t preload_pass2_t<L>(int);
 
 #define CUVGLS_INSTANTIATE_LEN(L)                                                   \
-    template cudaError_t launch_pass1_t<3, L>(const DevCurve *, int, const RecAB *, \
+    template cudaError_t launch_pass1_t<3, L>(const DevCurve *, int, int, const RecAB *, \
                                               const RecC *, const int *, const int *, \
                                               float2 *, const Plan &, cudaStream_t); \
-    template cudaError_t launch_pass1_t<1, L>(const DevCurve *, int, const RecAB *, \
+    template cudaError_t launch_pass1_t<1, L>(const DevCurve *, int, int, const RecAB *, \
                                               const RecC *, const int *, const int *, \
                                               float2 *, const Plan &, cudaStream_t); \
     template cudaError_t launch_pass2_gls_t<L>(const DevCurve *, int, int, const float2 *, \
