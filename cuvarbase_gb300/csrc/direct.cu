@@ -447,13 +447,16 @@ __host__ __device__ constexpr int mh_smem(int H) {
 // cluster share the points of the same frequencies, and the first adds their
 // sums and solves: 625 CTAs left a fifth of the FP64 pipes idle at the end
 // (4.1 CTAs per SM are 5 rounds).  Per point the
-// phasor from table_turn, its powers n = 2 .. 2H from half-way products (three
-// instructions for an even n), then the sums of
+// phasor from table_turn, its powers n = 2 .. 2H by the recurrence
+// z_n = 2 cos(phi) z_(n-1) - z_(n-2) (two instructions each; its rounding, 6e-16
+// rms at n = 6 and 2.4e-15 at n = 16, is that of the products z_n/2 z_n/2, which
+// took three or four, and far below that of the phase t f), then the sums of
 // cuvarbase/lombscargle.py:337-400 (mhdirect_sums) with the regulariser of
 // :403-447, the 2H x 2H system solved by Gaussian elimination with partial
 // pivoting, and the power of :497-536.  H = 3, 1,000 points, 20,000
-// frequencies, host to host: 4.93 -> 2.24 ms (the kernel 2.17 ms with the FP64
-// pipes 88 % busy: 54 instructions per point and frequency).
+// frequencies, host to host: 4.93 -> 2.24 ms with the table and the clusters
+// (54 FP64 instructions per point and frequency, the pipes 88 % busy), 1.97 ms
+// with the recurrence (48).
 template <int H>
 __global__ void __launch_bounds__(kDirThreads, H <= 4 ? 2 : 1)
 k_mhgls_direct(const double *__restrict__ t, const double *__restrict__ yw,
@@ -490,15 +493,14 @@ k_mhgls_direct(const double *__restrict__ t, const double *__restrict__ yw,
             const double wq = sw[q], yq = sy[q];
             double2 z[NH + 1];
             z[1] = table_turn(st[q] * f, turn);
+            const double hx = z[1].x + z[1].x;
 #pragma unroll
             for (int m = 1; m <= NH; ++m) {
-                if (m > 1 && m % 2 == 0) {
-                    const double2 h = z[m / 2];
-                    const double hx = h.x + h.x;
-                    z[m] = make_double2(fma(hx, h.x, -1.0), hx * h.y);
-                } else if (m > 1) {
-                    z[m] = zmul(z[m / 2], z[m - m / 2]);
-                }
+                if (m == 2)
+                    z[m] = make_double2(fma(hx, z[1].x, -1.0), hx * z[1].y);
+                else if (m > 2)
+                    z[m] = make_double2(fma(hx, z[m - 1].x, -z[m - 2].x),
+                                        fma(hx, z[m - 1].y, -z[m - 2].y));
                 c[m] = fma(wq, z[m].x, c[m]);
                 s[m] = fma(wq, z[m].y, s[m]);
                 if (m <= H) {
