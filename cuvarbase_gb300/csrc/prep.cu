@@ -690,6 +690,11 @@ cudaError_t launch_prep(const PrepArrays &a, const DescParam &d, const int *list
         return prep_kind<kPrepThreads, kPrepPpt, false>(a, d, list, n, 1, kPrepPoints, raw, ngrids,
                                                         fp32_positions, beside, s);
     }
+    if (cls == kPrepShort) {
+        if (max_n > kShortPoints) return cudaErrorInvalidValue;
+        return prep_kind<kShortThreads, kShortPpt, false>(a, d, list, n, 1, kShortPoints, raw,
+                                                          ngrids, fp32_positions, beside, s);
+    }
     if (cls == kPrepWide) {
         int csize = 1;
         while (csize * kWidePoints < max_n) csize *= 2;

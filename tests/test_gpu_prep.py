@@ -73,6 +73,30 @@ def test_several_plans_in_one_call(oracle):
             assert np.abs(P - alone).max() <= 2e-5
 
 
+@pytest.mark.parametrize("raw", [True, False])
+def test_short_curves_of_a_large_batch(oracle, raw):
+    """The class of short curves, which only a batch that fills the chip uses:
+    the edges of its sizes, beside longer curves."""
+    from cuvarbase_gb300 import _lib
+    from test_gpu_rows import _ref
+    sizes = ([1, 2, 63, 64, 65, 127, 383, 384, 385, 1024, 3000] * 70)
+    curves = [_curve(n, 31 * i + n) for i, n in enumerate(sizes)]
+    hh = _lib.Handle(sigma=2.0, m=8)
+    try:
+        nf = 500
+        k = np.arange(50, nf, 3)
+        for mode in (2, 1) if raw else (1,):
+            P = _raw(hh, curves, nf, mode) if raw else _prepared(hh, curves, nf)
+            for i in list(range(11)) + [400, 401, 402, 403, 404, 767, 768, 769]:
+                n = len(curves[i][0])
+                if n < 3 or (mode == 1 and n < 200):
+                    continue      # singular; nearly exact fits: rounding over rounding
+                ref = _ref(oracle, curves[i], k, mode)
+                assert np.abs(P[i][k] - ref).max() <= 2e-5 * max(1.0, np.abs(ref).max())
+    finally:
+        hh.close()
+
+
 @pytest.mark.parametrize("n", [300, 1500, 20000, 40000])
 def test_unsorted_and_far_times(oracle, n):
     """Positions of every sign and many turns: shuffled times, an origin far
