@@ -410,23 +410,35 @@ cudaError_t launch_gls_direct(const DevCurve *cv, int n_curves, int max_nf, int 
 // ---------------------------------------------------------------------------
 namespace {
 
-constexpr int kTurn = 256;  // phasors of the shared turn table
+// Phasors of the shared turn table, from kTurnCoarse by kTurnFine products.
+constexpr int kTurn = 2048, kTurnCoarse = 64, kTurnFine = kTurn / kTurnCoarse;
 
-// exp(2 pi i p) from the phasor at the nearest multiple of 1 / kTurn and the
-// Taylor series of the remaining angle d, |d| <= pi / kTurn: the first terms
-// left out are d^7 / 7! < 9e-18 and d^8 / 8! < 2e-20.  16 FP64 instructions
-// with the product p = t f, against about 28 for floor and sincospi.
+// A float as a double by its bits (zero becomes 2^-127; no FP64 instruction).
+__device__ __forceinline__ double widen(float x) {
+    const int b = __float_as_int(x);
+    return __hiloint2double((b & 0x80000000) | (((b & 0x7fffffff) >> 3) + 0x38000000), b << 29);
+}
+// exp(2 pi i p), NaN when p is not finite: the phasor at the nearest multiple
+// of 1 / kTurn turned by the remaining angle d, |d| <= pi / kTurn.  One SM
+// issues 64 other instructions in the time of an FP64 one, so the fraction of
+// p, the table index and the remainder are integers, and FP32 has what it is
+// exact enough for: d^3 / 6 - d^5 / 120 (6e-10) and d^4 / 24 (2e-13); the terms
+// left out are d^6 / 720 and d^7 / 5040, below 2e-20.  Eight FP64 instructions
+// after p (16 with all of it in FP64, about 28 for floor and sincospi).
 __device__ __forceinline__ double2 table_turn(double p, const double2 *tab) {
-    // from 2^40 turns on the index below would lose bits: reduce first
-    // (the exponent compared as an integer: no FP64 instruction)
-    if ((__double2hiint(p) & 0x7ff00000) >= (1023 + 40) << 20) p -= floor(p);
-    constexpr double kRound = 6755399441055744.0;  // 1.5 2^52: adding it rounds to an integer
-    const double z = fma(p, (double)kTurn, kRound);
-    const double2 e = tab[__double2loint(z) & (kTurn - 1)];
-    const double d = fma(z - kRound, -1.0 / kTurn, p) * 6.283185307179586477;
-    const double d2 = d * d;
-    const double sn = fma(d * d2, fma(d2, 1.0 / 120.0, -1.0 / 6.0), d);
-    const double cm = d2 * fma(d2, fma(d2, -1.0 / 720.0, 1.0 / 24.0), -0.5);  // cos d - 1
+    const u64 th = turns64(p);
+    const int k = (int)((th + (1ULL << 52)) >> 53);  // 0 .. kTurn
+    const double2 e = tab[k & (kTurn - 1)];
+    const long long r = (long long)(th - ((u64)k << 53));  // |r| <= 2^52, in 2^-64 turns
+    // d: r / 4 set into the mantissa of 1.5 2^52, scaled and taken off in one step
+    constexpr double kUnit = 6.283185307179586477 / 4611686018427387904.0;  // 2 pi 2^-62
+    const double d = fma(__longlong_as_double(0x4338000000000000LL + (r >> 2)), kUnit,
+                         -6755399441055744.0 * kUnit);
+    const float df = (float)(int)(r >> 21) * (float)(6.283185307179586477 / 8796093022208.0);
+    const float q = df * df;
+    double w3 = widen(df * q * fmaf(q, 1.f / 120.f, -1.f / 6.f));
+    if ((__double2hiint(p) & 0x7ff00000) == 0x7ff00000) w3 = __longlong_as_double(-1LL);
+    const double sn = d + w3, cm = fma(d * d, -0.5, widen(q * q * (1.f / 24.f)));
     return make_double2(fma(-e.y, sn, fma(e.x, cm, e.x)), fma(e.x, sn, fma(e.y, cm, e.y)));
 }
 
@@ -456,7 +468,8 @@ __host__ __device__ constexpr int mh_smem(int H) {
 // pivoting, and the power of :497-536.  H = 3, 1,000 points, 20,000
 // frequencies, host to host: 4.93 -> 2.24 ms with the table and the clusters
 // (54 FP64 instructions per point and frequency, the pipes 88 % busy), 1.97 ms
-// with the recurrence (48).
+// with the recurrence (48), 1.54 ms with the integer and FP32 parts of the
+// phasor (37).
 template <int H>
 __global__ void __launch_bounds__(kDirThreads, H <= 4 ? 2 : 1)
 k_mhgls_direct(const double *__restrict__ t, const double *__restrict__ yw,
@@ -468,8 +481,16 @@ k_mhgls_direct(const double *__restrict__ t, const double *__restrict__ yw,
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     double2 *turn = reinterpret_cast<double2 *>(sm);
     double *st = sm + 2 * kTurn + wid * 96, *sy = st + 32, *sw = st + 64;
-    for (int i = tid; i < kTurn; i += kDirThreads) turn[i] = zturn((double)i / kTurn);
-    __syncthreads();
+    {  // the coarse and fine steps (in the point tiles' memory), then their products
+        double2 *step = reinterpret_cast<double2 *>(sm + 2 * kTurn);
+        for (int i = tid; i < kTurnCoarse + kTurnFine; i += kDirThreads)
+            step[i] = zturn(i < kTurnCoarse ? (double)i / kTurnCoarse
+                                            : (double)(i - kTurnCoarse) / kTurn);
+        __syncthreads();
+        for (int i = tid; i < kTurn; i += kDirThreads)
+            turn[i] = zmul(step[i / kTurnFine], step[kTurnCoarse + i % kTurnFine]);
+        __syncthreads();
+    }
     const long long k = (long long)(blockIdx.x / csize) * 32 + lane;
     const double f = (k < nf) ? freqs[k] : 0.0;
     double c[NH + 1], s[NH + 1], yc[H + 1], ys[H + 1];
@@ -493,7 +514,9 @@ k_mhgls_direct(const double *__restrict__ t, const double *__restrict__ yw,
             const double wq = sw[q], yq = sy[q];
             double2 z[NH + 1];
             z[1] = table_turn(st[q] * f, turn);
-            const double hx = z[1].x + z[1].x;
+            // 2 cos, by the exponent (zero becomes 2^-1022)
+            const double hx = __hiloint2double(__double2hiint(z[1].x) + 0x00100000,
+                                               __double2loint(z[1].x));
 #pragma unroll
             for (int m = 1; m <= NH; ++m) {
                 if (m == 2)

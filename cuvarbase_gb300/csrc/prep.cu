@@ -21,22 +21,9 @@ namespace cuvgls {
 
 namespace {
 
-using u64 = unsigned long long;
-
 // ---------------------------------------------------------------------------
 // positions
 // ---------------------------------------------------------------------------
-// frac(x) as a 64-bit fraction, exact to 2^-64 (finite x).
-__device__ __forceinline__ u64 turns64(double x) {
-    const u64 b = (u64)__double_as_longlong(x);
-    const int sh = (int)((b >> 52) & 0x7ff) - 1011;  // mantissa 2^-52-scaled -> 2^-64
-    const u64 m = (b & 0xfffffffffffffULL) | 0x10000000000000ULL;
-    u64 f = 0;
-    if (sh >= 0) f = sh < 64 ? m << sh : 0;
-    else if (sh > -64) f = m >> -sh;  // (zero and denormals land here or at 0)
-    return (long long)b < 0 ? 0 - f : f;
-}
-
 // floor(f n) of a fraction f, which becomes frac(f n); n < 2^31.
 __device__ __forceinline__ int take_cells(u64 &f, unsigned n) {
     const u64 lo = (u64)(unsigned)f * n;
