@@ -1,8 +1,8 @@
-// Direct sums in FP64: use_fft=False (k_gls_direct), use_double
+// Direct sums in 64 bits: use_fft=False (k_gls_direct), use_double
 // (k_nfft_direct64) and the multi-harmonic model (k_mhgls_direct).
 //
-// GB300 issues about two FP64 multiply-adds per clock and SM, so these
-// kernels are bound by their FP64 instruction count and by nothing else; a
+// GB300 issues about two FP64 multiply-adds per clock and SM, so in FP64 these
+// kernels are bound by their instruction count and by nothing else; a
 // sincospi per (point, frequency) alone is some 25 of them.  On a uniform
 // frequency grid the phasors factor instead.  A lane owns the 2 M + 1
 // consecutive bins K - M .. K + M; with E = v exp(i K x) and the step phasors
@@ -41,65 +41,140 @@ __device__ __forceinline__ double2 zturn(double turns) {  // exp(2 pi i turns)
     return make_double2(c, s);
 }
 
+// ---- fixed point ----
+// Phasors are integers in units of 2^-56, values on them (E below) in units of
+// 2^-(55 - hr) of the power of two above the largest value; hr bits of headroom
+// keep the sums of a run below 2^62.  A factor is split into 27 low bits (signed)
+// and the rest, and a product takes three 32 x 32 -> 64 bit multiply-adds (the
+// low x low part, below 2^-2 of a unit, is left out).  These run at 24 or more
+// per clock and SM, against 2 of FP64: 2.4 FP64 instructions per bin become
+// 6 of them, with finer steps than FP64 has for values near one.
+using i64 = long long;
+struct Fx {
+    int h, l;  // h 2^27 + l, |l| <= 2^26
+};
+struct Cx {
+    Fx x, y;
+};
+__device__ __forceinline__ Fx fx_split(i64 v) {
+    const int h = (int)((v + (1 << 26)) >> 27);
+    return Fx{h, (int)((unsigned)v - ((unsigned)h << 27))};
+}
+__device__ __forceinline__ i64 fx_wide(int a, int b, i64 c) { return c + (i64)a * b; }
+// c + a b / 2^54
+__device__ __forceinline__ i64 fx_fma(Fx a, Fx b, i64 c) {
+    const i64 t = fx_wide(a.l, b.h, fx_wide(a.h, b.l, 1 << 26));
+    return fx_wide(a.h, b.h, c) + (t >> 27);
+}
+// a b, a unit phasor b: in the units of a
+__device__ __forceinline__ Cx fx_cmul(Cx a, Cx b) {
+    const i64 tr = fx_wide(-a.y.l, b.y.h, fx_wide(-a.y.h, b.y.l,
+                   fx_wide(a.x.l, b.x.h, fx_wide(a.x.h, b.x.l, 1 << 26))));
+    const i64 ti = fx_wide(a.y.l, b.x.h, fx_wide(a.y.h, b.x.l,
+                   fx_wide(a.x.l, b.y.h, fx_wide(a.x.h, b.y.l, 1 << 26))));
+    const i64 re = fx_wide(-a.y.h, b.y.h, fx_wide(a.x.h, b.x.h, tr >> 27));
+    const i64 im = fx_wide(a.y.h, b.x.h, fx_wide(a.x.h, b.y.h, ti >> 27));
+    return Cx{fx_split((re + 2) >> 2), fx_split((im + 2) >> 2)};
+}
+// a b of a value a and a unit phasor b
+__device__ __forceinline__ Cx fx_scale(Fx a, Cx b) {
+    return Cx{fx_split((fx_fma(a, b.x, 2) >> 2)), fx_split((fx_fma(a, b.y, 2) >> 2))};
+}
+__device__ __forceinline__ Cx fx_unit(double2 z) {
+    constexpr double kOne = 72057594037927936.0;  // 2^56
+    return Cx{fx_split(__double2ll_rn(z.x * kOne)), fx_split(__double2ll_rn(z.y * kOne))};
+}
+__device__ __forceinline__ int4 fx_pack(Cx v) { return make_int4(v.x.h, v.x.l, v.y.h, v.y.l); }
+__device__ __forceinline__ Cx fx_unpack(int4 v) { return Cx{Fx{v.x, v.y}, Fx{v.z, v.w}}; }
+__device__ __forceinline__ i64 fx_join(Fx a) { return ((i64)a.h << 27) + a.l; }
+
+// Points of a run (one CTA, sums in 64-bit integers) and its headroom: 2^(5 +
+// hr) terms per warp.
+constexpr int kDirRun = 1024 * kDirWarps;
+__device__ __forceinline__ int fx_headroom(i64 points) {
+    const int per = (int)((points + kDirThreads - 1) / kDirThreads) * 32;
+    int hr = 0;
+    while ((32 << hr) < per) ++hr;
+    return hr;
+}
+// Exponent ex with |v| < 2^ex for the largest finite |v| of the CTA's threads;
+// `sh` one shared word.
+__device__ __forceinline__ int fx_exponent(double mx, u64 *sh, int tid) {
+    if (tid == 0) *sh = 0;
+    __syncthreads();
+    u64 b = (u64)__double_as_longlong(mx);  // (not negative: ordered as integers)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const u64 v = __shfl_xor_sync(0xffffffffu, b, o);
+        b = v > b ? v : b;
+    }
+    if ((tid & 31) == 0) atomicMax(sh, b);
+    __syncthreads();
+    b = *sh;
+    return b >> 52 || !b ? (int)(b >> 52) - 1022 : -1010 - __clzll((i64)b);
+}
+
 // Phasor tables of a warp's tile of 32 points, one entry row of 32 points
 // each: NB step phasors exp(i b x), kCoarse centres exp(i (K0 + 8 W g) x),
 // kFine offsets exp(i W f x), W = 2 M + 1.
 template <int M, int NB>
 struct DirTable {
     static constexpr int kRows = NB + kCoarse + kFine;
-    double2 row[kRows][32];
+    int4 row[kRows][32];
 
     // This lane's point: x in turns per bin, th0 the phase of K0 in turns.
     // Two sincospi, the rest by products of depth at most 8.
     __device__ __forceinline__ void build(int lane, double x, double th0) {
         static_assert(NB >= M, "the centre step is built from step phasor M");
-        double2 z[NB + 1];
-        z[1] = zturn(x);
+        Cx z[NB + 1];
+        z[1] = fx_unit(zturn(x));
 #pragma unroll
-        for (int b = 2; b <= NB; ++b) z[b] = zmul(z[b / 2], z[b - b / 2]);
+        for (int b = 2; b <= NB; ++b) z[b] = fx_cmul(z[b / 2], z[b - b / 2]);
 #pragma unroll
-        for (int b = 1; b <= NB; ++b) row[b - 1][lane] = z[b];
-        const double2 w1 = zmul(zmul(z[M], z[M]), z[1]);  // exp(i W x)
-        double2 f[kFine];
-        f[0] = make_double2(1.0, 0.0);
+        for (int b = 1; b <= NB; ++b) row[b - 1][lane] = fx_pack(z[b]);
+        const Cx w1 = fx_cmul(fx_cmul(z[M], z[M]), z[1]);  // exp(i W x)
+        Cx f[kFine];
+        f[0] = Cx{Fx{1 << 29, 0}, Fx{0, 0}};
         f[1] = w1;
 #pragma unroll
-        for (int k = 2; k < kFine; ++k) f[k] = zmul(f[k / 2], f[k - k / 2]);
+        for (int k = 2; k < kFine; ++k) f[k] = fx_cmul(f[k / 2], f[k - k / 2]);
 #pragma unroll
-        for (int k = 0; k < kFine; ++k) row[NB + kCoarse + k][lane] = f[k];
-        const double2 w8 = zmul(f[kFine / 2], f[kFine / 2]);
-        double2 c = zturn(th0);
+        for (int k = 0; k < kFine; ++k) row[NB + kCoarse + k][lane] = fx_pack(f[k]);
+        const Cx w8 = fx_cmul(f[kFine / 2], f[kFine / 2]);
+        Cx c = fx_unit(zturn(th0));
 #pragma unroll
         for (int k = 0; k < kCoarse; ++k) {
-            row[NB + k][lane] = c;
-            c = zmul(c, w8);
+            row[NB + k][lane] = fx_pack(c);
+            c = fx_cmul(c, w8);
         }
     }
     // exp(i K x) of this lane's centre K = K0 + W lane at point p
-    __device__ __forceinline__ double2 centre(int lane, int p) const {
-        return zmul(row[NB + lane / kFine][p], row[NB + kCoarse + lane % kFine][p]);
+    __device__ __forceinline__ Cx centre(int lane, int p) const {
+        return fx_cmul(fx_unpack(row[NB + lane / kFine][p]),
+                       fx_unpack(row[NB + kCoarse + lane % kFine][p]));
     }
+    __device__ __forceinline__ Cx step(int b, int p) const { return fx_unpack(row[b][p]); }
 };
 
-// The sums of one value kind over a lane's 2 M + 1 bins.
+// The sums of one value kind over a lane's 2 M + 1 bins, over one run.
 template <int M>
 struct DirSums {
-    double c0 = 0.0, s0 = 0.0, p1[M], p2[M], p3[M], p4[M];
+    i64 c0 = 0, s0 = 0, p1[M], p2[M], p3[M], p4[M];
     __device__ __forceinline__ DirSums() {
 #pragma unroll
-        for (int b = 0; b < M; ++b) p1[b] = p2[b] = p3[b] = p4[b] = 0.0;
+        for (int b = 0; b < M; ++b) p1[b] = p2[b] = p3[b] = p4[b] = 0;
     }
-    __device__ __forceinline__ void centre(double2 e) { c0 += e.x; s0 += e.y; }
-    __device__ __forceinline__ void pair(int b, double2 e, double2 st) {
-        p1[b] = fma(e.x, st.x, p1[b]);
-        p2[b] = fma(e.y, st.y, p2[b]);
-        p3[b] = fma(e.y, st.x, p3[b]);
-        p4[b] = fma(e.x, st.y, p4[b]);
+    __device__ __forceinline__ void centre(Cx e) { c0 += fx_join(e.x); s0 += fx_join(e.y); }
+    __device__ __forceinline__ void pair(int b, Cx e, Cx st) {
+        p1[b] = fx_fma(e.x, st.x, p1[b]);
+        p2[b] = fx_fma(e.y, st.y, p2[b]);
+        p3[b] = fx_fma(e.y, st.x, p3[b]);
+        p4[b] = fx_fma(e.x, st.y, p4[b]);
     }
     // real and imaginary parts of the lane's bins into re[0 .. 2 M], im[...]
-    __device__ __forceinline__ void bins(double *re, double *im) const {
-        re[M] = c0;
-        im[M] = s0;
+    __device__ __forceinline__ void bins(i64 *re, i64 *im) const {
+        re[M] = c0 * 4;
+        im[M] = s0 * 4;
 #pragma unroll
         for (int b = 0; b < M; ++b) {
             re[M + 1 + b] = p1[b] - p2[b];
@@ -110,10 +185,10 @@ struct DirSums {
     }
 };
 
-// Sum of a value kind over the CTA's warps: bin tid + 256 q of the CTA's
-// 32 W bins into (re[q], im[q]).  `red` holds 2 x kDirWarps x 32 W doubles.
+// Adds the sums of a run over the CTA's warps: bin tid + 256 q of the CTA's 32 W
+// bins to out[q], in units of 2^unit.  `red` holds 2 x kDirWarps x 32 W words.
 template <int M>
-__device__ __forceinline__ void dir_reduce(const DirSums<M> &v, double *red, int tid,
+__device__ __forceinline__ void dir_reduce(const DirSums<M> &v, i64 *red, int tid, int unit,
                                            double2 *out) {
     constexpr int TB = 32 * (2 * M + 1);
     const int lane = tid & 31, wid = tid >> 5;
@@ -126,10 +201,11 @@ __device__ __forceinline__ void dir_reduce(const DirSums<M> &v, double *red, int
         double re = 0.0, im = 0.0;
         if (b < TB)
             for (int w = 0; w < kDirWarps; ++w) {
-                re += red[w * TB + b];
-                im += red[(kDirWarps + w) * TB + b];
+                re += (double)red[w * TB + b];
+                im += (double)red[(kDirWarps + w) * TB + b];
             }
-        out[q] = make_double2(re, im);
+        out[q].x += scalbn(re, unit);
+        out[q].y += scalbn(im, unit);
     }
 }
 
@@ -145,66 +221,87 @@ __device__ __forceinline__ bool dir_part(long long n, int splits, int z, long lo
 }
 
 // ---------------------------------------------------------------------------
-// adjoint NFFT (use_double): M = 8, 544 bins per CTA
+// adjoint NFFT (use_double): M = 6, 416 bins per CTA
 // ---------------------------------------------------------------------------
-constexpr int kNfM = 8, kNfBins = 32 * (2 * kNfM + 1);
+constexpr int kNfM = 6, kNfBins = 32 * (2 * kNfM + 1);
 using NfTable = DirTable<kNfM, kNfM>;
 constexpr int kNfSmem = kDirWarps * (int)sizeof(NfTable);
 static_assert(kNfSmem >= 2 * kDirWarps * kNfBins * 8, "the reduction reuses the tables");
 
 }  // namespace
 
-// One CTA per (544 bins, curve, part of its points); its eight warps take the
+// One CTA per (416 bins, curve, part of its points); its eight warps take the
 // points 32 at a time in turn, each with tables of its own, and are summed in
 // shared memory at the end.  A curve cut into several parts leaves partial
-// sums for k_nfft_direct64_sum.  2.4 FP64 instructions per (point, bin)
-// against 12 with a sincospi pair per point and 8 bins: 4 curves of 300 to
-// 2,000 points and 20,000 bins 5.33 -> 0.36 ms (FP64 pipes 93 % busy).
+// sums for k_nfft_direct64_sum.  Bound by the wide multiply-adds, and by the
+// FP64 sincospi of the tables.  4 curves of 300 to 2,000 points and 20,000
+// bins, host to host: 5.67 ms with a sincospi pair per point and 8 bins, 0.45 ms
+// with factored phasors in FP64 (2.4 instructions per bin, 93 % busy), 0.235 ms
+// in fixed point (0.242 ms with M = 8, 0.273 with M = 4); errors against 64 bits
+// 6.8e-13 in all of them.
 __global__ void __launch_bounds__(kDirThreads, 2)
 k_nfft_direct64(const Direct64Curve *__restrict__ cvs, const double *__restrict__ t,
                 const double *__restrict__ y, double2 *__restrict__ out,
                 double2 *__restrict__ part, long long part_stride) {
     extern __shared__ __align__(16) double sm[];
+    __shared__ u64 top;
     const Direct64Curve cv = cvs[blockIdx.y];
     const long long k0 = (long long)blockIdx.x * kNfBins;
     long long j0, j1;
     if (k0 >= cv.nf || !dir_part(cv.n, cv.splits, blockIdx.z, j0, j1)) return;  // whole CTA
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     NfTable &tab = reinterpret_cast<NfTable *>(sm)[wid];
-    DirSums<kNfM> acc;
-    bool odd = false;  // a value that is not finite, added below bin by bin
-    const double kc = (double)(k0 + kNfM);
-    for (long long base = j0 + wid * 32; base < j1; base += kDirThreads) {
-        const int cnt = (int)min(32LL, j1 - base);
-        __syncwarp();  // the previous tile is consumed
-        if (lane < cnt) {
-            const double tj = t[cv.pt_off + base + lane];
-            double yj = y[cv.pt_off + base + lane];
-            if (!isfinite(yj)) {
-                odd = true;
-                yj = 0.0;
-            }
-            double a = cv.f0 * tj, b = cv.df * tj;
-            a -= floor(a);
-            b -= floor(b);
-            tab.build(lane, b, fma(kc, b, a));
-#pragma unroll
-            for (int g = 0; g < kCoarse; ++g) {  // y rides on the coarse centres
-                double2 &c = tab.row[kNfM + g][lane];
-                c = make_double2(c.x * yj, c.y * yj);
-            }
-        }
-        __syncwarp();
-        for (int p = 0; p < cnt; ++p) {
-            const double2 e = tab.centre(lane, p);
-            acc.centre(e);
-#pragma unroll
-            for (int b = 0; b < kNfM; ++b) acc.pair(b, e, tab.row[b][p]);
-        }
-    }
     constexpr int NQ = (kNfBins + kDirThreads - 1) / kDirThreads;
     double2 v[NQ];
-    dir_reduce<kNfM>(acc, sm, tid, v);
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) v[q] = make_double2(0.0, 0.0);
+    bool odd = false;   // a value that is not finite, added below bin by bin
+    bool lost = false;  // a time that is not finite: no bin has a value
+    const double kc = (double)(k0 + kNfM);
+    for (long long r0 = j0; r0 < j1; r0 += kDirRun) {  // one run, but for very long parts
+        const long long r1 = min(j1, r0 + kDirRun);
+        double mx = 0.0;
+        for (long long j = r0 + tid; j < r1; j += kDirThreads) {
+            const double yj = fabs(y[cv.pt_off + j]);
+            mx = isfinite(yj) && yj > mx ? yj : mx;
+        }
+        const int ex = fx_exponent(mx, &top, tid), hr = fx_headroom(r1 - r0);
+        DirSums<kNfM> acc;
+        for (long long base = r0 + wid * 32; base < r1; base += kDirThreads) {
+            const int cnt = (int)min(32LL, r1 - base);
+            __syncwarp();  // the previous tile is consumed
+            if (lane < cnt) {
+                const double tj = t[cv.pt_off + base + lane];
+                double yj = y[cv.pt_off + base + lane];
+                if (!isfinite(yj)) {
+                    odd = true;
+                    yj = 0.0;
+                }
+                double a = cv.f0 * tj, b = cv.df * tj;
+                a -= floor(a);
+                b -= floor(b);
+                const double th = fma(kc, b, a);
+                lost = lost || !isfinite(th);
+                tab.build(lane, b, th);
+                const Fx yv = fx_split(__double2ll_rn(scalbn(yj, 55 - hr - ex)));
+#pragma unroll
+                for (int g = 0; g < kCoarse; ++g) {  // y rides on the coarse centres
+                    int4 &c = tab.row[kNfM + g][lane];
+                    c = fx_pack(fx_scale(yv, fx_unpack(c)));
+                }
+            }
+            __syncwarp();
+#pragma unroll 1
+            for (int p = 0; p < cnt; ++p) {
+                const Cx e = tab.centre(lane, p);
+                acc.centre(e);
+#pragma unroll
+                for (int b = 0; b < kNfM; ++b) acc.pair(b, e, tab.step(b, p));
+            }
+        }
+        dir_reduce<kNfM>(acc, reinterpret_cast<i64 *>(sm), tid, ex + hr - 57, v);
+        __syncthreads();  // the next run's tables
+    }
     if (__syncthreads_or(odd)) {  // inf cos and inf sin keep their own signs
         for (long long j = j0; j < j1; ++j) {
             const double tj = t[cv.pt_off + j], yj = y[cv.pt_off + j];
@@ -219,6 +316,10 @@ k_nfft_direct64(const Direct64Curve *__restrict__ cvs, const double *__restrict_
                 v[q].y = fma(yj, e.y, v[q].y);
             }
         }
+    }
+    if (__syncthreads_or(lost)) {
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) v[q] = make_double2(nan(""), nan(""));
     }
     double2 *dst = cv.splits > 1 ? part + blockIdx.z * part_stride + cv.part_off : out + cv.out_off;
 #pragma unroll
@@ -274,15 +375,15 @@ cudaError_t launch_nfft_direct64(const Direct64Curve *cv, int n_curves, long lon
 }
 
 // ---------------------------------------------------------------------------
-// GLS (use_fft=False): three sums, M = 4, 288 bins per CTA
+// GLS (use_fft=False): three sums, M = 3, 224 bins per CTA
 // ---------------------------------------------------------------------------
 namespace {
-constexpr int kGlM = 4, kGlBins = 32 * (2 * kGlM + 1);
+constexpr int kGlM = 3, kGlBins = 32 * (2 * kGlM + 1);
 // step phasors up to 2 M: those of the 2x sums are the even ones
 using GlTable = DirTable<kGlM, 2 * kGlM>;
 struct GlTile {
     GlTable tab;
-    double yw[32], w[32];
+    int2 yw[32], w[32];
 };
 constexpr int kGlSmem = kDirWarps * (int)sizeof(GlTile);
 static_assert(kGlSmem >= 2 * kDirWarps * kGlBins * 8, "the reduction reuses the tables");
@@ -299,58 +400,87 @@ __device__ __forceinline__ float gls_direct_power(const DevCurve &cv, const GlsP
 // phasors are the squares of the others), then the power.  The times are
 // taken from the curve's first point (the power does not depend on the time
 // origin), so the phases stay small.  A curve cut into parts leaves its six
-// partial sums for k_gls_direct_sum.  7.7 FP64 instructions per (point,
-// frequency) against about 45 with a sincospi each: 8 curves of 300 to 2,000
-// points and 10,000 frequencies 9.62 -> 1.10 ms (FP64 pipes 81 % busy).
-__global__ void __launch_bounds__(kDirThreads, 1)
+// partial sums for k_gls_direct_sum.  8 curves of 300 to 2,000 points and
+// 10,000 frequencies: 9.62 ms with a sincospi each, 1.10 ms with factored
+// phasors in FP64 (7.7 instructions per frequency, 81 % busy), 0.47 ms in fixed
+// point (0.61 ms with M = 4 and one CTA per SM); errors against 64 bits 2.8e-8
+// in all of them.
+__global__ void __launch_bounds__(kDirThreads, 2)
 k_gls_direct(const DevCurve *__restrict__ cvs, const double *__restrict__ t,
              const float *__restrict__ yw, const float *__restrict__ w, float *__restrict__ out,
              double2 *__restrict__ part, long long part_stride, GlsParams gp) {
     extern __shared__ __align__(16) double sm[];
+    __shared__ u64 top[2];
     const DevCurve cv = cvs[blockIdx.y];
     const long long k0 = (long long)blockIdx.x * kGlBins;
     long long j0, j1;
     if (k0 >= cv.nf || !dir_part(cv.n, cv.aux, blockIdx.z, j0, j1)) return;  // whole CTA
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     GlTile &tile = reinterpret_cast<GlTile *>(sm)[wid];
-    DirSums<kGlM> sa, sb, sc;
-    const double kc = cv.kc - (double)(cv.nf / 2) + (double)(k0 + kGlM);
-    const double t0 = t[cv.pt_off];
-    for (long long base = j0 + wid * 32; base < j1; base += kDirThreads) {
-        const int cnt = (int)min(32LL, j1 - base);
-        __syncwarp();  // the previous tile is consumed
-        if (lane < cnt) {
-            const long long j = cv.pt_off + base + lane;
-            const double x = (t[j] - t0) * cv.df;
-            tile.tab.build(lane, x, kc * x);
-            tile.yw[lane] = (double)yw[j];
-            tile.w[lane] = (double)w[j];
-        }
-        __syncwarp();
-#pragma unroll 1
-        for (int p = 0; p < cnt; ++p) {
-            const double2 e = tile.tab.centre(lane, p);
-            const double vy = tile.yw[p], vw = tile.w[p];
-            const double2 ea = make_double2(vy * e.x, vy * e.y);
-            const double2 eb = make_double2(vw * e.x, vw * e.y);
-            const double2 ec = make_double2(fma(eb.x, e.x, -eb.y * e.y), 2.0 * eb.x * e.y);
-            sa.centre(ea);
-            sb.centre(eb);
-            sc.centre(ec);
-#pragma unroll
-            for (int b = 0; b < kGlM; ++b) {
-                const double2 st = tile.tab.row[b][p];
-                sa.pair(b, ea, st);
-                sb.pair(b, eb, st);
-                sc.pair(b, ec, tile.tab.row[2 * b + 1][p]);
-            }
-        }
-    }
     constexpr int NQ = (kGlBins + kDirThreads - 1) / kDirThreads;
     double2 va[NQ], vb[NQ], vc[NQ];
-    dir_reduce<kGlM>(sa, sm, tid, va);
-    dir_reduce<kGlM>(sb, sm, tid, vb);
-    dir_reduce<kGlM>(sc, sm, tid, vc);
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) va[q] = vb[q] = vc[q] = make_double2(0.0, 0.0);
+    bool lost = false;  // something not finite: no power of the curve is valid
+    const double kc = cv.kc - (double)(cv.nf / 2) + (double)(k0 + kGlM);
+    const double t0 = t[cv.pt_off];
+    for (long long r0 = j0; r0 < j1; r0 += kDirRun) {  // one run, but for very long parts
+        const long long r1 = min(j1, r0 + kDirRun);
+        float my = 0.f, mw = 0.f;
+        for (long long j = cv.pt_off + r0 + tid; j < cv.pt_off + r1; j += kDirThreads) {
+            const float a = fabsf(yw[j]), b = fabsf(w[j]);
+            if (isfinite(a) && isfinite(b)) {
+                my = fmaxf(my, a);
+                mw = fmaxf(mw, b);
+            } else {
+                lost = true;
+            }
+        }
+        const int hr = fx_headroom(r1 - r0);
+        const int ey = fx_exponent(my, &top[0], tid), ew = fx_exponent(mw, &top[1], tid);
+        DirSums<kGlM> sa, sb, sc;
+        for (long long base = r0 + wid * 32; base < r1; base += kDirThreads) {
+            const int cnt = (int)min(32LL, r1 - base);
+            __syncwarp();  // the previous tile is consumed
+            if (lane < cnt) {
+                const long long j = cv.pt_off + base + lane;
+                const double x = (t[j] - t0) * cv.df;
+                lost = lost || !isfinite(kc * x);
+                tile.tab.build(lane, x, kc * x);
+                const Fx fy = fx_split(__double2ll_rn(scalbn((double)yw[j], 55 - hr - ey)));
+                const Fx fw = fx_split(__double2ll_rn(scalbn((double)w[j], 55 - hr - ew)));
+                tile.yw[lane] = make_int2(fy.h, fy.l);
+                tile.w[lane] = make_int2(fw.h, fw.l);
+            }
+            __syncwarp();
+#pragma unroll 1
+            for (int p = 0; p < cnt; ++p) {
+                const Cx e = tile.tab.centre(lane, p);
+                const int2 vy = tile.yw[p], vw = tile.w[p];
+                const Cx ea = fx_scale(Fx{vy.x, vy.y}, e), eb = fx_scale(Fx{vw.x, vw.y}, e);
+                const Cx ec = fx_cmul(eb, e);
+                sa.centre(ea);
+                sb.centre(eb);
+                sc.centre(ec);
+#pragma unroll
+                for (int b = 0; b < kGlM; ++b) {
+                    const Cx st = tile.tab.step(b, p);
+                    sa.pair(b, ea, st);
+                    sb.pair(b, eb, st);
+                    sc.pair(b, ec, tile.tab.step(2 * b + 1, p));
+                }
+            }
+        }
+        i64 *red = reinterpret_cast<i64 *>(sm);
+        dir_reduce<kGlM>(sa, red, tid, ey + hr - 57, va);
+        dir_reduce<kGlM>(sb, red, tid, ew + hr - 57, vb);
+        dir_reduce<kGlM>(sc, red, tid, ew + hr - 57, vc);
+        __syncthreads();  // the next run's tables
+    }
+    if (__syncthreads_or(lost)) {
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) va[q] = vb[q] = vc[q] = make_double2(nan(""), nan(""));
+    }
 #pragma unroll
     for (int q = 0; q < NQ; ++q) {
         const int b = tid + q * kDirThreads;

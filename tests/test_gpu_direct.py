@@ -1,5 +1,5 @@
-"""The FP64 direct-sum kernels at the edges of their tiles: bins per CTA (544
-for the NFFT, 288 for the GLS, 32 frequencies for the harmonics), points per
+"""The 64-bit direct-sum kernels at the edges of their tiles: bins per CTA (416
+for the NFFT, 224 for the GLS, 32 frequencies for the harmonics), points per
 warp and per CTA (32, 256), one part and several parts of the points, against
 the FP64 oracle."""
 import numpy as np
@@ -21,6 +21,7 @@ def curve(n, seed):
 @pytest.mark.parametrize("sizes", [
     [(2, 1), (3, 543), (31, 544)], [(32, 545), (33, 17)], [(256, 1088), (257, 1089)],
     [(1025, 3000), (255, 2999)],
+    [(40, 415), (41, 416)], [(70, 417), (300, 833)],
     [(40 + i, 20000) for i in range(40)],        # enough CTAs: one part
     [(70, 700000)],
 ])
@@ -37,6 +38,54 @@ def test_use_double_tiles(oracle, sizes):
         # phase rounding of both sides (a few units of f t), then the sums
         tol = np.abs(y).sum() * EPS * (8 * 2 * np.pi * (1 + f[-1] * t.max()) + len(t))
         assert np.abs(got - ref).max() <= tol
+
+
+@pytest.mark.parametrize("scale", [1e300, 1e-300, 5e-324 * 2 ** 20, 0.0, "mixed"])
+def test_use_double_scales(oracle, scale):
+    """Values near the ends of the double range, all zero, and over 24 orders
+    of magnitude in one curve."""
+    from cuvarbase_gb300.cunfft import NFFTAsyncProcess
+    t, y, _ = curve(300, 8)
+    y = y * 10.0 ** np.random.default_rng(9).uniform(-12, 12, 300) if scale == "mixed" else y * scale
+    p = NFFTAsyncProcess(use_double=True)
+    (got,) = p.run([(t, y, 500)], samples_per_peak=5, minimum_frequency=0.3)
+    p.finish()
+    f = 0.3 + np.arange(500) / (5 * (t.max() - t.min()))
+    # the oracle on values of order one (times the exact power of two; a value
+    # below the normal range is a whole number of the smallest one)
+    ex = 0 if scale in (0.0, "mixed") else int(np.floor(np.log2(np.abs(y).max())))
+    ref = oracle.nfft_direct(t, np.ldexp(y, -ex), f)
+    got = np.ldexp(got.real, -ex) + 1j * np.ldexp(got.imag, -ex)
+    tol = np.abs(np.ldexp(y, -ex)).sum() * EPS * (8 * 2 * np.pi * (1 + f[-1] * t.max()) + 300)
+    if ex < -1000:
+        # each of the two parts' real and imaginary sums rounds to half a unit
+        tol += 2 * np.sqrt(0.5) * np.ldexp(1.0, -1074 - ex)
+    assert np.abs(got - ref).max() <= tol
+
+
+def test_long_parts(oracle):
+    """More points per warp than one run of integer sums holds (enough bins
+    that the points are not cut into parts)."""
+    from cuvarbase_gb300.cunfft import NFFTAsyncProcess
+    from cuvarbase_gb300.lombscargle import LombScargleAsyncProcess
+    n, nf = 17000, 520000
+    t, y, dy = curve(n, 4)
+    k = np.unique(np.concatenate([np.arange(20, 60), np.arange(nf - 40, nf), np.arange(21, nf, 9001)]))
+    p = NFFTAsyncProcess(use_double=True)
+    (got,) = p.run([(t, y, nf)], samples_per_peak=5, minimum_frequency=0.3)
+    p.finish()
+    f = 0.3 + k / (5 * (t.max() - t.min()))
+    ref = oracle.nfft_direct(t, y, f)
+    tol = np.abs(y).sum() * EPS * (8 * 2 * np.pi * (1 + f[-1] * t.max()) + n)
+    assert np.abs(got[k] - ref).max() <= tol
+    p = LombScargleAsyncProcess(sigma=2, m=8)
+    f = (1 + np.arange(nf)) / (5 * (t.max() - t.min()))
+    ((_, got),) = p.run([(t, y, dy)], freqs=[f], use_fft=False)
+    p.finish()
+    tt, yw, w, YY, ybar = oracle.prepare_curve(t, y, dy)
+    ref = oracle.gls_tau(tt, yw.astype(np.float32).astype(np.float64),
+                         w.astype(np.float32).astype(np.float64), f[k], YY, ybar, mode=1)
+    assert np.abs(got[k] - ref).max() <= 2e-6 * max(1.0, np.abs(ref).max())
 
 
 def test_use_double_infinite_value():
