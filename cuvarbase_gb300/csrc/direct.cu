@@ -543,41 +543,35 @@ namespace {
 // Phasors of the shared turn table, from kTurnCoarse by kTurnFine products.
 constexpr int kTurn = 2048, kTurnCoarse = 64, kTurnFine = kTurn / kTurnCoarse;
 
-// A float as a double by its bits (zero becomes 2^-127; no FP64 instruction).
-__device__ __forceinline__ double widen(float x) {
-    const int b = __float_as_int(x);
-    return __hiloint2double((b & 0x80000000) | (((b & 0x7fffffff) >> 3) + 0x38000000), b << 29);
-}
-// exp(2 pi i p), NaN when p is not finite: the phasor at the nearest multiple
-// of 1 / kTurn turned by the remaining angle d, |d| <= pi / kTurn.  One SM
-// issues 64 other instructions in the time of an FP64 one, so the fraction of
-// p, the table index and the remainder are integers, and FP32 has what it is
-// exact enough for: d^3 / 6 - d^5 / 120 (6e-10) and d^4 / 24 (2e-13); the terms
-// left out are d^6 / 720 and d^7 / 5040, below 2e-20.  Eight FP64 instructions
-// after p (16 with all of it in FP64, about 28 for floor and sincospi).
-__device__ __forceinline__ double2 table_turn(double p, const double2 *tab) {
+// exp(2 pi i p) of a finite p: the phasor at the nearest multiple of 1 / kTurn
+// turned by the remaining angle d, |d| <= pi / kTurn, all of it in integers
+// (FP64 forms p only): d and sin d in units of 2^-61, cos d - 1 = -d^2 / 2 +
+// d^4 / 24 the same, the small terms d^3 / 6 - d^5 / 120 (6e-10) and d^4 / 24
+// (2e-13) in FP32; those left out are below 2e-20.
+__device__ __forceinline__ Cx table_turn(double p, const int4 *tab) {
     const u64 th = turns64(p);
     const int k = (int)((th + (1ULL << 52)) >> 53);  // 0 .. kTurn
-    const double2 e = tab[k & (kTurn - 1)];
-    const long long r = (long long)(th - ((u64)k << 53));  // |r| <= 2^52, in 2^-64 turns
-    // d: r / 4 set into the mantissa of 1.5 2^52, scaled and taken off in one step
-    constexpr double kUnit = 6.283185307179586477 / 4611686018427387904.0;  // 2 pi 2^-62
-    const double d = fma(__longlong_as_double(0x4338000000000000LL + (r >> 2)), kUnit,
-                         -6755399441055744.0 * kUnit);
-    const float df = (float)(int)(r >> 21) * (float)(6.283185307179586477 / 8796093022208.0);
-    const float q = df * df;
-    double w3 = widen(df * q * fmaf(q, 1.f / 120.f, -1.f / 6.f));
-    if ((__double2hiint(p) & 0x7ff00000) == 0x7ff00000) w3 = __longlong_as_double(-1LL);
-    const double sn = d + w3, cm = fma(d * d, -0.5, widen(q * q * (1.f / 24.f)));
-    return make_double2(fma(-e.y, sn, fma(e.x, cm, e.x)), fma(e.x, sn, fma(e.y, cm, e.y)));
+    const Cx e = fx_unpack(tab[k & (kTurn - 1)]);
+    const Fx r = fx_split((i64)(th - ((u64)k << 53)));  // |r| <= 2^52, in 2^-64 turns
+    constexpr i64 kTwoPi = 14148475504056880LL;        // 2 pi 2^51
+    constexpr int kHi = (int)((kTwoPi + (1 << 26)) >> 27), kLo = (int)(kTwoPi - ((i64)kHi << 27));
+    const i64 d = fx_fma(r, Fx{kHi, kLo}, 0);
+    const int dh = (int)(d >> 21), dl = (int)(d & ((1 << 21) - 1));
+    const float df = (float)dh * 9.094947017729282e-13f, q = df * df;  // 2^-40
+    const float kUp = 2305843009213693952.f;                           // 2^61
+    const Fx sn = fx_split(d + __float2int_rn(kUp * df * q * fmaf(q, 1.f / 120.f, -1.f / 6.f)));
+    const i64 d2 = fx_wide(dh, dh, fx_wide(dh, dl, 0) >> 20);  // 2^-80
+    const Fx cm = fx_split(__float2int_rn(kUp * q * q * (1.f / 24.f)) - (d2 >> 20));
+    // e + e (cm + i sn), the product in units of 2^-63
+    const i64 re = fx_fma(cm, e.x, 64) - fx_fma(sn, e.y, 0), im = fx_fma(cm, e.y, fx_fma(sn, e.x, 64));
+    return Cx{fx_split(fx_join(e.x) + (re >> 7)), fx_split(fx_join(e.y) + (im >> 7))};
 }
 
 // rows of sums a CTA reduces: c, s (2H each), yc, ys (H each), and sum w
 __host__ __device__ constexpr int mh_sums(int H) { return 6 * H + 1; }
 __host__ __device__ constexpr int mh_smem(int H) {
-    // turn table, the warps' point tiles, then (reused) the warps' sums
-    const int a = kTurn * 16 + kDirWarps * 32 * 24, b = (kDirWarps + 1) * mh_sums(H) * 32 * 8;
-    return a > b ? a : b;
+    // turn table, the warps' point tiles, the warps' sums and their totals
+    return kTurn * 16 + kDirWarps * 32 * 24 + (kDirWarps + 1) * mh_sums(H) * 32 * 8;
 }
 
 }  // namespace
@@ -590,16 +584,16 @@ __host__ __device__ constexpr int mh_smem(int H) {
 // sums and solves: 625 CTAs left a fifth of the FP64 pipes idle at the end
 // (4.1 CTAs per SM are 5 rounds).  Per point the
 // phasor from table_turn, its powers n = 2 .. 2H by the recurrence
-// z_n = 2 cos(phi) z_(n-1) - z_(n-2) (two instructions each; its rounding, 6e-16
-// rms at n = 6 and 2.4e-15 at n = 16, is that of the products z_n/2 z_n/2, which
-// took three or four, and far below that of the phase t f), then the sums of
-// cuvarbase/lombscargle.py:337-400 (mhdirect_sums) with the regulariser of
+// z_n = 2 cos(phi) z_(n-1) - z_(n-2), then the sums of
+// cuvarbase/lombscargle.py:337-400 (mhdirect_sums), all in fixed point; FP64
+// forms t f, adds the warps' sums, and from there on: the regulariser of
 // :403-447, the 2H x 2H system solved by Gaussian elimination with partial
 // pivoting, and the power of :497-536.  H = 3, 1,000 points, 20,000
-// frequencies, host to host: 4.93 -> 2.24 ms with the table and the clusters
-// (54 FP64 instructions per point and frequency, the pipes 88 % busy), 1.97 ms
-// with the recurrence (48), 1.54 ms with the integer and FP32 parts of the
-// phasor (37).
+// frequencies, host to host: 4.93 ms with a sincospi per point; in FP64 2.24 ms
+// with the table and the clusters (54 instructions per point and frequency, the
+// pipes 88 % busy), 1.97 ms with the recurrence, 1.54 ms with the phasor's
+// fraction in integers; 0.79 ms in fixed point (about 100 wide multiply-adds).
+// Errors against 64 bits 1.8e-13 in all of them: that of the FP64 phase t f.
 template <int H>
 __global__ void __launch_bounds__(kDirThreads, H <= 4 ? 2 : 1)
 k_mhgls_direct(const double *__restrict__ t, const double *__restrict__ yw,
@@ -609,83 +603,108 @@ k_mhgls_direct(const double *__restrict__ t, const double *__restrict__ yw,
     const int rank = blockIdx.x % csize;
     extern __shared__ __align__(16) double sm[];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    double2 *turn = reinterpret_cast<double2 *>(sm);
-    double *st = sm + 2 * kTurn + wid * 96, *sy = st + 32, *sw = st + 64;
+    __shared__ u64 top[2];
+    int4 *turn = reinterpret_cast<int4 *>(sm);
+    double *tiles = sm + 2 * kTurn, *sums = tiles + kDirWarps * 96;
+    double *st = tiles + wid * 96;
+    int2 *sy = reinterpret_cast<int2 *>(st + 32), *sw = sy + 32;
     {  // the coarse and fine steps (in the point tiles' memory), then their products
-        double2 *step = reinterpret_cast<double2 *>(sm + 2 * kTurn);
+        int4 *step = reinterpret_cast<int4 *>(tiles);
         for (int i = tid; i < kTurnCoarse + kTurnFine; i += kDirThreads)
-            step[i] = zturn(i < kTurnCoarse ? (double)i / kTurnCoarse
-                                            : (double)(i - kTurnCoarse) / kTurn);
+            step[i] = fx_pack(fx_unit(zturn(i < kTurnCoarse ? (double)i / kTurnCoarse
+                                                            : (double)(i - kTurnCoarse) / kTurn)));
         __syncthreads();
         for (int i = tid; i < kTurn; i += kDirThreads)
-            turn[i] = zmul(step[i / kTurnFine], step[kTurnCoarse + i % kTurnFine]);
+            turn[i] = fx_pack(fx_cmul(fx_unpack(step[i / kTurnFine]),
+                                      fx_unpack(step[kTurnCoarse + i % kTurnFine])));
         __syncthreads();
     }
     const long long k = (long long)(blockIdx.x / csize) * 32 + lane;
     const double f = (k < nf) ? freqs[k] : 0.0;
-    double c[NH + 1], s[NH + 1], yc[H + 1], ys[H + 1];
-#pragma unroll
-    for (int m = 0; m <= NH; ++m) { c[m] = 0.0; s[m] = 0.0; }
-#pragma unroll
-    for (int m = 0; m <= H; ++m) { yc[m] = 0.0; ys[m] = 0.0; }
-    double ws = 0.0;  // of the points this lane staged
-    for (long long base = rank * kDirThreads + wid * 32; base < n; base += csize * kDirThreads) {
-        const int cnt = (int)min(32LL, n - base);
-        __syncwarp();  // the previous tile is consumed
-        if (lane < cnt) {
-            st[lane] = t[base + lane];
-            sy[lane] = yw[base + lane];
-            sw[lane] = w[base + lane];
-            ws += sw[lane];
+    double ws = 0.0;    // of the points this lane staged
+    // a phase that is not finite (of this lane's frequency), a value that is not
+    bool lost = false, odd = false;
+    // the warps' sums, in shared memory as [warp][sum][lane]
+    double *r = sums + wid * NS * 32 + lane;
+    for (int i = 0; i < NS; ++i) r[i * 32] = 0.0;
+    const long long share = (n + csize - 1) / csize;
+    const long long j1 = min(n, (rank + 1) * share);
+    for (long long r0 = rank * share; r0 < j1; r0 += kDirRun) {  // one run, but for very long curves
+        const long long r1 = min(j1, r0 + kDirRun);
+        double my = 0.0, mw = 0.0;
+        for (long long j = r0 + tid; j < r1; j += kDirThreads) {
+            const double u = fabs(yw[j]), v = fabs(w[j]);
+            if (isfinite(u) && isfinite(v)) {
+                my = u > my ? u : my;
+                mw = v > mw ? v : mw;
+            } else {
+                odd = true;
+            }
         }
-        __syncwarp();
-#pragma unroll 1
-        for (int q = 0; q < cnt; ++q) {
-            const double wq = sw[q], yq = sy[q];
-            double2 z[NH + 1];
-            z[1] = table_turn(st[q] * f, turn);
-            // 2 cos, by the exponent (zero becomes 2^-1022)
-            const double hx = __hiloint2double(__double2hiint(z[1].x) + 0x00100000,
-                                               __double2loint(z[1].x));
+        const int hr = fx_headroom(r1 - r0);
+        const int ey = fx_exponent(my, &top[0], tid), ew = fx_exponent(mw, &top[1], tid);
+        i64 c[NH + 1], s[NH + 1], yc[H + 1], ys[H + 1];
 #pragma unroll
-            for (int m = 1; m <= NH; ++m) {
-                if (m == 2)
-                    z[m] = make_double2(fma(hx, z[1].x, -1.0), hx * z[1].y);
-                else if (m > 2)
-                    z[m] = make_double2(fma(hx, z[m - 1].x, -z[m - 2].x),
-                                        fma(hx, z[m - 1].y, -z[m - 2].y));
-                c[m] = fma(wq, z[m].x, c[m]);
-                s[m] = fma(wq, z[m].y, s[m]);
-                if (m <= H) {
-                    yc[m] = fma(yq, z[m].x, yc[m]);
-                    ys[m] = fma(yq, z[m].y, ys[m]);
+        for (int m = 0; m <= NH; ++m) c[m] = s[m] = 0;
+#pragma unroll
+        for (int m = 0; m <= H; ++m) yc[m] = ys[m] = 0;
+        for (long long base = r0 + wid * 32; base < r1; base += kDirThreads) {
+            const int cnt = (int)min(32LL, r1 - base);
+            __syncwarp();  // the previous tile is consumed
+            if (lane < cnt) {
+                st[lane] = t[base + lane];
+                ws += w[base + lane];
+                const Fx fy = fx_split(__double2ll_rn(scalbn(yw[base + lane], 55 - hr - ey)));
+                const Fx fw = fx_split(__double2ll_rn(scalbn(w[base + lane], 55 - hr - ew)));
+                sy[lane] = make_int2(fy.h, fy.l);
+                sw[lane] = make_int2(fw.h, fw.l);
+            }
+            __syncwarp();
+#pragma unroll 1
+            for (int q = 0; q < cnt; ++q) {
+                const int2 vw = sw[q], vy = sy[q];
+                const Fx wq{vw.x, vw.y}, yq{vy.x, vy.y};
+                const double p = st[q] * f;
+                lost = lost || (__double2hiint(p) & 0x7ff00000) == 0x7ff00000;
+                Cx z = table_turn(p, turn), zp{Fx{1 << 29, 0}, Fx{0, 0}};  // power m, m - 1
+                const Fx cc = fx_split(2 * fx_join(z.x));                 // 2 cos
+#pragma unroll
+                for (int m = 1; m <= NH; ++m) {
+                    if (m > 1) {
+                        const Cx zn{fx_split((fx_fma(cc, z.x, 2 - 4 * fx_join(zp.x))) >> 2),
+                                    fx_split((fx_fma(cc, z.y, 2 - 4 * fx_join(zp.y))) >> 2)};
+                        zp = z;
+                        z = zn;
+                    }
+                    c[m] = fx_fma(wq, z.x, c[m]);
+                    s[m] = fx_fma(wq, z.y, s[m]);
+                    if (m <= H) {
+                        yc[m] = fx_fma(yq, z.x, yc[m]);
+                        ys[m] = fx_fma(yq, z.y, ys[m]);
+                    }
                 }
             }
         }
-    }
-    // the eight warps' sums, in shared memory as [warp][sum][lane]
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ws += __shfl_xor_sync(0xffffffffu, ws, o);
-    __syncthreads();
-    {
-        double *r = sm + wid * NS * 32 + lane;
 #pragma unroll
         for (int m = 1; m <= NH; ++m) {
-            r[(m - 1) * 32] = c[m];
-            r[(NH + m - 1) * 32] = s[m];
+            r[(m - 1) * 32] += scalbn((double)c[m], ew + hr - 57);
+            r[(NH + m - 1) * 32] += scalbn((double)s[m], ew + hr - 57);
         }
 #pragma unroll
         for (int m = 1; m <= H; ++m) {
-            r[(2 * NH + m - 1) * 32] = yc[m];
-            r[(2 * NH + H + m - 1) * 32] = ys[m];
+            r[(2 * NH + m - 1) * 32] += scalbn((double)yc[m], ey + hr - 57);
+            r[(2 * NH + H + m - 1) * 32] += scalbn((double)ys[m], ey + hr - 57);
         }
-        r[6 * H * 32] = ws;
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ws += __shfl_xor_sync(0xffffffffu, ws, o);
+    if (__syncthreads_or(odd) || lost) ws = nan("");
+    r[6 * H * 32] = ws;
     __syncthreads();
-    double *tot = sm + kDirWarps * NS * 32;
+    double *tot = sums + kDirWarps * NS * 32;
     for (int i = tid; i < NS * 32; i += kDirThreads) {
         double v = 0.0;
-        for (int q = 0; q < kDirWarps; ++q) v += sm[q * NS * 32 + i];
+        for (int q = 0; q < kDirWarps; ++q) v += sums[q * NS * 32 + i];
         tot[i] = v;
     }
     if (csize > 1) {
@@ -702,6 +721,8 @@ k_mhgls_direct(const double *__restrict__ t, const double *__restrict__ yw,
     }
     __syncthreads();
     if (wid != 0 || k >= nf) return;
+    double c[NH + 1], s[NH + 1], yc[H + 1], ys[H + 1];
+    s[0] = 0.0;
 #pragma unroll
     for (int m = 1; m <= NH; ++m) {
         c[m] = tot[(m - 1) * 32 + lane];

@@ -150,3 +150,37 @@ def test_harmonics_large_phases(oracle):
     P = lomb_scargle_direct_sums(t, yw, w, f, YY, nharms=2, amplitude_priors=3.0)
     ref = oracle.mhgls_np(t, yw, w, f, YY, nharms=2, amplitude_priors=3.0)
     assert np.abs(P - ref).max() <= 1e-9
+
+
+@pytest.mark.parametrize("H", [1, 3])
+def test_harmonics_long_curve(oracle, H):
+    """More points per warp than one run of integer sums holds, and weights
+    over six orders of magnitude."""
+    from cuvarbase_gb300.lombscargle import lomb_scargle_direct_sums
+    t, y, dy = curve(40000, 6)
+    dy = dy * 10.0 ** np.random.default_rng(5).uniform(0, 3, len(t))
+    tt, yw, w, YY, _ = oracle.prepare_curve(t, y, dy)
+    f = (12 + np.arange(40)) / (5 * (t.max() - t.min()))
+    f[-1] = 1 / 3.3
+    P = lomb_scargle_direct_sums(tt, yw, w, f, YY, nharms=H, amplitude_priors=3.0)
+    ref = oracle.mhgls_np(tt, yw, w, f, YY, nharms=H, amplitude_priors=3.0)
+    assert np.abs(P - ref).max() <= 1e-9
+
+
+def test_harmonics_values_not_finite():
+    """A time or weight that is not finite leaves no frequency a power, a
+    frequency that is not finite none of its own."""
+    from cuvarbase_gb300.lombscargle import lomb_scargle_direct_sums
+    t, y, _ = curve(600, 2)
+    w = np.full(600, 1 / 600)
+    f = np.linspace(0.1, 2.0, 70)
+
+    def put(a, i, v):
+        a = a.copy()
+        a[i] = v
+        return a
+    for v in (np.nan, np.inf):
+        for args in ((put(t, 7, v), w * y, w, f), (t, w * y, put(w, 7, v), f)):
+            assert np.all(np.isnan(lomb_scargle_direct_sums(*args, 1.0, nharms=2)))
+        P = lomb_scargle_direct_sums(t, w * y, w, put(f, 5, v), 1.0, nharms=2)
+        assert np.isnan(P[5]) and np.isfinite(np.delete(P, 5)).all()
