@@ -389,14 +389,14 @@ int get_class(cuvgls_handle *h, long long nf, int ng, ClassTables **out) {
     p.es_im2 = (float)(1.0 / ((double)p.m * p.m));
     // tables (FFT tables of G1 and G2, inter-pass twiddles, and for the ES
     // window the deconvolution of |k'| <= G / 2) built on the device
-    const size_t n1 = (size_t)fft_table_len(G1), n2 = (size_t)fft_table_len(G2);
+    const size_t n1 = (size_t)fft_table_len(G1), n2 = (size_t)row_table_len(ng, G2);
     const size_t nd = p.win == kWinES ? (size_t)(G / 2 + 2) / 2 : 0;  // in float2 units
     const size_t nr = p.win == kWinES ? (size_t)(G + 1) / 2 : 0;
     CK(cudaMalloc(&c.d, (n1 + n2 + (size_t)G + nd + nr) * sizeof(float2)),
        "cudaMalloc(plan tables)");
     // on a stream of their own: a new class waits neither for batches nor for
     // result copies in flight
-    CK(launch_plan_tables(c.d, G1, G2, B, h->table_stream), "plan tables");
+    CK(launch_plan_tables(c.d, G1, G2, B, ng, h->table_stream), "plan tables");
     if (p.win == kWinES)
         CK(launch_es_deconv((float *)(c.d + n1 + n2 + G), G, p.m, beta, h->table_stream),
            "deconvolution table");

@@ -149,7 +149,8 @@ __device__ double fft_table_turns(int L, int e) {
     return 0.0;
 }
 
-__global__ void k_plan_tables(float2 *dst, int G1, int G2, int B, int n1, int n2) {
+// (ng: grids, which choose the row table's layout)
+__global__ void k_plan_tables(float2 *dst, int G1, int G2, int B, int ng, int n1, int n2) {
     const long long G = (long long)G1 * G2;
     const long long total = n1 + n2 + G;
     for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
@@ -158,7 +159,14 @@ __global__ void k_plan_tables(float2 *dst, int G1, int G2, int B, int n1, int n2
         if (e < n1) {
             turns = fft_table_turns(G1, (int)e);
         } else if (e < n1 + n2) {
-            turns = fft_table_turns(G2, (int)(e - n1));
+            const int x = (int)(e - n1);
+            if (pass2_deep(ng, G2)) {
+                const int N1 = G2 / deep_fac(G2, 0), y = x - G2;
+                turns = y < 0 ? (double)(x / N1 * (x % N1)) / (double)G2
+                              : (double)(y / 8 * (y % 8)) / (double)N1;
+            } else {
+                turns = fft_table_turns(G2, x);
+            }
         } else {
             // inter-pass twiddle in the intermediate's [cb][q1][c] order
             const long long i = e - n1 - n2;
@@ -232,11 +240,11 @@ cudaError_t launch_best_finish(const unsigned long long *keys, int n, int64_t *b
     return cudaGetLastError();
 }
 
-cudaError_t launch_plan_tables(float2 *dst, int G1, int G2, int B, cudaStream_t s) {
-    const int n1 = fft_table_len(G1), n2 = fft_table_len(G2);
+cudaError_t launch_plan_tables(float2 *dst, int G1, int G2, int B, int ng, cudaStream_t s) {
+    const int n1 = fft_table_len(G1), n2 = row_table_len(ng, G2);
     const long long total = n1 + n2 + (long long)G1 * G2;
     const int blocks = (int)std::min<long long>((total + 255) / 256, 4096);
-    k_plan_tables<<<blocks, 256, 0, s>>>(dst, G1, G2, B, n1, n2);
+    k_plan_tables<<<blocks, 256, 0, s>>>(dst, G1, G2, B, ng, n1, n2);
     return cudaGetLastError();
 }
 

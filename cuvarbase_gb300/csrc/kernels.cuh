@@ -101,8 +101,8 @@ cudaError_t launch_es_deconv(float *dst, long long G, int m, double beta, cudaSt
 cudaError_t launch_deconv_rows(const float *dtab, float *dst, int G1, int G2, int R, cudaStream_t s);
 
 // Fill the tables of a plan (FFT tables of G1 and G2, then the inter-pass
-// twiddles), fft_table_len(G1) + fft_table_len(G2) + G1 G2 entries at dst.
-cudaError_t launch_plan_tables(float2 *dst, int G1, int G2, int B, cudaStream_t s);
+// twiddles), fft_table_len(G1) + row_table_len(ng, G2) + G1 G2 entries at dst.
+cudaError_t launch_plan_tables(float2 *dst, int G1, int G2, int B, int ng, cudaStream_t s);
 
 // Host preparation of LombScargleMemory.setdata on the device for long raw
 // (t, y, dy) curves, over their segments (one double4 of partA and partB

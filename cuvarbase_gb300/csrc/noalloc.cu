@@ -124,7 +124,7 @@ extern "C" int cuvgls_gls_noalloc(double sigma, int32_t m, const cuvgls_gls_inpu
     p.binv = (float)(1.0 / bw);
     p.dc1 = (float)(bw * kPiN * kPiN / ((double)G * (double)G));
     p.dc2 = (float)(1.0 / sqrt(kPiN * bw));
-    const int n1 = fft_table_len(G1), n2 = fft_table_len(G2);
+    const int n1 = fft_table_len(G1), n2 = row_table_len(3, G2);
 
     // scratch layout
     size_t off = 0;
@@ -209,7 +209,7 @@ extern "C" int cuvgls_gls_noalloc(double sigma, int32_t m, const cuvgls_gls_inpu
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemsetAsync(d_flag, 0, sizeof(unsigned), s);
-    if (e == cudaSuccess) e = launch_plan_tables(tab, G1, G2, B, s);
+    if (e == cudaSuccess) e = launch_plan_tables(tab, G1, G2, B, 3, s);
     RecAB *recAB = (RecAB *)(base + o_ra);
     RecC *recC = (RecC *)(base + o_rc);
     SegEntry *segs = (SegEntry *)(base + o_seg);

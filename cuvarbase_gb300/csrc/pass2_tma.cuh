@@ -138,7 +138,9 @@ k_pass2_gls_reg(const __grid_constant__ CUtensorMap map, const DevCurve *cvs,
         if (tid == 0) atomicOr(gp.errflag, 2u);
         return;
     }
-    const int G1 = p.G1, G = (int)p.G, lb = p.B == 4 ? 2 : 1, nrb = G1 / R;
+    constexpr int lb = 2;
+    static_assert(1 << lb == kGlsCols, "blocks of four columns");
+    const int G1 = p.G1, G = (int)p.G, nrb = G1 / R;
     const int ntask = n_curves * nrb;
     if (tid == 0) {
         for (int b = 0; b < NB; ++b) mbar_init(&full[b]);
@@ -155,11 +157,11 @@ k_pass2_gls_reg(const __grid_constant__ CUtensorMap map, const DevCurve *cvs,
         if (!live(s)) return;
         const int t = blockIdx.x + (s / 3) * (int)gridDim.x, c = t / nrb, rb = t - c * nrb;
         mbar_expect(&full[s % NB], R * L2 * 8);
-        tma_load_3d(tiles + (s % NB) * TILE, &map, rb * R * 2 * p.B, 0, (first + c) * 3 + s % 3,
+        tma_load_3d(tiles + (s % NB) * TILE, &map, rb * R * 2 * kGlsCols, 0, (first + c) * 3 + s % 3,
                     &full[s % NB]);
         if (!live(s + 1)) return;
         const int u = blockIdx.x + ((s + 1) / 3) * (int)gridDim.x, d = u / nrb;
-        tma_prefetch_3d(&map, (u - d * nrb) * R * 2 * p.B, 0, (first + d) * 3 + (s + 1) % 3);
+        tma_prefetch_3d(&map, (u - d * nrb) * R * 2 * kGlsCols, 0, (first + d) * 3 + (s + 1) % 3);
     };
     if (tid == 0)
         for (int b = 0; b < NB; ++b) issue(b);
@@ -489,7 +491,7 @@ cudaError_t launch_pass2_reg_t(const DevCurve *cv, int n_curves, int first, cons
     e = pass2_map(map, inter, p, 3 * (first + n_curves), R);
     if (e != cudaSuccess) return e;
     const long long tasks = (long long)n_curves * (p.G1 / R);
-    if (tasks > 0x3fffffffLL) return cudaErrorInvalidValue;
+    if (tasks > 0x3fffffffLL || p.B != kGlsCols) return cudaErrorInvalidValue;
     Plan q = p;
     q.dependent = small_launch(tasks);
     return launch_pdl(k_pass2_gls_reg<L2, ES>, q.dependent,

@@ -8,10 +8,10 @@
 //                    twiddle exp(2 pi i q1 l2 / G) and writes the tile to the
 //                    intermediate buffer ([column block][q1][column]).
 //   k_pass1_long<L1> the same for one grid of the long columns.
-//   k_pass2_gls<L2>  one CTA per (curve, block of R rows).  Loads R rows of
-//                    the three grids, runs the length-L2 row FFTs and, in the
-//                    same kernel, deconvolves the window and evaluates the
-//                    GLS power of every in-band frequency.
+//   k_pass2_gls_deep<L2>  one CTA per (curve, block of R rows), rows of 512 to
+//                    2,048.  Runs the length-L2 row FFTs of the three grids
+//                    and, in the same kernel, deconvolves the window and
+//                    evaluates the GLS power of every in-band frequency.
 //   k_pass2_gls_cube the same for rows of 4,096.
 //   k_pass2_nfft<L2> the same for one grid, writing complex adjoint-NFFT
 //                    values with the absolute-time phase.
@@ -642,207 +642,6 @@ __device__ __forceinline__ void rows_fft_b(float2 *tile, const float2 *__restric
     }
 }
 
-template <int NG, int L2, int R, int NT, int LDS>
-__device__ __forceinline__ void rows_fft(float2 *tile, const float2 *__restrict__ src,
-                                         const float2 *__restrict__ tab, int G1, long long G,
-                                         int B, int rb, int tid) {
-    if (B == 8) rows_fft_b<NG, L2, R, NT, LDS, 8>(tile, src, tab, G1, G, rb, tid);
-    else if (B == 4) rows_fft_b<NG, L2, R, NT, LDS, 4>(tile, src, tab, G1, G, rb, tid);
-    else rows_fft_b<NG, L2, R, NT, LDS, 2>(tile, src, tab, G1, G, rb, tid);
-}
-
-// Deconvolution + GLS power of every in-band frequency of the R rows of a
-// pass-2 tile.  BEST: also fold each valid power into the curve's best key
-// (power bits << 32 | ~index, one atomicMax per warp; the caller guarantees
-// full warps), and out == nullptr skips the powers themselves.  Chosen once
-// per CTA, so the plain path carries no per-frequency cost for it.
-template <bool BEST, bool ES, int L2, int R, int NT, int LDS>
-__device__ __forceinline__ void gls_epilogue(const float2 *tile, const DevCurve &cv,
-                                             float *__restrict__ out, const GlsParams &gp,
-                                             const Plan &p, int rb, int tid) {
-    const int G = (int)p.G;  // < 2^23
-    const int G1 = p.G1;
-    const int nf = cv.nf, h = nf / 2;
-    const int lo_end = nf - h, hi_start = G - h;
-    float *outc = (!BEST || out) ? out + cv.out_off + h : nullptr;
-    unsigned long long key = 0;
-    const unsigned ibase = (unsigned)(cv.best_off + h);
-#pragma unroll 2
-    for (int e = tid; e < R * L2; e += NT) {
-        const int r = e % R, q2 = e / R;
-        const int q = rb * R + r + G1 * q2;
-        int kp;
-        if (q < lo_end) kp = q;
-        else if (q >= hi_start) kp = q - G;
-        else continue;
-        const float D = ES ? __ldg(p.drow + (long long)rb * R * L2 + e) : win_deconv<false>(kp, p);
-        const int o = phys2<L2>(q2);
-        const float2 A = tile[r * LDS + o];
-        const float2 Bv = tile[(R + r) * LDS + o];
-        const float2 Cv = tile[(2 * R + r) * LDS + o];
-        const float P = gls_from_sums<float>(
-            A.x * D, A.y * D, Bv.x * D, Bv.y * D, Cv.x * D, Cv.y * D, gp.mode,
-            gp.reg, cv.w_sum, cv.yw_sum, cv.ybar, cv.yy_inv);
-        if (!BEST || outc) outc[kp] = P;
-        if (BEST && P >= 0.f) {  // valid powers only (invalid ones are -1)
-            const unsigned long long k =
-                ((unsigned long long)__float_as_uint(P) << 32) |
-                (0xFFFFFFFFu - (ibase + (unsigned)kp));
-            key = k > key ? k : key;
-        }
-    }
-    if (BEST) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const unsigned long long v = __shfl_xor_sync(0xffffffffu, key, o);
-            key = v > key ? v : key;
-        }
-        if ((tid & 31) == 0 && key != 0) atomicMax(gp.best + cv.best_slot, key);
-    }
-}
-
-// Floating-mean GLS finish of a pass-2 tile (mode 1) with two frequencies
-// per thread evaluated together as packed FP32x2 arithmetic: lane 0 is row
-// element q2, lane 1 element q2 + NT / R of the same row.  Same quantities
-// as gls_from_sums (2x2 normal equations, invalid -> -1); BEST as in
-// gls_epilogue.
-template <bool BEST, bool ES, int L2, int R, int NT, int LDS>
-__device__ __forceinline__ void gls_epilogue_fm2(const float2 *tile, const DevCurve &cv,
-                                                 float *__restrict__ out, const GlsParams &gp,
-                                                 const Plan &p, int rb, int tid) {
-    static_assert(NT % R == 0 && NT % 32 == 0, "one row per thread, full warps");
-    constexpr int QS = NT / R;
-    const int G = (int)p.G;  // < 2^23
-    const int G1 = p.G1;
-    const int nf = cv.nf, h = nf / 2;
-    const int lo_end = nf - h, hi_start = G - h;
-    float *outc = (!BEST || out) ? out + cv.out_off + h : nullptr;
-    unsigned long long key = 0;
-    const unsigned ibase = (unsigned)(cv.best_off + h);
-    auto keep = [&](float P, int k) {  // fold a valid power into the best key
-        if (P >= 0.f) {
-            const unsigned long long kk = ((unsigned long long)__float_as_uint(P) << 32) |
-                                          (0xFFFFFFFFu - (ibase + (unsigned)k));
-            key = kk > key ? kk : key;
-        }
-    };
-    const int r = tid % R, q20 = tid / R;
-    const float2 *tA = tile + r * LDS, *tB = tile + (R + r) * LDS, *tC = tile + (2 * R + r) * LDS;
-    const float2 dc1 = make_float2(p.dc1, p.dc1), dc2 = make_float2(p.dc2, p.dc2);
-    const float2 nyw = make_float2(-cv.yw_sum, -cv.yw_sum);
-    const float hw0 = 0.5f * cv.w_sum + gp.reg;
-    const float2 hw = make_float2(hw0, hw0), half = make_float2(0.5f, 0.5f);
-    const float2 mhalf = make_float2(-0.5f, -0.5f), mtwo = make_float2(-2.f, -2.f);
-    const float2 pn = make_float2(cv.yy_inv, cv.yy_inv);
-#pragma unroll 1
-    for (int q2a = q20; q2a < L2; q2a += 2 * QS) {
-        const int q2b = q2a + QS;
-        const int qa = rb * R + r + G1 * q2a, qb = qa + G1 * QS;
-        const bool ina = qa < lo_end || qa >= hi_start;
-        const bool inb = q2b < L2 && (qb < lo_end || qb >= hi_start);
-        if (!ina && !inb) continue;
-        const int ka = qa < lo_end ? qa : qa - G, kb = qb < lo_end ? qb : qb - G;
-        const int oa = phys2<L2>(q2a), ob = phys2<L2>(q2b < L2 ? q2b : q2a);
-        const float2 A0 = tA[oa], A1 = tA[ob], B0 = tB[oa], B1 = tB[ob];
-        const float2 C0 = tC[oa], C1 = tC[ob];
-        // deconvolution per lane: the Gaussian's exp(b (pi k' / G)^2) / sqrt(pi b),
-        // or the plan's table
-        float2 D;
-        if constexpr (ES) {
-            // (a lane beyond the row repeats the first entry)
-            const float *dr = p.drow + (long long)rb * R * L2 + r;
-            D = make_float2(__ldg(dr + q2a * R), __ldg(dr + (q2b < L2 ? q2b : q2a) * R));
-        } else {
-            const float2 kf = make_float2((float)ka, (float)kb);
-            const float2 ex = __fmul2_rn(__fmul2_rn(kf, kf), dc1);
-            D = __fmul2_rn(make_float2(__expf(ex.x), __expf(ex.y)), dc2);
-        }
-        const float2 YCh = __fmul2_rn(make_float2(A0.x, A1.x), D);
-        const float2 YSh = __fmul2_rn(make_float2(A0.y, A1.y), D);
-        const float2 C = __fmul2_rn(make_float2(B0.x, B1.x), D);
-        const float2 S = __fmul2_rn(make_float2(B0.y, B1.y), D);
-        const float2 C2 = __fmul2_rn(make_float2(C0.x, C1.x), D);
-        const float2 S2 = __fmul2_rn(make_float2(C0.y, C1.y), D);
-        const float2 mC = make_float2(-C.x, -C.y), mS = make_float2(-S.x, -S.y);
-        const float2 YC = __ffma2_rn(nyw, C, YCh);
-        const float2 YS = __ffma2_rn(nyw, S, YSh);
-        const float2 CC = __ffma2_rn(mC, C, __ffma2_rn(half, C2, hw));
-        const float2 SS = __ffma2_rn(mS, S, __ffma2_rn(mhalf, C2, hw));
-        const float2 CS = __ffma2_rn(mC, S, __fmul2_rn(half, S2));
-        const float2 det = __ffma2_rn(make_float2(-CS.x, -CS.y), CS, __fmul2_rn(CC, SS));
-        const float2 a = __ffma2_rn(__fmul2_rn(mtwo, YS), CS, __fmul2_rn(YC, SS));
-        const float2 num = __ffma2_rn(YC, a, __fmul2_rn(__fmul2_rn(YS, YS), CC));
-        const float2 P = __fmul2_rn(make_float2(__fdividef(num.x, det.x),
-                                                __fdividef(num.y, det.y)), pn);
-        const float Pa = (P.x >= 0.f && !isinf(P.x)) ? P.x : -1.f;
-        const float Pb = (P.y >= 0.f && !isinf(P.y)) ? P.y : -1.f;
-        if (!BEST || outc) {
-            if (ina) outc[ka] = Pa;
-            if (inb) outc[kb] = Pb;
-        }
-        if (BEST) {
-            if (ina) keep(Pa, ka);
-            if (inb) keep(Pb, kb);
-        }
-    }
-    if (BEST) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const unsigned long long v = __shfl_xor_sync(0xffffffffu, key, o);
-            key = v > key ? v : key;
-        }
-        if ((tid & 31) == 0 && key != 0) atomicMax(gp.best + cv.best_slot, key);
-    }
-}
-
-template <int L2>
-__global__ void __launch_bounds__(pass2_threads(3, L2))
-k_pass2_gls(const DevCurve *cvs, const float2 *inter, float *__restrict__ out, Plan p,
-            GlsParams gp) {
-    constexpr int R = pass2_rows(3, L2);
-    constexpr int NT = pass2_threads(3, L2);
-    static_assert(NT % 32 == 0, "the best-power reduction needs full warps");
-    constexpr int LDS = row_stride(L2);
-    extern __shared__ __align__(16) float2 sm[];
-    float2 *tile = sm;
-    const int tid = threadIdx.x, rb = blockIdx.x;
-    if (p.dependent) {
-        pdl_trigger();
-        pdl_wait();
-    }
-    inter = written(inter);
-    const DevCurve cv = written(cvs)[blockIdx.y];
-    const int G1 = p.G1;
-    rows_fft<3, L2, R, NT, LDS>(tile, inter + cv.inter_off, p.st2, G1, p.G, p.B, rb, tid);
-    // The packed finish is compiled only into the 4-row tiles (rows of 256 to
-    // 1024: 256 threads at up to 64 registers, 4 CTAs per SM either way).
-    // In the 16-row tiles of short rows (480 threads) its extra registers
-    // would cost a CTA per SM (rows of 80: 37 -> 42 registers, 3 -> 2 CTAs,
-    // pass 2 43 -> 56 ms on 200,000 curves).
-    // (window and output kind chosen once per CTA: each finish is compiled
-    // for one window, with no per-frequency branch)
-    const bool es = p.win == kWinES;
-    if constexpr (R == 4) {
-        if (gp.mode == 1) {
-            if (es) {
-                if (gp.best) gls_epilogue_fm2<true, true, L2, R, NT, LDS>(tile, cv, out, gp, p, rb, tid);
-                else gls_epilogue_fm2<false, true, L2, R, NT, LDS>(tile, cv, out, gp, p, rb, tid);
-            } else {
-                if (gp.best) gls_epilogue_fm2<true, false, L2, R, NT, LDS>(tile, cv, out, gp, p, rb, tid);
-                else gls_epilogue_fm2<false, false, L2, R, NT, LDS>(tile, cv, out, gp, p, rb, tid);
-            }
-            return;
-        }
-    }
-    if (es) {
-        if (gp.best) gls_epilogue<true, true, L2, R, NT, LDS>(tile, cv, out, gp, p, rb, tid);
-        else gls_epilogue<false, true, L2, R, NT, LDS>(tile, cv, out, gp, p, rb, tid);
-    } else {
-        if (gp.best) gls_epilogue<true, false, L2, R, NT, LDS>(tile, cv, out, gp, p, rb, tid);
-        else gls_epilogue<false, false, L2, R, NT, LDS>(tile, cv, out, gp, p, rb, tid);
-    }
-}
-
 // Pass 2 of the GLS for rows of 4,096: one row of one curve per CTA of 256
 // threads.  Each grid's row is transformed in three levels of 16 with every
 // butterfly in registers: n = i + 256 k, i = j + 16 k', output
@@ -872,7 +671,8 @@ k_pass2_gls_cube(const DevCurve *cvs, const float2 *inter, float *__restrict__ o
     }
     inter = written(inter);
     const DevCurve cv = written(cvs)[blockIdx.y];
-    const int G1 = p.G1, G = (int)p.G, B = p.B;
+    constexpr int B = kGlsCols;
+    const int G1 = p.G1, G = (int)p.G;
     const int lo = tid & 15, hi = tid >> 4;
     // element l = tid + 256 k of the row lies at ((l / B) G1 + row) B + l % B
     const float2 *src = inter + cv.inter_off + ((long long)(tid / B) * G1 + q1r) * B + tid % B;
@@ -980,6 +780,150 @@ k_pass2_gls_cube(const DevCurve *cvs, const float2 *inter, float *__restrict__ o
     }
 }
 
+// Pass 2 of the GLS for rows of 512 to 2,048: R rows of one curve per CTA, each
+// grid transformed in three levels with every butterfly in registers, as
+// k_pass2_gls_cube: n = i + N1 k (N1 = 8 F1), i = j + 8 k', output q0 + F0 q1 +
+// F0 F1 qb.  Level 3 leaves the eight outputs of a thread in its registers for
+// the powers, which went back to shared memory and were read again before.
+// Per cell on grids of 320 columns: rows of 512 10.5 -> 7.1 ps, 640 8.5 -> 8.4,
+// 800 9.7 -> 8.8, 1,024 12.2 -> 10.1, 1,280 20.2 -> 11.2 (without the next grid's
+// loads ahead 7.6, 9.4, 10.5, 11.4, 11.8).  Held by latency: 13 to 24 warps per
+// SM between three barriers a grid.
+template <int L2, bool ES>
+__global__ void __launch_bounds__(deep_threads(L2), deep_ctas(L2))
+k_pass2_gls_deep(const DevCurve *cvs, const float2 *inter, float *__restrict__ out, const Plan p,
+                 const GlsParams gp) {
+    constexpr int R = deep_rows(L2), NT = deep_threads(L2);
+    constexpr int F0 = deep_fac(L2, 0), F1 = deep_fac(L2, 1), N1 = 8 * F1;
+    constexpr int P0 = deep_plane(L2), PR = deep_pitch(L2), T = L2 / 8;
+    static_assert(F0 * N1 == L2 && N1 % 4 == 0, "three levels");
+    extern __shared__ __align__(16) float2 sm[];
+    const int tid = threadIdx.x, rb = blockIdx.x;
+    if (p.dependent) {
+        pdl_trigger();
+        pdl_wait();
+    }
+    inter = written(inter);
+    const DevCurve cv = written(cvs)[blockIdx.y];
+    constexpr int lb = 2;
+    static_assert(1 << lb == kGlsCols, "blocks of four columns");
+    const int G1 = p.G1, G = (int)p.G;
+    const float2 *w1 = p.st2, *w2 = p.st2 + L2;
+    const float2 *src = inter + cv.inter_off + (long long)rb * R * kGlsCols;
+    const int kstride = N1 * G1;  // elements between column blocks of n and n + N1
+    const int r3 = tid % R, v3 = tid / R;  // level-3 unit: row, q1 = v3 % F1, q0 = v3 / F1
+    const bool act = NT == R * T || v3 < T;
+    float2 ya[8], yb[8], yc[8], x[F0];
+    // level-1 unit (ih, r, c), i = ih B + c
+    const bool one = N1 * R == NT || tid < N1 * R;
+    static_assert(N1 * R <= NT && F0 * 8 * R <= NT, "a unit per thread");
+    const int i1 = ((tid >> lb) / R << lb) + (tid & ((1 << lb) - 1)), r1 = (tid >> lb) % R;
+    src += (((long long)((tid >> lb) / R) * G1 + r1) << lb) + (tid & ((1 << lb) - 1));
+    // (volatile: the loads stay ahead of the levels they are to overlap)
+    auto fetch = [](const float2 *q) {
+        float2 v;
+        asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(q) : "memory");
+        return v;
+    };
+    if (one) {
+#pragma unroll
+        for (int k = 0; k < F0; ++k) x[k] = fetch(src + k * kstride);
+    }
+#pragma unroll
+    for (int g = 0; g < 3; ++g) {
+        if (one) RegDFT<F0>::run(x);
+        if (g) __syncthreads();  // the grid before is read
+        if (one) {
+            float2 *d = sm + r1 * PR + i1 + (i1 >> 3);
+            d[0] = x[0];
+#pragma unroll
+            for (int q = 1; q < F0; ++q) d[q * P0] = cmul(x[q], __ldg(w1 + q * N1 + i1));
+            if (g < 2) {  // the next grid's rows, in flight during levels 2 and 3
+                src += p.G;
+#pragma unroll
+                for (int k = 0; k < F0; ++k) x[k] = fetch(src + k * kstride);
+            }
+        }
+        __syncthreads();
+        // level 2: unit (r, q0, j), in place
+        if (F0 * 8 * R == NT || tid < F0 * 8 * R) {
+            const int j = tid & 7, q0 = (tid >> 3) % F0, r = (tid >> 3) / F0;
+            float2 *e = sm + r * PR + q0 * P0 + j, u[F1];
+#pragma unroll
+            for (int k = 0; k < F1; ++k) u[k] = e[9 * k];
+            RegDFT<F1>::run(u);
+            e[0] = u[0];
+#pragma unroll
+            for (int q = 1; q < F1; ++q) e[9 * q] = cmul(u[q], __ldg(w2 + q * 8 + j));
+        }
+        __syncthreads();
+        float2 *y = g == 0 ? ya : g == 1 ? yb : yc;
+        if (act) {
+            const float2 *e = sm + r3 * PR + (v3 / F1) * P0 + 9 * (v3 % F1);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) y[j] = e[j];
+            RegDFT<8>::run(y);
+        }
+    }
+    const int nf = cv.nf, h = nf / 2, lo_end = nf - h, hi_start = G - h;
+    const bool write = gp.best == nullptr || out != nullptr;
+    float *o = out + cv.out_off + h;
+    const int qv = v3 / F1 + F0 * (v3 % F1), q0 = rb * R + r3 + G1 * qv;
+    const float *drow = ES ? p.drow + ((long long)rb * L2 + qv) * R + r3 : nullptr;
+    const Fm2 fm(cv, gp.reg);
+    unsigned long long key = 0;
+    const unsigned ibase = (unsigned)(cv.best_off + h);
+    auto emit = [&](float P, int k) {
+        if (write) o[k] = P;
+        if (gp.best != nullptr && P >= 0.f) {  // valid powers only
+            const unsigned long long kk = ((unsigned long long)__float_as_uint(P) << 32) |
+                                          (0xFFFFFFFFu - (ibase + (unsigned)k));
+            key = kk > key ? kk : key;
+        }
+    };
+    // two frequencies at a time; f(qb, ka, kb, ina, inb, D)
+    auto pairs = [&](auto f) {
+#pragma unroll
+        for (int qb = 0; qb < 8; qb += 2) {
+            const int qA = q0 + G1 * T * qb, qB = qA + G1 * T;
+            const bool ina = qA < lo_end || qA >= hi_start;
+            const bool inb = qB < lo_end || qB >= hi_start;
+            if (!ina && !inb) continue;
+            const int ka = qA < lo_end ? qA : qA - G, kb = qB < lo_end ? qB : qB - G;
+            float2 D;
+            if constexpr (ES)
+                D = make_float2(__ldg(drow + T * R * qb), __ldg(drow + T * R * (qb + 1)));
+            else
+                D = make_float2(win_deconv<false>(ka, p), win_deconv<false>(kb, p));
+            f(qb, ka, kb, ina, inb, D);
+        }
+    };
+    if (act && gp.mode == 1) {
+        pairs([&](int qb, int ka, int kb, bool ina, bool inb, float2 D) {
+            const float2 pw = fm.power(ya[qb], ya[qb + 1], yb[qb], yb[qb + 1], yc[qb], yc[qb + 1], D);
+            if (ina) emit(pw.x, ka);
+            if (inb) emit(pw.y, kb);
+        });
+    } else if (act) {
+        auto one = [&](float2 A, float2 Bv, float2 C, float d) {
+            return gls_from_sums<float>(A.x * d, A.y * d, Bv.x * d, Bv.y * d, C.x * d, C.y * d,
+                                        gp.mode, gp.reg, cv.w_sum, cv.yw_sum, cv.ybar, cv.yy_inv);
+        };
+        pairs([&](int qb, int ka, int kb, bool ina, bool inb, float2 D) {
+            if (ina) emit(one(ya[qb], yb[qb], yc[qb], D.x), ka);
+            if (inb) emit(one(ya[qb + 1], yb[qb + 1], yc[qb + 1], D.y), kb);
+        });
+    }
+    if (gp.best != nullptr) {
+#pragma unroll
+        for (int of = 16; of > 0; of >>= 1) {
+            const unsigned long long v = __shfl_xor_sync(0xffffffffu, key, of);
+            key = v > key ? v : key;
+        }
+        if ((tid & 31) == 0 && key != 0) atomicMax(gp.best + cv.best_slot, key);
+    }
+}
+
 // Adjoint-NFFT finish of a pass-2 tile: deconvolution and the phase of the
 // absolute time origin, complex output per in-band frequency.
 template <bool ES, int L2, int R, int NT, int LDS>
@@ -1018,8 +962,7 @@ k_pass2_nfft(const DevCurve *cvs, const float2 *inter, float2 *__restrict__ out,
     inter = written(inter);
     aux = written(aux);
     const DevCurve cv = written(cvs)[blockIdx.y];
-    const int G1 = p.G1;
-    rows_fft<1, L2, R, NT, LDS>(tile, inter + cv.inter_off, p.st2, G1, p.G, p.B, rb, tid);
+    rows_fft_b<1, L2, R, NT, LDS, kNfftCols>(tile, inter + cv.inter_off, p.st2, p.G1, p.G, rb, tid);
 
     if (p.win == kWinES) nfft_finish<true, L2, R, NT, LDS>(tile, cv, out, aux, p, rb, tid);
     else nfft_finish<false, L2, R, NT, LDS>(tile, cv, out, aux, p, rb, tid);
@@ -1096,7 +1039,22 @@ cudaError_t launch_pass2_gls_t(const DevCurve *cv, int n_curves, int first, cons
     if constexpr (pass2_reg(3, L2)) {
         return p.win == kWinES ? launch_pass2_reg_t<L2, true>(cv, n_curves, first, inter, out, p, g, s)
                                : launch_pass2_reg_t<L2, false>(cv, n_curves, first, inter, out, p, g, s);
-    } else if constexpr (pass2_cube(3, L2)) {
+    } else if constexpr (pass2_deep(3, L2)) {
+        static size_t done[2][64] = {{0}};  // per window and device
+        const bool es = p.win == kWinES;
+        const size_t smem = (size_t)pass2_smem(3, L2);
+        cudaError_t e = es ? allow_smem(k_pass2_gls_deep<L2, true>, smem, done[1])
+                           : allow_smem(k_pass2_gls_deep<L2, false>, smem, done[0]);
+        if (e != cudaSuccess) return e;
+        const dim3 grid(p.G1 / deep_rows(L2), n_curves);
+        Plan q = p;
+        q.dependent = small_launch((long long)grid.x * grid.y);
+        return es ? launch_pdl(k_pass2_gls_deep<L2, true>, q.dependent, grid, deep_threads(L2), smem, s,
+                               cv, inter, out, q, g)
+                  : launch_pdl(k_pass2_gls_deep<L2, false>, q.dependent, grid, deep_threads(L2), smem, s,
+                               cv, inter, out, q, g);
+    } else {
+        static_assert(pass2_cube(3, L2), "no other rows");
         static size_t done[2][64] = {{0}};  // per window and device
         const bool es = p.win == kWinES;
         const size_t smem = (size_t)pass2_smem(3, L2);
@@ -1108,15 +1066,6 @@ cudaError_t launch_pass2_gls_t(const DevCurve *cv, int n_curves, int first, cons
         q.dependent = small_launch((long long)grid.x * grid.y);
         return es ? launch_pdl(k_pass2_gls_cube<true>, q.dependent, grid, 256, smem, s, cv, inter, out, q, g)
                   : launch_pdl(k_pass2_gls_cube<false>, q.dependent, grid, 256, smem, s, cv, inter, out, q, g);
-    } else {
-        static size_t done[64] = {0};  // per instantiation
-        cudaError_t e = allow_smem(k_pass2_gls<L2>, (size_t)pass2_smem(3, L2), done);
-        if (e != cudaSuccess) return e;
-        const dim3 grid(p.G1 / pass2_rows(3, L2), n_curves);
-        Plan q = p;
-        q.dependent = small_launch((long long)grid.x * grid.y);
-        return launch_pdl(k_pass2_gls<L2>, q.dependent, grid, pass2_threads(3, L2),
-                          (size_t)pass2_smem(3, L2), s, cv, inter, out, q, g);
     }
 }
 
@@ -1167,13 +1116,14 @@ cudaError_t preload_pass2_t(int ng) {
         }
         const cudaError_t e = cudaFuncGetAttributes(&a, k_pass2_gls_reg<L2, true>);
         return e != cudaSuccess ? e : cudaFuncGetAttributes(&a, k_pass2_gls_reg<L2, false>);
-    } else if constexpr (pass2_cube(3, L2)) {
+    } else if constexpr (pass2_deep(3, L2)) {
+        if (ng != 3) return cudaFuncGetAttributes(&a, k_pass2_nfft<L2>);
+        const cudaError_t e = cudaFuncGetAttributes(&a, k_pass2_gls_deep<L2, true>);
+        return e != cudaSuccess ? e : cudaFuncGetAttributes(&a, k_pass2_gls_deep<L2, false>);
+    } else {
         if (ng != 3) return cudaFuncGetAttributes(&a, k_pass2_nfft<L2>);
         const cudaError_t e = cudaFuncGetAttributes(&a, k_pass2_gls_cube<true>);
         return e != cudaSuccess ? e : cudaFuncGetAttributes(&a, k_pass2_gls_cube<false>);
-    } else {
-        return ng == 3 ? cudaFuncGetAttributes(&a, k_pass2_gls<L2>)
-                       : cudaFuncGetAttributes(&a, k_pass2_nfft<L2>);
     }
 }
 

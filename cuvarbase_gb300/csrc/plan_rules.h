@@ -211,16 +211,49 @@ CUVGLS_HD constexpr bool pass2_reg(int ng, int L2) {
 CUVGLS_HD constexpr bool pass2_cube(int ng, int L2) { return ng == 3 && L2 == 4096; }
 constexpr int kCubePitch = 257;   // of its exchange tile: 16 planes of 256 elements
 
-// Rows per pass-2 CTA for ng grids of row length L2: 16 for short rows, so
-// that a CTA still transforms a few thousand elements; 8 for the other
-// register rows (32-byte runs of powers); 4 for the three-grid GLS rows of
-// 512..1024 (more, smaller CTAs per SM overlap one CTA's loads with another's
-// arithmetic); 8 otherwise; halved until the tile fits (2 at least, 1 only for
-// the 4096-long rows).
+// Whether the GLS rows of this length go through k_pass2_gls_deep: three levels
+// F0, F1 and F2 = 8 (the outputs of each grid per thread); the exchange tile's
+// slot of element j + 8 k of plane q0 is q0 P0 + 9 k + j.
+CUVGLS_HD constexpr int deep_fac(int L2, int level) {
+    if (level == 2) return 8;
+    const int f0 = L2 == 512 ? 8 : L2 == 640 || L2 == 800 ? 10 : L2 == 1600 ? 20 : 16;
+    return level == 0 ? f0 : L2 / 8 / f0;
+}
+CUVGLS_HD constexpr bool pass2_deep(int ng, int L2) {
+    return ng == 3 && !pass2_reg(3, L2) && !pass2_cube(3, L2);
+}
+CUVGLS_HD constexpr int deep_rows(int L2) { return L2 <= 800 ? 4 : 2; }
+CUVGLS_HD constexpr int deep_threads(int L2) { return (deep_rows(L2) * L2 / 8 + 31) / 32 * 32; }
+// CTAs per SM: as many as the registers of three grids' outputs and one
+// butterfly allow (measured: 512 8.6 ps per cell with two, 7.1 with three; 1,024
+// 10.7 and 10.1; 640, 800 and 1,280 are slower with three).
+CUVGLS_HD constexpr int deep_ctas(int L2) {
+    return L2 == 512 || L2 == 1024 ? 3 : L2 == 2048 ? 1 : 2;
+}
+// pitches that keep every access free of bank conflicts: planes 8 (mod 16)
+// apart, rows 4 (of four) or 8 (of two)
+CUVGLS_HD constexpr int deep_plane(int L2) { return (9 * deep_fac(L2, 1) + 7) / 16 * 16 + 8; }
+CUVGLS_HD constexpr int deep_pitch(int L2) {
+    return (deep_fac(L2, 0) * deep_plane(L2) + 15) / 16 * 16 + 16 / deep_rows(L2);
+}
+// Entries of the row table: exp(2 pi i q0 i / L2) as [q0][i], then
+// exp(2 pi i q1 j / (8 F1)) as [q1][j].
+CUVGLS_HD constexpr int deep_table_len(int L2) { return L2 + L2 / deep_fac(L2, 0); }
+
+CUVGLS_HD constexpr int row_table_len(int ng, int L2) {
+    return pass2_deep(ng, L2) ? deep_table_len(L2) : fft_table_len(L2);
+}
+
+// Rows per pass-2 CTA for ng grids of row length L2: 16 for short register
+// rows, so that a CTA still transforms a few thousand elements; 8 for the other
+// register rows (32-byte runs of powers); 4 or 2 for the longer GLS rows, 1 for
+// those of 4,096; for the one-grid rows beyond, 16 or as many as fit the tile.
 CUVGLS_HD constexpr int pass2_rows(int ng, int L2) {
     if (pass2_reg(ng, L2)) return L2 <= 160 ? 16 : 8;
-    int r = (ng == 1 || L2 <= 160) ? 16 : (L2 <= 1024 ? 4 : 8);
-    while (r > (L2 > 2048 ? 1 : 2) && !tile_fits(ng * r, L2)) r /= 2;
+    if (pass2_deep(ng, L2)) return deep_rows(L2);
+    if (pass2_cube(ng, L2)) return 1;
+    int r = 16;
+    while (r > 2 && !tile_fits(ng * r, L2)) r /= 2;
     return r;
 }
 
@@ -252,13 +285,14 @@ CUVGLS_HD constexpr int pass2_reg_tile(int L2) {
 }
 // k_pass2_nfft_reg: in place in one tile, four CTAs per SM (1,000 curves of
 // 512 x 400 cells 0.431 ms; 0.442 with a tile ahead, 0.452 with five CTAs).
-constexpr int kNfftCols = 8;  // columns per pass-1 block of every one-grid plan
-CUVGLS_HD constexpr bool nfft_cols_ok() {
+// (columns per pass-1 block of every one-grid plan, and of every GLS plan)
+constexpr int kNfftCols = 8, kGlsCols = 4;
+CUVGLS_HD constexpr bool cols_ok() {
     for (int l : kLens)
-        if (pass1_cols(1, l) != kNfftCols) return false;
+        if (pass1_cols(1, l) != kNfftCols || pass1_cols(3, l) != kGlsCols) return false;
     return true;
 }
-static_assert(nfft_cols_ok(), "k_pass2_nfft_reg reads blocks of eight columns");
+static_assert(cols_ok(), "pass 2 reads blocks of eight and of four columns");
 constexpr int kNfftRegCtas = 4;
 CUVGLS_HD constexpr int nfft_reg_elems(int L2) {
     return pass2_reg_exch(L2) + L2 / two_level_la(L2);
@@ -356,6 +390,7 @@ CUVGLS_HD constexpr long long pass1_smem(int ng, int L1, long long G) {
 CUVGLS_HD constexpr long long pass2_smem(int ng, int L2) {
     if (pass2_reg(ng, L2))
         return ((ng == 3 ? pass2_reg_elems(L2) : nfft_reg_elems(L2)) + 2LL) * 8;
+    if (pass2_deep(ng, L2)) return 8LL * deep_rows(L2) * deep_pitch(L2);
     if (pass2_cube(ng, L2)) return (16LL * kCubePitch + L2) * 8;  // exchange tile, grid A
     return (long long)(ng * pass2_rows(ng, L2) * row_stride(L2) +
                        (two_level_la(L2) ? 0 : fft_table_len(L2))) * 8;
