@@ -88,6 +88,50 @@ __device__ __forceinline__ int4 fx_pack(Cx v) { return make_int4(v.x.h, v.x.l, v
 __device__ __forceinline__ Cx fx_unpack(int4 v) { return Cx{Fx{v.x, v.y}, Fx{v.z, v.w}}; }
 __device__ __forceinline__ i64 fx_join(Fx a) { return ((i64)a.h << 27) + a.l; }
 
+// Phasors of multiples of 1 / kTurn of a turn, as products of kTurnCoarse and
+// kTurnFine steps (in shared memory: the coarse ones, then the fine ones).
+constexpr int kTurn = 2048, kTurnCoarse = 64, kTurnFine = kTurn / kTurnCoarse;
+
+__device__ __forceinline__ void turn_steps(int4 *step, int tid) {
+    for (int i = tid; i < kTurnCoarse + kTurnFine; i += kDirThreads)
+        step[i] = fx_pack(fx_unit(zturn(i < kTurnCoarse ? (double)i / kTurnCoarse
+                                                        : (double)(i - kTurnCoarse) / kTurn)));
+}
+__device__ __forceinline__ Cx turn_product(const int4 *step, int k) {
+    return fx_cmul(fx_unpack(step[k / kTurnFine]), fx_unpack(step[kTurnCoarse + k % kTurnFine]));
+}
+
+// exp(2 pi i p) of a finite p: the phasor at the nearest multiple of 1 / kTurn
+// turned by the remaining angle d, |d| <= pi / kTurn, all of it in integers
+// (FP64 forms p only): d and sin d in units of 2^-61, cos d - 1 = -d^2 / 2 +
+// d^4 / 24 the same, the small terms d^3 / 6 - d^5 / 120 (6e-10) and d^4 / 24
+// (2e-13) in FP32; those left out are below 2e-20.
+template <typename Table>
+__device__ __forceinline__ Cx fx_turn(double p, Table table) {
+    const u64 th = turns64(p);
+    const int k = (int)((th + (1ULL << 52)) >> 53);  // 0 .. kTurn
+    const Cx e = table(k & (kTurn - 1));
+    const Fx r = fx_split((i64)(th - ((u64)k << 53)));  // |r| <= 2^52, in 2^-64 turns
+    constexpr i64 kTwoPi = 14148475504056880LL;        // 2 pi 2^51
+    constexpr int kHi = (int)((kTwoPi + (1 << 26)) >> 27), kLo = (int)(kTwoPi - ((i64)kHi << 27));
+    const i64 d = fx_fma(r, Fx{kHi, kLo}, 0);
+    const int dh = (int)(d >> 21), dl = (int)(d & ((1 << 21) - 1));
+    const float df = (float)dh * 9.094947017729282e-13f, q = df * df;  // 2^-40
+    const float kUp = 2305843009213693952.f;                           // 2^61
+    const Fx sn = fx_split(d + __float2int_rn(kUp * df * q * fmaf(q, 1.f / 120.f, -1.f / 6.f)));
+    const i64 d2 = fx_wide(dh, dh, fx_wide(dh, dl, 0) >> 20);  // 2^-80
+    const Fx cm = fx_split(__float2int_rn(kUp * q * q * (1.f / 24.f)) - (d2 >> 20));
+    // e + e (cm + i sn), the product in units of 2^-63
+    const i64 re = fx_fma(cm, e.x, 64) - fx_fma(sn, e.y, 0), im = fx_fma(cm, e.y, fx_fma(sn, e.x, 64));
+    return Cx{fx_split(fx_join(e.x) + (re >> 7)), fx_split(fx_join(e.y) + (im >> 7))};
+}
+
+// An eighth of a warp's sum, so that the eight warps' add up in integers: a
+// conversion to FP64 costs as much as an FP64 instruction (one per warp and sum:
+// 0.468 against 0.450 ms of the GLS sums).
+static_assert(kDirWarps == 8, "eighths");
+__device__ __forceinline__ i64 fx_eighth(i64 v) { return (v + 4) >> 3; }
+
 // Points of a run (one CTA, sums in 64-bit integers) and its headroom: 2^(5 +
 // hr) terms per warp.
 constexpr int kDirRun = 1024 * kDirWarps;
@@ -122,12 +166,14 @@ struct DirTable {
     static constexpr int kRows = NB + kCoarse + kFine;
     int4 row[kRows][32];
 
-    // This lane's point: x in turns per bin, th0 the phase of K0 in turns.
-    // Two sincospi, the rest by products of depth at most 8.
-    __device__ __forceinline__ void build(int lane, double x, double th0) {
+    // This lane's point: x in turns per bin, th0 the phase of K0 in turns;
+    // `steps` from turn_steps.  Two phasors, the rest by products of depth at
+    // most 8.
+    __device__ __forceinline__ void build(int lane, double x, double th0, const int4 *steps) {
+        auto table = [&](int k) { return turn_product(steps, k); };
         static_assert(NB >= M, "the centre step is built from step phasor M");
         Cx z[NB + 1];
-        z[1] = fx_unit(zturn(x));
+        z[1] = fx_turn(x, table);
 #pragma unroll
         for (int b = 2; b <= NB; ++b) z[b] = fx_cmul(z[b / 2], z[b - b / 2]);
 #pragma unroll
@@ -141,7 +187,7 @@ struct DirTable {
 #pragma unroll
         for (int k = 0; k < kFine; ++k) row[NB + kCoarse + k][lane] = fx_pack(f[k]);
         const Cx w8 = fx_cmul(f[kFine / 2], f[kFine / 2]);
-        Cx c = fx_unit(zturn(th0));
+        Cx c = fx_turn(th0, table);
 #pragma unroll
         for (int k = 0; k < kCoarse; ++k) {
             row[NB + k][lane] = fx_pack(c);
@@ -198,14 +244,15 @@ __device__ __forceinline__ void dir_reduce(const DirSums<M> &v, i64 *red, int ti
 #pragma unroll
     for (int q = 0; q < (TB + kDirThreads - 1) / kDirThreads; ++q) {
         const int b = tid + q * kDirThreads;
-        double re = 0.0, im = 0.0;
+        i64 re = 0, im = 0;
         if (b < TB)
+#pragma unroll
             for (int w = 0; w < kDirWarps; ++w) {
-                re += (double)red[w * TB + b];
-                im += (double)red[(kDirWarps + w) * TB + b];
+                re += fx_eighth(red[w * TB + b]);
+                im += fx_eighth(red[(kDirWarps + w) * TB + b]);
             }
-        out[q].x += scalbn(re, unit);
-        out[q].y += scalbn(im, unit);
+        out[q].x += scalbn((double)re, unit + 3);
+        out[q].y += scalbn((double)im, unit + 3);
     }
 }
 
@@ -233,24 +280,26 @@ static_assert(kNfSmem >= 2 * kDirWarps * kNfBins * 8, "the reduction reuses the 
 // One CTA per (416 bins, curve, part of its points); its eight warps take the
 // points 32 at a time in turn, each with tables of its own, and are summed in
 // shared memory at the end.  A curve cut into several parts leaves partial
-// sums for k_nfft_direct64_sum.  Bound by the wide multiply-adds, and by the
-// FP64 sincospi of the tables.  4 curves of 300 to 2,000 points and 20,000
+// sums for k_nfft_direct64_sum.  Bound by the wide multiply-adds.  4 curves of 300 to 2,000 points and 20,000
 // bins, host to host: 5.67 ms with a sincospi pair per point and 8 bins, 0.45 ms
 // with factored phasors in FP64 (2.4 instructions per bin, 93 % busy), 0.235 ms
-// in fixed point (0.242 ms with M = 8, 0.273 with M = 4); errors against 64 bits
-// 6.8e-13 in all of them.
+// in fixed point (0.242 ms with M = 8, 0.273 with M = 4), 0.223 ms with the
+// warps' sums and the phasors of the tables in integers too; errors against 64
+// bits 6.8e-13 in all of them.
 __global__ void __launch_bounds__(kDirThreads, 2)
 k_nfft_direct64(const Direct64Curve *__restrict__ cvs, const double *__restrict__ t,
                 const double *__restrict__ y, double2 *__restrict__ out,
                 double2 *__restrict__ part, long long part_stride) {
     extern __shared__ __align__(16) double sm[];
     __shared__ u64 top;
+    __shared__ int4 steps[kTurnCoarse + kTurnFine];
     const Direct64Curve cv = cvs[blockIdx.y];
     const long long k0 = (long long)blockIdx.x * kNfBins;
     long long j0, j1;
     if (k0 >= cv.nf || !dir_part(cv.n, cv.splits, blockIdx.z, j0, j1)) return;  // whole CTA
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     NfTable &tab = reinterpret_cast<NfTable *>(sm)[wid];
+    turn_steps(steps, tid);  // (the barriers below come before its first use)
     constexpr int NQ = (kNfBins + kDirThreads - 1) / kDirThreads;
     double2 v[NQ];
 #pragma unroll
@@ -282,7 +331,7 @@ k_nfft_direct64(const Direct64Curve *__restrict__ cvs, const double *__restrict_
                 b -= floor(b);
                 const double th = fma(kc, b, a);
                 lost = lost || !isfinite(th);
-                tab.build(lane, b, th);
+                tab.build(lane, b, th, steps);
                 const Fx yv = fx_split(__double2ll_rn(scalbn(yj, 55 - hr - ex)));
 #pragma unroll
                 for (int g = 0; g < kCoarse; ++g) {  // y rides on the coarse centres
@@ -403,7 +452,8 @@ __device__ __forceinline__ float gls_direct_power(const DevCurve &cv, const GlsP
 // partial sums for k_gls_direct_sum.  8 curves of 300 to 2,000 points and
 // 10,000 frequencies: 9.62 ms with a sincospi each, 1.10 ms with factored
 // phasors in FP64 (7.7 instructions per frequency, 81 % busy), 0.47 ms in fixed
-// point (0.61 ms with M = 4 and one CTA per SM); errors against 64 bits 2.8e-8
+// point (0.61 ms with M = 4 and one CTA per SM), 0.44 ms with the warps' sums
+// and the phasors of the tables in integers too; errors against 64 bits 2.8e-8
 // in all of them.
 __global__ void __launch_bounds__(kDirThreads, 2)
 k_gls_direct(const DevCurve *__restrict__ cvs, const double *__restrict__ t,
@@ -411,12 +461,14 @@ k_gls_direct(const DevCurve *__restrict__ cvs, const double *__restrict__ t,
              double2 *__restrict__ part, long long part_stride, GlsParams gp) {
     extern __shared__ __align__(16) double sm[];
     __shared__ u64 top[2];
+    __shared__ int4 steps[kTurnCoarse + kTurnFine];
     const DevCurve cv = cvs[blockIdx.y];
     const long long k0 = (long long)blockIdx.x * kGlBins;
     long long j0, j1;
     if (k0 >= cv.nf || !dir_part(cv.n, cv.aux, blockIdx.z, j0, j1)) return;  // whole CTA
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     GlTile &tile = reinterpret_cast<GlTile *>(sm)[wid];
+    turn_steps(steps, tid);  // (the barriers below come before its first use)
     constexpr int NQ = (kGlBins + kDirThreads - 1) / kDirThreads;
     double2 va[NQ], vb[NQ], vc[NQ];
 #pragma unroll
@@ -446,7 +498,7 @@ k_gls_direct(const DevCurve *__restrict__ cvs, const double *__restrict__ t,
                 const long long j = cv.pt_off + base + lane;
                 const double x = (t[j] - t0) * cv.df;
                 lost = lost || !isfinite(kc * x);
-                tile.tab.build(lane, x, kc * x);
+                tile.tab.build(lane, x, kc * x, steps);
                 const Fx fy = fx_split(__double2ll_rn(scalbn((double)yw[j], 55 - hr - ey)));
                 const Fx fw = fx_split(__double2ll_rn(scalbn((double)w[j], 55 - hr - ew)));
                 tile.yw[lane] = make_int2(fy.h, fy.l);
@@ -540,33 +592,6 @@ cudaError_t launch_gls_direct(const DevCurve *cv, int n_curves, int max_nf, int 
 // ---------------------------------------------------------------------------
 namespace {
 
-// Phasors of the shared turn table, from kTurnCoarse by kTurnFine products.
-constexpr int kTurn = 2048, kTurnCoarse = 64, kTurnFine = kTurn / kTurnCoarse;
-
-// exp(2 pi i p) of a finite p: the phasor at the nearest multiple of 1 / kTurn
-// turned by the remaining angle d, |d| <= pi / kTurn, all of it in integers
-// (FP64 forms p only): d and sin d in units of 2^-61, cos d - 1 = -d^2 / 2 +
-// d^4 / 24 the same, the small terms d^3 / 6 - d^5 / 120 (6e-10) and d^4 / 24
-// (2e-13) in FP32; those left out are below 2e-20.
-__device__ __forceinline__ Cx table_turn(double p, const int4 *tab) {
-    const u64 th = turns64(p);
-    const int k = (int)((th + (1ULL << 52)) >> 53);  // 0 .. kTurn
-    const Cx e = fx_unpack(tab[k & (kTurn - 1)]);
-    const Fx r = fx_split((i64)(th - ((u64)k << 53)));  // |r| <= 2^52, in 2^-64 turns
-    constexpr i64 kTwoPi = 14148475504056880LL;        // 2 pi 2^51
-    constexpr int kHi = (int)((kTwoPi + (1 << 26)) >> 27), kLo = (int)(kTwoPi - ((i64)kHi << 27));
-    const i64 d = fx_fma(r, Fx{kHi, kLo}, 0);
-    const int dh = (int)(d >> 21), dl = (int)(d & ((1 << 21) - 1));
-    const float df = (float)dh * 9.094947017729282e-13f, q = df * df;  // 2^-40
-    const float kUp = 2305843009213693952.f;                           // 2^61
-    const Fx sn = fx_split(d + __float2int_rn(kUp * df * q * fmaf(q, 1.f / 120.f, -1.f / 6.f)));
-    const i64 d2 = fx_wide(dh, dh, fx_wide(dh, dl, 0) >> 20);  // 2^-80
-    const Fx cm = fx_split(__float2int_rn(kUp * q * q * (1.f / 24.f)) - (d2 >> 20));
-    // e + e (cm + i sn), the product in units of 2^-63
-    const i64 re = fx_fma(cm, e.x, 64) - fx_fma(sn, e.y, 0), im = fx_fma(cm, e.y, fx_fma(sn, e.x, 64));
-    return Cx{fx_split(fx_join(e.x) + (re >> 7)), fx_split(fx_join(e.y) + (im >> 7))};
-}
-
 // rows of sums a CTA reduces: c, s (2H each), yc, ys (H each), and sum w
 __host__ __device__ constexpr int mh_sums(int H) { return 6 * H + 1; }
 __host__ __device__ constexpr int mh_smem(int H) {
@@ -592,7 +617,7 @@ __host__ __device__ constexpr int mh_smem(int H) {
 // frequencies, host to host: 4.93 ms with a sincospi per point; in FP64 2.24 ms
 // with the table and the clusters (54 instructions per point and frequency, the
 // pipes 88 % busy), 1.97 ms with the recurrence, 1.54 ms with the phasor's
-// fraction in integers; 0.79 ms in fixed point (about 100 wide multiply-adds).
+// fraction in integers; 0.76 ms in fixed point (about 100 wide multiply-adds).
 // Errors against 64 bits 1.8e-13 in all of them: that of the FP64 phase t f.
 template <int H>
 __global__ void __launch_bounds__(kDirThreads, H <= 4 ? 2 : 1)
@@ -605,18 +630,16 @@ k_mhgls_direct(const double *__restrict__ t, const double *__restrict__ yw,
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     __shared__ u64 top[2];
     int4 *turn = reinterpret_cast<int4 *>(sm);
-    double *tiles = sm + 2 * kTurn, *sums = tiles + kDirWarps * 96;
+    double *tiles = sm + 2 * kTurn;
+    i64 *sums = reinterpret_cast<i64 *>(tiles + kDirWarps * 96);
+    double *tot = tiles + kDirWarps * 96 + kDirWarps * NS * 32;
     double *st = tiles + wid * 96;
     int2 *sy = reinterpret_cast<int2 *>(st + 32), *sw = sy + 32;
-    {  // the coarse and fine steps (in the point tiles' memory), then their products
+    {  // the steps (in the point tiles' memory), then all their products
         int4 *step = reinterpret_cast<int4 *>(tiles);
-        for (int i = tid; i < kTurnCoarse + kTurnFine; i += kDirThreads)
-            step[i] = fx_pack(fx_unit(zturn(i < kTurnCoarse ? (double)i / kTurnCoarse
-                                                            : (double)(i - kTurnCoarse) / kTurn)));
+        turn_steps(step, tid);
         __syncthreads();
-        for (int i = tid; i < kTurn; i += kDirThreads)
-            turn[i] = fx_pack(fx_cmul(fx_unpack(step[i / kTurnFine]),
-                                      fx_unpack(step[kTurnCoarse + i % kTurnFine])));
+        for (int i = tid; i < kTurn; i += kDirThreads) turn[i] = fx_pack(turn_product(step, i));
         __syncthreads();
     }
     const long long k = (long long)(blockIdx.x / csize) * 32 + lane;
@@ -625,8 +648,8 @@ k_mhgls_direct(const double *__restrict__ t, const double *__restrict__ yw,
     // a phase that is not finite (of this lane's frequency), a value that is not
     bool lost = false, odd = false;
     // the warps' sums, in shared memory as [warp][sum][lane]
-    double *r = sums + wid * NS * 32 + lane;
-    for (int i = 0; i < NS; ++i) r[i * 32] = 0.0;
+    i64 *r = sums + wid * NS * 32 + lane;
+    for (int i = tid; i < NS * 32; i += kDirThreads) tot[i] = 0.0;
     const long long share = (n + csize - 1) / csize;
     const long long j1 = min(n, (rank + 1) * share);
     for (long long r0 = rank * share; r0 < j1; r0 += kDirRun) {  // one run, but for very long curves
@@ -666,7 +689,7 @@ k_mhgls_direct(const double *__restrict__ t, const double *__restrict__ yw,
                 const Fx wq{vw.x, vw.y}, yq{vy.x, vy.y};
                 const double p = st[q] * f;
                 lost = lost || (__double2hiint(p) & 0x7ff00000) == 0x7ff00000;
-                Cx z = table_turn(p, turn), zp{Fx{1 << 29, 0}, Fx{0, 0}};  // power m, m - 1
+                Cx z = fx_turn(p, [&](int i) { return fx_unpack(turn[i]); }), zp{Fx{1 << 29, 0}, Fx{0, 0}};  // power m, m - 1
                 const Fx cc = fx_split(2 * fx_join(z.x));                 // 2 cos
 #pragma unroll
                 for (int m = 1; m <= NH; ++m) {
@@ -687,25 +710,32 @@ k_mhgls_direct(const double *__restrict__ t, const double *__restrict__ yw,
         }
 #pragma unroll
         for (int m = 1; m <= NH; ++m) {
-            r[(m - 1) * 32] += scalbn((double)c[m], ew + hr - 57);
-            r[(NH + m - 1) * 32] += scalbn((double)s[m], ew + hr - 57);
+            r[(m - 1) * 32] = c[m];
+            r[(NH + m - 1) * 32] = s[m];
         }
 #pragma unroll
         for (int m = 1; m <= H; ++m) {
-            r[(2 * NH + m - 1) * 32] += scalbn((double)yc[m], ey + hr - 57);
-            r[(2 * NH + H + m - 1) * 32] += scalbn((double)ys[m], ey + hr - 57);
+            r[(2 * NH + m - 1) * 32] = yc[m];
+            r[(2 * NH + H + m - 1) * 32] = ys[m];
         }
+        __syncthreads();
+        for (int i = tid; i < (NS - 1) * 32; i += kDirThreads) {
+            i64 v = 0;
+            for (int q = 0; q < kDirWarps; ++q) v += fx_eighth(sums[q * NS * 32 + i]);
+            tot[i] += scalbn((double)v, (i < 2 * NH * 32 ? ew : ey) + hr - 54);
+        }
+        __syncthreads();  // before the next run's sums
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) ws += __shfl_xor_sync(0xffffffffu, ws, o);
+    // (a value that is not finite spoils every frequency, a phase its own)
     if (__syncthreads_or(odd) || lost) ws = nan("");
-    r[6 * H * 32] = ws;
+    r[6 * H * 32] = __double_as_longlong(ws);
     __syncthreads();
-    double *tot = sums + kDirWarps * NS * 32;
-    for (int i = tid; i < NS * 32; i += kDirThreads) {
+    if (tid < 32) {
         double v = 0.0;
-        for (int q = 0; q < kDirWarps; ++q) v += sums[q * NS * 32 + i];
-        tot[i] = v;
+        for (int q = 0; q < kDirWarps; ++q) v += __longlong_as_double(sums[(q * NS + 6 * H) * 32 + tid]);
+        tot[6 * H * 32 + tid] = v;
     }
     if (csize > 1) {
         cg::cluster_group cl = cg::this_cluster();
