@@ -36,7 +36,10 @@ constexpr int kNumRowLens = sizeof(kRowLens) / sizeof(kRowLens[0]);
 // curve and 6.1 would make 320 x 80 beat 160 x 160 at nf = 2e4, measured 8 %
 // slower on these curves.)  Pass 1
 // also pays per point (~0.23 ns per point of the curve, whatever the shape),
-// which the shape choice can leave out.
+// which the shape choice can leave out.  (The kernels have become faster since,
+// unevenly: rows of 400 6.3 ps, 160 5.6, 512 7.0, 640 8.4, 800 8.8, 1,024 10,
+// 1,280 11, 4,096 about 13, columns of 2,048 about 10.  The entries are kept, so
+// that a number of frequencies keeps its grid.)
 constexpr float kPass1PsPerCell[] = {18.f /*16*/, 8.f /*32*/, 7.5f /*64 **/, 8.6f /*80*/,
                                      7.f /*128 **/, 6.4f /*160*/, 7.1f /*256*/, 6.5f /*320*/,
                                      6.3f /*400*/, 6.8f /*512*/, 6.f /*640*/, 6.8f /*800*/,

@@ -61,7 +61,7 @@ extern "C" {
 #define CUVGLS_DEVERR_BINNING 4   /* binning count and scatter disagreed (records dropped) */
 
 /* largest number of points of one curve (kernels index points of a curve in
- * 32 bits, in segments of 1024) */
+ * 32 bits, in segments of 4096) */
 #define CUVGLS_MAX_CURVE_POINTS 2147482623LL
 
 typedef struct cuvgls_handle cuvgls_handle;
