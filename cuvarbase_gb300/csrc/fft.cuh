@@ -205,8 +205,8 @@ __device__ __forceinline__ void tile_fft(float2 *__restrict__ buf,
 //   stage B, per (vector, qa): X[qa + La qb] = sum_i Y_i[qa] W_Lb^(i qb),
 //            read from the contiguous block Lb qa .. Lb qa + Lb - 1.
 // Both DFTs run in registers with compile-time twiddles.  The stage-A
-// twiddles W_L^(i qa) come from a [qa][i] table (consecutive threads read
-// consecutive entries).  With the padding, the strided reads of stage B
+// twiddles W_L^(i qa) come from a table, two of a thread's to a load
+// (consecutive threads read consecutive entries).  With the padding, the strided reads of stage B
 // (stride Lb + 1, odd) and all other accesses are free of bank conflicts.
 // ===========================================================================
 
@@ -315,8 +315,18 @@ __device__ __forceinline__ void fft2_stage_a_regs(float2 (&x)[two_level_la(L)],
     constexpr int LA = two_level_la(L);
     constexpr int LB = L / LA;
     RegDFT<LA>::run(x);
+    if constexpr (tw_pairs(L)) {
+        const float4 *t = reinterpret_cast<const float4 *>(twa) + i;
 #pragma unroll
-    for (int qa = 1; qa < LA; ++qa) x[qa] = cmul(x[qa], __ldg(twa + qa * LB + i));
+        for (int p = 0; p < (LA + 1) / 2; ++p) {
+            const float4 w = __ldg(t + p * LB);
+            if (p > 0) x[2 * p] = cmul(x[2 * p], make_float2(w.x, w.y));
+            if (2 * p + 1 < LA) x[2 * p + 1] = cmul(x[2 * p + 1], make_float2(w.z, w.w));
+        }
+    } else {
+#pragma unroll
+        for (int qa = 1; qa < LA; ++qa) x[qa] = cmul(x[qa], __ldg(twa + qa * LB + i));
+    }
 }
 
 // Stage A over every vector of a tile, in place (no barrier at the end).

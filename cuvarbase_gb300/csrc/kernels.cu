@@ -124,12 +124,13 @@ cudaError_t launch_grid_finish(const GridFinishCurve *cv, int n_curves, long lon
 // plan tables (FP64 angles, rounded once to float)
 // ---------------------------------------------------------------------------
 // Turns (fraction of a full turn) of entry e of the FFT table of a length-L
-// transform, in the layout the pass kernels read: [qa][i] stage-A twiddles
-// i qa / L of a two-level length, else [stage][r - 1][k] Stockham twiddles.
+// transform, in the layout the pass kernels read: the stage-A twiddles i qa / L of
+// a two-level length (fft_table_len), else [stage][r - 1][k] Stockham twiddles.
 __device__ double fft_table_turns(int L, int e) {
     if (two_level_la(L) > 0) {
         const int LB = L / two_level_la(L);
-        const int qa = e / LB, i = e % LB;
+        const bool pr = tw_pairs(L);
+        const int i = pr ? e / 2 % LB : e % LB, qa = pr ? e / (2 * LB) * 2 + e % 2 : e / LB;
         return (double)(i * qa) / (double)L;
     }
     const FacList f = fft_factors(L);
