@@ -16,6 +16,10 @@
 // table's scattered reads.  2,000 curves of 320 x 400 cells 1.80 -> 1.61 ms
 // (now at 53 % issue, 51 % of the L1 pipe and of DRAM), 20,000 of 160 x 160
 // 4.11 -> 2.81 ms (the old tile also had two- to four-way bank conflicts).
+//   NARROW  sigma >= kNarrowSigma: only the outputs near both ends of a row can
+//     be in band; the rest are neither finished nor kept, and grid A is not
+//     parked.  400 curves of 1024 x 400 cells at sigma 4 833 -> 774 us (781 with a
+//     second tile in flight in the memory that frees, 981 with five CTAs per SM).
 #pragma once
 
 #include <cuda.h>
@@ -117,21 +121,21 @@ struct Fm2 {
     }
 };
 
-template <int L2, bool ES>
+template <int L2, bool ES, bool NARROW>
 __global__ void __launch_bounds__(pass2_reg_threads(L2), pass2_reg_ctas(L2))
 k_pass2_gls_reg(const __grid_constant__ CUtensorMap map, const DevCurve *cvs,
                 int n_curves, int first, float *__restrict__ out, const Plan p, const GlsParams gp) {
     constexpr int LA = two_level_la(L2), LB = L2 / LA;
     constexpr int R = pass2_rows(3, L2), NT = pass2_reg_threads(L2);
     constexpr int PITCH = pass2_reg_pitch(L2), TILE = pass2_reg_tile(L2);
-    constexpr bool IP = pass2_reg_inplace(L2);
+    constexpr bool IP = pass2_reg_inplace(L2), PARK = IP && !NARROW;
     constexpr int NB = IP ? 1 : 2;  // tiles in flight
     constexpr int AU = R * LB, UPT = (AU + NT - 1) / NT;  // stage-A units per grid and thread
     // tiles in flight (at the 128 bytes a TMA tile needs: no static shared
     // memory lies before them), exchange tile or parked outputs, barriers
     extern __shared__ __align__(1024) unsigned char sm_tiles[];
     float2 *tiles = reinterpret_cast<float2 *>(sm_tiles), *rest = tiles + NB * TILE;
-    unsigned long long *full = reinterpret_cast<unsigned long long *>(tiles + pass2_reg_elems(L2));
+    unsigned long long *full = reinterpret_cast<unsigned long long *>(tiles + (IP && NARROW ? TILE : pass2_reg_elems(L2)));
     const int tid = threadIdx.x;
     if (p.dependent) pdl_trigger();
     if (smem_addr(tiles) & 127) {  // uniform; a copy there would fault
@@ -229,14 +233,13 @@ k_pass2_gls_reg(const __grid_constant__ CUtensorMap map, const DevCurve *cvs,
                 if (tid == 0) issue(s + NB);
             }
             if (act) RegDFT<LB>::run(y);
-            if constexpr (IP) {
+            if constexpr (PARK) {
                 if (g == 0) {  // grid A parked, read back by the same thread
 #pragma unroll
                     for (int qb = 0; qb < LB; ++qb) rest[qb * NT + tid] = ya[qb];
                 }
-            } else {
-                __syncthreads();  // the exchange tile is written next
             }
+            if constexpr (!IP) __syncthreads();  // the exchange tile is written next
         }
         // power of the outputs q2 = qa + LA qb
         const DevCurve cv = cvs[ci];
@@ -263,11 +266,12 @@ k_pass2_gls_reg(const __grid_constant__ CUtensorMap map, const DevCurve *cvs,
             for (int qb = 0; qb < LB; qb += 2) {
                 // (no band reaches the middle fifth of the grid: sigma >= 1.25)
                 if (5 * qb >= 2 * LB && 5 * (qb + 2) <= 3 * LB) continue;
+                if (NARROW && !narrow_pair(L2, qb)) continue;
                 const int qA = q0 + G1 * LA * qb, qB = qA + G1 * LA;
                 const bool ina = qA < lo_end || qA >= hi_start;
                 const bool inb = qB < lo_end || qB >= hi_start;
                 if (!ina && !inb) continue;
-                if constexpr (IP) {
+                if constexpr (PARK) {
                     ya[qb] = rest[qb * NT + tid];
                     ya[qb + 1] = rest[(qb + 1) * NT + tid];
                 }
@@ -477,13 +481,13 @@ cudaError_t launch_nfft_reg_t(const DevCurve *cv, int n_curves, int first, const
                       n_curves, first, out, aux, errflag, q);
 }
 
-template <int L2, bool ES>
+template <int L2, bool ES, bool NARROW>
 cudaError_t launch_pass2_reg_t(const DevCurve *cv, int n_curves, int first, const float2 *inter,
                                float *out, const Plan &p, GlsParams g, cudaStream_t s) {
     static int slots[64] = {0};  // resident CTAs, per instantiation and device
     constexpr int NT = pass2_reg_threads(L2), R = pass2_rows(3, L2);
-    const int smem = (int)pass2_smem(3, L2);
-    cudaError_t e = resident_ctas(k_pass2_gls_reg<L2, ES>, NT, smem, slots);
+    const int smem = NARROW && pass2_reg_inplace(L2) ? (pass2_reg_tile(L2) + 2) * 8 : (int)pass2_smem(3, L2);
+    cudaError_t e = resident_ctas(k_pass2_gls_reg<L2, ES, NARROW>, NT, smem, slots);
     if (e != cudaSuccess) return e;
     int dev = 0;
     cudaGetDevice(&dev);
@@ -494,7 +498,7 @@ cudaError_t launch_pass2_reg_t(const DevCurve *cv, int n_curves, int first, cons
     if (tasks > 0x3fffffffLL || p.B != kGlsCols) return cudaErrorInvalidValue;
     Plan q = p;
     q.dependent = small_launch(tasks);
-    return launch_pdl(k_pass2_gls_reg<L2, ES>, q.dependent,
+    return launch_pdl(k_pass2_gls_reg<L2, ES, NARROW>, q.dependent,
                       dim3((int)(tasks < slots[dev] ? tasks : slots[dev])), NT, smem, s, map, cv,
                       n_curves, first, out, q, g);
 }

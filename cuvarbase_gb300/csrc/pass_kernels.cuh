@@ -1037,8 +1037,11 @@ template <int L2>
 cudaError_t launch_pass2_gls_t(const DevCurve *cv, int n_curves, int first, const float2 *inter,
                                float *out, const Plan &p, GlsParams g, cudaStream_t s) {
     if constexpr (pass2_reg(3, L2)) {
-        return p.win == kWinES ? launch_pass2_reg_t<L2, true>(cv, n_curves, first, inter, out, p, g, s)
-                               : launch_pass2_reg_t<L2, false>(cv, n_curves, first, inter, out, p, g, s);
+        if (p.win == kWinES)  // (sigma 1.28)
+            return launch_pass2_reg_t<L2, true, false>(cv, n_curves, first, inter, out, p, g, s);
+        return p.narrow
+                   ? launch_pass2_reg_t<L2, false, true>(cv, n_curves, first, inter, out, p, g, s)
+                   : launch_pass2_reg_t<L2, false, false>(cv, n_curves, first, inter, out, p, g, s);
     } else if constexpr (pass2_deep(3, L2)) {
         static size_t done[2][64] = {{0}};  // per window and device
         const bool es = p.win == kWinES;
@@ -1114,8 +1117,9 @@ cudaError_t preload_pass2_t(int ng) {
             const cudaError_t e = cudaFuncGetAttributes(&a, k_pass2_nfft_reg<L2, true>);
             return e != cudaSuccess ? e : cudaFuncGetAttributes(&a, k_pass2_nfft_reg<L2, false>);
         }
-        const cudaError_t e = cudaFuncGetAttributes(&a, k_pass2_gls_reg<L2, true>);
-        return e != cudaSuccess ? e : cudaFuncGetAttributes(&a, k_pass2_gls_reg<L2, false>);
+        cudaError_t e = cudaFuncGetAttributes(&a, k_pass2_gls_reg<L2, true, false>);
+        if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_pass2_gls_reg<L2, false, true>);
+        return e != cudaSuccess ? e : cudaFuncGetAttributes(&a, k_pass2_gls_reg<L2, false, false>);
     } else if constexpr (pass2_deep(3, L2)) {
         if (ng != 3) return cudaFuncGetAttributes(&a, k_pass2_nfft<L2>);
         const cudaError_t e = cudaFuncGetAttributes(&a, k_pass2_gls_deep<L2, true>);

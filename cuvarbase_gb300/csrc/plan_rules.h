@@ -292,6 +292,14 @@ CUVGLS_HD constexpr int pass2_reg_exch(int L2) {
 CUVGLS_HD constexpr int pass2_reg_tile(int L2) {
     return pass2_reg_inplace(L2) ? pass2_reg_exch(L2) : pass2_rows(3, L2) * L2;
 }
+// Upsampling from which the band reaches only the first and the last 5/34 of the
+// rows' outputs (nf <= G / 3.4): there k_pass2_gls_reg keeps the outputs qb of
+// those (in pairs) and nothing else.
+constexpr double kNarrowSigma = 3.4;
+CUVGLS_HD constexpr bool narrow_pair(int L2, int qb) {  // of outputs qb, qb + 1
+    const int la = two_level_la(L2), reach = 5 * L2 / 34 + 1;
+    return qb * la <= reach || (qb + 2) * la > L2 - reach - 1;
+}
 // k_pass2_nfft_reg: in place in one tile, four CTAs per SM (1,000 curves of
 // 512 x 400 cells 0.431 ms; 0.442 with a tile ahead, 0.452 with five CTAs).
 // (columns per pass-1 block of every one-grid plan, and of every GLS plan)

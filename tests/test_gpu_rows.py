@@ -55,6 +55,36 @@ def test_row_lengths(oracle, G2, G1):
             h.close()
 
 
+@pytest.mark.parametrize("sigma", [3.39, 3.4, 4.0, 8.0])
+@pytest.mark.parametrize("G2", [32, 64, 80, 128, 160, 256, 320, 400, 512])
+def test_narrow_bands(oracle, G2, sigma):
+    """Around and above the upsampling from which rows up to 400 keep the ends
+    of their outputs only, with as many frequencies as the grid may hold."""
+    from cuvarbase_gb300 import _lib
+    curves = [_curve(n, n + G2) for n in (300, 700)]
+    G1 = 160
+    h = _lib.Handle(sigma=sigma, m=8)
+    try:
+        nf = int(G1 * G2 / sigma)
+        h.plan_pin(nf, G1, G2)
+        assert h.plan(nf)[1:3] == (G1, G2)
+        k = np.unique(np.concatenate([np.arange(30, 90), np.arange(nf - 60, nf),
+                                      np.arange(nf // 2 - 40, nf // 2 + 40),
+                                      np.arange(31, nf, max(1, nf // 200))]))
+        for mode in (1, 0, 2):
+            P = _raw(h, curves, nf, mode)
+            for c, got in zip(curves, P):
+                ref = _ref(oracle, c, k, mode)
+                assert np.abs(got[k] - ref).max() <= 2e-5 * max(1.0, np.abs(ref).max())
+        bk, bp = _raw(h, curves, nf, best=True)
+        P = _raw(h, curves, nf)
+        for i in range(len(curves)):
+            assert P[i][bk[i]] >= P[i].max() - 1e-6
+            assert abs(float(bp[i]) - float(P[i].max())) <= 1e-6
+    finally:
+        h.close()
+
+
 @pytest.mark.parametrize("sigma", ["auto", 2])
 @pytest.mark.parametrize("nf", [150, 700, 2500, 5000, 12800, 20000, 31000, 50000, 100000, 160000,
                                 250000, 600000])
