@@ -39,6 +39,10 @@ bool cuvgls_internal_choose_plan(long long nf, double sigma, int m, int ng, int 
 namespace {
 
 constexpr size_t kScratchBytes = (size_t)CUVGLS_NOALLOC_SCRATCH_BYTES;
+// Room beside the documented bytes for what the row tables of three levels hold
+// more than those of one exchange (at most 144 entries), so that a batch that
+// just fits still does.
+constexpr size_t kScratchSpare = 4096;
 constexpr int kMaxDevices = 64;
 constexpr size_t kAlignN = 256;
 constexpr double kPiN = 3.14159265358979323846;
@@ -52,7 +56,7 @@ std::mutex g_scratch_mutex;
 }  // namespace
 
 // The scratch array itself (device memory, fixed size).
-static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
+static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes + kScratchSpare];
 
 // Descriptors handed to the device as a kernel parameter, kDescPerLaunch at
 // a time (32 x 96 bytes stays under the classic 4 KB parameter limit).
@@ -139,7 +143,8 @@ extern "C" int cuvgls_gls_noalloc(double sigma, int32_t m, const cuvgls_gls_inpu
     const size_t nbin = (size_t)nc * (p.nb + 1);
     const size_t o_bins = off; off += up(4 * nbin * sizeof(int));  // counts, cursors
     const size_t o_in = off;  off += up((size_t)nc * 3 * G * sizeof(float2));
-    if (off > kScratchBytes) {
+    const size_t spare = (size_t)(n2 - fft_table_len(G2)) * sizeof(float2) + 2 * kAlignN;
+    if (off > kScratchBytes + std::min(spare, kScratchSpare)) {
         snprintf(msg, sizeof msg,
                  "batch needs %zu bytes of scratch; cuvgls_gls_noalloc holds %zu "
                  "(use fewer curves per call or cuvgls_gls_batch)", off, kScratchBytes);
