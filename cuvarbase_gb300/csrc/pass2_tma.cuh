@@ -13,9 +13,9 @@
 // What it replaces (a CTA per R rows; the three grids' outputs back to shared
 // memory and read again) was held by the L1 data pipe: 75 % busy, of which a
 // third was the outputs' way through shared memory and the deconvolution
-// table's scattered reads.  2,000 curves of 320 x 400 cells 1.80 -> 1.61 ms
-// (now at 53 % issue, 51 % of the L1 pipe and of DRAM), 20,000 of 160 x 160
-// 4.11 -> 2.81 ms (the old tile also had two- to four-way bank conflicts).
+// table's scattered reads.  2,000 curves of 320 x 400 cells 1.80 -> 1.61 ms,
+// 1.585 with the next tile in L2 and two twiddles to a load (now at 54 % issue,
+// 54 % of the L1 pipe and of DRAM), 20,000 of 160 x 160 4.11 -> 2.82 ms (the old tile also had two- to four-way bank conflicts).
 //   NARROW  sigma >= kNarrowSigma: only the outputs near both ends of a row can
 //     be in band; the rest are neither finished nor kept, and grid A is not
 //     parked.  400 curves of 1024 x 400 cells at sigma 4 833 -> 774 us (781 with a
