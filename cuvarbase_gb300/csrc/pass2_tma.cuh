@@ -70,6 +70,13 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, i
         : "memory");
 }
 
+// Orders this thread's own loads and stores of shared memory before the copies
+// into the same bytes that another thread issues after the next barrier: the
+// copies are the async proxy's, and a barrier alone orders one proxy only.
+__device__ __forceinline__ void before_copy() {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
 // Asks for the same box in L2, ahead of its load.
 __device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap *map, int x, int y, int z) {
     asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(map),
@@ -148,7 +155,7 @@ k_pass2_gls_reg(const __grid_constant__ CUtensorMap map, const DevCurve *cvs,
     const int ntask = n_curves * nrb;
     if (tid == 0) {
         for (int b = 0; b < NB; ++b) mbar_init(&full[b]);
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        before_copy();
     }
     __syncthreads();
     if (p.dependent) pdl_wait();  // the intermediate and the descriptors
@@ -229,6 +236,7 @@ k_pass2_gls_reg(const __grid_constant__ CUtensorMap map, const DevCurve *cvs,
                 for (int i = 0; i < LB; ++i) y[i] = e[i];
             }
             if constexpr (IP) {
+                before_copy();
                 __syncthreads();  // all read: the tile is free
                 if (tid == 0) issue(s + NB);
             }
@@ -348,7 +356,7 @@ k_pass2_nfft_reg(const __grid_constant__ CUtensorMap map, const DevCurve *cvs,
     const int ntask = n_curves * nrb;
     if (tid == 0) {
         mbar_init(full);
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        before_copy();
     }
     __syncthreads();
     if (p.dependent) pdl_wait();  // the intermediate and the descriptors
@@ -414,6 +422,7 @@ k_pass2_nfft_reg(const __grid_constant__ CUtensorMap map, const DevCurve *cvs,
 #pragma unroll
             for (int i = 0; i < LB; ++i) y[i] = e[i];
         }
+        before_copy();
         __syncthreads();  // all read: the tile is free
         if (tid == 0) issue(s + 1);
         const int nf = cv.nf, h = nf / 2, lo_end = nf - h, hi_start = G - h;
