@@ -32,9 +32,6 @@ constexpr int kDirThreads = 256;
 constexpr int kDirWarps = kDirThreads / 32;
 constexpr int kCoarse = 4, kFine = 8;  // 32 centres
 
-__device__ __forceinline__ double2 zmul(double2 a, double2 b) {
-    return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));
-}
 __device__ __forceinline__ double2 zturn(double turns) {  // exp(2 pi i turns)
     double s, c;
     sincospi(2.0 * (turns - floor(turns)), &s, &c);
@@ -42,13 +39,20 @@ __device__ __forceinline__ double2 zturn(double turns) {  // exp(2 pi i turns)
 }
 
 // ---- fixed point ----
-// Phasors are integers in units of 2^-56, values on them (E below) in units of
-// 2^-(55 - hr) of the power of two above the largest value; hr bits of headroom
-// keep the sums of a run below 2^62.  A factor is split into 27 low bits (signed)
-// and the rest, and a product takes three 32 x 32 -> 64 bit multiply-adds (the
-// low x low part, below 2^-2 of a unit, is left out).  These run at 24 or more
-// per clock and SM, against 2 of FP64: 2.4 FP64 instructions per bin become
-// 6 of them, with finer steps than FP64 has for values near one.
+// Phasors are integers in units of 2^-56, and so are values on them (E below),
+// of the power of two above the largest value of a run.  The step phasors that
+// multiply E for the sums are in units of 2^-54, which makes those products
+// units of E too, and a run is short enough that its sums stay within 2^62.  A
+// factor is split into 27 low bits (signed) and the rest, and a product takes
+// three 32 x 32 -> 64 bit multiply-adds (the low x low part, below 2^-2 of a
+// unit, is left out).  These run at 24 or more per clock and SM, against 2 of
+// FP64: 2.4 FP64 instructions per bin become 6 of them.  2^-56 of the largest
+// value is less than what a sum in FP64 that holds this value rounds to at every
+// addition: one value a thousand times the others, error of the sums relative to
+// it (rms over bins, worst place of the value within its power of two), in FP64
+// in sequence and here: 60 points 2.7e-16 and 1.4e-16, 300 points 6.4e-16 and
+// 3.2e-16, 2,000 points 1.6e-15 and 3.6e-16, 8,192 points 3.3e-15 and 5.2e-16
+// (7.1e-14 with one run for all of them).
 using i64 = long long;
 struct Fx {
     int h, l;  // h 2^27 + l, |l| <= 2^26
@@ -56,10 +60,11 @@ struct Fx {
 struct Cx {
     Fx x, y;
 };
-__device__ __forceinline__ Fx fx_split(i64 v) {
+__host__ __device__ constexpr Fx fx_split(i64 v) {
     const int h = (int)((v + (1 << 26)) >> 27);
     return Fx{h, (int)((unsigned)v - ((unsigned)h << 27))};
 }
+__device__ __forceinline__ i64 fx_join(Fx a) { return ((i64)a.h << 27) + a.l; }
 __device__ __forceinline__ i64 fx_wide(int a, int b, i64 c) { return c + (i64)a * b; }
 // c + a b / 2^54
 __device__ __forceinline__ i64 fx_fma(Fx a, Fx b, i64 c) {
@@ -80,35 +85,76 @@ __device__ __forceinline__ Cx fx_cmul(Cx a, Cx b) {
 __device__ __forceinline__ Cx fx_scale(Fx a, Cx b) {
     return Cx{fx_split((fx_fma(a, b.x, 2) >> 2)), fx_split((fx_fma(a, b.y, 2) >> 2))};
 }
-__device__ __forceinline__ Cx fx_unit(double2 z) {
-    constexpr double kOne = 72057594037927936.0;  // 2^56
-    return Cx{fx_split(__double2ll_rn(z.x * kOne)), fx_split(__double2ll_rn(z.y * kOne))};
+// a unit phasor in units of 2^-54
+__device__ __forceinline__ Cx fx_step(Cx v) {
+    return Cx{fx_split((fx_join(v.x) + 2) >> 2), fx_split((fx_join(v.y) + 2) >> 2)};
 }
 __device__ __forceinline__ int4 fx_pack(Cx v) { return make_int4(v.x.h, v.x.l, v.y.h, v.y.l); }
 __device__ __forceinline__ Cx fx_unpack(int4 v) { return Cx{Fx{v.x, v.y}, Fx{v.z, v.w}}; }
-__device__ __forceinline__ i64 fx_join(Fx a) { return ((i64)a.h << 27) + a.l; }
 
 // Phasors of multiples of 1 / kTurn of a turn, as products of kTurnCoarse and
-// kTurnFine steps (in shared memory: the coarse ones, then the fine ones).
+// kTurnFine steps (in shared memory: the coarse ones, then the fine ones).  The
+// steps are rounded once, to 2^-56: from sincospi their error would be the 2^-54
+// of FP64, and every product of phasors adds its factors' errors up.
 constexpr int kTurn = 2048, kTurnCoarse = 64, kTurnFine = kTurn / kTurnCoarse;
+constexpr int kTurnSteps = kTurnCoarse + kTurnFine;
+
+// cos and sin of pi num / den (at most pi / 2) by their series, in units of 2^-62.
+struct HostPhasor {
+    i64 c, s;
+};
+constexpr HostPhasor host_phasor(int num, int den) {
+    constexpr unsigned long long kPi = 0xC90FDAA22168C234ULL;  // pi 2^62
+    const __int128 x = ((__int128)kPi * num + den / 2) / den;
+    __int128 term = (__int128)1 << 62, sum[2] = {term, 0};
+    for (int n = 1; n < 32; ++n) {  // x^n / n!
+        const __int128 p = term * x, d = ((__int128)n) << 62;
+        term = (p + d / 2) / d;
+        sum[n & 1] += n & 2 ? -term : term;
+    }
+    return HostPhasor{(i64)sum[0], (i64)sum[1]};
+}
+struct TurnSteps {
+    int v[kTurnSteps][4];
+    constexpr TurnSteps() : v() {
+        for (int i = 0; i < kTurnSteps; ++i) {
+            const int k = i < kTurnCoarse ? i : i - kTurnCoarse;
+            const int quarter = i < kTurnCoarse ? kTurnCoarse / 4 : kTurn / 4;
+            const HostPhasor z = host_phasor(k % quarter, 2 * quarter);
+            i64 c = z.c, s = z.s;
+            for (int q = k / quarter; q > 0; --q) {  // a quarter turn on
+                const i64 t = c;
+                c = -s;
+                s = t;
+            }
+            const Fx x = fx_split((c + 32) >> 6), y = fx_split((s + 32) >> 6);
+            v[i][0] = x.h;
+            v[i][1] = x.l;
+            v[i][2] = y.h;
+            v[i][3] = y.l;
+        }
+    }
+};
+__device__ constexpr TurnSteps kTurnStepTable;
 
 __device__ __forceinline__ void turn_steps(int4 *step, int tid) {
-    for (int i = tid; i < kTurnCoarse + kTurnFine; i += kDirThreads)
-        step[i] = fx_pack(fx_unit(zturn(i < kTurnCoarse ? (double)i / kTurnCoarse
-                                                        : (double)(i - kTurnCoarse) / kTurn)));
+    if (tid < kTurnSteps) {
+        const int *v = kTurnStepTable.v[tid];
+        step[tid] = make_int4(v[0], v[1], v[2], v[3]);
+    }
 }
+static_assert(kTurnSteps <= kDirThreads, "a step per thread");
 __device__ __forceinline__ Cx turn_product(const int4 *step, int k) {
     return fx_cmul(fx_unpack(step[k / kTurnFine]), fx_unpack(step[kTurnCoarse + k % kTurnFine]));
 }
 
-// exp(2 pi i p) of a finite p: the phasor at the nearest multiple of 1 / kTurn
-// turned by the remaining angle d, |d| <= pi / kTurn, all of it in integers
-// (FP64 forms p only): d and sin d in units of 2^-61, cos d - 1 = -d^2 / 2 +
-// d^4 / 24 the same, the small terms d^3 / 6 - d^5 / 120 (6e-10) and d^4 / 24
-// (2e-13) in FP32; those left out are below 2e-20.
+// exp(2 pi i th) of a 64-bit fraction of a turn: the phasor at the nearest
+// multiple of 1 / kTurn turned by the remaining angle d, |d| <= pi / kTurn, all of
+// it in integers: d and sin d in units of 2^-61, cos d - 1 = -d^2 / 2 + d^4 / 24
+// the same, the small terms d^5 / 120 (7e-17) and d^4 / 24 (2e-13) in FP32; those
+// left out are below 2e-20.
 template <typename Table>
-__device__ __forceinline__ Cx fx_turn(double p, Table table) {
-    const u64 th = turns64(p);
+__device__ __forceinline__ Cx fx_turn(u64 th, Table table) {
     const int k = (int)((th + (1ULL << 52)) >> 53);  // 0 .. kTurn
     const Cx e = table(k & (kTurn - 1));
     const Fx r = fx_split((i64)(th - ((u64)k << 53)));  // |r| <= 2^52, in 2^-64 turns
@@ -118,29 +164,36 @@ __device__ __forceinline__ Cx fx_turn(double p, Table table) {
     const int dh = (int)(d >> 21), dl = (int)(d & ((1 << 21) - 1));
     const float df = (float)dh * 9.094947017729282e-13f, q = df * df;  // 2^-40
     const float kUp = 2305843009213693952.f;                           // 2^61
-    const Fx sn = fx_split(d + __float2int_rn(kUp * df * q * fmaf(q, 1.f / 120.f, -1.f / 6.f)));
-    const i64 d2 = fx_wide(dh, dh, fx_wide(dh, dl, 0) >> 20);  // 2^-80
+    const i64 d2 = fx_wide(dh, dh, fx_wide(dh, dl, 0) >> 20);          // 2^-80
+    // d^3 in 2^-59 (below 2^31), times 2^31 4 / 6
+    const int d3 = (int)(fx_wide(dh, (int)(d2 >> 31), 1 << 29) >> 30);
+    const i64 d36 = fx_wide(d3, 1431655765, 1 << 30) >> 31;
+    const Fx sn = fx_split(d - d36 + __float2int_rn(kUp * df * q * q * (1.f / 120.f)));
     const Fx cm = fx_split(__float2int_rn(kUp * q * q * (1.f / 24.f)) - (d2 >> 20));
     // e + e (cm + i sn), the product in units of 2^-63
     const i64 re = fx_fma(cm, e.x, 64) - fx_fma(sn, e.y, 0), im = fx_fma(cm, e.y, fx_fma(sn, e.x, 64));
     return Cx{fx_split(fx_join(e.x) + (re >> 7)), fx_split(fx_join(e.y) + (im >> 7))};
 }
 
-// An eighth of a warp's sum, so that the eight warps' add up in integers: a
-// conversion to FP64 costs as much as an FP64 instruction (one per warp and sum:
-// 0.468 against 0.450 ms of the GLS sums).
-static_assert(kDirWarps == 8, "eighths");
-__device__ __forceinline__ i64 fx_eighth(i64 v) { return (v + 4) >> 3; }
+// The warps' sums added up exactly, in two halves of 32 bits: a conversion to
+// FP64 costs as much as an FP64 instruction (one per warp and sum: 0.468 against
+// 0.450 ms of the GLS sums).
+struct FxTotal {
+    i64 hi = 0, lo = 0;
+    __device__ __forceinline__ void add(i64 v) {
+        hi += v >> 32;
+        lo += (unsigned)v;
+    }
+    // in units of 2^unit
+    __device__ __forceinline__ double value(int unit) const {
+        return scalbn(fma((double)hi, 4294967296.0, (double)lo), unit);
+    }
+};
 
-// Points of a run (one CTA, sums in 64-bit integers) and its headroom: 2^(5 +
-// hr) terms per warp.
-constexpr int kDirRun = 1024 * kDirWarps;
-__device__ __forceinline__ int fx_headroom(i64 points) {
-    const int per = (int)((points + kDirThreads - 1) / kDirThreads) * 32;
-    int hr = 0;
-    while ((32 << hr) < per) ++hr;
-    return hr;
-}
+// Points of a run (one CTA, sums in 64-bit integers): 64 terms per warp, of at
+// most 2^56.
+constexpr int kDirRun = 64 * kDirWarps;
+constexpr int kFxBits = 56;
 // Exponent ex with |v| < 2^ex for the largest finite |v| of the CTA's threads;
 // `sh` one shared word.
 __device__ __forceinline__ int fx_exponent(double mx, u64 *sh, int tid) {
@@ -166,27 +219,28 @@ struct DirTable {
     static constexpr int kRows = NB + kCoarse + kFine;
     int4 row[kRows][32];
 
-    // This lane's point: x in turns per bin, th0 the phase of K0 in turns;
-    // `steps` from turn_steps.  Two phasors, the rest by products of depth at
-    // most 8.
-    __device__ __forceinline__ void build(int lane, double x, double th0, const int4 *steps) {
+    // This lane's point: x in turns per bin, th0 the phase of K0, both as
+    // fractions of a turn; `steps` from turn_steps.  Four phasors (the multiples
+    // of x are exact), the rest by products of at most eight of one: an error of
+    // a phasor counts as often as the phasor does, and from two phasors alone the
+    // last bin would hold that of x 400 times.
+    __device__ __forceinline__ void build(int lane, u64 x, u64 th0, const int4 *steps) {
         auto table = [&](int k) { return turn_product(steps, k); };
-        static_assert(NB >= M, "the centre step is built from step phasor M");
         Cx z[NB + 1];
         z[1] = fx_turn(x, table);
 #pragma unroll
         for (int b = 2; b <= NB; ++b) z[b] = fx_cmul(z[b / 2], z[b - b / 2]);
 #pragma unroll
-        for (int b = 1; b <= NB; ++b) row[b - 1][lane] = fx_pack(z[b]);
-        const Cx w1 = fx_cmul(fx_cmul(z[M], z[M]), z[1]);  // exp(i W x)
+        for (int b = 1; b <= NB; ++b) row[b - 1][lane] = fx_pack(fx_step(z[b]));
+        constexpr int W = 2 * M + 1;
         Cx f[kFine];
         f[0] = Cx{Fx{1 << 29, 0}, Fx{0, 0}};
-        f[1] = w1;
+        f[1] = fx_turn(W * x, table);
 #pragma unroll
         for (int k = 2; k < kFine; ++k) f[k] = fx_cmul(f[k / 2], f[k - k / 2]);
 #pragma unroll
         for (int k = 0; k < kFine; ++k) row[NB + kCoarse + k][lane] = fx_pack(f[k]);
-        const Cx w8 = fx_cmul(f[kFine / 2], f[kFine / 2]);
+        const Cx w8 = fx_turn(W * kFine * x, table);
         Cx c = fx_turn(th0, table);
 #pragma unroll
         for (int k = 0; k < kCoarse; ++k) {
@@ -219,8 +273,8 @@ struct DirSums {
     }
     // real and imaginary parts of the lane's bins into re[0 .. 2 M], im[...]
     __device__ __forceinline__ void bins(i64 *re, i64 *im) const {
-        re[M] = c0 * 4;
-        im[M] = s0 * 4;
+        re[M] = c0;
+        im[M] = s0;
 #pragma unroll
         for (int b = 0; b < M; ++b) {
             re[M + 1 + b] = p1[b] - p2[b];
@@ -244,20 +298,20 @@ __device__ __forceinline__ void dir_reduce(const DirSums<M> &v, i64 *red, int ti
 #pragma unroll
     for (int q = 0; q < (TB + kDirThreads - 1) / kDirThreads; ++q) {
         const int b = tid + q * kDirThreads;
-        i64 re = 0, im = 0;
+        FxTotal re, im;
         if (b < TB)
 #pragma unroll
             for (int w = 0; w < kDirWarps; ++w) {
-                re += fx_eighth(red[w * TB + b]);
-                im += fx_eighth(red[(kDirWarps + w) * TB + b]);
+                re.add(red[w * TB + b]);
+                im.add(red[(kDirWarps + w) * TB + b]);
             }
-        out[q].x += scalbn((double)re, unit + 3);
-        out[q].y += scalbn((double)im, unit + 3);
+        out[q].x += re.value(unit);
+        out[q].y += im.value(unit);
     }
 }
 
 // Points [j0, j1) of split z of a curve of n points cut into `splits` equal
-// parts; false when the part is empty.
+// parts (the last ones may hold none); false when there is no such part.
 __device__ __forceinline__ bool dir_part(long long n, int splits, int z, long long &j0,
                                          long long &j1) {
     if (z >= splits) return false;
@@ -283,16 +337,16 @@ static_assert(kNfSmem >= 2 * kDirWarps * kNfBins * 8, "the reduction reuses the 
 // sums for k_nfft_direct64_sum.  Bound by the wide multiply-adds.  4 curves of 300 to 2,000 points and 20,000
 // bins, host to host: 5.67 ms with a sincospi pair per point and 8 bins, 0.45 ms
 // with factored phasors in FP64 (2.4 instructions per bin, 93 % busy), 0.235 ms
-// in fixed point (0.242 ms with M = 8, 0.273 with M = 4), 0.223 ms with the
+// in fixed point (0.242 ms with M = 8, 0.273 with M = 4), 0.219 ms with the
 // warps' sums and the phasors of the tables in integers too; errors against 64
-// bits 6.8e-13 in all of them.
+// bits 6.8e-13 in all of them, that of the phases.
 __global__ void __launch_bounds__(kDirThreads, 2)
 k_nfft_direct64(const Direct64Curve *__restrict__ cvs, const double *__restrict__ t,
                 const double *__restrict__ y, double2 *__restrict__ out,
                 double2 *__restrict__ part, long long part_stride) {
     extern __shared__ __align__(16) double sm[];
     __shared__ u64 top;
-    __shared__ int4 steps[kTurnCoarse + kTurnFine];
+    __shared__ int4 steps[kTurnSteps];
     const Direct64Curve cv = cvs[blockIdx.y];
     const long long k0 = (long long)blockIdx.x * kNfBins;
     long long j0, j1;
@@ -307,14 +361,14 @@ k_nfft_direct64(const Direct64Curve *__restrict__ cvs, const double *__restrict_
     bool odd = false;   // a value that is not finite, added below bin by bin
     bool lost = false;  // a time that is not finite: no bin has a value
     const double kc = (double)(k0 + kNfM);
-    for (long long r0 = j0; r0 < j1; r0 += kDirRun) {  // one run, but for very long parts
+    for (long long r0 = j0; r0 < j1; r0 += kDirRun) {
         const long long r1 = min(j1, r0 + kDirRun);
         double mx = 0.0;
         for (long long j = r0 + tid; j < r1; j += kDirThreads) {
             const double yj = fabs(y[cv.pt_off + j]);
             mx = isfinite(yj) && yj > mx ? yj : mx;
         }
-        const int ex = fx_exponent(mx, &top, tid), hr = fx_headroom(r1 - r0);
+        const int ex = fx_exponent(mx, &top, tid);
         DirSums<kNfM> acc;
         for (long long base = r0 + wid * 32; base < r1; base += kDirThreads) {
             const int cnt = (int)min(32LL, r1 - base);
@@ -331,8 +385,8 @@ k_nfft_direct64(const Direct64Curve *__restrict__ cvs, const double *__restrict_
                 b -= floor(b);
                 const double th = fma(kc, b, a);
                 lost = lost || !isfinite(th);
-                tab.build(lane, b, th, steps);
-                const Fx yv = fx_split(__double2ll_rn(scalbn(yj, 55 - hr - ex)));
+                tab.build(lane, turns64(b), turns64(th), steps);
+                const Fx yv = fx_split(__double2ll_rn(scalbn(yj, kFxBits - ex)));
 #pragma unroll
                 for (int g = 0; g < kCoarse; ++g) {  // y rides on the coarse centres
                     int4 &c = tab.row[kNfM + g][lane];
@@ -348,7 +402,7 @@ k_nfft_direct64(const Direct64Curve *__restrict__ cvs, const double *__restrict_
                 for (int b = 0; b < kNfM; ++b) acc.pair(b, e, tab.step(b, p));
             }
         }
-        dir_reduce<kNfM>(acc, reinterpret_cast<i64 *>(sm), tid, ex + hr - 57, v);
+        dir_reduce<kNfM>(acc, reinterpret_cast<i64 *>(sm), tid, ex - kFxBits, v);
         __syncthreads();  // the next run's tables
     }
     if (__syncthreads_or(odd)) {  // inf cos and inf sin keep their own signs
@@ -452,7 +506,7 @@ __device__ __forceinline__ float gls_direct_power(const DevCurve &cv, const GlsP
 // partial sums for k_gls_direct_sum.  8 curves of 300 to 2,000 points and
 // 10,000 frequencies: 9.62 ms with a sincospi each, 1.10 ms with factored
 // phasors in FP64 (7.7 instructions per frequency, 81 % busy), 0.47 ms in fixed
-// point (0.61 ms with M = 4 and one CTA per SM), 0.44 ms with the warps' sums
+// point (0.61 ms with M = 4 and one CTA per SM), 0.435 ms with the warps' sums
 // and the phasors of the tables in integers too; errors against 64 bits 2.8e-8
 // in all of them.
 __global__ void __launch_bounds__(kDirThreads, 2)
@@ -461,7 +515,7 @@ k_gls_direct(const DevCurve *__restrict__ cvs, const double *__restrict__ t,
              double2 *__restrict__ part, long long part_stride, GlsParams gp) {
     extern __shared__ __align__(16) double sm[];
     __shared__ u64 top[2];
-    __shared__ int4 steps[kTurnCoarse + kTurnFine];
+    __shared__ int4 steps[kTurnSteps];
     const DevCurve cv = cvs[blockIdx.y];
     const long long k0 = (long long)blockIdx.x * kGlBins;
     long long j0, j1;
@@ -476,7 +530,7 @@ k_gls_direct(const DevCurve *__restrict__ cvs, const double *__restrict__ t,
     bool lost = false;  // something not finite: no power of the curve is valid
     const double kc = cv.kc - (double)(cv.nf / 2) + (double)(k0 + kGlM);
     const double t0 = t[cv.pt_off];
-    for (long long r0 = j0; r0 < j1; r0 += kDirRun) {  // one run, but for very long parts
+    for (long long r0 = j0; r0 < j1; r0 += kDirRun) {
         const long long r1 = min(j1, r0 + kDirRun);
         float my = 0.f, mw = 0.f;
         for (long long j = cv.pt_off + r0 + tid; j < cv.pt_off + r1; j += kDirThreads) {
@@ -488,7 +542,6 @@ k_gls_direct(const DevCurve *__restrict__ cvs, const double *__restrict__ t,
                 lost = true;
             }
         }
-        const int hr = fx_headroom(r1 - r0);
         const int ey = fx_exponent(my, &top[0], tid), ew = fx_exponent(mw, &top[1], tid);
         DirSums<kGlM> sa, sb, sc;
         for (long long base = r0 + wid * 32; base < r1; base += kDirThreads) {
@@ -498,9 +551,9 @@ k_gls_direct(const DevCurve *__restrict__ cvs, const double *__restrict__ t,
                 const long long j = cv.pt_off + base + lane;
                 const double x = (t[j] - t0) * cv.df;
                 lost = lost || !isfinite(kc * x);
-                tile.tab.build(lane, x, kc * x, steps);
-                const Fx fy = fx_split(__double2ll_rn(scalbn((double)yw[j], 55 - hr - ey)));
-                const Fx fw = fx_split(__double2ll_rn(scalbn((double)w[j], 55 - hr - ew)));
+                tile.tab.build(lane, turns64(x), turns64(kc * x), steps);
+                const Fx fy = fx_split(__double2ll_rn(scalbn((double)yw[j], kFxBits - ey)));
+                const Fx fw = fx_split(__double2ll_rn(scalbn((double)w[j], kFxBits - ew)));
                 tile.yw[lane] = make_int2(fy.h, fy.l);
                 tile.w[lane] = make_int2(fw.h, fw.l);
             }
@@ -524,9 +577,9 @@ k_gls_direct(const DevCurve *__restrict__ cvs, const double *__restrict__ t,
             }
         }
         i64 *red = reinterpret_cast<i64 *>(sm);
-        dir_reduce<kGlM>(sa, red, tid, ey + hr - 57, va);
-        dir_reduce<kGlM>(sb, red, tid, ew + hr - 57, vb);
-        dir_reduce<kGlM>(sc, red, tid, ew + hr - 57, vc);
+        dir_reduce<kGlM>(sa, red, tid, ey - kFxBits, va);
+        dir_reduce<kGlM>(sb, red, tid, ew - kFxBits, vb);
+        dir_reduce<kGlM>(sc, red, tid, ew - kFxBits, vc);
         __syncthreads();  // the next run's tables
     }
     if (__syncthreads_or(lost)) {
@@ -592,6 +645,11 @@ cudaError_t launch_gls_direct(const DevCurve *cv, int n_curves, int max_nf, int 
 // ---------------------------------------------------------------------------
 namespace {
 
+// Points of a run and the bits of its values.  The phasors keep their 2^-56
+// here (the recurrence needs them), so the products are quarter units and a
+// value has fewer bits; it is rounded once, not at each of E's two products.
+constexpr int kMhRun = 64 * kDirWarps, kMhBits = 54;
+
 // rows of sums a CTA reduces: c, s (2H each), yc, ys (H each), and sum w
 __host__ __device__ constexpr int mh_sums(int H) { return 6 * H + 1; }
 __host__ __device__ constexpr int mh_smem(int H) {
@@ -608,7 +666,7 @@ __host__ __device__ constexpr int mh_smem(int H) {
 // cluster share the points of the same frequencies, and the first adds their
 // sums and solves: 625 CTAs left a fifth of the FP64 pipes idle at the end
 // (4.1 CTAs per SM are 5 rounds).  Per point the
-// phasor from table_turn, its powers n = 2 .. 2H by the recurrence
+// phasor from fx_turn, its powers n = 2 .. 2H by the recurrence
 // z_n = 2 cos(phi) z_(n-1) - z_(n-2), then the sums of
 // cuvarbase/lombscargle.py:337-400 (mhdirect_sums), all in fixed point; FP64
 // forms t f, adds the warps' sums, and from there on: the regulariser of
@@ -617,7 +675,7 @@ __host__ __device__ constexpr int mh_smem(int H) {
 // frequencies, host to host: 4.93 ms with a sincospi per point; in FP64 2.24 ms
 // with the table and the clusters (54 instructions per point and frequency, the
 // pipes 88 % busy), 1.97 ms with the recurrence, 1.54 ms with the phasor's
-// fraction in integers; 0.76 ms in fixed point (about 100 wide multiply-adds).
+// fraction in integers; 0.79 ms in fixed point (about 100 wide multiply-adds).
 // Errors against 64 bits 1.8e-13 in all of them: that of the FP64 phase t f.
 template <int H>
 __global__ void __launch_bounds__(kDirThreads, H <= 4 ? 2 : 1)
@@ -652,8 +710,8 @@ k_mhgls_direct(const double *__restrict__ t, const double *__restrict__ yw,
     for (int i = tid; i < NS * 32; i += kDirThreads) tot[i] = 0.0;
     const long long share = (n + csize - 1) / csize;
     const long long j1 = min(n, (rank + 1) * share);
-    for (long long r0 = rank * share; r0 < j1; r0 += kDirRun) {  // one run, but for very long curves
-        const long long r1 = min(j1, r0 + kDirRun);
+    for (long long r0 = rank * share; r0 < j1; r0 += kMhRun) {
+        const long long r1 = min(j1, r0 + kMhRun);
         double my = 0.0, mw = 0.0;
         for (long long j = r0 + tid; j < r1; j += kDirThreads) {
             const double u = fabs(yw[j]), v = fabs(w[j]);
@@ -664,7 +722,6 @@ k_mhgls_direct(const double *__restrict__ t, const double *__restrict__ yw,
                 odd = true;
             }
         }
-        const int hr = fx_headroom(r1 - r0);
         const int ey = fx_exponent(my, &top[0], tid), ew = fx_exponent(mw, &top[1], tid);
         i64 c[NH + 1], s[NH + 1], yc[H + 1], ys[H + 1];
 #pragma unroll
@@ -677,8 +734,8 @@ k_mhgls_direct(const double *__restrict__ t, const double *__restrict__ yw,
             if (lane < cnt) {
                 st[lane] = t[base + lane];
                 ws += w[base + lane];
-                const Fx fy = fx_split(__double2ll_rn(scalbn(yw[base + lane], 55 - hr - ey)));
-                const Fx fw = fx_split(__double2ll_rn(scalbn(w[base + lane], 55 - hr - ew)));
+                const Fx fy = fx_split(__double2ll_rn(scalbn(yw[base + lane], kMhBits - ey)));
+                const Fx fw = fx_split(__double2ll_rn(scalbn(w[base + lane], kMhBits - ew)));
                 sy[lane] = make_int2(fy.h, fy.l);
                 sw[lane] = make_int2(fw.h, fw.l);
             }
@@ -689,7 +746,7 @@ k_mhgls_direct(const double *__restrict__ t, const double *__restrict__ yw,
                 const Fx wq{vw.x, vw.y}, yq{vy.x, vy.y};
                 const double p = st[q] * f;
                 lost = lost || (__double2hiint(p) & 0x7ff00000) == 0x7ff00000;
-                Cx z = fx_turn(p, [&](int i) { return fx_unpack(turn[i]); }), zp{Fx{1 << 29, 0}, Fx{0, 0}};  // power m, m - 1
+                Cx z = fx_turn(turns64(p), [&](int i) { return fx_unpack(turn[i]); }), zp{Fx{1 << 29, 0}, Fx{0, 0}};  // power m, m - 1
                 const Fx cc = fx_split(2 * fx_join(z.x));                 // 2 cos
 #pragma unroll
                 for (int m = 1; m <= NH; ++m) {
@@ -720,9 +777,9 @@ k_mhgls_direct(const double *__restrict__ t, const double *__restrict__ yw,
         }
         __syncthreads();
         for (int i = tid; i < (NS - 1) * 32; i += kDirThreads) {
-            i64 v = 0;
-            for (int q = 0; q < kDirWarps; ++q) v += fx_eighth(sums[q * NS * 32 + i]);
-            tot[i] += scalbn((double)v, (i < 2 * NH * 32 ? ew : ey) + hr - 54);
+            FxTotal v;
+            for (int q = 0; q < kDirWarps; ++q) v.add(sums[q * NS * 32 + i]);
+            tot[i] += v.value((i < 2 * NH * 32 ? ew : ey) - kMhBits - 2);
         }
         __syncthreads();  // before the next run's sums
     }

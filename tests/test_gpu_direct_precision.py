@@ -1,0 +1,68 @@
+"""The 64-bit direct sums with one value that dominates a long curve: no coarser
+than the same sums in FP64.  Times, frequencies and their products are exact, so
+that the sums are all that rounds."""
+import numpy as np
+import pytest
+
+LD = np.longdouble
+TWO_PI = 2 * LD("3.14159265358979323846264338327950288")
+
+
+def _curve(n, seed):
+    """Times of 30 bits over 1,024; a value of nearly 2 among ones of 10^-3."""
+    rng = np.random.default_rng(seed)
+    t = np.sort(rng.integers(1, (1 << 30) - 1, n)) / 2.0 ** 20
+    t[0], t[-1] = 0.0, 1024.0
+    y = rng.standard_normal(n) * 1e-3
+    y[n // 7] = 1.98
+    return t, y
+
+
+def _sums(t, v, f):
+    """sum v exp(2 pi i t f) per frequency, in extended precision."""
+    out = np.empty((len(f), 2), LD)
+    for i, x in enumerate(f):
+        ph = t * x                       # exact
+        a = TWO_PI * (ph - np.floor(ph)).astype(LD)
+        out[i] = (v.astype(LD) * np.cos(a)).sum(), (v.astype(LD) * np.sin(a)).sum()
+    return out
+
+
+def _rms_fp64(n):
+    """A sum in FP64 that holds a value in [1, 2) rounds to units of 2^-52: 0.29
+    of them per addition (rms)."""
+    return 0.29 * 2.0 ** -52 * np.sqrt(n)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,nf", [(300, 400), (2000, 520000), (8192, 520000)])
+def test_use_double_one_value_dominates(n, nf):
+    """Both with the points in parts and, with enough bins, in one part."""
+    from cuvarbase_gb300.cunfft import NFFTAsyncProcess
+    t, y = _curve(n, n)
+    p = NFFTAsyncProcess(use_double=True)
+    (got,) = p.run([(t, y, nf)], samples_per_peak=1)
+    p.finish()
+    k = np.random.default_rng(1).integers(0, nf, 120)
+    ref = _sums(t, y, k / 1024.0)
+    err = np.concatenate([got.real[k] - ref[:, 0], got.imag[k] - ref[:, 1]]).astype(float)
+    assert np.sqrt(np.mean(err ** 2)) <= _rms_fp64(n)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [500, 2000, 32768])
+def test_harmonics_one_value_dominates(n):
+    from cuvarbase_gb300.lombscargle import lomb_scargle_direct_sums
+    t, yw = _curve(n, n + 1)
+    w = np.full(n, 2.0 ** -20)           # exact, as is their sum
+    f = np.random.default_rng(2).integers(1 << 12, 1 << 18, 96) / 1024.0
+    P = lomb_scargle_direct_sums(t, yw, w, f, 1.0, nharms=1)
+    W = n * LD(2) ** -20
+    C, S = _sums(t, w, f).T
+    C2, S2 = _sums(t, w, 2 * f).T
+    YC, YS = (_sums(t, yw, f) - LD(np.cumsum(yw)[-1]) * _sums(t, w, f)).T
+    CC, SS, CS = (W + C2) / 2 - C * C, (W - C2) / 2 - S * S, S2 / 2 - C * S
+    ref = (YC * YC * SS - 2 * YC * YS * CS + YS * YS * CC) / (CC * SS - CS * CS)
+    # P goes as the squares of YC and YS, whose larger one is 1.4 or more
+    err = ((P - ref) / ref).astype(float)
+    assert np.sqrt(np.mean(err ** 2)) <= 2 * _rms_fp64(n) / 1.4 + 16 * 2.0 ** -53
