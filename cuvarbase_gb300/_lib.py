@@ -334,13 +334,14 @@ class PinnedBuffer:
         self._lib = L
         self._np = np
 
-    def view(self, dtype, count, offset_bytes=0):
-        """numpy view of the buffer; the view keeps the buffer alive."""
+    def view(self, dtype, count, offset_bytes=0, owner=None):
+        """numpy view of the buffer; the view keeps the buffer (and ``owner``)
+        alive."""
         np = self._np
         dt = np.dtype(dtype)
         if offset_bytes + dt.itemsize * count > self.nbytes:
             raise ValueError("view outside the pinned buffer")
-        return np.asarray(_View(self, self.ptr.value + offset_bytes, dt, count))
+        return np.asarray(_View(owner or self, self.ptr.value + offset_bytes, dt, count))
 
     def close(self):
         if getattr(self, "ptr", None):

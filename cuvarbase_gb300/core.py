@@ -1,9 +1,55 @@
 """Asynchronous-process base class (mirrors cuvarbase/core.py:13-56)."""
 from __future__ import annotations
 
-import sys
-
 from . import _lib
+
+
+class ResultPool:
+    """Page-locked buffers for the results of one process.  Page-locking a
+    megabyte takes a few hundred microseconds, longer than most calls' kernels,
+    so buffers whose results are gone are kept, the last ``KEEP`` of them; the
+    others are given back at once.  A result takes no buffer of more than twice
+    its size (or a megabyte), so that results which a program keeps hold little
+    more than themselves."""
+
+    KEEP = 4
+    SMALL = 1 << 20
+
+    def __init__(self):
+        self._free = []
+
+    def take(self, nbytes):
+        """A lease on a buffer of at least nbytes."""
+        nbytes = (max(int(nbytes), 1) + 4095) // 4096 * 4096
+        fit = [b for b in list(self._free)
+               if nbytes <= b.nbytes <= max(2 * nbytes, self.SMALL)]
+        for buf in sorted(fit, key=lambda b: b.nbytes):
+            try:
+                self._free.remove(buf)
+            except ValueError:  # taken by another thread
+                continue
+            break
+        else:
+            buf = _lib.PinnedBuffer(nbytes)
+        return ResultBuffer(self, buf)
+
+    def give(self, buf):
+        self._free.append(buf)
+        del self._free[:-self.KEEP]
+
+
+class ResultBuffer:
+    """A lease on a page-locked buffer; it ends with the last view."""
+
+    def __init__(self, pool, buf):
+        self._pool, self._buf = pool, buf
+        self.ptr, self.nbytes = buf.ptr, buf.nbytes
+
+    def view(self, dtype, count, offset_bytes=0):
+        return self._buf.view(dtype, count, offset_bytes, owner=self)
+
+    def __del__(self):
+        self._pool.give(self._buf)
 
 
 class GPUAsyncProcess:
@@ -24,6 +70,7 @@ class GPUAsyncProcess:
         self.results = []
         self._adjust_nstreams = self.nstreams is None
         self._handles = {}
+        self._result_pool = ResultPool()
         if self.nstreams is not None:
             self._create_streams(self.nstreams)
         self.prepared_functions = {}
@@ -47,19 +94,9 @@ class GPUAsyncProcess:
         return h
 
     def _result_buffer(self, nbytes):
-        """A page-locked result buffer of the process: a pooled one that no
-        earlier result views any more, else a new one (free buffers that are
-        too small are given back then).  Page-locking a megabyte takes a few
-        hundred microseconds, longer than most calls' kernels."""
-        pool = self.__dict__.setdefault('_result_pool', [])
-        for buf in pool:
-            # references: the pool, the loop variable, getrefcount's argument
-            if buf.nbytes >= nbytes and sys.getrefcount(buf) <= 3:
-                return buf
-        buf = None
-        new = _lib.PinnedBuffer(max(int(nbytes), 1 << 20))
-        pool[:] = [b for b in pool if sys.getrefcount(b) > 3] + [new]
-        return new
+        """A page-locked result buffer, the process's again when the last
+        array that views it is gone."""
+        return self._result_pool.take(nbytes)
 
     def _compile_and_prepare_functions(self, **kwargs):
         """Kernels are compiled ahead of time into libcuvgls.so; this only
