@@ -424,15 +424,25 @@ int ensure_ws(cuvgls_handle *h, size_t need) {
                     "batch needs " + std::to_string(need) +
                         " workspace bytes, budget is " +
                         std::to_string(h->opts.workspace_bytes));
+    size_t sz = std::max(need, (size_t)64 << 20);
+    sz = std::min(sz, (size_t)h->opts.workspace_bytes);
     if (h->ws) {
+        // an arena that cannot grow is kept for what it holds
+        size_t left = 0, total = 0;
+        CK(cudaMemGetInfo(&left, &total), "cudaMemGetInfo");
+        if (left + h->ws_size < sz)
+            return cuda_fail(h, cudaErrorMemoryAllocation, "workspace growth");
         CK(cudaDeviceSynchronize(), "sync before workspace growth");
         cudaFree(h->ws);
         h->ws = nullptr;
         h->ws_size = 0;
     }
-    size_t sz = std::max(need, (size_t)64 << 20);
-    sz = std::min(sz, (size_t)h->opts.workspace_bytes);
-    CK(cudaMalloc(&h->ws, sz), "cudaMalloc(workspace)");
+    const cudaError_t e = cudaMalloc(&h->ws, sz);
+    if (e != cudaSuccess) {
+        cudaGetLastError();  // (a smaller arena may do: no launch is to find it)
+        h->ws = nullptr;
+        return cuda_fail(h, e, "cudaMalloc(workspace)");
+    }
     h->ws_size = sz;
     return CUVGLS_OK;
 }
@@ -738,8 +748,7 @@ int run_batch(cuvgls_handle *h, const Work &wk, std::vector<DevCurve> &cvs,
         sum_inter += align_up(g.inter_bytes);
         all_bins += (long long)g.count * (g.cls->plan.nb + 1);
     }
-    const bool merged = nph == 1 && all_rec + max_inter <= avail && all_bins < 0x7fffffffLL;
-    if (merged) max_group_bytes = all_rec + max_inter;
+    bool merged = nph == 1 && all_rec + max_inter <= avail && all_bins < 0x7fffffffLL;
     // Groups prepared together whose intermediates all fit run beside each
     // other; else one after the other over one intermediate.
     bool beside = merged && groups.size() > 1 && sum_inter <= inter_budget &&
@@ -749,7 +758,6 @@ int run_batch(cuvgls_handle *h, const Work &wk, std::vector<DevCurve> &cvs,
         CK(cudaStreamIsCapturing(s, &cap), "capture status");
         beside = cap == cudaStreamCaptureStatusNone;
     }
-    if (beside) max_group_bytes = all_rec + sum_inter;
     if (beside && !h->side[0]) {
         for (cudaStream_t &x : h->side)
             CK(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking), "side stream");
@@ -765,10 +773,17 @@ int run_batch(cuvgls_handle *h, const Work &wk, std::vector<DevCurve> &cvs,
             h->chunk_events.push_back(e);
         }
     }
-    // arena layout
-    size_t need = fixed + max_group_bytes + 8 * kAlign;
-    rc = ensure_ws(h, need);
+    // arena layout; where the device has no memory for it, that of the form
+    // that takes less
+    for (;;) {
+        const size_t form = beside ? all_rec + sum_inter : merged ? all_rec + max_inter : max_group_bytes;
+        rc = ensure_ws(h, fixed + form + 8 * kAlign);
+        if (rc != CUVGLS_ENOMEM || !merged || groups.size() == 1) break;
+        if (beside) beside = false;
+        else merged = false;
+    }
     if (rc) return rc;
+    h->err.clear();
     char *base = h->ws;
     size_t off = 0;
     auto take = [&](size_t bytes) { char *p = base + off; off += align_up(bytes); return p; };
