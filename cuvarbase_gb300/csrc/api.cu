@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "../../include/cuvgls.h"
+#include "all_or_none.h"
 #include "kernels.cuh"
 
 using namespace cuvgls;
@@ -87,10 +88,12 @@ struct cuvgls_handle {
     cudaStream_t copy_stream = nullptr;   // device-to-host copies of the outputs
     cudaStream_t in_stream = nullptr;     // second-phase host-to-device input copies
     cudaStream_t table_stream = nullptr;  // builds the tables of new plan classes
-    // passes of groups that run beside the caller's stream (created when a
-    // batch first has several groups), with the events that fork and join them
+    // passes of groups that run beside the caller's stream (created by
+    // cuvgls_warm, or when a batch first has several groups), with the events
+    // that fork and join them
     cudaStream_t side[kSideStreams] = {};
     cudaEvent_t side_ev[kSideStreams + 1] = {};
+    bool side_ready = false;  // all of them are there
     cudaEvent_t done = nullptr;       // last enqueued work of this handle
     cudaStream_t last_stream = nullptr;
     bool have_last = false;
@@ -463,6 +466,40 @@ int ensure_host_cv(cuvgls_handle *h, size_t n) {
     return CUVGLS_OK;
 }
 
+int ensure_chunk_events(cuvgls_handle *h, int n) {
+    while ((int)h->chunk_events.size() < n) {
+        cudaEvent_t e;
+        CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
+        h->chunk_events.push_back(e);
+    }
+    return CUVGLS_OK;
+}
+
+// The side streams and their events, all of them or none (a batch then runs
+// its plans on the caller's stream).
+bool make_side_streams(cuvgls_handle *h) {
+    if (h->side_ready) return true;
+    if (make_all(h->side, kSideStreams,
+                 [](cudaStream_t *x) {
+                     return cudaStreamCreateWithFlags(x, cudaStreamNonBlocking) == cudaSuccess;
+                 },
+                 cudaStreamDestroy)) {
+        h->side_ready = make_all(h->side_ev, kSideStreams + 1,
+                                 [](cudaEvent_t *x) {
+                                     return cudaEventCreateWithFlags(x, cudaEventDisableTiming) ==
+                                            cudaSuccess;
+                                 },
+                                 cudaEventDestroy);
+        if (!h->side_ready)
+            for (cudaStream_t &x : h->side) {
+                cudaStreamDestroy(x);
+                x = nullptr;
+            }
+    }
+    if (!h->side_ready) cudaGetLastError();
+    return h->side_ready;
+}
+
 int order_stream(cuvgls_handle *h, cudaStream_t s) {
     CK(cudaSetDevice(h->device), "cudaSetDevice");
     if (h->have_last && h->last_stream != s)
@@ -753,26 +790,15 @@ int run_batch(cuvgls_handle *h, const Work &wk, std::vector<DevCurve> &cvs,
     // other; else one after the other over one intermediate.
     bool beside = merged && groups.size() > 1 && sum_inter <= inter_budget &&
                   all_rec + sum_inter <= avail;
-    if (beside && !h->side[0]) {  // (nothing is created while the caller captures)
+    if (beside && !h->side_ready) {  // (nothing is created while the caller captures)
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         CK(cudaStreamIsCapturing(s, &cap), "capture status");
-        beside = cap == cudaStreamCaptureStatusNone;
+        beside = cap == cudaStreamCaptureStatusNone && make_side_streams(h);
     }
-    if (beside && !h->side[0]) {
-        for (cudaStream_t &x : h->side)
-            CK(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking), "side stream");
-        for (cudaEvent_t &x : h->side_ev)
-            CK(cudaEventCreateWithFlags(&x, cudaEventDisableTiming), "side event");
-    }
-    if ((int)h->chunk_events.size() < 3 + nph) {
-        // two for alternating chunk copies, the start of the later phases'
-        // input copies, then the end of each later phase's copies
-        while ((int)h->chunk_events.size() < 3 + nph) {
-            cudaEvent_t e;
-            CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
-            h->chunk_events.push_back(e);
-        }
-    }
+    // two for alternating chunk copies, the start of the later phases'
+    // input copies, then the end of each later phase's copies
+    rc = ensure_chunk_events(h, 3 + nph);
+    if (rc) return rc;
     // arena layout; where the device has no memory for it, that of the form
     // that takes less
     for (;;) {
@@ -1972,8 +1998,15 @@ int cuvgls_warm(cuvgls_handle *h, int64_t nf_min, int64_t nf_max, int32_t reserv
         }
         nf = hi;
     }
-    if (reserve) return ensure_ws(h, (size_t)h->opts.workspace_bytes);
-    return CUVGLS_OK;
+    // what the first batches would otherwise load and create: the preparation
+    // kernels (which one depends on a batch's lengths), the side streams, the
+    // descriptor staging of an ordinary batch, the events of its chunks
+    CK(preload_prep_kernels(3, h->opts.precision == CUVGLS_PREC_FP32), "preload preparation");
+    make_side_streams(h);
+    int rc = ensure_host_cv(h, 1);
+    if (!rc) rc = ensure_chunk_events(h, 16);
+    if (!rc && reserve) rc = ensure_ws(h, (size_t)h->opts.workspace_bytes);
+    return rc;
 }
 
 int cuvgls_batch_bytes(cuvgls_handle *h, int32_t n_curves, const int64_t *n,

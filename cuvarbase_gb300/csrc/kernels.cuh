@@ -93,6 +93,8 @@ template <int L2>
 cudaError_t preload_pass2_t(int ng);
 // Load the pass-1 and pass-2 kernels of a (G1, G2) plan for ngrids grids.
 cudaError_t preload_pass_kernels(int G1, int G2, int ngrids);
+// Load every preparation kernel of ngrids grids (prep.cu).
+cudaError_t preload_prep_kernels(int ngrids, int fp32_positions);
 
 // Fill the deconvolution table of an ES-window plan: G / 2 + 1 floats
 // 1 / phihat(k'), |k'| <= G / 2 (kernels.cu: k_es_deconv).

@@ -665,7 +665,41 @@ cudaError_t prep_kind(const PrepArrays &a, const DescParam &d, const int *list, 
                : prep_t<NT, PPT, CL, false, 1, false>(a, d, list, n, csize, chunk, beside, s);
 }
 
+// Loads a kernel that a first launch would load.
+template <typename K>
+cudaError_t load(K kernel) {
+    cudaFuncAttributes a;
+    return cudaFuncGetAttributes(&a, kernel);
+}
+template <int NG, bool F32, bool RAW>
+cudaError_t load_prep() {
+    cudaError_t e = load(k_prep<kPrepThreads, kPrepPpt, false, RAW, NG, F32>);
+    if (e == cudaSuccess) e = load(k_prep<kPrepThreads, kPrepPpt, true, RAW, NG, F32>);
+    if (e == cudaSuccess) e = load(k_prep<kShortThreads, kShortPpt, false, RAW, NG, F32>);
+    if (e == cudaSuccess) e = load(k_prep<kWideThreads, kWidePpt, true, RAW, NG, F32>);
+    return e;
+}
+template <int NG, bool F32>
+cudaError_t load_all() {
+    cudaError_t e = load_prep<NG, F32, false>();
+    if constexpr (NG == 3) {
+        if (e == cudaSuccess) e = load_prep<NG, F32, true>();
+        if (e == cudaSuccess) e = load(k_raw_sums);
+        if (e == cudaSuccess) e = load(k_raw_finish);
+        if (e == cudaSuccess) e = load(k_fill_desc);
+    }
+    if (e == cudaSuccess) e = load(k_bin_count<NG, F32>);
+    if (e == cudaSuccess) e = load(k_bin_scan);
+    if (e == cudaSuccess) e = load(k_bin_scatter<NG, F32>);
+    return e;
+}
+
 }  // namespace
+
+cudaError_t preload_prep_kernels(int ngrids, int fp32_positions) {
+    if (ngrids == 3) return fp32_positions ? load_all<3, true>() : load_all<3, false>();
+    return fp32_positions ? load_all<1, true>() : load_all<1, false>();
+}
 
 cudaError_t launch_prep(const PrepArrays &a, const DescParam &d, const int *list, int n, int cls,
                         int max_n, int raw, int ngrids, int fp32_positions, bool beside,

@@ -358,9 +358,10 @@ int cuvgls_plan_nf(double sigma, int32_t m, int64_t nf, int64_t *G, int32_t *G1,
                    int32_t *G2);
 
 /* Build the grid tables of every plan the handle would choose for GLS
- * bands of nf_min..nf_max frequencies (and for the sub-bands of wider ones)
+ * bands of nf_min..nf_max frequencies (and for the sub-bands of wider ones),
+ * load the kernels and create the streams and events that their batches use
  * and, with reserve != 0, allocate its whole workspace budget now, so that
- * later batches in that range allocate and build nothing.  No reference
+ * later batches in that range allocate, build and load nothing.  No reference
  * counterpart (cuvarbase creates cuFFT plans per curve,
  * cuvarbase/cunfft.py:82-92). */
 int cuvgls_warm(cuvgls_handle *h, int64_t nf_min, int64_t nf_max, int32_t reserve);

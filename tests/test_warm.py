@@ -1,0 +1,110 @@
+"""Warm-up: the first batches of a warmed handle create and load nothing, and
+the streams that plans run beside each other on are made together or not at
+all."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+_MAKE_ALL = r"""
+#include <cassert>
+#include <set>
+#include "all_or_none.h"
+int main() {
+    for (int fail = 0; fail <= 5; ++fail) {      // the call that fails (5: none)
+        std::set<int *> live;
+        int calls = 0;
+        int *a[5] = {};
+        const bool ok = cuvgls::make_all(a, 5,
+            [&](int **x) {
+                if (calls++ == fail) return false;
+                *x = new int(0);
+                live.insert(*x);
+                return true;
+            },
+            [&](int *x) { assert(live.erase(x) == 1); delete x; });
+        assert(ok == (fail == 5));
+        assert(live.size() == (ok ? 5u : 0u));
+        for (int *x : a) assert((x != nullptr) == ok);
+        for (int *x : live) delete x;
+    }
+    return 0;
+}
+"""
+
+
+def test_objects_are_made_together_or_not_at_all(tmp_path):
+    src = tmp_path / "t.cpp"
+    src.write_text(_MAKE_ALL)
+    exe = tmp_path / "t"
+    subprocess.run(["g++", "-std=c++17", "-I", os.path.join(ROOT, "cuvarbase_gb300", "csrc"),
+                    str(src), "-o", str(exe)], check=True)
+    assert subprocess.run([str(exe)]).returncode == 0
+
+
+# host time of enqueueing the first and the later batches, in microseconds
+_FIRST = r"""
+import ctypes, json, sys, time
+import numpy as np, torch
+from cuvarbase_gb300 import _lib
+L = _lib.load()
+def batch(sizes):
+    n = sum(s[0] for s in sizes)
+    cv, o = (_lib.Curve * len(sizes))(), 0
+    for c, (m, nf) in zip(cv, sizes):
+        c.pt_off, c.n, c.nf, c.k0, c.df = o, m, nf, 1, 1 / 5000.0
+        c.yy, c.w_sum, c.out_off = 1.0, 1.0, 0
+        o += m
+    t = torch.sort(torch.rand(n, dtype=torch.float64, device="cuda") * 1000)[0]
+    v = torch.full((n,), 1.0 / n, device="cuda")
+    inp = _lib.GlsInput()
+    inp.n_curves, inp.mode, inp.flags = len(sizes), 1, 0
+    inp.curves = ctypes.cast(cv, ctypes.c_void_p)
+    inp.t, inp.yw, inp.w = t.data_ptr(), v.data_ptr(), v.data_ptr()
+    inp.n_points_total, inp.n_out_total = n, max(s[1] for s in sizes)
+    out = torch.empty(inp.n_out_total, device="cuda")
+    torch.cuda.synchronize()
+    return inp, out, (cv, t, v)
+def time_call(h, b):
+    t0 = time.perf_counter()
+    h.check(L.cuvgls_gls_batch(h.ptr, ctypes.byref(b[0]), b[1].data_ptr(), None), "batch")
+    dt = 1e6 * (time.perf_counter() - t0)
+    h.sync(None, -1)
+    return dt
+def warm():
+    h = _lib.Handle(sigma=-1.0, workspace_bytes=1 << 30, chunk_mb=512)
+    h.check(L.cuvgls_warm(h.ptr, 2000, 60000, 1), "warm")
+    return h
+kinds = {"two": [(60, 3000)] * 2, "cluster": [(1500, 3000)], "wide": [(20000, 3000)],
+         "long": [(40000, 3000)], "short": [(60, 3000)] * 3000}
+h = warm()
+time_call(h, batch([(60, 3000)]))     # the process's first call
+r = {}
+for k, s in kinds.items():
+    b = batch(s)
+    r[k] = [time_call(h, b) for _ in range(6)]
+plans = batch([(60, 3000), (80, 9000), (70, 20000), (60, 55000)])
+r["plans"] = [[time_call(g, plans) for _ in range(6)] for g in [warm() for _ in range(8)]]
+print(json.dumps(r))
+"""
+
+
+@pytest.mark.gpu
+def test_first_batches_create_and_load_nothing():
+    """Loading a kernel or creating the seven streams takes 0.2 ms and more, a
+    later enqueue less than that: the first one of each kind takes no more than
+    1.5 times the later ones and 0.1 ms (the kinds once in a process of its own,
+    the streams as the best of eight handles)."""
+    import json
+    p = subprocess.run([sys.executable, "-c", _FIRST], cwd=ROOT, capture_output=True, text=True,
+                       timeout=300)
+    assert p.returncode == 0, p.stderr
+    r = json.loads(p.stdout.strip().splitlines()[-1])
+    plans = r.pop("plans")
+    later = sorted(x for h in plans for x in h[1:])
+    assert min(h[0] for h in plans) <= 1.5 * later[len(later) // 2] + 20.0, plans
+    slow = {k: v for k, v in r.items() if v[0] > 1.5 * sorted(v[1:])[2] + 100.0}
+    assert not slow, r
