@@ -43,12 +43,11 @@ __device__ __forceinline__ void mbar_expect(unsigned long long *b, unsigned byte
                  "r"(bytes)
                  : "memory");
 }
-// Waits for the phase of the given parity, a bounded number of times; false
-// when that ran out.
-__device__ __forceinline__ bool mbar_wait(unsigned long long *b, unsigned parity) {
-    constexpr int kTries = 1 << 18;  // each suspends for up to some microseconds
+// Waits for the phase of the given parity, a bounded number of times (each
+// suspends for up to some microseconds); false when that ran out.
+__device__ __forceinline__ bool mbar_wait(unsigned long long *b, unsigned parity, int tries) {
     const unsigned a = smem_addr(b);
-    for (int k = 0; k < kTries; ++k) {
+    for (int k = 0; k < tries; ++k) {
         unsigned done;
         asm volatile(
             "{\n .reg .pred p;\n"
@@ -184,7 +183,7 @@ k_pass2_gls_reg(const __grid_constant__ CUtensorMap map, const DevCurve *cvs,
         float2 ya[LB], yb[LB], yc[LB];
 #pragma unroll
         for (int g = 0; g < 3; ++g, ++s) {
-            const bool ok = mbar_wait(&full[s % NB], (s / NB) & 1);
+            const bool ok = mbar_wait(&full[s % NB], (s / NB) & 1, p.wait_tries);
             float2 *in = tiles + (s % NB) * TILE;
             float2 *ex = IP ? in : rest;
             // stage A: unit u = (ih, r, c) reads in[u + k AU], i.e. elements
@@ -212,11 +211,13 @@ k_pass2_gls_reg(const __grid_constant__ CUtensorMap map, const DevCurve *cvs,
                     store(x[0], u);
                 }
             }
-            if (__syncthreads_or(!ok)) {  // a copy never came: leave, all threads
+            // a copy never came: all threads leave, after a second bounded wait
+            // for the copies in flight
+            if (__syncthreads_or(!ok)) {
                 if (tid == 0) {
                     atomicOr(gp.errflag, 2u);
                     for (int k = s; k < s + NB; ++k)
-                        if (live(k)) mbar_wait(&full[k % NB], (k / NB) & 1);
+                        if (live(k)) mbar_wait(&full[k % NB], (k / NB) & 1, kWaitTries);
                 }
                 __syncthreads();
                 return;
@@ -376,7 +377,7 @@ k_pass2_nfft_reg(const __grid_constant__ CUtensorMap map, const DevCurve *cvs,
         const int t = blockIdx.x + s * (int)gridDim.x, ci = t / nrb, rb = t - ci * nrb;
         const DevCurve cv = cvs[ci];
         const ulonglong2 ax = aux[cv.aux];
-        const bool ok = mbar_wait(full, s & 1);
+        const bool ok = mbar_wait(full, s & 1, p.wait_tries);
         float2 x[UPT][LA];
 #pragma unroll
         for (int v = 0; v < UPT; ++v) {
@@ -392,10 +393,10 @@ k_pass2_nfft_reg(const __grid_constant__ CUtensorMap map, const DevCurve *cvs,
                 fft2_stage_a_regs<L2>(x[v], p.st2, i);
             }
         }
-        if (__syncthreads_or(!ok)) {  // a copy never came: leave, all threads
+        if (__syncthreads_or(!ok)) {  // as in k_pass2_gls_reg
             if (tid == 0) {
                 atomicOr(errflag, 2u);
-                mbar_wait(full, s & 1);
+                mbar_wait(full, s & 1, kWaitTries);
             }
             __syncthreads();
             return;
