@@ -384,7 +384,6 @@ int get_class(cuvgls_handle *h, long long nf, int ng, ClassTables **out) {
     const double sig = pk.sigma;
     p.win = pk.win;
     p.narrow = sig >= kNarrowSigma;
-    p.wait_tries = kWaitTries;
     const double b = 2.0 * sig * p.m / ((2.0 * sig - 1.0) * kPi);
     p.binv = (float)(1.0 / b);
     p.dc1 = (float)(b * kPi * kPi / ((double)G * (double)G));

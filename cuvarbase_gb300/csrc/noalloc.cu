@@ -125,7 +125,6 @@ extern "C" int cuvgls_gls_noalloc(double sigma, int32_t m, const cuvgls_gls_inpu
     memset(&p, 0, sizeof p);
     p.G1 = G1; p.G2 = G2; p.G = G; p.m = m; p.B = B; p.R = R; p.nb = G2 / B;
     p.narrow = sigma >= kNarrowSigma;
-    p.wait_tries = kWaitTries;
     const double bw = 2.0 * sigma * m / ((2.0 * sigma - 1.0) * kPiN);
     p.binv = (float)(1.0 / bw);
     p.dc1 = (float)(bw * kPiN * kPiN / ((double)G * (double)G));

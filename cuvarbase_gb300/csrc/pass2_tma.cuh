@@ -43,11 +43,13 @@ __device__ __forceinline__ void mbar_expect(unsigned long long *b, unsigned byte
                  "r"(bytes)
                  : "memory");
 }
-// Waits for the phase of the given parity, a bounded number of times (each
-// suspends for up to some microseconds); false when that ran out.
-__device__ __forceinline__ bool mbar_wait(unsigned long long *b, unsigned parity, int tries) {
+// Waits for the phase of the given parity, a bounded number of times; false
+// when that ran out.
+constexpr int kWaitTries = 1 << 18;  // each suspends for up to some microseconds
+template <int TRIES = kWaitTries>
+__device__ __forceinline__ bool mbar_wait(unsigned long long *b, unsigned parity) {
     const unsigned a = smem_addr(b);
-    for (int k = 0; k < tries; ++k) {
+    for (int k = 0; k < TRIES; ++k) {
         unsigned done;
         asm volatile(
             "{\n .reg .pred p;\n"
@@ -127,7 +129,8 @@ struct Fm2 {
     }
 };
 
-template <int L2, bool ES, bool NARROW>
+// (TRIES: the limit of the waits for a tile, which a test lets run out)
+template <int L2, bool ES, bool NARROW, int TRIES>
 __global__ void __launch_bounds__(pass2_reg_threads(L2), pass2_reg_ctas(L2))
 k_pass2_gls_reg(const __grid_constant__ CUtensorMap map, const DevCurve *cvs,
                 int n_curves, int first, float *__restrict__ out, const Plan p, const GlsParams gp) {
@@ -183,7 +186,7 @@ k_pass2_gls_reg(const __grid_constant__ CUtensorMap map, const DevCurve *cvs,
         float2 ya[LB], yb[LB], yc[LB];
 #pragma unroll
         for (int g = 0; g < 3; ++g, ++s) {
-            const bool ok = mbar_wait(&full[s % NB], (s / NB) & 1, p.wait_tries);
+            const bool ok = mbar_wait<TRIES>(&full[s % NB], (s / NB) & 1);
             float2 *in = tiles + (s % NB) * TILE;
             float2 *ex = IP ? in : rest;
             // stage A: unit u = (ih, r, c) reads in[u + k AU], i.e. elements
@@ -217,7 +220,7 @@ k_pass2_gls_reg(const __grid_constant__ CUtensorMap map, const DevCurve *cvs,
                 if (tid == 0) {
                     atomicOr(gp.errflag, 2u);
                     for (int k = s; k < s + NB; ++k)
-                        if (live(k)) mbar_wait(&full[k % NB], (k / NB) & 1, kWaitTries);
+                        if (live(k)) mbar_wait(&full[k % NB], (k / NB) & 1);
                 }
                 __syncthreads();
                 return;
@@ -329,7 +332,7 @@ k_pass2_gls_reg(const __grid_constant__ CUtensorMap map, const DevCurve *cvs,
 // the kernel at 68 % issue (half of it integer and conversion instructions).
 // 1,000 curves of 512 x 400 cells 0.797 -> 0.431 ms (2.4 GB moved: 0.36 ms at
 // the measured copy rate).
-template <int L2, bool ES>
+template <int L2, bool ES, int TRIES>
 __global__ void __launch_bounds__(pass2_reg_threads(L2), kNfftRegCtas)
 k_pass2_nfft_reg(const __grid_constant__ CUtensorMap map, const DevCurve *cvs,
                  int n_curves, int first, float2 *__restrict__ out,
@@ -377,7 +380,7 @@ k_pass2_nfft_reg(const __grid_constant__ CUtensorMap map, const DevCurve *cvs,
         const int t = blockIdx.x + s * (int)gridDim.x, ci = t / nrb, rb = t - ci * nrb;
         const DevCurve cv = cvs[ci];
         const ulonglong2 ax = aux[cv.aux];
-        const bool ok = mbar_wait(full, s & 1, p.wait_tries);
+        const bool ok = mbar_wait<TRIES>(full, s & 1);
         float2 x[UPT][LA];
 #pragma unroll
         for (int v = 0; v < UPT; ++v) {
@@ -396,7 +399,7 @@ k_pass2_nfft_reg(const __grid_constant__ CUtensorMap map, const DevCurve *cvs,
         if (__syncthreads_or(!ok)) {  // as in k_pass2_gls_reg
             if (tid == 0) {
                 atomicOr(errflag, 2u);
-                mbar_wait(full, s & 1, kWaitTries);
+                mbar_wait(full, s & 1);
             }
             __syncthreads();
             return;
@@ -468,14 +471,14 @@ cudaError_t resident_ctas(K kernel, int threads, int smem, int (&slots)[64]) {
     return e;
 }
 
-template <int L2, bool ES>
+template <int L2, bool ES, int TRIES = kWaitTries>
 cudaError_t launch_nfft_reg_t(const DevCurve *cv, int n_curves, int first, const float2 *inter,
                               float2 *out, const ulonglong2 *aux, unsigned *errflag, const Plan &p,
                               cudaStream_t s) {
     static int slots[64] = {0};  // resident CTAs, per instantiation and device
     constexpr int NT = pass2_reg_threads(L2), R = pass2_rows(1, L2);
     const int smem = (int)pass2_smem(1, L2);
-    cudaError_t e = resident_ctas(k_pass2_nfft_reg<L2, ES>, NT, smem, slots);
+    cudaError_t e = resident_ctas(k_pass2_nfft_reg<L2, ES, TRIES>, NT, smem, slots);
     if (e != cudaSuccess) return e;
     int dev = 0;
     cudaGetDevice(&dev);
@@ -486,18 +489,18 @@ cudaError_t launch_nfft_reg_t(const DevCurve *cv, int n_curves, int first, const
     if (tasks > 0x3fffffffLL || p.B != kNfftCols) return cudaErrorInvalidValue;
     Plan q = p;
     q.dependent = small_launch(tasks);
-    return launch_pdl(k_pass2_nfft_reg<L2, ES>, q.dependent,
+    return launch_pdl(k_pass2_nfft_reg<L2, ES, TRIES>, q.dependent,
                       dim3((int)(tasks < slots[dev] ? tasks : slots[dev])), NT, smem, s, map, cv,
                       n_curves, first, out, aux, errflag, q);
 }
 
-template <int L2, bool ES, bool NARROW>
+template <int L2, bool ES, bool NARROW, int TRIES = kWaitTries>
 cudaError_t launch_pass2_reg_t(const DevCurve *cv, int n_curves, int first, const float2 *inter,
                                float *out, const Plan &p, GlsParams g, cudaStream_t s) {
     static int slots[64] = {0};  // resident CTAs, per instantiation and device
     constexpr int NT = pass2_reg_threads(L2), R = pass2_rows(3, L2);
     const int smem = NARROW && pass2_reg_inplace(L2) ? (pass2_reg_tile(L2) + 2) * 8 : (int)pass2_smem(3, L2);
-    cudaError_t e = resident_ctas(k_pass2_gls_reg<L2, ES, NARROW>, NT, smem, slots);
+    cudaError_t e = resident_ctas(k_pass2_gls_reg<L2, ES, NARROW, TRIES>, NT, smem, slots);
     if (e != cudaSuccess) return e;
     int dev = 0;
     cudaGetDevice(&dev);
@@ -508,7 +511,7 @@ cudaError_t launch_pass2_reg_t(const DevCurve *cv, int n_curves, int first, cons
     if (tasks > 0x3fffffffLL || p.B != kGlsCols) return cudaErrorInvalidValue;
     Plan q = p;
     q.dependent = small_launch(tasks);
-    return launch_pdl(k_pass2_gls_reg<L2, ES, NARROW>, q.dependent,
+    return launch_pdl(k_pass2_gls_reg<L2, ES, NARROW, TRIES>, q.dependent,
                       dim3((int)(tasks < slots[dev] ? tasks : slots[dev])), NT, smem, s, map, cv,
                       n_curves, first, out, q, g);
 }

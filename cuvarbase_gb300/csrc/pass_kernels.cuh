@@ -1114,12 +1114,12 @@ cudaError_t preload_pass2_t(int ng) {
     cudaFuncAttributes a;
     if constexpr (pass2_reg(3, L2)) {
         if (ng != 3) {
-            const cudaError_t e = cudaFuncGetAttributes(&a, k_pass2_nfft_reg<L2, true>);
-            return e != cudaSuccess ? e : cudaFuncGetAttributes(&a, k_pass2_nfft_reg<L2, false>);
+            const cudaError_t e = cudaFuncGetAttributes(&a, k_pass2_nfft_reg<L2, true, kWaitTries>);
+            return e != cudaSuccess ? e : cudaFuncGetAttributes(&a, k_pass2_nfft_reg<L2, false, kWaitTries>);
         }
-        cudaError_t e = cudaFuncGetAttributes(&a, k_pass2_gls_reg<L2, true, false>);
-        if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_pass2_gls_reg<L2, false, true>);
-        return e != cudaSuccess ? e : cudaFuncGetAttributes(&a, k_pass2_gls_reg<L2, false, false>);
+        cudaError_t e = cudaFuncGetAttributes(&a, k_pass2_gls_reg<L2, true, false, kWaitTries>);
+        if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_pass2_gls_reg<L2, false, true, kWaitTries>);
+        return e != cudaSuccess ? e : cudaFuncGetAttributes(&a, k_pass2_gls_reg<L2, false, false, kWaitTries>);
     } else if constexpr (pass2_deep(3, L2)) {
         if (ng != 3) return cudaFuncGetAttributes(&a, k_pass2_nfft<L2>);
         const cudaError_t e = cudaFuncGetAttributes(&a, k_pass2_gls_deep<L2, true>);

@@ -1,6 +1,6 @@
-"""A wait for a tile's copy that runs out (its limit set to no tries at all; the
-copy itself arrives): the CTAs leave, the device error word says so, and the
-device goes on."""
+"""A wait for a tile's copy that runs out (kernels compiled with a limit of no
+tries at all; the copy itself arrives): the CTAs leave, the device error word
+says so, and the device goes on."""
 import os
 import shutil
 import subprocess
@@ -12,20 +12,20 @@ pytestmark = pytest.mark.gpu
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 PKG = os.path.join(ROOT, "cuvarbase_gb300")
 
-# argv: grids, row length, tries (-1: the library's).  Prints the error word, the
-# outputs written, and the word of the same launch after it with the library's
-# limit.
+# argv: grids, row length.  Prints the error word, the outputs written and their
+# number: with no tries, then with the library's kernels.
 _SRC = r"""
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
 #include <vector>
 #include "kernels.cuh"
+#include "pass2_tma.cuh"
 using namespace cuvgls;
 #define OK(x) do { cudaError_t e = (x); if (e != cudaSuccess) { \
     fprintf(stderr, "%s: %s\n", #x, cudaGetErrorString(e)); return 1; } } while (0)
 int main(int, char **argv) {
-    const int ng = atoi(argv[1]), G2 = atoi(argv[2]), tries = atoi(argv[3]), G1 = 160, curves = 40;
+    const int ng = atoi(argv[1]), G2 = atoi(argv[2]), G1 = 160, curves = 40;
     Plan p;
     memset(&p, 0, sizeof p);
     p.G1 = G1; p.G2 = G2; p.G = (long long)G1 * G2; p.m = 8;
@@ -54,13 +54,20 @@ int main(int, char **argv) {
     }
     OK(cudaMemcpy(cv, h.data(), curves * sizeof(DevCurve), cudaMemcpyHostToDevice));
     for (int k = 0; k < 2; ++k) {
-        p.wait_tries = k || tries < 0 ? kWaitTries : tries;
         OK(cudaMemset(flag, 0, 4));
         OK(cudaMemset(out, 0xff, on * 8));
-        if (ng == 3)
-            OK(launch_pass2_gls(cv, curves, 0, inter, (float *)out, p, GlsParams{1, 0.f, nullptr, flag}, 0));
-        else
+        const GlsParams g{1, 0.f, nullptr, flag};
+        if (k && ng == 3)
+            OK(launch_pass2_gls(cv, curves, 0, inter, (float *)out, p, g, 0));
+        else if (k)
             OK(launch_pass2_nfft(cv, curves, 0, inter, out, aux, flag, p, 0));
+        else if (ng == 3)
+            OK(G2 == 160 ? (launch_pass2_reg_t<160, false, false, 0>(cv, curves, 0, inter, (float *)out, p, g, 0))
+             : G2 == 256 ? (launch_pass2_reg_t<256, false, false, 0>(cv, curves, 0, inter, (float *)out, p, g, 0))
+                         : (launch_pass2_reg_t<400, false, false, 0>(cv, curves, 0, inter, (float *)out, p, g, 0)));
+        else
+            OK(G2 == 160 ? (launch_nfft_reg_t<160, false, 0>(cv, curves, 0, inter, out, aux, flag, p, 0))
+                         : (launch_nfft_reg_t<400, false, 0>(cv, curves, 0, inter, out, aux, flag, p, 0)));
         OK(cudaDeviceSynchronize());
         unsigned f;
         std::vector<unsigned> o(on * (ng == 3 ? 1 : 2));
@@ -90,14 +97,8 @@ def harness(tmp_path_factory):
 @pytest.mark.parametrize("grids,G2", [(3, 160), (3, 256), (3, 400), (1, 160), (1, 400)])
 def test_wait_runs_out(harness, grids, G2):
     from cuvarbase_gb300 import _lib
-
-    def run(tries):
-        r = subprocess.run([harness, str(grids), str(G2), str(tries)], capture_output=True,
-                           text=True, timeout=60)
-        assert r.returncode == 0, r.stderr
-        return [tuple(map(int, line.split())) for line in r.stdout.splitlines()]
-    first, after = run(0)
+    r = subprocess.run([harness, str(grids), str(G2)], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stderr
+    first, after = [tuple(map(int, line.split())) for line in r.stdout.splitlines()]
     assert first[0] == _lib.DEVERR_TIMEOUT and first[1] == 0
     assert after[0] == 0 and after[1] == after[2]
-    for flag, written, total in run(-1):
-        assert flag == 0 and written == total
