@@ -527,7 +527,10 @@ k_gls_direct(const DevCurve *__restrict__ cvs, const double *__restrict__ t,
     double2 va[NQ], vb[NQ], vc[NQ];
 #pragma unroll
     for (int q = 0; q < NQ; ++q) va[q] = vb[q] = vc[q] = make_double2(0.0, 0.0);
-    bool lost = false;  // something not finite: no power of the curve is valid
+    // something not finite: no power of the curve is valid (the window's powers
+    // are of the weights alone)
+    bool lost = false;
+    const bool window = gp.mode == 2;
     const double kc = cv.kc - (double)(cv.nf / 2) + (double)(k0 + kGlM);
     const double t0 = t[cv.pt_off];
     for (long long r0 = j0; r0 < j1; r0 += kDirRun) {
@@ -535,12 +538,10 @@ k_gls_direct(const DevCurve *__restrict__ cvs, const double *__restrict__ t,
         float my = 0.f, mw = 0.f;
         for (long long j = cv.pt_off + r0 + tid; j < cv.pt_off + r1; j += kDirThreads) {
             const float a = fabsf(yw[j]), b = fabsf(w[j]);
-            if (isfinite(a) && isfinite(b)) {
-                my = fmaxf(my, a);
-                mw = fmaxf(mw, b);
-            } else {
-                lost = true;
-            }
+            if (isfinite(a)) my = fmaxf(my, a);
+            else lost = lost || !window;
+            if (isfinite(b)) mw = fmaxf(mw, b);
+            else lost = true;
         }
         const int ey = fx_exponent(my, &top[0], tid), ew = fx_exponent(mw, &top[1], tid);
         DirSums<kGlM> sa, sb, sc;
@@ -552,7 +553,8 @@ k_gls_direct(const DevCurve *__restrict__ cvs, const double *__restrict__ t,
                 const double x = (t[j] - t0) * cv.df;
                 lost = lost || !isfinite(kc * x);
                 tile.tab.build(lane, turns64(x), turns64(kc * x), steps);
-                const Fx fy = fx_split(__double2ll_rn(scalbn((double)yw[j], kFxBits - ey)));
+                const double yj = isfinite(yw[j]) ? (double)yw[j] : 0.0;
+                const Fx fy = fx_split(__double2ll_rn(scalbn(yj, kFxBits - ey)));
                 const Fx fw = fx_split(__double2ll_rn(scalbn((double)w[j], kFxBits - ew)));
                 tile.yw[lane] = make_int2(fy.h, fy.l);
                 tile.w[lane] = make_int2(fw.h, fw.l);

@@ -66,3 +66,46 @@ def test_harmonics_one_value_dominates(n):
     # P goes as the squares of YC and YS, whose larger one is 1.4 or more
     err = ((P - ref) / ref).astype(float)
     assert np.sqrt(np.mean(err ** 2)) <= 2 * _rms_fp64(n) / 1.4 + 16 * 2.0 ** -53
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bad", [np.nan, np.inf, 1e30])
+def test_window_needs_no_values(bad):
+    """The spectral window (mode "window") is that of the weights: a value that
+    is not finite, or not in float32, leaves its powers alone; in the other
+    modes it leaves the curve none."""
+    import ctypes
+    from cuvarbase_gb300 import _lib
+    rng = np.random.default_rng(7)
+    n, nf = 300, 700
+    t = np.sort(rng.uniform(0, 900.0, n))
+    w = np.full(n, 1 / n, np.float32)
+    yw = (rng.standard_normal(n) / n).astype(np.float32)
+
+    def powers(yw, mode):
+        c = _lib.Curve()
+        c.pt_off, c.n, c.nf, c.k0, c.df, c.out_off = 0, n, nf, 1, 1 / 4500.0, 0
+        c.yy, c.ybar, c.yw_sum, c.w_sum = 1.0, 0.0, float(yw.sum()), float(w.sum())
+        inp = _lib.GlsInput()
+        inp.n_curves, inp.mode = 1, mode
+        inp.curves = ctypes.addressof(c)
+        inp.t, inp.yw, inp.w = t.ctypes.data, yw.ctypes.data, w.ctypes.data
+        inp.flags = _lib.HOST_INPUT | _lib.HOST_OUTPUT
+        inp.n_points_total, inp.n_out_total = n, nf
+        P = np.empty(nf, np.float32)
+        h.check(_lib.load().cuvgls_gls_direct_batch(h.ptr, ctypes.byref(inp), P.ctypes.data, None),
+                "direct")
+        h.sync(None, -1)
+        return P
+    h = _lib.Handle(sigma=2.0, m=8)
+    try:
+        spoilt = yw.copy()
+        with np.errstate(over="ignore"):
+            spoilt[11] = np.float32(bad) * np.float32(1e10)
+        want = powers(yw, _lib.MODE_WINDOW)
+        assert np.all(want >= 0)
+        assert np.array_equal(powers(spoilt, _lib.MODE_WINDOW), want)
+        for mode in (_lib.MODE_STANDARD, _lib.MODE_FLOATING_MEAN):
+            assert np.all(powers(spoilt, mode) == -1)
+    finally:
+        h.close()
