@@ -14,11 +14,12 @@
 //                grid (shared-memory float atomics), runs the length-G1 column
 //                FFTs in shared memory, applies the inter-pass twiddle and
 //                writes the tile to the intermediate buffer.
-//   k_pass2_*    one CTA per (curve, R-row block).  Loads R rows of every
-//                grid, runs the length-G2 row FFTs in shared memory and, in
-//                the same kernel, deconvolves the Gaussian window and either
-//                evaluates the GLS power (3 grids) or applies the output phase
-//                of the adjoint NFFT (1 grid).
+//   k_pass2_*    a task or CTA per (curve, R-row block).  Runs the length-G2
+//                row FFTs of every grid, the butterflies in registers and the
+//                exchange between them in shared memory, and, in the same
+//                kernel, deconvolves the window and either evaluates the GLS
+//                power (3 grids) or applies the output phase of the adjoint
+//                NFFT (1 grid).
 // The grid itself never exists in HBM: spreading is fused into pass 1.
 #include <cuda.h>
 #include <cudaTypedefs.h>

@@ -117,7 +117,7 @@ cudaError_t launch_raw_long(const SegEntry *segs, int n_segs, const DevCurve *cv
 cudaError_t launch_fill_desc(DevCurve *cv, const int *list, int n, const double4 *partA,
                              const double4 *partB, int mode, cudaStream_t s);
 
-// Per-curve best keys of k_pass2_gls to (index, power); -1 / -1 where a
+// Per-curve best keys of the GLS pass 2 to (index, power); -1 / -1 where a
 // curve had no valid power.
 cudaError_t launch_best_finish(const unsigned long long *keys, int n, int64_t *best_k,
                                float *best_p, cudaStream_t s);

@@ -73,7 +73,8 @@ __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, i
 
 // Orders this thread's own loads and stores of shared memory before the copies
 // into the same bytes that another thread issues after the next barrier: the
-// copies are the async proxy's, and a barrier alone orders one proxy only.
+// copies are the async proxy's, and a barrier alone orders one proxy only.  (2,000
+// curves of 320 x 400 cells 3.537 -> 3.553 ms, 1,000 NFFTs 0.941 -> 0.948.)
 __device__ __forceinline__ void before_copy() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }

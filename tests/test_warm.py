@@ -96,15 +96,21 @@ print(json.dumps(r))
 def test_first_batches_create_and_load_nothing():
     """Loading a kernel or creating the seven streams takes 0.2 ms and more, a
     later enqueue less than that: the first one of each kind takes no more than
-    1.5 times the later ones and 0.1 ms (the kinds once in a process of its own,
-    the streams as the best of eight handles)."""
+    1.5 times the later ones and 0.1 ms (the streams 0.02 ms).  Each is the best
+    of several, so that a pause of the host does not count: the kinds of three
+    processes, the streams of eight handles in each."""
     import json
-    p = subprocess.run([sys.executable, "-c", _FIRST], cwd=ROOT, capture_output=True, text=True,
-                       timeout=300)
-    assert p.returncode == 0, p.stderr
-    r = json.loads(p.stdout.strip().splitlines()[-1])
-    plans = r.pop("plans")
-    later = sorted(x for h in plans for x in h[1:])
-    assert min(h[0] for h in plans) <= 1.5 * later[len(later) // 2] + 20.0, plans
-    slow = {k: v for k, v in r.items() if v[0] > 1.5 * sorted(v[1:])[2] + 100.0}
-    assert not slow, r
+    first, later, plans = {}, {}, []
+    for _ in range(3):
+        p = subprocess.run([sys.executable, "-c", _FIRST], cwd=ROOT, capture_output=True,
+                           text=True, timeout=300)
+        assert p.returncode == 0, p.stderr
+        r = json.loads(p.stdout.strip().splitlines()[-1])
+        plans += r.pop("plans")
+        for k, v in r.items():
+            first[k] = min(first.get(k, v[0]), v[0])
+            later.setdefault(k, []).extend(v[1:])
+    rest = sorted(x for h in plans for x in h[1:])
+    assert min(h[0] for h in plans) <= 1.5 * rest[len(rest) // 2] + 20.0, plans
+    for k, v in later.items():
+        assert first[k] <= 1.5 * sorted(v)[len(v) // 2] + 100.0, (k, first, later)
